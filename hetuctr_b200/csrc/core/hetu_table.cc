@@ -324,11 +324,11 @@ void HetuTable::reserveShared(size_t batch) {
 void HetuTable::preprocess(index_t *data_ptr, size_t batch_size) {
   HCTR_CUDA(cudaSetDevice(device_id_));
   // A single-rank table never waits for its dedupe here: the next reduction reads the batch's sizes on the device.
-  if (nrank_ == 1) flushDedupe(cur_batch_);  // two preprocess calls in a row: the first one's dedupe is still due
-  else finalizePending();
+  // A dedupe that is still due (serving, or two preprocess calls in a row) stays due until its gradients come.
+  if (nrank_ > 1) finalizePending();
   batch_open_ = true;
   profile_ = profile_every_ > 0 && (profile_step_++ % (size_t)profile_every_) == 0;
-  flushOrdering(cur_batch_);  // normally done by push_pull already; two preprocess calls in a row get here
+  if (nrank_ > 1) flushOrdering(cur_batch_);  // normally done by push_pull already; two preprocess calls in a row get here
   std::swap(cur_batch_, prev_batch_);
   BatchDesc &cur = cur_batch_, &prev = prev_batch_;
   cur.decided = false;
@@ -353,6 +353,11 @@ void HetuTable::preprocess(index_t *data_ptr, size_t batch_size) {
   // A single-rank table ingests on the (idle) stream of its reduction: stream_main_ may still hold the previous
   // batch's dedupe, which nothing here has to wait for.  The dedupe of this batch waits for ev_keys_.
   cudaStream_t ks = n == 1 ? stream_reduce_ : stream_main_;
+  if (n == 1 && cur.dedupe_in_flight) {  // no reduction has waited for the dedupe of the batch this descriptor held
+    HCTR_CUDA(cudaStreamWaitEvent(ks, cur.ev_scatter, 0));
+    if (cur.order_recorded) HCTR_CUDA(cudaStreamWaitEvent(ks, cur.ev_order, 0));
+    cur.dedupe_in_flight = false;
+  }
   const int64_t *key_src = reinterpret_cast<const int64_t *>(data_ptr);
   if (!keys_on_device) {
     HCTR_CUDA(cudaMemcpyAsync(cur.keys.p, data_ptr, sizeof(index_t) * batch_size, cudaMemcpyDefault, ks));
@@ -362,53 +367,10 @@ void HetuTable::preprocess(index_t *data_ptr, size_t batch_size) {
                                     (unsigned)meta_words, d_row_of_.as<int32_t>(), kEmbeddingIDMax,
                                     cur.pos_row.as<int32_t>(), d_ingest_err_, ks));
   HCTR_CUDA(cudaEventRecord(ev_keys_, ks));
-  if (n == 1) HCTR_CUDA(cudaStreamWaitEvent(stream_main_, ev_keys_, 0));
-
-  if (!key_stride_known_ && batch_size >= 4096) detectKeyStride(cur);  // once per table
-  hctr_dedupe_args a;
-  a.stride = key_stride_;
-  a.keys = cur.keys.as<int64_t>();
-  a.batch = batch_size;
-  a.length = kEmbeddingIDMax;
-  a.length_pad = length_pad_;
-  a.nrank = n;
-  a.owner_of = d_root_.as<uint8_t>();
-  a.row_of = d_row_of_.as<int32_t>();
-  a.bits = d_bits_.as<unsigned long long>();
-  a.chain_scratch = d_blk_cnt_.as<uint32_t>();
-  a.epoch = nextEpoch();
-  a.blk_flag = d_blk_flag_.as<uint8_t>();
-  a.word_base = d_word_base_.as<uint32_t>();
-  a.scan_scratch = d_chain_.as<uint32_t>();
-  a.sk = d_sk_.as<unsigned long long>();
-  a.rank_in_run = cur.rank.as<uint32_t>();
-  a.heavy_list = cur.heavy.as<uint32_t>();
-  a.pos_row = nullptr;  // resolved by the key ingest above
-  a.uniq = cur.uniq.as<int64_t>();
-  a.uniq_owner = cur.uniq_owner.as<uint8_t>();
-  a.uniq_row = cur.uniq_row.as<int32_t>();
-  a.cnt = d_cnt_.as<uint32_t>();
-  a.run_start = cur.run_start.as<uint32_t>();
-  a.sorted_pos = cur.sorted_pos.as<uint32_t>();
-  a.idx_map = cur.idx_map.as<int32_t>();
-  a.meta = cur.meta.as<uint32_t>();
-  // run ordering happens on stream_side_, off this stream's critical path; the reduction of this batch
-  // (next step) waits on the batch's own event.  The ordering stages through the batch's own rank buffer, so the
-  // ordering of the previous batch may still run while this batch is deduplicated; only the descriptor being
-  // recycled (two batches old) must be out of use.
-  if (cur.order_recorded) HCTR_CUDA(cudaStreamWaitEvent(stream_main_, cur.ev_order, 0));
-  if (!cur.ev_order) HCTR_CUDA(cudaEventCreateWithFlags(&cur.ev_order, cudaEventDisableTiming));
-  if (!cur.ev_scatter) HCTR_CUDA(cudaEventCreateWithFlags(&cur.ev_scatter, cudaEventDisableTiming));
-  a.side_stream = stream_side_;
-  a.fork_event = cur.ev_scatter;
-  // The ordering kernels are not even enqueued here: push_pull enqueues them after the gradient reduction,
-  // which brings the reduction (it only starts once push_pull is called) several launches forward.
-  a.join_event = nullptr;
-  cur.order_recorded = false;
   cur.scatter_recorded = false;
   cur.light_ordered = false;
+  cur.dedupe_pending = true;
   cur.order_pending = true;
-  cur.order_args = a;
   // The push decision for the previous batch goes first: the gradient reduction (on its own stream, started
   // by the next push_pull) only needs this, not the dedupe of the new batch that follows.
 
@@ -418,7 +380,6 @@ void HetuTable::preprocess(index_t *data_ptr, size_t batch_size) {
   if (decide && !prev.decided) launchPushDecide(prev);  // normally done at the end of the previous push_pull
   HCTR_CUDA(cudaEventRecord(ev_decide_, stream_reduce_));
   prev_push_valid_ = decide;
-  cur.dedupe_pending = true;
   cur.pending = true;
   if (n == 1) {
     // Single rank: nothing of this step reads what the dedupe produces (the expansion has the rows from the key
@@ -521,9 +482,53 @@ void HetuTable::launchPushDecide(BatchDesc &b) {
 void HetuTable::flushDedupe(BatchDesc &b) {
   if (!b.dedupe_pending) return;
   b.dedupe_pending = false;
+  if (nrank_ == 1) HCTR_CUDA(cudaStreamWaitEvent(stream_main_, ev_keys_, 0));
+  if (!key_stride_known_ && b.batch_size >= 4096) detectKeyStride(b);  // once per table
+  // run ordering happens on stream_side_, off this stream's critical path; the reduction of this batch
+  // (next step) waits on the batch's own event.  The ordering stages through the batch's own rank buffer, so the
+  // ordering of the previous batch may still run while this batch is deduplicated; only the descriptor being
+  // recycled (two batches old) must be out of use.
+  if (b.order_recorded) HCTR_CUDA(cudaStreamWaitEvent(stream_main_, b.ev_order, 0));
+  if (!b.ev_order) HCTR_CUDA(cudaEventCreateWithFlags(&b.ev_order, cudaEventDisableTiming));
+  if (!b.ev_scatter) HCTR_CUDA(cudaEventCreateWithFlags(&b.ev_scatter, cudaEventDisableTiming));
+  b.order_recorded = false;
+  // (built here and not at preprocess: a larger batch in between may have moved the shared scratch)
+  hctr_dedupe_args &a = b.order_args;
+  a.stride = key_stride_;
+  a.keys = b.keys.as<int64_t>();
+  a.batch = b.batch_size;
+  a.length = kEmbeddingIDMax;
+  a.length_pad = length_pad_;
+  a.nrank = nrank_;
+  a.owner_of = d_root_.as<uint8_t>();
+  a.row_of = d_row_of_.as<int32_t>();
+  a.bits = d_bits_.as<unsigned long long>();
+  a.chain_scratch = d_blk_cnt_.as<uint32_t>();
+  a.epoch = nextEpoch();
+  a.blk_flag = d_blk_flag_.as<uint8_t>();
+  a.word_base = d_word_base_.as<uint32_t>();
+  a.scan_scratch = d_chain_.as<uint32_t>();
+  a.cnt = d_cnt_.as<uint32_t>();
+  a.sk = d_sk_.as<unsigned long long>();
+  a.rank_in_run = b.rank.as<uint32_t>();
+  a.heavy_list = b.heavy.as<uint32_t>();
+  a.pos_row = nullptr;  // resolved by the key ingest
+  a.uniq = b.uniq.as<int64_t>();
+  a.uniq_owner = b.uniq_owner.as<uint8_t>();
+  a.uniq_row = b.uniq_row.as<int32_t>();
+  a.run_start = b.run_start.as<uint32_t>();
+  a.sorted_pos = b.sorted_pos.as<uint32_t>();
+  a.idx_map = b.idx_map.as<int32_t>();
+  a.meta = b.meta.as<uint32_t>();
+  a.side_stream = stream_side_;
+  a.fork_event = b.ev_scatter;
+  // The ordering kernels are enqueued by flushOrdering, after the gradient reduction, which brings the reduction (it
+  // only starts once push_pull is called) several launches forward.
+  a.join_event = nullptr;
   int sp = tic(kPhDedupe);
-  HCTR_LAUNCH(hctr_dedupe_map(&b.order_args, stream_main_));  // records b.ev_scatter behind its last kernel
+  HCTR_LAUNCH(hctr_dedupe_map(&a, stream_main_));  // records b.ev_scatter behind its last kernel
   b.scatter_recorded = true;
+  b.dedupe_in_flight = true;
   toc(sp);
   const size_t meta_words = HCTR_META_WORDS + nrank_ + 1;
   HCTR_CUDA(cudaMemcpyAsync(b.h_meta, b.meta.p, meta_words * sizeof(uint32_t), cudaMemcpyDeviceToHost, stream_main_));
@@ -596,6 +601,7 @@ void HetuTable::finalizePrev() {
 
 void HetuTable::finalizePending() {
   if (!cur_batch_.pending && !prev_batch_.pending) return;
+  flushDedupe(prev_batch_);
   flushDedupe(cur_batch_);
   HCTR_CUDA(cudaStreamSynchronize(stream_main_));
   collectSpans();
@@ -631,8 +637,15 @@ void HetuTable::pushPull(embed_t *grad, embed_t *dst) {
     prev.batch_size = 0;
     prev.unique_size = 0;
     prev.n_heavy = 0;
+    if (n == 1) prev.dedupe_pending = prev.order_pending = prev.pending = false;  // nobody will ask for its runs
     std::fill(prev.push_send.begin(), prev.push_send.end(), 0);
     std::fill(prev.push_recv.begin(), prev.push_recv.end(), 0);
+  }
+
+  // The batch before was pulled without gradients (its dedupe was not due then) and gets some now.
+  if (n == 1 && prev.dedupe_pending) {
+    flushDedupe(prev);
+    flushOrdering(prev);
   }
 
   // dst (and grad) are normally device memory; host buffers are staged
@@ -737,6 +750,7 @@ void HetuTable::pushPull(embed_t *grad, embed_t *dst) {
     int sp = tic(kPhReduce, stream_reduce_);
     HCTR_LAUNCH(hctr_grad_reduce_apply_pack(&r, stream_reduce_));
     toc(sp, stream_reduce_);
+    prev.dedupe_in_flight = false;  // stream_reduce_ has waited for it
     HCTR_CUDA(cudaEventRecord(ev_reduce_, stream_reduce_));
     // everything below reads rows / versions the reduction updates (a single-rank table runs it on the reduction's
     // own stream instead, and its dedupe on stream_main_ needs nothing from here)
@@ -764,9 +778,12 @@ void HetuTable::pushPull(embed_t *grad, embed_t *dst) {
     toc(sp, tail);
     // The dedupe of this batch goes behind the step's critical path on stream_main_ (low priority): only the next
     // step's reduction needs it.  (Holding it back until the reduction has ended was measured and is slower: the
-    // dedupe then ends after the expansion and the next reduction waits for it.)
-    flushDedupe(cur);
-    flushOrdering(cur);
+    // dedupe then ends after the expansion and the next reduction waits for it.)  A step without gradients is taken
+    // for serving: the dedupe of its batch stays due until gradients for it come, which they normally never do.
+    if (grad != nullptr) {
+      flushDedupe(cur);
+      flushOrdering(cur);
+    }
   } else if (use_p2p_) {
     exchangeP2P(dst_dev);
   } else {

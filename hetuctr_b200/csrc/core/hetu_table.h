@@ -63,10 +63,11 @@ struct BatchDesc {
   bool order_recorded = false;
   cudaEvent_t ev_scatter = nullptr;  // this batch's positions are in their runs (end of the dedupe pipeline)
   bool scatter_recorded = false;
+  bool dedupe_in_flight = false;     // the dedupe was enqueued and the reduction's stream has not waited for it yet
   bool light_ordered = false;        // runs of up to HCTR_LIGHT_RUN positions have been put in ascending order
   bool decided = false;            // the push decision for this batch has been enqueued
   bool order_pending = false;      // the run-ordering kernels of this batch are not enqueued yet
-  bool dedupe_pending = false;     // single-rank tables: the dedupe pipeline of this batch is not enqueued yet
+  bool dedupe_pending = false;     // the dedupe pipeline of this batch is not enqueued yet
   hctr_dedupe_args order_args;     // what both will be launched with
   DevBuf keys, idx_map, sorted_pos, uniq, uniq_owner, uniq_row, run_start, meta, pos_row, heavy;
   // Push decision of this batch (multi-rank tables): flag and send slot per unique key.  They belong to the batch
