@@ -10,6 +10,7 @@
 #include "core/transport.h"
 #include "hctr_kernels.h"
 #include "utils/errors.h"
+#include "utils/stage_keys.h"
 
 namespace hetuCTR {
 
@@ -339,17 +340,6 @@ void HetuTable::preprocess(index_t *data_ptr, size_t batch_size) {
   const int n = nrank_;
   const size_t meta_words = HCTR_META_WORDS + n + 1;
 
-  bool keys_on_device = false;
-  if (batch_size > 0) {
-    cudaPointerAttributes attr;
-    if (cudaPointerGetAttributes(&attr, data_ptr) == cudaSuccess)
-      keys_on_device = attr.type == cudaMemoryTypeDevice || attr.type == cudaMemoryTypeManaged;
-    else
-      cudaGetLastError();
-  }
-  // One launch in front of the pipeline: private copy of the keys (host keys are copied first, then taken in place),
-  // cleared meta words, and the local row of every batch position - which is all the row expansion needs for keys
-  // that are stored here, so a single-rank table starts it without waiting for the dedupe.
   // A single-rank table ingests on the (idle) stream of its reduction: stream_main_ may still hold the previous
   // batch's dedupe, which nothing here has to wait for.  The dedupe of this batch waits for ev_keys_.
   cudaStream_t ks = n == 1 ? stream_reduce_ : stream_main_;
@@ -358,19 +348,12 @@ void HetuTable::preprocess(index_t *data_ptr, size_t batch_size) {
     if (cur.order_recorded) HCTR_CUDA(cudaStreamWaitEvent(ks, cur.ev_order, 0));
     cur.dedupe_in_flight = false;
   }
-  const int64_t *key_src = reinterpret_cast<const int64_t *>(data_ptr);
-  if (!keys_on_device) {
-    HCTR_CUDA(cudaMemcpyAsync(cur.keys.p, data_ptr, sizeof(index_t) * batch_size, cudaMemcpyDefault, ks));
-    key_src = cur.keys.as<int64_t>();
-  }
-  HCTR_LAUNCH(hctr_ingest_keys_rows(key_src, cur.keys.as<int64_t>(), batch_size, cur.meta.as<uint32_t>(),
-                                    (unsigned)meta_words, d_row_of_.as<int32_t>(), kEmbeddingIDMax,
-                                    cur.pos_row.as<int32_t>(), d_ingest_err_, ks));
-  HCTR_CUDA(cudaEventRecord(ev_keys_, ks));
   cur.scatter_recorded = false;
   cur.light_ordered = false;
   cur.dedupe_pending = true;
   cur.order_pending = true;
+  cur.pending = true;
+  ingestKeys(cur, data_ptr, batch_size, ks);
   // The push decision for the previous batch goes first: the gradient reduction (on its own stream, started
   // by the next push_pull) only needs this, not the dedupe of the new batch that follows.
 
@@ -378,24 +361,14 @@ void HetuTable::preprocess(index_t *data_ptr, size_t batch_size) {
   // row is owned, nothing is ever pushed.
   const bool decide = n > 1 && prev.unique_size > 0;
   if (decide && !prev.decided) launchPushDecide(prev);  // normally done at the end of the previous push_pull
-  HCTR_CUDA(cudaEventRecord(ev_decide_, stream_reduce_));
+  if (n > 1) HCTR_CUDA(cudaEventRecord(ev_decide_, stream_reduce_));
   prev_push_valid_ = decide;
-  cur.pending = true;
   if (n == 1) {
     // Single rank: nothing of this step reads what the dedupe produces (the expansion has the rows from the key
     // ingest), so its launches are left to push_pull, AFTER the reduction and the expansion have been enqueued: the
-    // host reaches those sooner.  Wait only until the caller's key buffer has been consumed.
-    HCTR_CUDA(cudaEventSynchronize(ev_keys_));
-    if (*h_ingest_err_) {
-      // a key outside the table: drop the batch (its dedupe is not enqueued yet) and report right away
-      *h_ingest_err_ = 0;
-      cur.dedupe_pending = cur.order_pending = cur.pending = false;
-      cur.batch_size = cur.unique_size = cur.n_heavy = 0;
-      throw std::runtime_error("preprocess: a key is outside [0, length)");
-    }
+    // host reaches those sooner.
     return;
   }
-  *h_ingest_err_ = 0;  // multi-rank tables learn about bad keys from the dedupe (which also checks the owners)
   flushDedupe(cur);
   int sp;
   uint32_t *h_cnt_s = h_pinned_ + meta_words;
@@ -417,15 +390,100 @@ void HetuTable::preprocess(index_t *data_ptr, size_t batch_size) {
   }
   if (use_p2p_) {
     // (The device-driven exchange, where counts never visit the host.)
-    // Nothing on the host depends on the result before push_pull: wait only until the caller's key
-    // buffer has been consumed and let the rest of the pipeline run under the next call's launches.
+    // Nothing on the host depends on the result before push_pull: the rest of the pipeline runs under the next
+    // call's launches.
     // The batch's sizes (and a key-range error, if any) are picked up at the next synchronisation.
-    HCTR_CUDA(cudaEventSynchronize(ev_keys_));
     return;
   }
   transport_->waitStream(stream_main_);  // an NCCL group is in the stream: wait with a deadline
   collectSpans();
   finalizeBatch();
+}
+
+// One launch in front of the pipeline: private copy of the keys, cleared meta words, and the local row of every batch
+// position - which is all the row expansion needs for keys that are stored here, so a single-rank table starts it
+// without waiting for the dedupe.  Records ev_keys_; returns when the caller's buffer may be reused.
+//  * Keys in pageable memory (and small pinned batches) are copied into pinned staging by this thread, which checks
+//    their range on the way: nothing is left to wait for, and the kernel reads the staged keys over the host link.
+//    Big batches go in chunks, so that the link works while the next chunk is being copied.
+//  * Keys the device can address - device, managed or pinned memory - are read in place and the call waits for the
+//    kernel that has read them all.
+void HetuTable::ingestKeys(BatchDesc &b, const void *keys, size_t n, cudaStream_t s) {
+  // Staging a pinned batch costs ~0.2 us per 1000 keys, waiting for the kernel to read it in place ~8 us plus the
+  // transfer.
+  constexpr size_t kStagePinned = 16384;
+  constexpr size_t kChunk = 65536;
+  const unsigned meta_words = (unsigned)(HCTR_META_WORDS + nrank_ + 1);
+  const void *in_place = n == 0 ? nullptr : keys;
+  bool pageable = false;
+  if (n > 0) {
+    cudaPointerAttributes attr;
+    if (cudaPointerGetAttributes(&attr, keys) != cudaSuccess) {
+      cudaGetLastError();
+      attr.type = cudaMemoryTypeUnregistered;
+    }
+    const bool pinned = attr.type == cudaMemoryTypeHost && attr.devicePointer != nullptr;
+    pageable = !(attr.type == cudaMemoryTypeDevice || attr.type == cudaMemoryTypeManaged || pinned);
+    if (pinned) in_place = attr.devicePointer;
+    if (pageable || (pinned && n <= kStagePinned)) {
+      const bool narrow = kEmbeddingIDMax <= ((size_t)1 << 31);
+      const size_t each = narrow ? sizeof(int32_t) : sizeof(int64_t);
+      if (b.h_keys_busy) HCTR_CUDA(cudaEventSynchronize(ev_keys_));
+      b.h_keys_busy = false;
+      if (b.h_keys_bytes < n * each) {
+        if (b.h_keys) HCTR_CUDA(cudaFreeHost(b.h_keys));
+        b.h_keys = nullptr;
+        b.h_keys_bytes = 0;
+        const size_t want = round_up(std::max(n, b.capacity) * each, 4096);
+        HCTR_CUDA(cudaHostAlloc(&b.h_keys, want, cudaHostAllocMapped));
+        b.h_keys_bytes = want;
+      }
+      void *dev = nullptr;
+      HCTR_CUDA(cudaHostGetDevicePointer(&dev, b.h_keys, 0));
+      const int64_t *src = static_cast<const int64_t *>(keys);
+      bool good = true;
+      for (size_t off = 0; off < n && good; off += kChunk) {
+        const size_t m = std::min(kChunk, n - off);
+        char *to = static_cast<char *>(b.h_keys) + off * each;
+        good = narrow ? stage_keys(src + off, reinterpret_cast<int32_t *>(to), m, kEmbeddingIDMax)
+                      : stage_keys(src + off, reinterpret_cast<int64_t *>(to), m, kEmbeddingIDMax);
+        if (!good) break;
+        HCTR_LAUNCH(hctr_ingest_keys_rows(static_cast<const char *>(dev) + off * each, (int)each,
+                                          b.keys.as<int64_t>() + off, m, b.meta.as<uint32_t>(),
+                                          off == 0 ? meta_words : 0u, d_row_of_.as<int32_t>(), kEmbeddingIDMax,
+                                          b.pos_row.as<int32_t>() + off, nullptr, s));
+        b.h_keys_busy = true;
+      }
+      if (good) {
+        HCTR_CUDA(cudaEventRecord(ev_keys_, s));
+        return;
+      }
+      HCTR_CUDA(cudaStreamSynchronize(s));  // chunks in front of the bad one may still be on their way
+      b.h_keys_busy = false;
+      if (nrank_ == 1) dropBadBatch(b);
+      // a multi-rank table takes the whole batch to the dedupe, which reports the key at the end of the step
+    }
+  }
+  if (pageable) {
+    HCTR_CUDA(cudaMemcpyAsync(b.keys.p, keys, sizeof(index_t) * n, cudaMemcpyDefault, s));
+    in_place = b.keys.p;
+  }
+  HCTR_LAUNCH(hctr_ingest_keys_rows(in_place, (int)sizeof(index_t), b.keys.as<int64_t>(), n, b.meta.as<uint32_t>(),
+                                    meta_words, d_row_of_.as<int32_t>(), kEmbeddingIDMax, b.pos_row.as<int32_t>(),
+                                    d_ingest_err_, s));
+  HCTR_CUDA(cudaEventRecord(ev_keys_, s));
+  if (n == 0 || (nrank_ > 1 && !use_p2p_)) return;  // (NCCL: the count exchange that follows waits for the stream)
+  HCTR_CUDA(cudaEventSynchronize(ev_keys_));
+  const bool bad = *h_ingest_err_ != 0;
+  *h_ingest_err_ = 0;
+  if (bad && nrank_ == 1) dropBadBatch(b);  // (multi-rank tables hear of it from the dedupe, which also checks owners)
+}
+
+// A key outside the table: the batch is dropped (its dedupe is not enqueued yet) and the caller told right away.
+void HetuTable::dropBadBatch(BatchDesc &b) {
+  b.dedupe_pending = b.order_pending = b.pending = false;
+  b.batch_size = b.unique_size = b.n_heavy = 0;
+  throw std::runtime_error("preprocess: a key is outside [0, length)");
 }
 
 // The row expansion: the register kernel, or (HCTR_EXPAND=bulk) the bulk-copy engine variant.
@@ -739,7 +797,7 @@ void HetuTable::pushPull(embed_t *grad, embed_t *dst) {
     r.join_event = ev_rjoin_;
     // Own stream: overlaps the (still running) dedupe of the current batch.  It needs the push decision of
     // the previous batch (ev_decide_) and nothing else from stream_main_.
-    HCTR_CUDA(cudaStreamWaitEvent(stream_reduce_, ev_decide_, 0));
+    if (n > 1) HCTR_CUDA(cudaStreamWaitEvent(stream_reduce_, ev_decide_, 0));
     // the batch's runs must exist (end of its dedupe); the ordering of its long runs only concerns the long-run
     // kernel, and the short runs are ordered by the streaming kernel as it loads them (or here, for the row
     // widths and gradient buffers that kernel does not take)
@@ -751,10 +809,12 @@ void HetuTable::pushPull(embed_t *grad, embed_t *dst) {
     HCTR_LAUNCH(hctr_grad_reduce_apply_pack(&r, stream_reduce_));
     toc(sp, stream_reduce_);
     prev.dedupe_in_flight = false;  // stream_reduce_ has waited for it
-    HCTR_CUDA(cudaEventRecord(ev_reduce_, stream_reduce_));
     // everything below reads rows / versions the reduction updates (a single-rank table runs it on the reduction's
     // own stream instead, and its dedupe on stream_main_ needs nothing from here)
-    if (n > 1) HCTR_CUDA(cudaStreamWaitEvent(stream_main_, ev_reduce_, 0));
+    if (n > 1) {
+      HCTR_CUDA(cudaEventRecord(ev_reduce_, stream_reduce_));
+      HCTR_CUDA(cudaStreamWaitEvent(stream_main_, ev_reduce_, 0));
+    }
   }
   if (n > 1) flushOrdering(cur);  // the current batch's run ordering, deferred by preprocess
 
@@ -762,9 +822,8 @@ void HetuTable::pushPull(embed_t *grad, embed_t *dst) {
   cudaStream_t tail = n == 1 ? stream_reduce_ : stream_main_;
   if (n == 1) {
     // Single rank: every key is owned and stored here; the pull is a local gather that only needs the rows the
-    // key ingest resolved (ev_keys_) and the reduction in front of it on this stream.  The dedupe of this batch
+    // key ingest resolved and the reduction, both in front of it on this stream.  The dedupe of this batch
     // keeps running on stream_main_; nothing of this step reads its results.
-    HCTR_CUDA(cudaStreamWaitEvent(tail, ev_keys_, 0));
     int sp = tic(kPhExpand, tail);
     if (split_expand) {
       HCTR_LAUNCH(hctr_expand_rows_subset(cur.batch_size, W, cur.pos_row.as<int32_t>(), cur.keys.as<int64_t>(),
@@ -773,7 +832,7 @@ void HetuTable::pushPull(embed_t *grad, embed_t *dst) {
       HCTR_CUDA(cudaStreamWaitEvent(tail, ev_early_, 0));  // the step ends when both halves are in dst
     } else {
       HCTR_LAUNCH(expandRows(cur.batch_size, W, cur.pos_row.as<int32_t>(), cur.idx_map.as<int32_t>(), nullptr,
-                                   nullptr, d_embedding_.as<float>(), dst_dev, d_ingest_err_ + 1, tail));
+                             nullptr, d_embedding_.as<float>(), dst_dev, d_ingest_err_ + 1, tail));
     }
     toc(sp, tail);
     // The dedupe of this batch goes behind the step's critical path on stream_main_ (low priority): only the next
@@ -974,9 +1033,10 @@ void HetuTable::pushPull(embed_t *grad, embed_t *dst) {
 
   if (dst_staged)
     HCTR_CUDA(cudaMemcpyAsync(dst, dst_dev, cur.batch_size * W * sizeof(embed_t), cudaMemcpyDeviceToHost, tail));
-  // the expand kernel reports a bounded wait that ran out through a mapped pinned word: nothing to copy back
+  // the bulk-copy expansion reports a bounded wait that ran out through a mapped pinned word: nothing to copy back
   if (transport_ && !use_p2p_) transport_->waitStream(tail);
   else HCTR_CUDA(cudaStreamSynchronize(tail));
+  cur.h_keys_busy = false;  // the step has read its keys
   collectSpans();
   if (h_ingest_err_[1]) {
     h_ingest_err_[1] = 0;
@@ -1325,6 +1385,8 @@ void HetuTable::releaseAll() {
     b->ev_scatter = nullptr;
     if (b->h_meta) cudaFreeHost(b->h_meta);
     b->h_meta = nullptr;
+    if (b->h_keys) cudaFreeHost(b->h_keys);
+    b->h_keys = nullptr;
   }
   if (h_ingest_err_) cudaFreeHost(h_ingest_err_);
   h_ingest_err_ = d_ingest_err_ = nullptr;

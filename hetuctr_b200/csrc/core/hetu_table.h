@@ -77,6 +77,10 @@ struct BatchDesc {
   // rank of every position inside its run; later the staging area of the batch's run ordering (its own buffer, so
   // that the ordering of one batch can overlap the dedupe of the next)
   DevBuf rank;
+  // mapped pinned staging of a batch handed over in host memory (32-bit keys where the table's length allows)
+  void *h_keys = nullptr;
+  size_t h_keys_bytes = 0;
+  bool h_keys_busy = false;        // an ingest kernel may still be reading it
   uint32_t *h_meta = nullptr;      // pinned: the batch's meta words (sizes, segment starts, error bits) as read back
   std::vector<size_t> seg;         // [n+1] first unique of each owner
   std::vector<size_t> query_send;  // [n] unique keys addressed to each owner
@@ -244,9 +248,11 @@ class HetuTable {
   void *h_src_ = nullptr;         // pinned staging of the per-source list descriptors
   size_t p2p_off_cap_ = 0;        // mailbox capacity d_src_off_ was filled for
   uint32_t *h_pinned_ = nullptr;  // pinned mirror for counts read back from the device
-  // Mapped pinned word the key ingest reports an out-of-range key through: the host reads it right after the
-  // ingest without a copy.
+  // Mapped pinned words: [0] the key ingest reports an out-of-range key through (the host reads it right after the
+  // ingest without a copy), [1] error bits of the bulk-copy expansion.
   uint32_t *h_ingest_err_ = nullptr, *d_ingest_err_ = nullptr;
+  void dropBadBatch(BatchDesc &b);
+  void ingestKeys(BatchDesc &b, const void *keys, size_t n, cudaStream_t s);
   size_t h_pinned_words_ = 0;
 
   BatchDesc cur_batch_, prev_batch_;

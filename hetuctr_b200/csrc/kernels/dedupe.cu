@@ -333,37 +333,71 @@ __global__ void __launch_bounds__(kThreads) ingest_keys(const long long *__restr
 
 // The same, plus the local row of every batch position (pos_row[i] = row_of[key] or HCTR_INVALID_ROW): all the
 // row expansion needs to know about a batch whose keys are stored here, so that it does not have to wait for the
-// dedupe pipeline.  src may equal dst (keys already in place).  A key outside [0, length) sets bit
-// HCTR_ERR_KEY_RANGE in *err.
-__global__ void __launch_bounds__(kThreads) ingest_keys_rows(const long long *__restrict__ src,
-                                                             long long *__restrict__ dst, size_t n,
+// dedupe pipeline.  src may equal dst (keys already in place) and may be mapped host memory; K is the width the keys
+// arrive in.  A key outside [0, length) sets HCTR_ERR_KEY_RANGE in *err.
+// Bound: the latency of two dependent accesses (key, row), so a thread takes ITEMS independent ones.
+template <class K, int ITEMS>
+__global__ void __launch_bounds__(kThreads) ingest_keys_rows(const K *src, long long *dst, size_t n,
                                                              u32 *__restrict__ meta, unsigned meta_words,
                                                              const int32_t *__restrict__ row_of, size_t length,
-                                                             int32_t *__restrict__ pos_row, u32 *__restrict__ err) {
-  const size_t i = (size_t)blockIdx.x * kThreads + threadIdx.x;
-  if (i < meta_words) meta[i] = 0;
-  if (i < n) {
-    const long long k = src[i];
-    if (src != dst) dst[i] = k;
-    int32_t row = HCTR_INVALID_ROW;
-    if (k >= 0 && (size_t)k < length) row = row_of[k];
-    else atomicOr(err, HCTR_ERR_KEY_RANGE);
-    pos_row[i] = row;
+                                                             int32_t *__restrict__ pos_row, u32 *err) {
+  const size_t base = (size_t)blockIdx.x * kThreads * ITEMS + threadIdx.x;
+  for (unsigned m = blockIdx.x * kThreads + threadIdx.x; m < meta_words; m += gridDim.x * kThreads) meta[m] = 0;
+  long long k[ITEMS];
+  int32_t row[ITEMS];
+  bool bad = false;
+#pragma unroll
+  for (int j = 0; j < ITEMS; j++) {
+    const size_t i = base + (size_t)j * kThreads;
+    k[j] = i < n ? (long long)src[i] : 0;
   }
+#pragma unroll
+  for (int j = 0; j < ITEMS; j++) {
+    const size_t i = base + (size_t)j * kThreads;
+    row[j] = HCTR_INVALID_ROW;
+    if (i < n) {
+      if (k[j] >= 0 && (size_t)k[j] < length) row[j] = row_of[k[j]];
+      else bad = true;
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < ITEMS; j++) {
+    const size_t i = base + (size_t)j * kThreads;
+    if (i < n) {
+      if ((const void *)src != (const void *)dst) dst[i] = k[j];
+      pos_row[i] = row[j];
+    }
+  }
+  if (bad && err) atomicOr(err, HCTR_ERR_KEY_RANGE);
 }
 
 }  // namespace hctr
 
 using namespace hctr;
 
-extern "C" int hctr_ingest_keys_rows(const int64_t *src, int64_t *dst, size_t n, uint32_t *meta, unsigned meta_words,
-                                     const int32_t *row_of, size_t length, int32_t *pos_row, uint32_t *err,
-                                     void *stream) {
-  const size_t items = n > meta_words ? n : meta_words;
-  ingest_keys_rows<<<grid_for(items ? items : 1, kThreads), kThreads, 0, (cudaStream_t)stream>>>(
-      (const long long *)src, (long long *)dst, n, meta, meta_words, row_of, length, pos_row, err);
+template <class K>
+static int launch_ingest(const K *src, int64_t *dst, size_t n, uint32_t *meta, unsigned meta_words,
+                         const int32_t *row_of, size_t length, int32_t *pos_row, uint32_t *err, void *stream) {
+  cudaStream_t s = (cudaStream_t)stream;
+  // four keys per thread where that still leaves every SM a block
+  if (n >= (size_t)kThreads * 4 * kSMs)
+    ingest_keys_rows<K, 4><<<grid_for(n, kThreads * 4), kThreads, 0, s>>>(src, (long long *)dst, n, meta, meta_words,
+                                                                         row_of, length, pos_row, err);
+  else
+    ingest_keys_rows<K, 1><<<grid_for(n, kThreads), kThreads, 0, s>>>(src, (long long *)dst, n, meta, meta_words,
+                                                                     row_of, length, pos_row, err);
   count_launches(1);
   return launch_status();
+}
+
+extern "C" int hctr_ingest_keys_rows(const void *src, int key_bytes, int64_t *dst, size_t n, uint32_t *meta,
+                                     unsigned meta_words, const int32_t *row_of, size_t length, int32_t *pos_row,
+                                     uint32_t *err, void *stream) {
+  if (key_bytes == 8)
+    return launch_ingest((const long long *)src, dst, n, meta, meta_words, row_of, length, pos_row, err, stream);
+  if (key_bytes == 4)
+    return launch_ingest((const int32_t *)src, dst, n, meta, meta_words, row_of, length, pos_row, err, stream);
+  return (int)cudaErrorInvalidValue;
 }
 
 extern "C" int hctr_detect_key_stride(const int64_t *keys, size_t n, uint32_t *scores, void *stream) {

@@ -189,10 +189,11 @@ int hctr_detect_key_stride(const int64_t *keys, size_t n, uint32_t *scores, void
  * copy, so that the caller may reuse its buffer) and meta[0..meta_words) = 0, in one launch. */
 int hctr_ingest_keys(const int64_t *src, int64_t *dst, size_t n, uint32_t *meta, unsigned meta_words, void *stream);
 /* hctr_ingest_keys plus pos_row[i] = row_of[keys[i]] (HCTR_INVALID_ROW for a key that is not stored here or lies
- * outside [0, length); the latter also sets HCTR_ERR_KEY_RANGE in *err).  With pos_row known this early the row
- * expansion of a batch whose keys are all stored locally does not depend on the dedupe pipeline at all.  src may
- * equal dst.  Part of what cvt_embedding_idx_2_offset did, csrc/core/preprocess.cu:62-76. */
-int hctr_ingest_keys_rows(const int64_t *src, int64_t *dst, size_t n, uint32_t *meta, unsigned meta_words,
+ * outside [0, length)).  With pos_row known this early the row expansion of a batch whose keys are all stored locally
+ * does not depend on the dedupe pipeline at all.  src holds keys of key_bytes (4 or 8) bytes, may equal dst and may be
+ * mapped host memory.  Part of what cvt_embedding_idx_2_offset did, csrc/core/preprocess.cu:62-76.
+ * A key out of range sets HCTR_ERR_KEY_RANGE in *err (null: the caller has checked). */
+int hctr_ingest_keys_rows(const void *src, int key_bytes, int64_t *dst, size_t n, uint32_t *meta, unsigned meta_words,
                           const int32_t *row_of, size_t length, int32_t *pos_row, uint32_t *err, void *stream);
 
 /* The run-ordering half of the pipeline alone (positions of every unique key's run in ascending batch order
