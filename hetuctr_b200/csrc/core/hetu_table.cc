@@ -222,11 +222,12 @@ void HetuTable::initTable(const worker_t *root, const index_t *storage) {
   HCTR_CUDA(cudaMemsetAsync(d_gradient_.p, 0, d_gradient_.bytes, stream_main_));
   HCTR_CUDA(cudaMemsetAsync(d_updates_.p, 0, d_updates_.bytes, stream_main_));
   HCTR_LAUNCH(hctr_table_build(d_stored_keys_.as<int64_t>(), S, kNonLocalStorageMax, N, d_row_of_.as<int32_t>(),
-                               d_version_.as<int64_t>(), err, stream_main_));
+                               d_version_.as<int64_t>(), err, err + 48, stream_main_));
   HCTR_LAUNCH(hctr_count_owned(d_root_.as<uint8_t>(), N, rank_, owned_cnt, stream_main_));
-  uint32_t h_err = 0;
+  uint32_t h_err = 0, h_moved = 0;
   unsigned long long h_owned = 0;
   HCTR_CUDA(cudaMemcpyAsync(&h_err, err, sizeof(h_err), cudaMemcpyDeviceToHost, stream_main_));
+  HCTR_CUDA(cudaMemcpyAsync(&h_moved, err + 48, sizeof(h_moved), cudaMemcpyDeviceToHost, stream_main_));
   HCTR_CUDA(cudaMemcpyAsync(&h_owned, owned_cnt, sizeof(h_owned), cudaMemcpyDeviceToHost, stream_main_));
   HCTR_CUDA(cudaStreamSynchronize(stream_main_));
   raw.release();
@@ -239,6 +240,7 @@ void HetuTable::initTable(const worker_t *root, const index_t *storage) {
   // The owner answers every query for its rows (csrc/core/handle_query.cu:12-15 asserts it), so a
   // rank must store all rows it owns.
   HCTR_CHECK(h_owned == S - kNonLocalStorageMax, "storage_arr must contain every key whose root_arr entry is this rank");
+  rows_are_keys_ = nrank_ == 1 && S == N && h_moved == 0;
 
   if (nrank_ > 1) {
     // owner-side apply: one source-mask word per owned row, and the per-source list descriptors
@@ -250,7 +252,16 @@ void HetuTable::initTable(const worker_t *root, const index_t *storage) {
     d_src_cnt_.ensure(((size_t)nrank_ + 1) * sizeof(uint32_t));
   }
 
-  // dedupe scratch over the (owner, key) space: all-zero at rest
+  d_group_hist_.ensure(2048 * sizeof(uint32_t));
+  d_group_tiles_.ensure((6 + 512) * HCTR_GROUP_MAX_TILES * sizeof(uint32_t));
+  HCTR_CUDA(cudaMemsetAsync(d_group_hist_.p, 0, d_group_hist_.bytes, stream_main_));
+  HCTR_CUDA(cudaMemsetAsync(d_group_tiles_.p, 0, 6 * HCTR_GROUP_MAX_TILES * sizeof(uint32_t), stream_main_));
+  HCTR_CUDA(cudaStreamSynchronize(stream_main_));
+}
+
+// Scratch of the bitmap ranking (batches the radix grouping does not serve): table-sized, all-zero at rest.
+void HetuTable::reserveBitmap() {
+  if (d_bits_.p) return;
   const size_t words = (size_t)nrank_ * length_pad_ / HCTR_WORD_BITS;
   const size_t blocks = (size_t)nrank_ * length_pad_ / HCTR_BLOCK_KEYS;
   d_bits_.ensure(words * sizeof(unsigned long long));
@@ -277,7 +288,12 @@ void HetuTable::reserveBatch(BatchDesc &b, size_t batch) {
   b.meta.ensure((HCTR_META_WORDS + nrank_ + 1) * sizeof(uint32_t));
   b.pos_row.ensure(batch * sizeof(int32_t));
   b.heavy.ensure((batch / 32 + 2) * sizeof(uint32_t));
-  b.rank.ensure(batch * sizeof(uint32_t));
+  if (!hctr_group_fits(batch, kEmbeddingIDMax, nrank_)) b.rank.ensure(batch * sizeof(uint32_t));
+  b.chunk_key.ensure((batch / HCTR_CHUNK_POS + 2) * sizeof(uint32_t));
+  if (nrank_ == 1) {  // every key is rank 0's, once and for all
+    HCTR_CUDA(cudaMemsetAsync(b.uniq_owner.p, 0, b.uniq_owner.bytes, stream_main_));
+    HCTR_CUDA(cudaStreamSynchronize(stream_main_));
+  }
   if (nrank_ > 1) {
     b.need_push.ensure((batch + 1) * sizeof(uint32_t));
     b.push_slot.ensure((batch + 1) * sizeof(uint32_t));
@@ -297,8 +313,14 @@ void HetuTable::reserveShared(size_t batch) {
   HCTR_CUDA(cudaMemsetAsync(d_chain3_.p, 0, d_chain3_.bytes, stream_main_));
   HCTR_CUDA(cudaStreamSynchronize(stream_main_));  // the scratch is used from other streams as well
   d_sk_.ensure(batch * sizeof(unsigned long long));
-  d_cnt_.ensure((batch + 1) * sizeof(uint32_t));  // all-zero between calls, like the bitmap
-  HCTR_CUDA(cudaMemsetAsync(d_cnt_.p, 0, d_cnt_.bytes, stream_main_));
+  d_pairs_.ensure(batch * sizeof(unsigned long long));
+  d_sort_keys_.ensure(batch * sizeof(uint32_t));
+  if (!hctr_group_fits(batch, kEmbeddingIDMax, nrank_)) {
+    reserveBitmap();
+    d_cnt_.ensure((batch + 1) * sizeof(uint32_t));  // all-zero between calls, like the bitmap
+    HCTR_CUDA(cudaMemsetAsync(d_cnt_.p, 0, d_cnt_.bytes, stream_main_));
+    HCTR_CUDA(cudaStreamSynchronize(stream_main_));
+  }
   d_push_count_.ensure((size_t)nrank_ * sizeof(uint32_t));
   d_push_base_.ensure((size_t)nrank_ * sizeof(uint32_t));
   d_recv_idx_.ensure((batch + 1) * sizeof(uint32_t));
@@ -414,6 +436,7 @@ void HetuTable::ingestKeys(BatchDesc &b, const void *keys, size_t n, cudaStream_
   constexpr size_t kStagePinned = 16384;
   constexpr size_t kChunk = 65536;
   const unsigned meta_words = (unsigned)(HCTR_META_WORDS + nrank_ + 1);
+  const int32_t *row_of = rows_are_keys_ ? nullptr : d_row_of_.as<int32_t>();
   const void *in_place = n == 0 ? nullptr : keys;
   bool pageable = false;
   if (n > 0) {
@@ -450,7 +473,7 @@ void HetuTable::ingestKeys(BatchDesc &b, const void *keys, size_t n, cudaStream_
         if (!good) break;
         HCTR_LAUNCH(hctr_ingest_keys_rows(static_cast<const char *>(dev) + off * each, (int)each,
                                           b.keys.as<int64_t>() + off, m, b.meta.as<uint32_t>(),
-                                          off == 0 ? meta_words : 0u, d_row_of_.as<int32_t>(), kEmbeddingIDMax,
+                                          off == 0 ? meta_words : 0u, row_of, kEmbeddingIDMax,
                                           b.pos_row.as<int32_t>() + off, nullptr, s));
         b.h_keys_busy = true;
       }
@@ -469,7 +492,7 @@ void HetuTable::ingestKeys(BatchDesc &b, const void *keys, size_t n, cudaStream_
     in_place = b.keys.p;
   }
   HCTR_LAUNCH(hctr_ingest_keys_rows(in_place, (int)sizeof(index_t), b.keys.as<int64_t>(), n, b.meta.as<uint32_t>(),
-                                    meta_words, d_row_of_.as<int32_t>(), kEmbeddingIDMax, b.pos_row.as<int32_t>(),
+                                    meta_words, row_of, kEmbeddingIDMax, b.pos_row.as<int32_t>(),
                                     d_ingest_err_, s));
   HCTR_CUDA(cudaEventRecord(ev_keys_, s));
   if (n == 0 || (nrank_ > 1 && !use_p2p_)) return;  // (NCCL: the count exchange that follows waits for the stream)
@@ -541,14 +564,64 @@ void HetuTable::flushDedupe(BatchDesc &b) {
   if (!b.dedupe_pending) return;
   b.dedupe_pending = false;
   if (nrank_ == 1) HCTR_CUDA(cudaStreamWaitEvent(stream_main_, ev_keys_, 0));
+  if (!b.ev_order) HCTR_CUDA(cudaEventCreateWithFlags(&b.ev_order, cudaEventDisableTiming));
+  if (!b.ev_scatter) HCTR_CUDA(cudaEventCreateWithFlags(&b.ev_scatter, cudaEventDisableTiming));
+  b.scatter_recorded = true;
+  b.dedupe_in_flight = true;
+  if (hctr_group_fits(b.batch_size, kEmbeddingIDMax, nrank_)) groupKeys(b);
+  else rankKeys(b);
+  if (nrank_ == 1) return;  // whoever wants the sizes on the host copies them then
+  const size_t meta_words = HCTR_META_WORDS + nrank_ + 1;
+  HCTR_CUDA(cudaMemcpyAsync(b.h_meta, b.meta.p, meta_words * sizeof(uint32_t), cudaMemcpyDeviceToHost, stream_main_));
+}
+
+// The usual form: a stable radix sort of (owner, key) and position.  Runs come out in batch order.
+void HetuTable::groupKeys(BatchDesc &b) {
+  hctr_group_args a{};
+  a.keys = b.keys.as<int64_t>();
+  a.batch = b.batch_size;
+  a.length = kEmbeddingIDMax;
+  a.nrank = nrank_;
+  a.owner_of = d_root_.as<uint8_t>();
+  a.pos_row = b.pos_row.as<int32_t>();
+  a.pairs0 = d_sk_.as<unsigned long long>();
+  a.pairs1 = d_pairs_.as<unsigned long long>();
+  a.sort_keys = d_sort_keys_.as<uint32_t>();
+  a.hist = d_group_hist_.as<uint32_t>();
+  a.tile_flags = d_group_tiles_.as<uint32_t>();
+  a.chain_scratch = a.tile_flags + 4 * HCTR_GROUP_MAX_TILES;
+  a.tile_counts = a.tile_flags + 6 * HCTR_GROUP_MAX_TILES;
+  a.epoch = nextEpoch();
+  a.uniq = b.uniq.as<int64_t>();
+  a.uniq_owner = b.uniq_owner.as<uint8_t>();
+  a.uniq_row = b.uniq_row.as<int32_t>();
+  a.run_start = b.run_start.as<uint32_t>();
+  a.sorted_pos = b.sorted_pos.as<uint32_t>();
+  a.idx_map = nrank_ > 1 ? b.idx_map.as<int32_t>() : nullptr;  // (one rank: for dump only, made there)
+  a.chunk_key = b.chunk_key.as<uint32_t>();
+  a.heavy_list = b.heavy.as<uint32_t>();
+  a.meta = b.meta.as<uint32_t>();
+  b.index_map_due = nrank_ == 1;
+  // (this descriptor's batch of two steps ago may have been ordered on the side stream)
+  if (b.order_recorded) HCTR_CUDA(cudaStreamWaitEvent(stream_main_, b.ev_order, 0));
+  b.order_pending = false;
+  b.order_recorded = false;
+  b.light_ordered = true;
+  int sp = tic(kPhDedupe);
+  HCTR_LAUNCH(hctr_group_keys(&a, stream_main_));
+  HCTR_CUDA(cudaEventRecord(b.ev_scatter, stream_main_));
+  toc(sp);
+}
+
+// Batches beyond that (more than 2 M keys, or (owner, key) pairs of more than 32 bits): bitmap ranking.
+void HetuTable::rankKeys(BatchDesc &b) {
+  b.index_map_due = false;
   if (!key_stride_known_ && b.batch_size >= 4096) detectKeyStride(b);  // once per table
   // run ordering happens on stream_side_, off this stream's critical path; the reduction of this batch
   // (next step) waits on the batch's own event.  The ordering stages through the batch's own rank buffer, so the
   // ordering of the previous batch may still run while this batch is deduplicated; only the descriptor being
   // recycled (two batches old) must be out of use.
   if (b.order_recorded) HCTR_CUDA(cudaStreamWaitEvent(stream_main_, b.ev_order, 0));
-  if (!b.ev_order) HCTR_CUDA(cudaEventCreateWithFlags(&b.ev_order, cudaEventDisableTiming));
-  if (!b.ev_scatter) HCTR_CUDA(cudaEventCreateWithFlags(&b.ev_scatter, cudaEventDisableTiming));
   b.order_recorded = false;
   // (built here and not at preprocess: a larger batch in between may have moved the shared scratch)
   hctr_dedupe_args &a = b.order_args;
@@ -585,19 +658,16 @@ void HetuTable::flushDedupe(BatchDesc &b) {
   a.join_event = nullptr;
   int sp = tic(kPhDedupe);
   HCTR_LAUNCH(hctr_dedupe_map(&a, stream_main_));  // records b.ev_scatter behind its last kernel
-  b.scatter_recorded = true;
-  b.dedupe_in_flight = true;
   toc(sp);
-  const size_t meta_words = HCTR_META_WORDS + nrank_ + 1;
-  HCTR_CUDA(cudaMemcpyAsync(b.h_meta, b.meta.p, meta_words * sizeof(uint32_t), cudaMemcpyDeviceToHost, stream_main_));
 }
 
 // The long runs (hot keys) are ordered on stream_side_; only the long-run kernel of the next reduction waits for
 // that.  The short runs are ordered by the reduction itself where its kernel can (orderLightRuns otherwise).
 void HetuTable::flushOrdering(BatchDesc &b) {
   if (!b.order_pending) return;
-  b.order_pending = false;
   flushDedupe(b);
+  if (!b.order_pending) return;  // came out in order
+  b.order_pending = false;
   HCTR_CUDA(cudaStreamWaitEvent(stream_side_, b.ev_scatter, 0));
   HCTR_LAUNCH(hctr_dedupe_order_heavy(&b.order_args, stream_side_));
   HCTR_CUDA(cudaEventRecord(b.ev_order, stream_side_));
@@ -661,6 +731,11 @@ void HetuTable::finalizePending() {
   if (!cur_batch_.pending && !prev_batch_.pending) return;
   flushDedupe(prev_batch_);
   flushDedupe(cur_batch_);
+  if (nrank_ == 1)
+    for (BatchDesc *b : {&prev_batch_, &cur_batch_})
+      if (b->pending)
+        HCTR_CUDA(cudaMemcpyAsync(b->h_meta, b->meta.p, (HCTR_META_WORDS + 2) * sizeof(uint32_t), cudaMemcpyDeviceToHost,
+                                  stream_main_));
   HCTR_CUDA(cudaStreamSynchronize(stream_main_));
   collectSpans();
   finalizePrev();  // (the dedupe of the previous batch sits in front of this one's on the same stream)
@@ -1372,7 +1447,7 @@ void HetuTable::releaseAll() {
   p2p_.reset();
   transport_.reset();
   DevBuf *all[] = {&d_embedding_, &d_gradient_, &d_updates_, &d_version_, &d_root_, &d_row_of_, &d_stored_keys_,
-                   &d_bits_, &d_blk_cnt_, &d_blk_flag_, &d_chain_, &d_chain3_, &d_ent_row_, &d_ent_next_, &d_row_mask_, &d_row_head_, &d_src_off_, &d_src_cnt_, &d_word_base_, &d_scan_, &d_sk_, &d_cnt_,
+                   &d_bits_, &d_blk_cnt_, &d_blk_flag_, &d_chain_, &d_chain3_, &d_ent_row_, &d_ent_next_, &d_row_mask_, &d_row_head_, &d_src_off_, &d_src_cnt_, &d_word_base_, &d_scan_, &d_sk_, &d_cnt_, &d_pairs_, &d_sort_keys_, &d_group_hist_, &d_group_tiles_,
                    &d_push_count_, &d_push_base_, &d_recv_idx_, &d_err_, &d_cnt_s_, &d_cnt_r_, &d_qver_s_,
                    &d_qkey_r_, &d_qver_r_, &d_pkey_s_, &d_pupd_s_, &d_pval_s_, &d_pkey_r_, &d_pupd_r_, &d_pval_r_,
                    &d_flag_s_, &d_flag_r_, &d_flag32_, &d_ret_slot_, &d_recv_slot_, &d_seg_r_, &d_retcnt_s_,
@@ -1392,7 +1467,7 @@ void HetuTable::releaseAll() {
   h_ingest_err_ = d_ingest_err_ = nullptr;
   for (BatchDesc *b : {&cur_batch_, &prev_batch_})
     for (DevBuf *d : {&b->keys, &b->idx_map, &b->sorted_pos, &b->uniq, &b->uniq_owner, &b->uniq_row,
-                      &b->run_start, &b->meta, &b->pos_row, &b->heavy, &b->need_push, &b->push_slot, &b->rank})
+                      &b->run_start, &b->meta, &b->pos_row, &b->heavy, &b->chunk_key, &b->need_push, &b->push_slot, &b->rank})
       d->release();
   for (Span &sp : spans_) {
     cudaEventDestroy(sp.a);

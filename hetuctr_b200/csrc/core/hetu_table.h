@@ -69,7 +69,8 @@ struct BatchDesc {
   bool order_pending = false;      // the run-ordering kernels of this batch are not enqueued yet
   bool dedupe_pending = false;     // the dedupe pipeline of this batch is not enqueued yet
   hctr_dedupe_args order_args;     // what both will be launched with
-  DevBuf keys, idx_map, sorted_pos, uniq, uniq_owner, uniq_row, run_start, meta, pos_row, heavy;
+  bool index_map_due = false;      // idx_map has not been filled (nothing but dump reads it on a single-rank table)
+  DevBuf keys, idx_map, sorted_pos, uniq, uniq_owner, uniq_row, run_start, meta, pos_row, heavy, chunk_key;
   // Push decision of this batch (multi-rank tables): flag and send slot per unique key.  They belong to the batch
   // because the decision is taken at the end of the batch's own push_pull and consumed by the next one; a larger
   // batch arriving in between must not move them.
@@ -192,6 +193,9 @@ class HetuTable {
                  const float *recv_val, const float *embedding, float *dst, uint32_t *err, cudaStream_t stream);
   void launchPushDecide(BatchDesc &b);
   void flushOrdering(BatchDesc &b);  // enqueues a batch's deferred run ordering
+  void groupKeys(BatchDesc &b);
+  void rankKeys(BatchDesc &b);
+  void reserveBitmap();
   void flushDedupe(BatchDesc &b);    // enqueues a batch's deferred dedupe pipeline (single-rank tables)
   void orderLightRuns(BatchDesc &b, cudaStream_t s);  // the short-run half of the ordering, where somebody needs it
   void quiesce();  // every stream drained, pending batch sizes read back
@@ -231,6 +235,8 @@ class HetuTable {
 
   // dedupe scratch (persistent, all-zero between calls) and per-step scratch
   DevBuf d_bits_, d_blk_cnt_, d_blk_flag_, d_chain_, d_chain3_, d_ent_row_, d_ent_next_, d_row_mask_, d_row_head_, d_src_off_, d_src_cnt_, d_word_base_, d_scan_, d_sk_, d_cnt_;
+  DevBuf d_pairs_, d_sort_keys_, d_group_hist_, d_group_tiles_;  // radix grouping; d_sk_ holds its other half of the pairs
+  bool rows_are_keys_ = false;  // single rank, every key stored in key order: row = key, no lookup
   DevBuf d_push_count_, d_push_base_, d_recv_idx_, d_err_;
   size_t shared_capacity_ = 0;
   uint32_t dedupe_epoch_ = 0;

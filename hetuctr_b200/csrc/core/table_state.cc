@@ -72,8 +72,16 @@ void HetuTable::quiesce() {
   finalizePending();
   flushOrdering(cur_batch_);
   // whoever looks at a batch's position lists expects every run in ascending order
-  for (BatchDesc *b : {&cur_batch_, &prev_batch_})
-    if (b->batch_size > 0) orderLightRuns(*b, stream_side_);
+  for (BatchDesc *b : {&cur_batch_, &prev_batch_}) {
+    if (b->batch_size == 0) continue;
+    orderLightRuns(*b, stream_side_);
+    if (b->index_map_due && b->scatter_recorded) {
+      HCTR_CUDA(cudaStreamWaitEvent(stream_side_, b->ev_scatter, 0));
+      HCTR_LAUNCH(hctr_group_index_map(b->meta.as<uint32_t>(), b->run_start.as<uint32_t>(),
+                                       b->sorted_pos.as<uint32_t>(), b->idx_map.as<int32_t>(), stream_side_));
+      b->index_map_due = false;
+    }
+  }
   for (cudaStream_t s : {stream_main_, stream_side_, stream_reduce_, stream_reduce_side_})
     if (s) HCTR_CUDA(cudaStreamSynchronize(s));
 }

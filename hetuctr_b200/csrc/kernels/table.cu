@@ -36,11 +36,12 @@ __global__ void __launch_bounds__(kThreads) storage_layout(const long long *__re
 
 __global__ void __launch_bounds__(kThreads) table_build(const long long *__restrict__ stored_keys, size_t n,
                                                         size_t n_cached, size_t length, int32_t *row_of,
-                                                        long long *__restrict__ version, u32 *err) {
+                                                        long long *__restrict__ version, u32 *err, u32 *moved) {
   const size_t i = (size_t)blockIdx.x * kThreads + threadIdx.x;
   if (i >= n) return;
   version[i] = i < n_cached ? INT64_MIN : 0;
   const long long k = stored_keys[i];
+  if (k != (long long)i) *moved = 1;
   if (k < 0 || (size_t)k >= length) {
     atomicOr(err, HCTR_ERR_KEY_RANGE);
     return;
@@ -104,13 +105,13 @@ extern "C" int hctr_storage_layout(const int64_t *storage, size_t n, const uint3
 }
 
 extern "C" int hctr_table_build(const int64_t *stored_keys, size_t n, size_t n_cached, size_t length,
-                                int32_t *row_of, int64_t *version, uint32_t *err, void *stream) {
+                                int32_t *row_of, int64_t *version, uint32_t *err, uint32_t *moved, void *stream) {
   cudaStream_t s = (cudaStream_t)stream;
   cudaError_t e = cudaMemsetAsync(row_of, 0xFF, length * sizeof(int32_t), s);
   if (e != cudaSuccess) return (int)e;
   if (n == 0) return 0;
   table_build<<<grid_for(n, kThreads), kThreads, 0, s>>>((const long long *)stored_keys, n, n_cached, length, row_of,
-                                                         (long long *)version, err);
+                                                         (long long *)version, err, moved);
   return launch_status();
 }
 

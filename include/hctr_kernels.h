@@ -41,6 +41,9 @@ extern "C" {
 #define HCTR_BLOCK_WORDS 64
 #define HCTR_BLOCK_KEYS 4096
 #define HCTR_SCAN_TILE 4096
+#define HCTR_LONG_RUN 256 /* runs longer than this are summed by a whole thread block */
+#define HCTR_CHUNK_POS 32 /* batch positions of one chunk_key entry, see hctr_group_args */
+#define HCTR_GROUP_MAX_TILES 256
 #define HCTR_LIGHT_RUN 32 /* runs up to this many positions are "short" */
 
 /* Kernels this library has enqueued since it was loaded (all launchers, all streams). */
@@ -90,10 +93,10 @@ const char *hctr_noalloc_last_error(void);
 /* row_of[key] = local row of every stored key, HCTR_INVALID_ROW elsewhere; version[row] = INT64_MIN for
  * cached rows (row < n_cached), 0 for owned rows.  `stored_keys` is the storage list already put in
  * layout order (cached rows first, each group in caller order).  Sets HCTR_ERR_KEY_RANGE for a key outside
- * [0,length) and HCTR_ERR_CAPACITY for a key listed twice.
+ * [0,length) and HCTR_ERR_CAPACITY for a key listed twice, and *moved = 1 when some key's row is not the key itself.
  * Replaces the hash-map build and version fill of csrc/core/table_initialize.cu:84-87,108-112. */
 int hctr_table_build(const int64_t *stored_keys, size_t n_stored, size_t n_cached, size_t length,
-                     int32_t *row_of, int64_t *version, uint32_t *err, void *stream);
+                     int32_t *row_of, int64_t *version, uint32_t *err, uint32_t *moved, void *stream);
 
 /* Stable partition flags for the storage list: is_cached[i] = owner_of[storage[i]] != rank, and
  * dst[i] = final local row (cached keys first, both groups in input order), given the exclusive scan
@@ -173,6 +176,7 @@ typedef struct hctr_dedupe_args {
 #define HCTR_META_ERR 1      /* error word (HCTR_ERR_*)                         */
 #define HCTR_META_NHEAVY 2   /* number of runs longer than HCTR_LIGHT_RUN       */
 #define HCTR_META_SEG 4      /* seg_start[0..nrank]: first unique of each owner */
+#define HCTR_META_NLONG 3    /* number of runs longer than HCTR_LONG_RUN (hctr_group_keys) */
 #define HCTR_META_WORDS 4
 
 /* Enqueues the whole dedupe pipeline.  On completion meta[HCTR_META_UNIQUE] = U, meta[HCTR_META_SEG+p]
@@ -189,12 +193,50 @@ int hctr_detect_key_stride(const int64_t *keys, size_t n, uint32_t *scores, void
  * copy, so that the caller may reuse its buffer) and meta[0..meta_words) = 0, in one launch. */
 int hctr_ingest_keys(const int64_t *src, int64_t *dst, size_t n, uint32_t *meta, unsigned meta_words, void *stream);
 /* hctr_ingest_keys plus pos_row[i] = row_of[keys[i]] (HCTR_INVALID_ROW for a key that is not stored here or lies
- * outside [0, length)).  With pos_row known this early the row expansion of a batch whose keys are all stored locally
+ * outside [0, length)); row_of = null means that every key's row is the key itself.  With pos_row known this early the row expansion of a batch whose keys are all stored locally
  * does not depend on the dedupe pipeline at all.  src holds keys of key_bytes (4 or 8) bytes, may equal dst and may be
  * mapped host memory.  Part of what cvt_embedding_idx_2_offset did, csrc/core/preprocess.cu:62-76.
  * A key out of range sets HCTR_ERR_KEY_RANGE in *err (null: the caller has checked). */
 int hctr_ingest_keys_rows(const void *src, int key_bytes, int64_t *dst, size_t n, uint32_t *meta, unsigned meta_words,
                           const int32_t *row_of, size_t length, int32_t *pos_row, uint32_t *err, void *stream);
+
+/* Grouping of a batch by a stable radix sort: the outputs of hctr_dedupe_map (positions of every run ascending) without
+ * table-sized scratch.  Serves batches of up to 8192 * HCTR_GROUP_MAX_TILES keys whose (owner, key) pairs fit 32 bits,
+ * see hctr_group_fits; up to 65,536 keys take one launch, more take 2 + the number of sort passes.  A key out of range
+ * (or with an owner >= nrank) sets HCTR_ERR_KEY_RANGE in meta[HCTR_META_ERR], gets idx_map = -1 and stands in no run.
+ * Replaces csrc/core/preprocess.cu:11-141, like hctr_dedupe_map. */
+typedef struct hctr_group_args {
+  const int64_t *keys;     /* [B] batch keys (device) */
+  size_t batch;            /* B */
+  size_t length;           /* table length N */
+  int nrank;
+  const uint8_t *owner_of; /* [N]; not read when nrank == 1 */
+  const int32_t *pos_row;  /* [B] local row of every position (hctr_ingest_keys_rows) */
+  /* scratch: pairs0, pairs1 [B] 64-bit, sort_keys [B], tile_counts [512 * HCTR_GROUP_MAX_TILES] need no initial value;
+   * hist [2048] all-zero between calls; tile_flags [4 * HCTR_GROUP_MAX_TILES] and chain_scratch [2 *
+   * HCTR_GROUP_MAX_TILES] (8-byte aligned) zero-initialised ONCE */
+  unsigned long long *pairs0, *pairs1;
+  uint32_t *sort_keys, *tile_counts, *hist, *tile_flags, *chain_scratch;
+  uint32_t epoch;          /* non-zero, different from every earlier call's on the same scratch */
+  /* outputs, as in hctr_dedupe_args; uniq_owner is not written when nrank == 1, idx_map may be null */
+  int64_t *uniq;
+  uint8_t *uniq_owner;
+  int32_t *uniq_row;
+  uint32_t *run_start;
+  uint32_t *sorted_pos;
+  int32_t *idx_map;
+  uint32_t *chunk_key;     /* [B/32 + 2] entry c = first unique key whose run starts at position 32 c of sorted_pos or
+                              later; the entry behind the last chunk = U */
+  uint32_t *heavy_list;    /* [B/32 + 2] unique indices of runs longer than HCTR_LIGHT_RUN, from the front
+                              (meta[HCTR_META_NHEAVY]); of runs longer than HCTR_LONG_RUN, from the back
+                              (meta[HCTR_META_NLONG]), which are in the front part too */
+  uint32_t *meta;          /* [HCTR_META_WORDS + nrank + 1], all-zero on entry */
+} hctr_group_args;
+int hctr_group_fits(size_t batch, size_t length, int nrank);
+int hctr_group_keys(const hctr_group_args *a, void *stream);
+/* idx_map of a finished grouping that was made without one (positions of invalid keys are left alone) */
+int hctr_group_index_map(const uint32_t *meta, const uint32_t *run_start, const uint32_t *sorted_pos, int32_t *idx_map,
+                         void *stream);
 
 /* The run-ordering half of the pipeline alone (positions of every unique key's run in ascending batch order
  * inside sorted_pos), for callers that deferred it: same args as the hctr_dedupe_map call it completes, on a
