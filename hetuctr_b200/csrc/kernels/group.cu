@@ -6,12 +6,13 @@
 // inside arrays of the batch's size (L2-resident); the only thing that grows with the table is the number of key bits:
 // three passes of nine bits serve 2^27 (owner, key) pairs.  (The bitmap ranking of dedupe.cu touches table-sized
 // arrays at random - bitmap, word ranks, owners, rows - which on tables of 1e8 keys is bound by address translation:
-// 851,968 keys cost 158 us there, XX here.)
+// 851,968 keys cost 158 us there, 87 here; 212,992 keys of a table of
+// 3.4e7 59 and 54, the former without putting long runs in order.)
 //
-// A tile is 8192 consecutive pairs held by one block of 1024 threads, eight pairs per thread, in the order
-// (warp, item, lane).  Per pass a tile ranks its pairs by digit (rank_tile), learns how many pairs of each digit stand
+// A tile is 1024 * ITEMS consecutive pairs held by one block of 1024 threads, ITEMS (1..8) pairs per thread, in the
+// order (warp, item, lane).  Per pass a tile ranks its pairs by digit (rank_tile), learns how many pairs of each digit stand
 // in front of it, and scatters.  What is in front comes from the tiles' digit counts:
-//   group_cluster   up to eight tiles: ONE launch for the whole job, a cluster of one block per tile; counts are read
+//   group_cluster   up to 32,768 pairs: ONE launch for the whole job, a cluster of one block per tile; counts are read
 //                   through distributed shared memory, passes are separated by cluster barriers.
 //   group_pass ...  more tiles: histogram of all digits, one launch per pass (a tile publishes its counts and waits,
 //                   bounded, for those of the tiles before it - blocks are dispatched in index order, so these are
@@ -26,12 +27,15 @@ namespace cg = cooperative_groups;
 
 constexpr int kTileThreads = 1024;
 constexpr int kTileWarps = kTileThreads / 32;
-constexpr int kItems = 8;
-constexpr u32 kTile = kTileThreads * kItems;
+constexpr int kMaxItems = 8;
 constexpr int kMaxDigits = 512;
 constexpr int kMaxPasses = 4;
 constexpr u32 kMaxTiles = HCTR_GROUP_MAX_TILES;
 constexpr u32 kMaxCluster = 8;
+// Tiles of the multi-launch form before a thread takes more pairs: a tile adds up the counts of all tiles in front of
+// it, and ranking and scattering a tile cost what they cost per SM, so the batch is spread over about as many SMs as
+// there are (212,992 keys as 26 tiles of 8192: 16 us per pass, as 104 tiles of 2048: 9).
+constexpr u32 kSpreadTiles = 112;
 
 struct TileSmem {
   uint16_t cnt[kTileWarps][kMaxDigits];  // pairs of a digit in a warp, then in the warps before it
@@ -64,9 +68,17 @@ __device__ __forceinline__ u32 sort_key(const hctr_group_args &a, const GroupPla
   return g.sentinel;
 }
 
-// index of a thread's j-th pair inside its tile
-__device__ __forceinline__ u32 tile_slot(int j) {
-  return (threadIdx.x >> 5) * (32 * kItems) + j * 32 + (threadIdx.x & 31);
+// index in the batch of a thread's j-th pair
+template <int ITEMS>
+__device__ __forceinline__ u32 pair_index(u32 tile, int j) {
+  return tile * (kTileThreads * ITEMS) + (threadIdx.x >> 5) * (32 * ITEMS) + j * 32 + (threadIdx.x & 31);
+}
+
+// Barrier over the cluster's threads, global and shared memory included; the warps are brought together first (divergent
+// code stands in front of every use).
+__device__ __forceinline__ void sync_cluster() {
+  __syncwarp();
+  cg::this_cluster().sync();
 }
 
 // Exclusive prefix of v over the block's threads, in thread order; *total = sum.  Two barriers.
@@ -92,67 +104,101 @@ __device__ __forceinline__ u32 block_prefix(u32 v, u32 *warp_sum, u32 *total) {
 }
 
 // Stable rank of every pair among the tile's pairs of the same digit; s.total = pairs per digit.  A warp counts in its
-// own row of s.cnt: equal digits among its lanes find each other with one match, the lowest lane moves the counter.
-__device__ __forceinline__ void rank_tile(TileSmem &s, const u32 (&digit)[kItems], const bool (&act)[kItems],
-                                          u32 (&rank)[kItems]) {
+// own row of s.cnt: equal digits among its lanes find each other with one ballot per digit bit, the lowest lane moves
+// the counter.  (__match_any_sync instead of the ballots: 1650 cycles per item with 32 warps on the SM, 1000 with them.)
+template <int ITEMS>
+__device__ __forceinline__ void rank_tile(TileSmem &s, const u32 (&digit)[ITEMS], const bool (&act)[ITEMS],
+                                          int digit_bits, u32 (&rank)[ITEMS]) {
   const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint16_t *mine = s.cnt[warp];
 #pragma unroll
   for (int k = 0; k < kMaxDigits / 64; k++) reinterpret_cast<u32 *>(mine)[k * 32 + lane] = 0;
+  unsigned peers[ITEMS];
+#pragma unroll
+  for (int j = 0; j < ITEMS; j++) peers[j] = __ballot_sync(0xffffffffu, act[j]);
+  for (int b = 0; b < digit_bits; b++) {
+#pragma unroll
+    for (int j = 0; j < ITEMS; j++) {
+      const bool one = (digit[j] >> b) & 1u;
+      const unsigned m = __ballot_sync(0xffffffffu, one);
+      peers[j] &= one ? m : ~m;
+    }
+  }
   __syncwarp();
 #pragma unroll
-  for (int j = 0; j < kItems; j++) {
-    const unsigned peers = __match_any_sync(0xffffffffu, act[j] ? digit[j] : 0x80000000u);
-    const unsigned leader = (unsigned)(__ffs(peers) - 1);
+  for (int j = 0; j < ITEMS; j++) {
+    const unsigned leader = act[j] ? (unsigned)(__ffs(peers[j]) - 1) : lane;
     u32 old = 0;
     if (act[j] && lane == leader) {
       old = mine[digit[j]];
-      mine[digit[j]] = (uint16_t)(old + __popc(peers));
+      mine[digit[j]] = (uint16_t)(old + __popc(peers[j]));
     }
     old = __shfl_sync(0xffffffffu, old, leader);
-    rank[j] = old + __popc(peers & ((1u << lane) - 1u));
+    rank[j] = old + __popc(peers[j] & ((1u << lane) - 1u));
     __syncwarp();
   }
   __syncthreads();
   if (threadIdx.x < kMaxDigits) {
     u32 sum = 0;
-#pragma unroll 8
-    for (int w = 0; w < kTileWarps; w++) {
-      const u32 c = s.cnt[w][threadIdx.x];
-      s.cnt[w][threadIdx.x] = (uint16_t)sum;
-      sum += c;
+#pragma unroll
+    for (int w0 = 0; w0 < kTileWarps; w0 += 16) {
+      u32 c[16];
+#pragma unroll
+      for (int w = 0; w < 16; w++) c[w] = s.cnt[w0 + w][threadIdx.x];
+#pragma unroll
+      for (int w = 0; w < 16; w++) {
+        s.cnt[w0 + w][threadIdx.x] = (uint16_t)sum;
+        sum += c[w];
+      }
     }
     s.total[threadIdx.x] = sum;
   }
   __syncthreads();
 #pragma unroll
-  for (int j = 0; j < kItems; j++)
+  for (int j = 0; j < ITEMS; j++)
     if (act[j]) rank[j] += s.cnt[warp][digit[j]];
 }
 
 // The sorted pairs of one tile -> unique keys, runs, positions.  before(heads) returns the number of heads (first pairs
 // of a key) in the tiles in front, given the tile's own; every thread calls it.
-template <class F>
+template <int ITEMS, class F>
 __device__ __forceinline__ void finish_tile(TileSmem &s, const hctr_group_args &a, const GroupPlan &g,
                                             const u64 *pairs, u32 tile, F before) {
   const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const u32 n = (u32)a.batch;
-  u32 sk[kItems], pos[kItems], heads[kItems];
+  u32 sk[ITEMS], pos[ITEMS], prev[ITEMS], next[ITEMS], heads[ITEMS];
+#pragma unroll
+  for (int j = 0; j < ITEMS; j++) {
+    const u32 q = pair_index<ITEMS>(tile, j);
+    const u64 w = q < n ? __ldcg(pairs + q) : ((u64)g.sentinel << 32);
+    sk[j] = (u32)(w >> 32);
+    pos[j] = (u32)w;
+    // neighbours across the warp's edges (the others come by shuffle)
+    prev[j] = next[j] = g.sentinel;
+    if (lane == 0 && q > 0 && q < n) prev[j] = (u32)(__ldcg(pairs + q - 1) >> 32);
+    if (lane == 31 && q + 1 < n) next[j] = (u32)(__ldcg(pairs + q + 1) >> 32);
+  }
   u32 in_warp = 0;
 #pragma unroll
-  for (int j = 0; j < kItems; j++) {
-    const u32 q = tile * kTile + tile_slot(j);
-    const u64 w = q < n ? __ldcg(pairs + q) : ~0ull;
-    sk[j] = q < n ? (u32)(w >> 32) : g.sentinel;
-    pos[j] = (u32)w;
-  }
-#pragma unroll
-  for (int j = 0; j < kItems; j++) {
-    const u32 q = tile * kTile + tile_slot(j);
-    u32 prev = __shfl_up_sync(0xffffffffu, sk[j], 1);
-    if (lane == 0 && q > 0 && q < n) prev = (u32)(__ldcg(pairs + q - 1) >> 32);
-    heads[j] = __ballot_sync(0xffffffffu, sk[j] != g.sentinel && (q == 0 || prev != sk[j]));
+  for (int j = 0; j < ITEMS; j++) {
+    const u32 up = __shfl_up_sync(0xffffffffu, sk[j], 1), down = __shfl_down_sync(0xffffffffu, sk[j], 1);
+    if (lane != 0) prev[j] = up;
+    if (lane != 31) next[j] = down;
+    const u32 q = pair_index<ITEMS>(tile, j);
+    heads[j] = __ballot_sync(0xffffffffu, sk[j] != g.sentinel && (q == 0 || prev[j] != sk[j]));
     in_warp += __popc(heads[j]);
+  }
+  // what the heads need from elsewhere, all of it in flight while the tiles add up their counts
+  int32_t row[ITEMS];
+  bool heavy[ITEMS], very[ITEMS];
+#pragma unroll
+  for (int j = 0; j < ITEMS; j++) {
+    const u32 q = pair_index<ITEMS>(tile, j);
+    const bool head = (heads[j] >> lane) & 1u;
+    row[j] = head ? a.pos_row[pos[j]] : 0;
+    const bool run = head && next[j] == sk[j];
+    heavy[j] = run && q + HCTR_LIGHT_RUN < n && (u32)(__ldcg(pairs + q + HCTR_LIGHT_RUN) >> 32) == sk[j];
+    very[j] = run && q + HCTR_LONG_RUN < n && (u32)(__ldcg(pairs + q + HCTR_LONG_RUN) >> 32) == sk[j];
   }
   __syncthreads();
   if (lane == 0) s.warp_sum[warp] = in_warp;
@@ -163,54 +209,48 @@ __device__ __forceinline__ void finish_tile(TileSmem &s, const hctr_group_args &
   u32 base = before(all) + first;  // heads in front of this warp's next item
   const u32 key_mask = g.key_bits >= 32 ? 0xffffffffu : (1u << g.key_bits) - 1u;
 #pragma unroll
-  for (int j = 0; j < kItems; j++) {
-    const u32 q = tile * kTile + tile_slot(j);
+  for (int j = 0; j < ITEMS; j++) {
+    const u32 q = pair_index<ITEMS>(tile, j);
     const bool valid = sk[j] != g.sentinel;
     const bool head = (heads[j] >> lane) & 1u;
     const u32 upto = base + __popc(heads[j] & ((1u << lane) - 1u));  // heads at positions before q
     const u32 u = upto + (head ? 1u : 0u) - 1u;                      // this pair's unique index (if valid)
     base += __popc(heads[j]);
-    u32 next = __shfl_down_sync(0xffffffffu, sk[j], 1);
-    if (q >= n) continue;
-    if (lane == 31) next = q + 1 < n ? (u32)(__ldcg(pairs + q + 1) >> 32) : g.sentinel;
-    if (q + 1 == n) next = g.sentinel;
-    if (q % HCTR_CHUNK_POS == 0) a.chunk_key[q / HCTR_CHUNK_POS] = upto;
-    a.sorted_pos[q] = pos[j];
-    if (a.idx_map) a.idx_map[pos[j]] = valid ? (int32_t)u : -1;
-    const u32 owner = a.nrank > 1 ? sk[j] >> g.key_bits : 0u;
-    if (head) {
-      const u32 key = sk[j] & key_mask;
-      a.run_start[u] = q;
-      a.uniq[u] = key;
-      a.uniq_row[u] = a.pos_row[pos[j]];
-      if (a.nrank > 1) {
-        a.uniq_owner[u] = (uint8_t)owner;
-        // segments of the owners between the key before and this one start here
-        const u32 from = q == 0 ? 0u : (u32)(__ldcg(pairs + q - 1) >> 32 >> g.key_bits) + 1u;
-        for (u32 p = from; p <= owner; p++) a.meta[HCTR_META_SEG + p] = u;
-      }
-      if (next == sk[j]) {
+    if (q < n) {
+      if (q % HCTR_CHUNK_POS == 0) a.chunk_key[q / HCTR_CHUNK_POS] = upto;
+      a.sorted_pos[q] = pos[j];
+      if (a.idx_map) a.idx_map[pos[j]] = valid ? (int32_t)u : -1;
+      const u32 owner = a.nrank > 1 ? sk[j] >> g.key_bits : 0u;
+      if (head) {
+        a.run_start[u] = q;
+        a.uniq[u] = sk[j] & key_mask;
+        a.uniq_row[u] = row[j];
+        if (a.nrank > 1) {
+          a.uniq_owner[u] = (uint8_t)owner;
+          // segments of the owners between the key before and this one start here
+          const u32 from = q == 0 ? 0u : (prev[j] >> g.key_bits) + 1u;
+          for (u32 p = from; p <= owner; p++) a.meta[HCTR_META_SEG + p] = u;
+        }
         // long runs are listed from the front, very long ones from the back as well (both fit: a very long run is one
         // entry of each and takes the place of several long ones)
-        if (q + HCTR_LIGHT_RUN < n && (u32)(__ldcg(pairs + q + HCTR_LIGHT_RUN) >> 32) == sk[j])
-          a.heavy_list[atomicAdd(&a.meta[HCTR_META_NHEAVY], 1u)] = u;
-        if (q + HCTR_LONG_RUN < n && (u32)(__ldcg(pairs + q + HCTR_LONG_RUN) >> 32) == sk[j])
-          a.heavy_list[n / 32 + 1 - atomicAdd(&a.meta[HCTR_META_NLONG], 1u)] = u;
+        if (heavy[j]) a.heavy_list[atomicAdd(&a.meta[HCTR_META_NHEAVY], 1u)] = u;
+        if (very[j]) a.heavy_list[n / 32 + 1 - atomicAdd(&a.meta[HCTR_META_NLONG], 1u)] = u;
       }
+      if (valid && (q + 1 == n || next[j] == g.sentinel)) {  // the last key of the batch
+        const u32 U = u + 1;
+        a.meta[HCTR_META_UNIQUE] = U;
+        a.run_start[U] = q + 1;
+        a.chunk_key[(q + HCTR_CHUNK_POS) / HCTR_CHUNK_POS] = U;
+        for (u32 p = owner + 1; p <= (u32)a.nrank; p++) a.meta[HCTR_META_SEG + p] = U;
+      }
+      if (q == 0 && !valid) a.run_start[0] = a.chunk_key[0] = 0;  // nothing but invalid keys
     }
-    if (valid && next == g.sentinel) {  // the last key of the batch
-      const u32 U = u + 1;
-      a.meta[HCTR_META_UNIQUE] = U;
-      a.run_start[U] = q + 1;
-      a.chunk_key[(q + HCTR_CHUNK_POS) / HCTR_CHUNK_POS] = U;
-      for (u32 p = owner + 1; p <= (u32)a.nrank; p++) a.meta[HCTR_META_SEG + p] = U;
-    }
-    if (q == 0 && !valid) a.run_start[0] = a.chunk_key[0] = 0;  // nothing but invalid keys
   }
   if (n == 0 && tile == 0 && threadIdx.x == 0) a.run_start[0] = a.chunk_key[0] = 0;
 }
 
-// Up to eight tiles, one launch.  Bound: a chain of short phases (per pass ~2 us of ranking and two cluster barriers).
+// One launch, a cluster of up to eight tiles.  Bound: a chain of short phases (per pass ~2 us of ranking and two cluster barriers).
+template <int ITEMS>
 __global__ void __launch_bounds__(kTileThreads) group_cluster(hctr_group_args a, GroupPlan g) {
   extern __shared__ __align__(16) unsigned char group_smem[];
   TileSmem &s = *reinterpret_cast<TileSmem *>(group_smem);
@@ -221,23 +261,24 @@ __global__ void __launch_bounds__(kTileThreads) group_cluster(hctr_group_args a,
   const u64 *in = nullptr;
   u64 *out = reinterpret_cast<u64 *>(a.pairs0);
   for (int pass = 0; pass < g.passes; pass++) {
-    u64 pair[kItems];
-    u32 digit[kItems], rank[kItems];
-    bool act[kItems];
+    u64 pair[ITEMS];
+    u32 digit[ITEMS], rank[ITEMS];
+    bool act[ITEMS];
 #pragma unroll
-    for (int j = 0; j < kItems; j++) {
-      const u32 q = tile * kTile + tile_slot(j);
+    for (int j = 0; j < ITEMS; j++) {
+      const u32 q = pair_index<ITEMS>(tile, j);
       act[j] = q < n;
       pair[j] = 0;
       if (act[j]) pair[j] = pass == 0 ? ((u64)sort_key(a, g, q) << 32) | q : __ldcg(in + q);
       digit[j] = digit_of((u32)(pair[j] >> 32), g, pass);
     }
-    rank_tile(s, digit, act, rank);
-    cluster.sync();
+    rank_tile<ITEMS>(s, digit, act, g.digit_bits, rank);
+    sync_cluster();
     u32 all = 0, before = 0;
     if (tid < kMaxDigits) {
-      for (u32 t = 0; t < tiles; t++) {
-        const u32 v = tiles == 1 ? s.total[tid] : *cluster.map_shared_rank(&s.total[tid], t);
+#pragma unroll
+      for (u32 t = 0; t < kMaxCluster; t++) {
+        const u32 v = t < tiles ? *cluster.map_shared_rank(&s.total[tid], t < tiles ? t : tile) : 0u;
         if (t < tile) before += v;
         all += v;
       }
@@ -247,21 +288,21 @@ __global__ void __launch_bounds__(kTileThreads) group_cluster(hctr_group_args a,
     if (tid < kMaxDigits) s.start[tid] = base + before;
     __syncthreads();
 #pragma unroll
-    for (int j = 0; j < kItems; j++)
+    for (int j = 0; j < ITEMS; j++)
       if (act[j]) out[s.start[digit[j]] + rank[j]] = pair[j];
-    cluster.sync();  // pairs in place for everybody; nobody reads s.total any more
+    sync_cluster();  // pairs in place for everybody; nobody reads s.total any more
     in = out;
     out = reinterpret_cast<u64 *>(in == reinterpret_cast<u64 *>(a.pairs0) ? a.pairs1 : a.pairs0);
   }
-  finish_tile(s, a, g, in, tile, [&](u32 heads) -> u32 {
+  finish_tile<ITEMS>(s, a, g, in, tile, [&](u32 heads) -> u32 {
     if (tiles == 1) return 0u;
     if (tid == 0) s.heads = heads;
-    cluster.sync();
+    sync_cluster();
     u32 before = 0;
     for (u32 t = 0; t < tile; t++) before += *cluster.map_shared_rank(&s.heads, t);
     return before;
   });
-  cluster.sync();  // the blocks behind have read this block's count
+  sync_cluster();  // the blocks behind have read this block's count
 }
 
 // Sort keys of the batch and, for every pass, how many have each digit (hist: all-zero on entry).
@@ -281,6 +322,7 @@ __global__ void __launch_bounds__(512) group_histogram(hctr_group_args a, GroupP
   }
 }
 
+template <int ITEMS>
 __global__ void __launch_bounds__(kTileThreads) group_pass(hctr_group_args a, GroupPlan g, int pass) {
   extern __shared__ __align__(16) unsigned char group_smem[];
   TileSmem &s = *reinterpret_cast<TileSmem *>(group_smem);
@@ -289,18 +331,18 @@ __global__ void __launch_bounds__(kTileThreads) group_pass(hctr_group_args a, Gr
   const u32 n = (u32)a.batch;
   const u64 *in = reinterpret_cast<const u64 *>(pass & 1 ? a.pairs0 : a.pairs1);
   u64 *out = reinterpret_cast<u64 *>(pass & 1 ? a.pairs1 : a.pairs0);
-  u64 pair[kItems];
-  u32 digit[kItems], rank[kItems];
-  bool act[kItems];
+  u64 pair[ITEMS];
+  u32 digit[ITEMS], rank[ITEMS];
+  bool act[ITEMS];
 #pragma unroll
-  for (int j = 0; j < kItems; j++) {
-    const u32 q = tile * kTile + tile_slot(j);
+  for (int j = 0; j < ITEMS; j++) {
+    const u32 q = pair_index<ITEMS>(tile, j);
     act[j] = q < n;
     pair[j] = 0;
     if (act[j]) pair[j] = pass == 0 ? ((u64)a.sort_keys[q] << 32) | q : __ldcg(in + q);
     digit[j] = digit_of((u32)(pair[j] >> 32), g, pass);
   }
-  rank_tile(s, digit, act, rank);
+  rank_tile<ITEMS>(s, digit, act, g.digit_bits, rank);
   u32 *flags = a.tile_flags + pass * kMaxTiles;
   if (tid < kMaxDigits) a.tile_counts[tile * kMaxDigits + tid] = s.total[tid];
   __syncthreads();
@@ -325,25 +367,26 @@ __global__ void __launch_bounds__(kTileThreads) group_pass(hctr_group_args a, Gr
   }
   __syncthreads();
   u32 before = 0;
-#pragma unroll 8
+#pragma unroll 16
   for (u32 t = tid / kMaxDigits; t < tile; t += kTileThreads / kMaxDigits)
     before += __ldcg(a.tile_counts + t * kMaxDigits + tid % kMaxDigits);
   atomicAdd(&s.start[tid % kMaxDigits], before);
   __syncthreads();
 #pragma unroll
-  for (int j = 0; j < kItems; j++)
+  for (int j = 0; j < ITEMS; j++)
     if (act[j]) {
       const u32 to = s.start[digit[j]] + rank[j];
       if (to < n) out[to] = pair[j];  // (always, unless a wait ran out)
     }
 }
 
+template <int ITEMS>
 __global__ void __launch_bounds__(kTileThreads) group_finish(hctr_group_args a, GroupPlan g) {
   __shared__ TileSmem s;
   const u64 *in = reinterpret_cast<const u64 *>(g.passes & 1 ? a.pairs0 : a.pairs1);
   if (blockIdx.x == 0)
     for (int i = threadIdx.x; i < g.passes * kMaxDigits; i += kTileThreads) a.hist[i] = 0;  // at rest again
-  finish_tile(s, a, g, in, blockIdx.x, [&](u32 heads) {
+  finish_tile<ITEMS>(s, a, g, in, blockIdx.x, [&](u32 heads) {
     return chained_cta_prefix(reinterpret_cast<u64 *>(a.chain_scratch), a.epoch, blockIdx.x, heads,
                               &a.meta[HCTR_META_ERR]);
   });
@@ -378,47 +421,59 @@ static bool group_plan(size_t length, int nrank, GroupPlan *g) {
   return true;
 }
 
+template <int ITEMS>
+static int launch_cluster(const hctr_group_args &a, const GroupPlan &g, cudaStream_t s) {
+  const u32 tiles = a.batch ? (u32)((a.batch + kTileThreads * ITEMS - 1) / (kTileThreads * ITEMS)) : 1u;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(tiles);
+  cfg.blockDim = dim3(kTileThreads);
+  cfg.dynamicSmemBytes = sizeof(TileSmem);
+  cfg.stream = s;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = tiles;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, group_cluster<ITEMS>, a, g);
+  count_launches(1);
+  return e != cudaSuccess ? (int)e : launch_status();
+}
+
+template <int ITEMS>
+static int launch_passes(const hctr_group_args &a, const GroupPlan &g, cudaStream_t s) {
+  const u32 tiles = (u32)((a.batch + kTileThreads * ITEMS - 1) / (kTileThreads * ITEMS));
+  group_histogram<<<kSMs, 512, 0, s>>>(a, g);
+  for (int p = 0; p < g.passes; p++) group_pass<ITEMS><<<tiles, kTileThreads, sizeof(TileSmem), s>>>(a, g, p);
+  group_finish<ITEMS><<<tiles, kTileThreads, 0, s>>>(a, g);
+  count_launches(g.passes + 2);
+  return launch_status();
+}
+
 extern "C" int hctr_group_fits(size_t batch, size_t length, int nrank) {
   GroupPlan g;
-  return batch <= (size_t)kTile * kMaxTiles && group_plan(length, nrank, &g) ? 1 : 0;
+  return batch <= (size_t)kTileThreads * kMaxItems * kMaxTiles && group_plan(length, nrank, &g) ? 1 : 0;
 }
 
 extern "C" int hctr_group_keys(const hctr_group_args *ap, void *stream) {
   cudaStream_t s = (cudaStream_t)stream;
   const hctr_group_args a = *ap;
   GroupPlan g;
-  if (a.epoch == 0 || a.batch > (size_t)kTile * kMaxTiles || !group_plan(a.length, a.nrank, &g))
+  if (a.epoch == 0 || a.batch > (size_t)kTileThreads * kMaxItems * kMaxTiles || !group_plan(a.length, a.nrank, &g))
     return (int)cudaErrorInvalidValue;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(group_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TileSmem));
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(group_pass, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TileSmem));
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
+  // One launch while a cluster's blocks take at most four pairs per thread: beyond, the few SMs of a cluster take longer
+  // (53,248 keys: 61 us) than the launches of the other form cost.
+  if (a.batch <= (size_t)kTileThreads * 4 * kMaxCluster) {
+    const size_t per = (size_t)kTileThreads * kMaxCluster;
+    return a.batch <= per       ? launch_cluster<1>(a, g, s)
+           : a.batch <= per * 2 ? launch_cluster<2>(a, g, s)
+                                : launch_cluster<4>(a, g, s);
   }
-  const u32 tiles = a.batch ? (u32)((a.batch + kTile - 1) / kTile) : 1u;
-  if (tiles <= kMaxCluster) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(tiles);
-    cfg.blockDim = dim3(kTileThreads);
-    cfg.dynamicSmemBytes = sizeof(TileSmem);
-    cfg.stream = s;
-    cudaLaunchAttribute at;
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = tiles;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, group_cluster, a, g);
-    count_launches(1);
-    return e != cudaSuccess ? (int)e : launch_status();
-  }
-  group_histogram<<<kSMs, 512, 0, s>>>(a, g);
-  for (int p = 0; p < g.passes; p++) group_pass<<<tiles, kTileThreads, sizeof(TileSmem), s>>>(a, g, p);
-  group_finish<<<tiles, kTileThreads, 0, s>>>(a, g);
-  count_launches(g.passes + 2);
-  return launch_status();
+  const size_t per = (size_t)kTileThreads * kSpreadTiles;
+  return a.batch <= per       ? launch_passes<1>(a, g, s)
+         : a.batch <= per * 2 ? launch_passes<2>(a, g, s)
+         : a.batch <= per * 4 ? launch_passes<4>(a, g, s)
+                              : launch_passes<8>(a, g, s);
 }
 
 extern "C" int hctr_group_index_map(const uint32_t *meta, const uint32_t *run_start, const uint32_t *sorted_pos,
