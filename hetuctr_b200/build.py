@@ -22,7 +22,8 @@ INCLUDE = os.path.join(ROOT, "include")
 CUDA_HOME = os.environ.get("CUDA_HOME", "/usr/local/cuda")
 NVCC = os.path.join(CUDA_HOME, "bin", "nvcc")
 
-CU_SOURCES = ["kernels/scan.cu", "kernels/dedupe.cu", "kernels/group.cu", "kernels/update.cu", "kernels/query.cu", "kernels/table.cu",
+CU_SOURCES = ["kernels/scan.cu", "kernels/dedupe.cu", "kernels/group.cu", "kernels/reduce.cu",
+              "kernels/update.cu", "kernels/query.cu", "kernels/table.cu",
               "kernels/p2p.cu", "kernels/p2p_pull.cu"]
 CC_SOURCES = ["core/hetu_table.cc", "core/table_state.cc", "core/c_api.cc", "core/transport.cc", "core/p2p.cc", "utils/rendezvous.cc",
               "utils/stage_keys.cc"]

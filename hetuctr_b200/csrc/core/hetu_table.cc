@@ -100,17 +100,15 @@ HetuTable::HetuTable(const int rank, const int nrank, const int device_id, const
     HCTR_CUDA(cudaDeviceGetStreamPriorityRange(&lo, &hi));
     const bool single = nrank == 1;
     HCTR_CUDA(cudaStreamCreateWithPriority(&stream_main_, cudaStreamNonBlocking, single ? lo : hi));
-    // the side stream carries the few long-run CTAs that should start ahead of the bulk kernels
+    // the side stream carries the run ordering of batches that are ranked through the bitmap
     HCTR_CUDA(cudaStreamCreateWithPriority(&stream_side_, cudaStreamNonBlocking, single ? lo : hi));
     HCTR_CUDA(cudaStreamCreateWithPriority(&stream_reduce_, cudaStreamNonBlocking, single ? hi : lo));
-    HCTR_CUDA(cudaStreamCreateWithPriority(&stream_reduce_side_, cudaStreamNonBlocking, hi));
+    if (!single) HCTR_CUDA(cudaStreamCreateWithPriority(&stream_reduce_side_, cudaStreamNonBlocking, hi));
   }
   HCTR_CUDA(cudaEventCreateWithFlags(&ev_rfork_, cudaEventDisableTiming));
   HCTR_CUDA(cudaEventCreateWithFlags(&ev_rjoin_, cudaEventDisableTiming));
   HCTR_CUDA(cudaEventCreateWithFlags(&ev_decide_, cudaEventDisableTiming));
   HCTR_CUDA(cudaEventCreateWithFlags(&ev_reduce_, cudaEventDisableTiming));
-  HCTR_CUDA(cudaEventCreateWithFlags(&ev_fork_, cudaEventDisableTiming));
-  HCTR_CUDA(cudaEventCreateWithFlags(&ev_join_, cudaEventDisableTiming));
   HCTR_CUDA(cudaEventCreateWithFlags(&ev_keys_, cudaEventDisableTiming));
   HCTR_CUDA(cudaEventCreateWithFlags(&ev_early_, cudaEventDisableTiming));
   if (const char *e = std::getenv("HCTR_SPLIT_HOST_EXPAND")) split_host_expand_ = std::atoi(e) != 0;
@@ -351,7 +349,6 @@ void HetuTable::preprocess(index_t *data_ptr, size_t batch_size) {
   if (nrank_ > 1) finalizePending();
   batch_open_ = true;
   profile_ = profile_every_ > 0 && (profile_step_++ % (size_t)profile_every_) == 0;
-  if (nrank_ > 1) flushOrdering(cur_batch_);  // normally done by push_pull already; two preprocess calls in a row get here
   std::swap(cur_batch_, prev_batch_);
   BatchDesc &cur = cur_batch_, &prev = prev_batch_;
   cur.decided = false;
@@ -371,9 +368,7 @@ void HetuTable::preprocess(index_t *data_ptr, size_t batch_size) {
     cur.dedupe_in_flight = false;
   }
   cur.scatter_recorded = false;
-  cur.light_ordered = false;
   cur.dedupe_pending = true;
-  cur.order_pending = true;
   cur.pending = true;
   ingestKeys(cur, data_ptr, batch_size, ks);
   // The push decision for the previous batch goes first: the gradient reduction (on its own stream, started
@@ -504,7 +499,7 @@ void HetuTable::ingestKeys(BatchDesc &b, const void *keys, size_t n, cudaStream_
 
 // A key outside the table: the batch is dropped (its dedupe is not enqueued yet) and the caller told right away.
 void HetuTable::dropBadBatch(BatchDesc &b) {
-  b.dedupe_pending = b.order_pending = b.pending = false;
+  b.dedupe_pending = b.pending = false;
   b.batch_size = b.unique_size = b.n_heavy = 0;
   throw std::runtime_error("preprocess: a key is outside [0, length)");
 }
@@ -604,9 +599,7 @@ void HetuTable::groupKeys(BatchDesc &b) {
   b.index_map_due = nrank_ == 1;
   // (this descriptor's batch of two steps ago may have been ordered on the side stream)
   if (b.order_recorded) HCTR_CUDA(cudaStreamWaitEvent(stream_main_, b.ev_order, 0));
-  b.order_pending = false;
   b.order_recorded = false;
-  b.light_ordered = true;
   int sp = tic(kPhDedupe);
   HCTR_LAUNCH(hctr_group_keys(&a, stream_main_));
   HCTR_CUDA(cudaEventRecord(b.ev_scatter, stream_main_));
@@ -617,14 +610,12 @@ void HetuTable::groupKeys(BatchDesc &b) {
 void HetuTable::rankKeys(BatchDesc &b) {
   b.index_map_due = false;
   if (!key_stride_known_ && b.batch_size >= 4096) detectKeyStride(b);  // once per table
-  // run ordering happens on stream_side_, off this stream's critical path; the reduction of this batch
-  // (next step) waits on the batch's own event.  The ordering stages through the batch's own rank buffer, so the
-  // ordering of the previous batch may still run while this batch is deduplicated; only the descriptor being
-  // recycled (two batches old) must be out of use.
+  // The runs are put in order on stream_side_, off this stream's critical path; the reduction of this batch (next step)
+  // waits on the batch's own event.  The ordering stages through the batch's own rank buffer, so the ordering of the
+  // previous batch may still run while this batch is deduplicated; only the descriptor being recycled (two batches
+  // old) must be out of use.
   if (b.order_recorded) HCTR_CUDA(cudaStreamWaitEvent(stream_main_, b.ev_order, 0));
-  b.order_recorded = false;
-  // (built here and not at preprocess: a larger batch in between may have moved the shared scratch)
-  hctr_dedupe_args &a = b.order_args;
+  hctr_dedupe_args a{};
   a.stride = key_stride_;
   a.keys = b.keys.as<int64_t>();
   a.batch = b.batch_size;
@@ -653,32 +644,13 @@ void HetuTable::rankKeys(BatchDesc &b) {
   a.meta = b.meta.as<uint32_t>();
   a.side_stream = stream_side_;
   a.fork_event = b.ev_scatter;
-  // The ordering kernels are enqueued by flushOrdering, after the gradient reduction, which brings the reduction (it
-  // only starts once push_pull is called) several launches forward.
-  a.join_event = nullptr;
+  a.join_event = b.ev_order;
   int sp = tic(kPhDedupe);
-  HCTR_LAUNCH(hctr_dedupe_map(&a, stream_main_));  // records b.ev_scatter behind its last kernel
+  HCTR_LAUNCH(hctr_dedupe_map(&a, stream_main_));  // records b.ev_scatter behind its last kernel on this stream
   toc(sp);
-}
-
-// The long runs (hot keys) are ordered on stream_side_; only the long-run kernel of the next reduction waits for
-// that.  The short runs are ordered by the reduction itself where its kernel can (orderLightRuns otherwise).
-void HetuTable::flushOrdering(BatchDesc &b) {
-  if (!b.order_pending) return;
-  flushDedupe(b);
-  if (!b.order_pending) return;  // came out in order
-  b.order_pending = false;
-  HCTR_CUDA(cudaStreamWaitEvent(stream_side_, b.ev_scatter, 0));
-  HCTR_LAUNCH(hctr_dedupe_order_heavy(&b.order_args, stream_side_));
+  HCTR_LAUNCH(hctr_run_chunks(b.batch_size, a.run_start, b.chunk_key.as<uint32_t>(), a.heavy_list, a.meta, stream_side_));
   HCTR_CUDA(cudaEventRecord(b.ev_order, stream_side_));
   b.order_recorded = true;
-}
-
-void HetuTable::orderLightRuns(BatchDesc &b, cudaStream_t s) {
-  if (b.light_ordered || !b.scatter_recorded) return;
-  HCTR_CUDA(cudaStreamWaitEvent(s, b.ev_scatter, 0));
-  HCTR_LAUNCH(hctr_dedupe_order_light(&b.order_args, s));
-  b.light_ordered = true;
 }
 
 // Reads the counts the preprocess pipeline copied to pinned memory into the batch descriptors.
@@ -755,6 +727,56 @@ const void *HetuTable::stageIn(const void *ptr, size_t bytes, DevBuf &buf, cudaS
   return buf.p;
 }
 
+// Duplicate-gradient reduction + local apply (+ pack of pushed rows) of batch b, on stream_reduce_ (generateGradient).
+void HetuTable::reduceGradients(BatchDesc &b, const embed_t *grad) {
+  if (nrank_ == 1) {
+    hctr_local_reduce_args r{};
+    r.batch = b.batch_size;
+    r.width = kEmbeddingWidth;
+    r.neg_lr = -learning_rate_;
+    r.grad = grad;
+    r.run_start = b.run_start.as<uint32_t>();
+    r.sorted_pos = b.sorted_pos.as<uint32_t>();
+    r.chunk_key = b.chunk_key.as<uint32_t>();
+    r.heavy_list = b.heavy.as<uint32_t>();
+    r.uniq_row = b.uniq_row.as<int32_t>();
+    r.meta = b.meta.as<uint32_t>();
+    r.embedding = d_embedding_.as<float>();
+    r.version = d_version_.as<int64_t>();
+    HCTR_LAUNCH(hctr_grad_reduce_local(&r, stream_reduce_));
+    return;
+  }
+  hctr_reduce_args r{};
+  r.n_unique = b.unique_size;
+  r.width = kEmbeddingWidth;
+  r.n_cached = kNonLocalStorageMax;
+  r.neg_lr = -learning_rate_;
+  r.grad = grad;
+  r.run_start = b.run_start.as<uint32_t>();
+  r.sorted_pos = b.sorted_pos.as<uint32_t>();
+  r.heavy_list = b.heavy.as<uint32_t>();
+  r.n_heavy = b.n_heavy;
+  r.uniq = b.uniq.as<int64_t>();
+  r.uniq_row = b.uniq_row.as<int32_t>();
+  r.need_push = b.need_push.as<uint32_t>();
+  r.push_slot = b.push_slot.as<uint32_t>();
+  r.embedding = d_embedding_.as<float>();
+  r.version = d_version_.as<int64_t>();
+  r.pending = d_gradient_.as<float>();
+  r.pending_cnt = d_updates_.as<int64_t>();
+  r.push_key = d_pkey_s_.as<int64_t>();
+  r.push_updates = d_pupd_s_.as<int64_t>();
+  r.push_val = d_pval_s_.as<float>();
+  r.work_counter = d_err_.as<uint32_t>() + 32;
+  r.p2p = use_p2p_ ? &p2p_->ctx() : nullptr;
+  r.uniq_owner = b.uniq_owner.as<uint8_t>();
+  r.push_base = d_push_base_.as<uint32_t>();
+  r.side_stream = stream_reduce_side_;
+  r.fork_event = ev_rfork_;
+  r.join_event = ev_rjoin_;
+  HCTR_LAUNCH(hctr_grad_reduce_apply_pack(&r, stream_reduce_));
+}
+
 // ------------------------------------------------------------------------------------------------
 // pushPull — csrc/core/hetu_gpu_table.cu:9-41
 // ------------------------------------------------------------------------------------------------
@@ -770,16 +792,13 @@ void HetuTable::pushPull(embed_t *grad, embed_t *dst) {
     prev.batch_size = 0;
     prev.unique_size = 0;
     prev.n_heavy = 0;
-    if (n == 1) prev.dedupe_pending = prev.order_pending = prev.pending = false;  // nobody will ask for its runs
+    if (n == 1) prev.dedupe_pending = prev.pending = false;  // nobody will ask for its runs
     std::fill(prev.push_send.begin(), prev.push_send.end(), 0);
     std::fill(prev.push_recv.begin(), prev.push_recv.end(), 0);
   }
 
   // The batch before was pulled without gradients (its dedupe was not due then) and gets some now.
-  if (n == 1 && prev.dedupe_pending) {
-    flushDedupe(prev);
-    flushOrdering(prev);
-  }
+  if (n == 1) flushDedupe(prev);
 
   // dst (and grad) are normally device memory; host buffers are staged
   embed_t *dst_dev = dst, *dst_mapped = nullptr;
@@ -837,53 +856,16 @@ void HetuTable::pushPull(embed_t *grad, embed_t *dst) {
   stats_.queried_keys = q_recv;
 
   // A. duplicate-gradient reduction + local apply + pack (generateGradient)
-  // A single-rank table has not read the previous batch's sizes (that would mean waiting for its dedupe on the
-  // host): the kernels take them from the batch's meta words on the device, the host passes upper bounds.
-  const bool sizes_on_device = n == 1 && prev.pending;
-  if (sizes_on_device ? prev.batch_size > 0 : prev.unique_size > 0) {
-    hctr_reduce_args r;
-    r.meta = sizes_on_device ? prev.meta.as<uint32_t>() : nullptr;
-    r.n_unique = sizes_on_device ? prev.batch_size : prev.unique_size;
-    r.width = W;
-    r.n_cached = kNonLocalStorageMax;
-    r.neg_lr = -learning_rate_;
-    r.grad = grad_dev;
-    r.run_start = prev.run_start.as<uint32_t>();
-    r.sorted_pos = prev.sorted_pos.as<uint32_t>();
-    r.heavy_list = prev.heavy.as<uint32_t>();
-    r.n_heavy = sizes_on_device ? prev.batch_size / (HCTR_LIGHT_RUN + 1) + 1 : prev.n_heavy;
-    r.uniq = prev.uniq.as<int64_t>();
-    r.uniq_row = prev.uniq_row.as<int32_t>();
-    r.need_push = n > 1 ? prev.need_push.as<uint32_t>() : nullptr;
-    r.push_slot = n > 1 ? prev.push_slot.as<uint32_t>() : nullptr;
-    r.embedding = d_embedding_.as<float>();
-    r.version = d_version_.as<int64_t>();
-    r.pending = d_gradient_.as<float>();
-    r.pending_cnt = d_updates_.as<int64_t>();
-    r.push_key = d_pkey_s_.as<int64_t>();
-    r.push_updates = d_pupd_s_.as<int64_t>();
-    r.push_val = d_pval_s_.as<float>();
-    r.work_counter = d_err_.as<uint32_t>() + 32;
-    r.p2p = use_p2p_ ? &p2p_->ctx() : nullptr;
-    r.uniq_owner = prev.uniq_owner.as<uint8_t>();
-    r.push_base = d_push_base_.as<uint32_t>();
-    r.side_stream = stream_reduce_side_;
-    r.fork_event = ev_rfork_;
-    r.join_event = ev_rjoin_;
-    // Own stream: overlaps the (still running) dedupe of the current batch.  It needs the push decision of
-    // the previous batch (ev_decide_) and nothing else from stream_main_.
+  if (prev.batch_size > 0 && (n == 1 || prev.unique_size > 0)) {
+    // Own stream: overlaps the (still running) dedupe of the current batch.  It needs the runs of the previous batch
+    // (end of its dedupe), the push decision (ev_decide_) and nothing else from stream_main_.
     if (n > 1) HCTR_CUDA(cudaStreamWaitEvent(stream_reduce_, ev_decide_, 0));
-    // the batch's runs must exist (end of its dedupe); the ordering of its long runs only concerns the long-run
-    // kernel, and the short runs are ordered by the streaming kernel as it loads them (or here, for the row
-    // widths and gradient buffers that kernel does not take)
     if (prev.scatter_recorded) HCTR_CUDA(cudaStreamWaitEvent(stream_reduce_, prev.ev_scatter, 0));
-    if (!prev.light_ordered && !hctr_reduce_orders_short_runs(W, grad_dev)) orderLightRuns(prev, stream_reduce_);
-    r.short_runs_unordered = prev.light_ordered ? 0 : 1;
-    r.long_wait_event = prev.order_recorded ? prev.ev_order : nullptr;
+    if (prev.order_recorded) HCTR_CUDA(cudaStreamWaitEvent(stream_reduce_, prev.ev_order, 0));
+    prev.dedupe_in_flight = false;
     int sp = tic(kPhReduce, stream_reduce_);
-    HCTR_LAUNCH(hctr_grad_reduce_apply_pack(&r, stream_reduce_));
+    reduceGradients(prev, grad_dev);
     toc(sp, stream_reduce_);
-    prev.dedupe_in_flight = false;  // stream_reduce_ has waited for it
     // everything below reads rows / versions the reduction updates (a single-rank table runs it on the reduction's
     // own stream instead, and its dedupe on stream_main_ needs nothing from here)
     if (n > 1) {
@@ -891,7 +873,6 @@ void HetuTable::pushPull(embed_t *grad, embed_t *dst) {
       HCTR_CUDA(cudaStreamWaitEvent(stream_main_, ev_reduce_, 0));
     }
   }
-  if (n > 1) flushOrdering(cur);  // the current batch's run ordering, deferred by preprocess
 
   // the stream the step ends on
   cudaStream_t tail = n == 1 ? stream_reduce_ : stream_main_;
@@ -914,10 +895,7 @@ void HetuTable::pushPull(embed_t *grad, embed_t *dst) {
     // step's reduction needs it.  (Holding it back until the reduction has ended was measured and is slower: the
     // dedupe then ends after the expansion and the next reduction waits for it.)  A step without gradients is taken
     // for serving: the dedupe of its batch stays due until gradients for it come, which they normally never do.
-    if (grad != nullptr) {
-      flushDedupe(cur);
-      flushOrdering(cur);
-    }
+    if (grad != nullptr) flushDedupe(cur);
   } else if (use_p2p_) {
     exchangeP2P(dst_dev);
   } else {
@@ -1480,8 +1458,6 @@ void HetuTable::releaseAll() {
   h_src_ = nullptr;
   if (ev_epoch_) cudaEventDestroy(ev_epoch_);
   ev_epoch_ = nullptr;
-  if (ev_fork_) cudaEventDestroy(ev_fork_);
-  if (ev_join_) cudaEventDestroy(ev_join_);
   if (ev_keys_) cudaEventDestroy(ev_keys_);
   if (ev_early_) cudaEventDestroy(ev_early_);
   ev_early_ = nullptr;
@@ -1494,7 +1470,7 @@ void HetuTable::releaseAll() {
   stream_reduce_side_ = nullptr;
   if (stream_reduce_) cudaStreamDestroy(stream_reduce_);
   stream_reduce_ = nullptr;
-  ev_fork_ = ev_join_ = ev_keys_ = nullptr;
+  ev_keys_ = nullptr;
   if (stream_side_) cudaStreamDestroy(stream_side_);
   stream_side_ = nullptr;
   if (stream_main_) cudaStreamDestroy(stream_main_);

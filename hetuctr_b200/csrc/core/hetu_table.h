@@ -57,18 +57,15 @@ struct BatchDesc {
   size_t batch_size = 0;
   size_t unique_size = 0;
   size_t capacity = 0;
-  size_t n_heavy = 0;  // runs longer than HCTR_LIGHT_RUN
+  size_t n_heavy = 0;  // runs longer than HCTR_LIGHT_RUN (multi-rank tables)
   bool pending = false;  // sizes not yet read back from the device (single-rank tables defer this)
   cudaEvent_t ev_order = nullptr;  // completion of the ordering of this batch's long runs (on the ordering stream)
   bool order_recorded = false;
   cudaEvent_t ev_scatter = nullptr;  // this batch's positions are in their runs (end of the dedupe pipeline)
   bool scatter_recorded = false;
   bool dedupe_in_flight = false;     // the dedupe was enqueued and the reduction's stream has not waited for it yet
-  bool light_ordered = false;        // runs of up to HCTR_LIGHT_RUN positions have been put in ascending order
   bool decided = false;            // the push decision for this batch has been enqueued
-  bool order_pending = false;      // the run-ordering kernels of this batch are not enqueued yet
   bool dedupe_pending = false;     // the dedupe pipeline of this batch is not enqueued yet
-  hctr_dedupe_args order_args;     // what both will be launched with
   bool index_map_due = false;      // idx_map has not been filled (nothing but dump reads it on a single-rank table)
   DevBuf keys, idx_map, sorted_pos, uniq, uniq_owner, uniq_row, run_start, meta, pos_row, heavy, chunk_key;
   // Push decision of this batch (multi-rank tables): flag and send slot per unique key.  They belong to the batch
@@ -192,25 +189,24 @@ class HetuTable {
   int expandRows(size_t batch, size_t width, const int32_t *pos_row, const int32_t *idx_map, const uint32_t *recv_slot,
                  const float *recv_val, const float *embedding, float *dst, uint32_t *err, cudaStream_t stream);
   void launchPushDecide(BatchDesc &b);
-  void flushOrdering(BatchDesc &b);  // enqueues a batch's deferred run ordering
+  void reduceGradients(BatchDesc &b, const embed_t *grad);
   void groupKeys(BatchDesc &b);
   void rankKeys(BatchDesc &b);
   void reserveBitmap();
   void flushDedupe(BatchDesc &b);    // enqueues a batch's deferred dedupe pipeline (single-rank tables)
-  void orderLightRuns(BatchDesc &b, cudaStream_t s);  // the short-run half of the ordering, where somebody needs it
   void quiesce();  // every stream drained, pending batch sizes read back
   void exchangeP2P(embed_t *dst_dev);
   const void *stageIn(const void *ptr, size_t bytes, DevBuf &buf, cudaStream_t s);
 
   cudaStream_t stream_main_ = nullptr;
-  cudaStream_t stream_side_ = nullptr;  // overlaps the long-run kernels with their short-run twins
+  cudaStream_t stream_side_ = nullptr;  // run ordering of batches that are ranked through the bitmap
   // The gradient reduction of the PREVIOUS batch runs here, concurrently with the dedupe of the current
   // batch on stream_main_ (they touch disjoint data); stream_main_ joins it before the first kernel that
   // reads updated rows or versions.
   cudaStream_t stream_reduce_ = nullptr;
-  cudaStream_t stream_reduce_side_ = nullptr;  // long-run reduce kernel, forked from stream_reduce_
+  cudaStream_t stream_reduce_side_ = nullptr;  // multi-rank tables: long-run reduce kernel, forked from stream_reduce_
   cudaEvent_t ev_decide_ = nullptr, ev_reduce_ = nullptr, ev_rfork_ = nullptr, ev_rjoin_ = nullptr;
-  cudaEvent_t ev_fork_ = nullptr, ev_join_ = nullptr, ev_keys_ = nullptr;
+  cudaEvent_t ev_keys_ = nullptr;
   cudaEvent_t ev_early_ = nullptr;   // end of the gradient-independent half of a split row expansion
   bool split_host_expand_ = true;    // HCTR_SPLIT_HOST_EXPAND=0 switches the split off
   bool fused_refresh_expand_ = true; // HCTR_P2P_FUSED_EXPAND=0: cache refresh and row expansion as two launches

@@ -70,11 +70,9 @@ struct Pinned {
 void HetuTable::quiesce() {
   HCTR_CUDA(cudaSetDevice(device_id_));
   finalizePending();
-  flushOrdering(cur_batch_);
-  // whoever looks at a batch's position lists expects every run in ascending order
+  // the batch -> unique map of a single-rank table is only made when somebody looks
   for (BatchDesc *b : {&cur_batch_, &prev_batch_}) {
     if (b->batch_size == 0) continue;
-    orderLightRuns(*b, stream_side_);
     if (b->index_map_due && b->scatter_recorded) {
       HCTR_CUDA(cudaStreamWaitEvent(stream_side_, b->ev_scatter, 0));
       HCTR_LAUNCH(hctr_group_index_map(b->meta.as<uint32_t>(), b->run_start.as<uint32_t>(),

@@ -401,6 +401,19 @@ __global__ void __launch_bounds__(256) group_index_map(const u32 *__restrict__ m
     for (u32 q = run_start[u] + lane; q < run_start[u + 1]; q += 32) idx_map[sorted_pos[q]] = (int32_t)u;
 }
 
+// What hctr_group_keys leaves for the reduction, from runs that were made otherwise.
+__global__ void __launch_bounds__(256) run_chunks(u32 n, const u32 *__restrict__ run_start, u32 *__restrict__ chunk_key,
+                                                  u32 *__restrict__ heavy_list, u32 *meta) {
+  const u32 U = meta[HCTR_META_UNIQUE];
+  for (u32 u = blockIdx.x * 256 + threadIdx.x; u <= U; u += gridDim.x * 256) {
+    // chunks that begin behind the start of the key before and not behind this one's
+    const u32 here = u < U ? run_start[u] : run_start[U] + HCTR_CHUNK_POS - 1;
+    const u32 from = u == 0 ? 0u : run_start[u - 1] / HCTR_CHUNK_POS + 1;
+    for (u32 c = from; c <= here / HCTR_CHUNK_POS; c++) chunk_key[c] = u;
+    if (u < U && run_start[u + 1] - here > HCTR_LONG_RUN) heavy_list[n / 32 + 1 - atomicAdd(&meta[HCTR_META_NLONG], 1u)] = u;
+  }
+}
+
 }  // namespace hctr
 
 using namespace hctr;
@@ -479,6 +492,13 @@ extern "C" int hctr_group_keys(const hctr_group_args *ap, void *stream) {
 extern "C" int hctr_group_index_map(const uint32_t *meta, const uint32_t *run_start, const uint32_t *sorted_pos,
                                     int32_t *idx_map, void *stream) {
   group_index_map<<<kSMs * 4, 256, 0, (cudaStream_t)stream>>>(meta, run_start, sorted_pos, idx_map);
+  count_launches(1);
+  return launch_status();
+}
+
+extern "C" int hctr_run_chunks(size_t batch, const uint32_t *run_start, uint32_t *chunk_key, uint32_t *heavy_list,
+                               uint32_t *meta, void *stream) {
+  run_chunks<<<kSMs * 4, 256, 0, (cudaStream_t)stream>>>((u32)batch, run_start, chunk_key, heavy_list, meta);
   count_launches(1);
   return launch_status();
 }

@@ -115,11 +115,6 @@ __global__ void push_counts(const u32 *__restrict__ meta, int nrank, const u32 *
 //   type 2  cached, push    -> emb += s, pending += s, push pending, clear it, version += pending count
 //   type 3  cached, hold    -> emb += s, pending += s, pending count += count
 
-// number of unique keys / of long runs of the batch: from the batch's meta words when the host passed them
-__device__ __forceinline__ size_t unique_count(const hctr_reduce_args &a) {
-  return a.meta ? (size_t)a.meta[HCTR_META_UNIQUE] : a.n_unique;
-}
-
 struct RowTarget {
   int type;
   size_t slot;
@@ -220,7 +215,7 @@ __global__ void __launch_bounds__(kThreads) grad_reduce_short(ReduceKernelArgs k
   typedef typename R::T T;
   const size_t u = ((size_t)blockIdx.x * kThreads + threadIdx.x) / LANES;
   const unsigned gl = threadIdx.x % LANES;
-  if (u >= unique_count(a)) return;
+  if (u >= a.n_unique) return;
   const u32 l = a.run_start[u], r = a.run_start[u + 1];
   if (r - l > HCTR_LIGHT_RUN) return;  // handled by grad_reduce_long
   PushDest dest;
@@ -284,7 +279,7 @@ __global__ void __launch_bounds__(kThreads) grad_reduce_short_wide(ReduceKernelA
   T *emb_base = reinterpret_cast<T *>(a.embedding);
   T *pend_base = reinterpret_cast<T *>(a.pending);
   // (A one-wave grid with chunks drawn from a shared counter was measured and was slower: 105 us vs 92 us.)
-  const size_t n_unique = unique_count(a);
+  const size_t n_unique = a.n_unique;
   for (size_t u0 = warp * kWideChunk; u0 < n_unique; u0 += n_warps * kWideChunk) {
     const size_t my_u = u0 + lane;
     u32 l = 0, len = 0, p0 = 0;
@@ -461,14 +456,11 @@ __global__ void __launch_bounds__(kThreads) grad_reduce_short_stream(ReduceKerne
   const u64 warp = (u64)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
   const u64 n_warps = ((u64)gridDim.x * kThreads) >> 5;
   const size_t E = EC ? (size_t)EC : a.width / 4;
-  const u32 U = (u32)unique_count(a);
+  const u32 U = (u32)a.n_unique;
   const T *grad = reinterpret_cast<const T *>(a.grad);
   T *emb_base = reinterpret_cast<T *>(a.embedding);
   T *pend_base = reinterpret_cast<T *>(a.pending);
   T *ring = ring_all + (size_t)(threadIdx.x >> 5) * D * E;
-  __shared__ u32 sort_all[kThreads];  // 32 words per warp
-  u32 *sort_buf = sort_all + (threadIdx.x & ~31u);
-  const bool unordered = a.short_runs_unordered != 0;
   const u64 once = l2_evict_first_policy();
   const u32 n_pos = a.run_start[U];
   const u64 total = (u64)n_pos + 2ull * U;
@@ -513,24 +505,6 @@ __global__ void __launch_bounds__(kThreads) grad_reduce_short_stream(ReduceKerne
           src = emb_base + (size_t)P.row * E;
         } else {
           const u32 q = P.l + (u32)P.j;
-          if (unordered && P.j == 0 && P.len >= 2) {
-            // First gradient row of a key whose run is still in arrival order: bring the whole run (at most 32
-            // positions) into the window, then put it in ascending order - a lane's place is the number of smaller
-            // positions in the run (positions are distinct).  Sums stay in batch order without a separate pass.
-            if (!have_window || q - q_base + P.len > 32u) {
-              q_base = q;
-              have_window = true;
-              sp = q_base + lane < n_pos ? a.sorted_pos[q_base + lane] : 0u;
-            }
-            const u32 s0 = q - q_base;
-            const bool in_run = lane - s0 < P.len;
-            u32 place = 0;
-            for (u32 k2 = 0; k2 < P.len; k2++) place += __shfl_sync(0xffffffffu, sp, (int)(s0 + k2)) < sp ? 1u : 0u;
-            if (in_run) sort_buf[place] = sp;
-            __syncwarp();
-            if (in_run) sp = sort_buf[lane - s0];
-            __syncwarp();
-          }
           if (!have_window || q - q_base >= 32u) {
             q_base = q;
             have_window = true;
@@ -635,9 +609,8 @@ __device__ __forceinline__ void cp_async_elem(void *smem_dst, const void *gsrc, 
 }
 
 template <bool VEC>
-__global__ void __launch_bounds__(kLongThreads) grad_reduce_long(ReduceKernelArgs ka, u32 n_heavy_host, u32 *work_counter) {
+__global__ void __launch_bounds__(kLongThreads) grad_reduce_long(ReduceKernelArgs ka, u32 n_heavy, u32 *work_counter) {
   const hctr_reduce_args &a = ka.a;
-  const u32 n_heavy = a.meta ? a.meta[HCTR_META_NHEAVY] : n_heavy_host;
   const u64 once = l2_evict_first_policy();
   typedef RowT<VEC> R;
   typedef typename R::T T;
@@ -1154,12 +1127,7 @@ extern "C" int hctr_push_decide_fused(const uint32_t *meta, int nrank, int rank,
   return launch_status();
 }
 
-// the streaming short-run kernel is the variant that can order its runs itself
 static bool streaming_shape(size_t width, bool aligned) { return aligned && width % 4 == 0 && width >= 128 && width <= 512; }
-
-extern "C" int hctr_reduce_orders_short_runs(size_t width, const float *grad) {
-  return streaming_shape(width, host_aligned16(grad)) ? 1 : 0;
-}
 
 extern "C" int hctr_grad_reduce_apply_pack(const hctr_reduce_args *ap, void *stream) {
   cudaStream_t s = (cudaStream_t)stream;
@@ -1175,19 +1143,16 @@ extern "C" int hctr_grad_reduce_apply_pack(const hctr_reduce_args *ap, void *str
     cudaError_t e = cudaEventRecord((cudaEvent_t)a.fork_event, s);
     if (e != cudaSuccess) return (int)e;
   }
-  if (a.short_runs_unordered && !streaming_shape(a.width, al)) return (int)cudaErrorInvalidValue;
 
   // Two kernels: the long runs (one thread block per hot key) and everything else.  They touch different keys, so
   // with a second stream they run side by side.  The long-run kernel is launched FIRST and with at most
   // `long_per_sm` blocks per SM, the short-run kernel then fills what is left of every SM: launched the other way
   // round, the short-run kernel's single resident round of blocks occupies all SMs and the long runs only start
   // when it ends.
-  // (Measured on config 2, one GPU: 1 long-run block + 3 short-run blocks per SM gave 0.146 ms per step; 2 + 4,
-  // 3 + 3 and the old order - short-run kernel first - 0.147, 0.147 and 0.160.)
   // A multi-rank table runs the dedupe of the next batch beside this reduction, and both are on the step's critical
   // path: two short-run blocks per SM leave its small kernels room (config 2, two GPUs: 0.314 ms per step against
   // 0.323 with three blocks and 0.369 with one; the dedupe 108 against 122 us, the reduction 113 against 120 us).
-  const int long_per_sm = 1, short_cap = a.need_push ? 2 : 3;
+  const int long_per_sm = 1, short_cap = 2;
   const bool forked = a.n_heavy > 0 && a.side_stream && a.fork_event && a.join_event;
   cudaStream_t ls = forked ? (cudaStream_t)a.side_stream : s;
   if (a.n_heavy > 0) {
@@ -1203,10 +1168,6 @@ extern "C" int hctr_grad_reduce_apply_pack(const hctr_reduce_args *ap, void *str
     }
     if (forked) {
       cudaError_t e = cudaStreamWaitEvent(ls, (cudaEvent_t)a.fork_event, 0);
-      if (e != cudaSuccess) return (int)e;
-    }
-    if (a.long_wait_event) {  // ordering of the long runs, done on another stream
-      cudaError_t e = cudaStreamWaitEvent(ls, (cudaEvent_t)a.long_wait_event, 0);
       if (e != cudaSuccess) return (int)e;
     }
     cudaError_t em = cudaMemsetAsync(a.work_counter, 0, 2 * sizeof(u32), ls);

@@ -234,6 +234,9 @@ typedef struct hctr_group_args {
 } hctr_group_args;
 int hctr_group_fits(size_t batch, size_t length, int nrank);
 int hctr_group_keys(const hctr_group_args *a, void *stream);
+/* chunk_key and the very long runs' half of heavy_list for runs that another launcher made (hctr_dedupe_map) */
+int hctr_run_chunks(size_t batch, const uint32_t *run_start, uint32_t *chunk_key, uint32_t *heavy_list, uint32_t *meta,
+                    void *stream);
 /* idx_map of a finished grouping that was made without one (positions of invalid keys are left alone) */
 int hctr_group_index_map(const uint32_t *meta, const uint32_t *run_start, const uint32_t *sorted_pos, int32_t *idx_map,
                          void *stream);
@@ -244,8 +247,7 @@ int hctr_group_index_map(const uint32_t *meta, const uint32_t *run_start, const 
  * of sorted_pos) needs it. */
 int hctr_dedupe_order(const hctr_dedupe_args *a, void *stream);
 /* The two halves of hctr_dedupe_order: runs of 2..HCTR_LIGHT_RUN positions (one warp per run) and longer runs
- * (a thread block per run).  The short-run half is not needed when the consumer orders short runs itself, see
- * hctr_reduce_orders_short_runs. */
+ * (a thread block per run). */
 int hctr_dedupe_order_light(const hctr_dedupe_args *a, void *stream);
 int hctr_dedupe_order_heavy(const hctr_dedupe_args *a, void *stream);
 
@@ -428,23 +430,27 @@ typedef struct hctr_reduce_args {
   void *side_stream;
   void *fork_event;
   void *join_event;
-  /* optional: the batch's meta words on the device.  When non-null the kernels read the number of unique keys and
-   * of long runs from meta[HCTR_META_UNIQUE] / meta[HCTR_META_NHEAVY] - the host need not have seen them - and
-   * n_unique / n_heavy are only upper bounds that size the grids. */
-  const uint32_t *meta;
-  /* runs of up to HCTR_LIGHT_RUN positions are in arbitrary order in sorted_pos (hctr_dedupe_order_light has not
-   * run): the kernel puts each of them in ascending order as it loads them.  Only legal when
-   * hctr_reduce_orders_short_runs(width, grad) is non-zero. */
-  int short_runs_unordered;
-  /* optional cudaEvent_t the long-run kernel waits for before it starts (the ordering of the long runs, when that
-   * runs on another stream); the short-run kernel does not wait for it */
-  void *long_wait_event;
 } hctr_reduce_args;
 
 int hctr_grad_reduce_apply_pack(const hctr_reduce_args *a, void *stream);
-/* Non-zero when, for rows of `width` floats and this gradient buffer, the short-run kernel is the one that can
- * order its runs itself (short_runs_unordered). */
-int hctr_reduce_orders_short_runs(size_t width, const float *grad);
+
+/* The same for a single-rank table (every key owned: rows and versions are all there is to update), in one launch.  The
+ * batch's sizes are read from its meta words on the device. */
+typedef struct hctr_local_reduce_args {
+  size_t batch;               /* B_prev, keys of the previous batch */
+  size_t width;               /* W */
+  float neg_lr;               /* -learning_rate */
+  const float *grad;          /* [B_prev, W] caller's gradients */
+  const uint32_t *run_start;  /* run_start .. meta: outputs of hctr_group_keys */
+  const uint32_t *sorted_pos;
+  const uint32_t *chunk_key;
+  const uint32_t *heavy_list;
+  const int32_t *uniq_row;
+  const uint32_t *meta;
+  float *embedding;           /* [S, W] */
+  int64_t *version;           /* [S] */
+} hctr_local_reduce_args;
+int hctr_grad_reduce_local(const hctr_local_reduce_args *a, void *stream);
 
 /* ---------------------------------------------------------------------------------------------
  * Query generation.  Replaces lookup_version_kernel, csrc/core/generate_query.cu:91-106.

@@ -108,3 +108,38 @@ def test_grouping_matches_numpy(batch, length, nrank):
             torch.cuda.synchronize()
             assert np.array_equal(t["idx_map"].cpu().numpy()[:batch], exp_map)
         assert int(t["hist"].abs().sum()) == 0
+
+
+def test_batch_beyond_the_grouping_limit(oracle_mod):
+    # more keys than hctr_group_keys serves: the bitmap ranking makes the runs, hctr_run_chunks what the reduction needs
+    from test_gpu_parity import make_worlds, run_steps
+
+    N, W, B = 50_000, 2, 8192 * TILES + 5
+    gw, ow = make_worlds(oracle_mod, 1, N, W, 0, 0, 0.5, np.zeros(N, dtype=np.uint8), [np.arange(N)])
+    rng = np.random.RandomState(9)
+    keys = rng.randint(N, size=B)
+    keys[rng.rand(B) < 0.02] = 77
+    grads = [None, [rng.normal(0, 1, size=(B, W)).astype(np.float32)]]
+    run_steps(gw, ow, [[keys], [rng.randint(N, size=1000)]], grads)
+    gw.close()
+
+
+@pytest.mark.parametrize("width", [1, 2, 6, 12, 31, 32, 33, 60, 64, 66, 128, 130, 200, 516, 1030])
+def test_reduction_run_lengths(oracle_mod, width):
+    # runs on both sides of every limit of the reduction (short / long / very long, tiles of its rings), keys seen
+    # once between them, at widths of every element size and number of lanes
+    from test_gpu_parity import make_worlds, run_steps
+
+    N = 3000
+    gw, ow = make_worlds(oracle_mod, 1, N, width, 0, 0, 0.5, np.zeros(N, dtype=np.uint8),
+                         [np.random.RandomState(4).permutation(N)])
+    rng = np.random.RandomState(width)
+    runs = [1, 2, 3, 4, 5, 31, 32, 33, 39, 40, 41, 63, 64, 65, 96, 255, 256, 257, 383, 384, 385, 511, 512, 640, 1300]
+    key = np.repeat(rng.permutation(N)[:len(runs)], runs)
+    b0 = np.concatenate([key, rng.randint(N, size=900)])
+    rng.shuffle(b0)
+    b1 = np.full(300, 11)
+    batches = [[b0], [b1], [np.arange(N)]]
+    grads = [None] + [[rng.normal(0, 1, size=(len(b[0]), width)).astype(np.float32)] for b in batches[:-1]]
+    run_steps(gw, ow, batches, grads)
+    gw.close()
