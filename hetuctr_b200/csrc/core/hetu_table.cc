@@ -880,6 +880,12 @@ void HetuTable::pushPull(embed_t *grad, embed_t *dst) {
     // Single rank: every key is owned and stored here; the pull is a local gather that only needs the rows the
     // key ingest resolved and the reduction, both in front of it on this stream.  The dedupe of this batch
     // keeps running on stream_main_; nothing of this step reads its results.
+    // The grouping of a small batch is enqueued between reduction and expansion: the host's launch hides behind the
+    // reduction, and the few SMs it takes are free once the reduction drains.  (Behind the expansion it would start when
+    // that drains, before the reduction the host reaches both later.)
+    if (grad != nullptr && cur.batch_size > 0 && hctr_group_is_small(cur.batch_size) &&
+        hctr_group_fits(cur.batch_size, kEmbeddingIDMax, n))
+      flushDedupe(cur);
     int sp = tic(kPhExpand, tail);
     if (split_expand) {
       HCTR_LAUNCH(hctr_expand_rows_subset(cur.batch_size, W, cur.pos_row.as<int32_t>(), cur.keys.as<int64_t>(),

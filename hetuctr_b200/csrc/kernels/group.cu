@@ -12,7 +12,7 @@
 // A tile is 1024 * ITEMS consecutive pairs held by one block of 1024 threads, ITEMS (1..8) pairs per thread, in the
 // order (warp, item, lane).  Per pass a tile ranks its pairs by digit (rank_tile), learns how many pairs of each digit stand
 // in front of it, and scatters.  What is in front comes from the tiles' digit counts:
-//   group_cluster   up to 32,768 pairs: ONE launch for the whole job, a cluster of one block per tile; counts are read
+//   group_cluster   up to 65,536 pairs: ONE launch for the whole job, a cluster of one block per tile; counts are read
 //                   through distributed shared memory, passes are separated by cluster barriers.
 //   group_pass ...  more tiles: histogram of all digits, one launch per pass (a tile publishes its counts and waits,
 //                   bounded, for those of the tiles before it - blocks are dispatched in index order, so these are
@@ -31,7 +31,7 @@ constexpr int kMaxItems = 8;
 constexpr int kMaxDigits = 512;
 constexpr int kMaxPasses = 4;
 constexpr u32 kMaxTiles = HCTR_GROUP_MAX_TILES;
-constexpr u32 kMaxCluster = 8;
+constexpr u32 kMaxCluster = 16;  // (more than 8 blocks is not portable: see cluster_blocks)
 // Tiles of the multi-launch form before a thread takes more pairs: a tile adds up the counts of all tiles in front of
 // it, and ranking and scattering a tile cost what they cost per SM, so the batch is spread over about as many SMs as
 // there are (212,992 keys as 26 tiles of 8192: 16 us per pass, as 104 tiles of 2048: 9).
@@ -249,7 +249,7 @@ __device__ __forceinline__ void finish_tile(TileSmem &s, const hctr_group_args &
   if (n == 0 && tile == 0 && threadIdx.x == 0) a.run_start[0] = a.chunk_key[0] = 0;
 }
 
-// One launch, a cluster of up to eight tiles.  Bound: a chain of short phases (per pass ~2 us of ranking and two cluster barriers).
+// One launch, a cluster of up to 16 tiles.  Bound: a chain of short phases (per pass ~2 us of ranking and two cluster barriers).
 template <int ITEMS>
 __global__ void __launch_bounds__(kTileThreads) group_cluster(hctr_group_args a, GroupPlan g) {
   extern __shared__ __align__(16) unsigned char group_smem[];
@@ -435,19 +435,40 @@ static bool group_plan(size_t length, int nrank, GroupPlan *g) {
 }
 
 template <int ITEMS>
-static int launch_cluster(const hctr_group_args &a, const GroupPlan &g, cudaStream_t s) {
-  const u32 tiles = a.batch ? (u32)((a.batch + kTileThreads * ITEMS - 1) / (kTileThreads * ITEMS)) : 1u;
+static cudaLaunchConfig_t cluster_config(u32 tiles, cudaStream_t s, cudaLaunchAttribute *at) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(tiles);
   cfg.blockDim = dim3(kTileThreads);
   cfg.dynamicSmemBytes = sizeof(TileSmem);
   cfg.stream = s;
-  cudaLaunchAttribute at;
-  at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = tiles;
-  at.val.clusterDim.y = at.val.clusterDim.z = 1;
-  cfg.attrs = &at;
+  at->id = cudaLaunchAttributeClusterDimension;
+  at->val.clusterDim.x = tiles;
+  at->val.clusterDim.y = at->val.clusterDim.z = 1;
+  cfg.attrs = at;
   cfg.numAttrs = 1;
+  return cfg;
+}
+
+// Blocks a cluster of this kernel may have here: 16 where the device places such a cluster, else the portable 8.
+static u32 cluster_blocks() {
+  static u32 most = 0;
+  if (most) return most;
+  bool big = true;
+  for (const void *k : {(const void *)group_cluster<1>, (const void *)group_cluster<2>, (const void *)group_cluster<4>})
+    big = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess && big;
+  int clusters = 0;
+  cudaLaunchAttribute at;
+  const cudaLaunchConfig_t cfg = cluster_config<4>(kMaxCluster, nullptr, &at);
+  big = big && cudaOccupancyMaxActiveClusters(&clusters, group_cluster<4>, &cfg) == cudaSuccess && clusters > 0;
+  cudaGetLastError();
+  return most = big ? kMaxCluster : 8u;
+}
+
+template <int ITEMS>
+static int launch_cluster(const hctr_group_args &a, const GroupPlan &g, cudaStream_t s) {
+  const u32 tiles = a.batch ? (u32)((a.batch + kTileThreads * ITEMS - 1) / (kTileThreads * ITEMS)) : 1u;
+  cudaLaunchAttribute at;
+  const cudaLaunchConfig_t cfg = cluster_config<ITEMS>(tiles, s, &at);
   const cudaError_t e = cudaLaunchKernelEx(&cfg, group_cluster<ITEMS>, a, g);
   count_launches(1);
   return e != cudaSuccess ? (int)e : launch_status();
@@ -468,6 +489,8 @@ extern "C" int hctr_group_fits(size_t batch, size_t length, int nrank) {
   return batch <= (size_t)kTileThreads * kMaxItems * kMaxTiles && group_plan(length, nrank, &g) ? 1 : 0;
 }
 
+extern "C" int hctr_group_is_small(size_t batch) { return batch <= (size_t)kTileThreads * 4 * cluster_blocks() ? 1 : 0; }
+
 extern "C" int hctr_group_keys(const hctr_group_args *ap, void *stream) {
   cudaStream_t s = (cudaStream_t)stream;
   const hctr_group_args a = *ap;
@@ -475,13 +498,11 @@ extern "C" int hctr_group_keys(const hctr_group_args *ap, void *stream) {
   if (a.epoch == 0 || a.batch > (size_t)kTileThreads * kMaxItems * kMaxTiles || !group_plan(a.length, a.nrank, &g))
     return (int)cudaErrorInvalidValue;
   // One launch while a cluster's blocks take at most four pairs per thread: beyond, the few SMs of a cluster take longer
-  // (53,248 keys: 61 us) than the launches of the other form cost.
-  if (a.batch <= (size_t)kTileThreads * 4 * kMaxCluster) {
-    const size_t per = (size_t)kTileThreads * kMaxCluster;
-    return a.batch <= per       ? launch_cluster<1>(a, g, s)
-           : a.batch <= per * 2 ? launch_cluster<2>(a, g, s)
-                                : launch_cluster<4>(a, g, s);
-  }
+  // (53,248 keys with eight pairs per thread on eight SMs: 61 us) than the launches of the other form cost.
+  const size_t one = (size_t)kTileThreads * cluster_blocks();
+  if (a.batch <= one) return launch_cluster<1>(a, g, s);
+  if (a.batch <= one * 2) return launch_cluster<2>(a, g, s);
+  if (a.batch <= one * 4) return launch_cluster<4>(a, g, s);
   const size_t per = (size_t)kTileThreads * kSpreadTiles;
   return a.batch <= per       ? launch_passes<1>(a, g, s)
          : a.batch <= per * 2 ? launch_passes<2>(a, g, s)

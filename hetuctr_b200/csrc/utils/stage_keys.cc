@@ -1,11 +1,15 @@
 #include "utils/stage_keys.h"
 
+#if defined(__x86_64__)
+#include <immintrin.h>
+#endif
+
 namespace hetuCTR {
 
 namespace {
 // The sign bit of (k | length - 1 - k) is set exactly when k < 0 or k >= length (k >= 0 makes the difference exact), so
 // one OR per key collects the verdict and the loop has no branch: it vectorises and runs at the speed of the copy
-// (53,248 keys in cache: 11 us; wider vectors than the baseline's measured the same).
+// (53,248 keys in cache: 15 us).
 template <class T>
 __attribute__((optimize("O3"))) bool copy_checked(const int64_t *__restrict__ src, T *__restrict__ dst, size_t n,
                                                   size_t length) {
@@ -18,9 +22,36 @@ __attribute__((optimize("O3"))) bool copy_checked(const int64_t *__restrict__ sr
   }
   return n == 0 || (length > 0 && (int64_t)bad >= 0);
 }
+
+#if defined(__x86_64__)
+// Eight keys at a time in 32-byte registers: on a Xeon of the GPU boxes 53,248 keys that are no longer in cache take 23 us
+// against 29 for the loop above (26,624: 14 against 21).  Prefetches, stores past the cache and several streams at once
+// were all slower there (42 to 140 us).
+__attribute__((target("avx2"))) bool copy_checked_avx2(const int64_t *src, int32_t *dst, size_t n, size_t length) {
+  const __m256i last = _mm256_set1_epi64x((long long)length - 1), even = _mm256_setr_epi32(0, 2, 4, 6, 0, 2, 4, 6);
+  __m256i bad = _mm256_setzero_si256();
+  size_t i = 0;
+  for (; i + 8 <= n; i += 8) {
+    const __m256i a = _mm256_loadu_si256(reinterpret_cast<const __m256i *>(src + i));
+    const __m256i b = _mm256_loadu_si256(reinterpret_cast<const __m256i *>(src + i + 4));
+    bad = _mm256_or_si256(bad, _mm256_or_si256(a, _mm256_sub_epi64(last, a)));
+    bad = _mm256_or_si256(bad, _mm256_or_si256(b, _mm256_sub_epi64(last, b)));
+    const __m256i low = _mm256_permutevar8x32_epi32(a, even), high = _mm256_permutevar8x32_epi32(b, even);
+    _mm256_storeu_si256(reinterpret_cast<__m256i *>(dst + i), _mm256_blend_epi32(low, high, 0xF0));
+  }
+  const bool good = _mm256_movemask_pd(_mm256_castsi256_pd(bad)) == 0;  // no sign bit among them
+  return copy_checked(src + i, dst + i, n - i, length) && (i == 0 || (length > 0 && good));
+}
+#endif
 }  // namespace
 
-bool stage_keys(const int64_t *src, int32_t *dst, size_t n, size_t length) { return copy_checked(src, dst, n, length); }
+bool stage_keys(const int64_t *src, int32_t *dst, size_t n, size_t length) {
+#if defined(__x86_64__)
+  static const bool avx2 = __builtin_cpu_supports("avx2");
+  if (avx2) return copy_checked_avx2(src, dst, n, length);
+#endif
+  return copy_checked(src, dst, n, length);
+}
 bool stage_keys(const int64_t *src, int64_t *dst, size_t n, size_t length) { return copy_checked(src, dst, n, length); }
 
 }  // namespace hetuCTR

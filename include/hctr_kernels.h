@@ -202,7 +202,7 @@ int hctr_ingest_keys_rows(const void *src, int key_bytes, int64_t *dst, size_t n
 
 /* Grouping of a batch by a stable radix sort: the outputs of hctr_dedupe_map (positions of every run ascending) without
  * table-sized scratch.  Serves batches of up to 8192 * HCTR_GROUP_MAX_TILES keys whose (owner, key) pairs fit 32 bits,
- * see hctr_group_fits; up to 32,768 keys take one launch, more take 2 + the number of sort passes.  A key out of range
+ * see hctr_group_fits; up to 65,536 keys take one launch, more take 2 + the number of sort passes.  A key out of range
  * (or with an owner >= nrank) sets HCTR_ERR_KEY_RANGE in meta[HCTR_META_ERR], gets idx_map = -1 and stands in no run.
  * Replaces csrc/core/preprocess.cu:11-141, like hctr_dedupe_map. */
 typedef struct hctr_group_args {
@@ -233,6 +233,8 @@ typedef struct hctr_group_args {
   uint32_t *meta;          /* [HCTR_META_WORDS + nrank + 1], all-zero on entry */
 } hctr_group_args;
 int hctr_group_fits(size_t batch, size_t length, int nrank);
+/* non-zero when hctr_group_keys takes one launch on few SMs for a batch of this size */
+int hctr_group_is_small(size_t batch);
 int hctr_group_keys(const hctr_group_args *a, void *stream);
 /* chunk_key and the very long runs' half of heavy_list for runs that another launcher made (hctr_dedupe_map) */
 int hctr_run_chunks(size_t batch, const uint32_t *run_start, uint32_t *chunk_key, uint32_t *heavy_list, uint32_t *meta,

@@ -27,7 +27,7 @@ class GroupArgs(ctypes.Structure):  # field order of hctr_group_args
 
 
 @pytest.mark.parametrize("length,nrank", [(200, 1), (70_000, 3), (1 << 22, 1), (40_000_000, 5)])
-@pytest.mark.parametrize("batch", [0, 1, 31, 33, 8191, 8192, 8193, 32_768, 32_769, 114_689, 200_001])
+@pytest.mark.parametrize("batch", [0, 1, 31, 33, 8193, 16_385, 32_769, 65_536, 65_537, 114_689, 200_001])
 def test_grouping_matches_numpy(batch, length, nrank):
     L = hb.lib()
     L.hctr_group_keys.argtypes = [ctypes.POINTER(GroupArgs), vp]
