@@ -295,6 +295,8 @@ void HetuTable::reserveBatch(BatchDesc &b, size_t batch) {
   if (nrank_ > 1) {
     b.need_push.ensure((batch + 1) * sizeof(uint32_t));
     b.push_slot.ensure((batch + 1) * sizeof(uint32_t));
+    b.push_count.ensure((size_t)nrank_ * sizeof(uint32_t));
+    b.push_base.ensure((size_t)nrank_ * sizeof(uint32_t));
   }
   b.capacity = batch;
 }
@@ -319,8 +321,6 @@ void HetuTable::reserveShared(size_t batch) {
     HCTR_CUDA(cudaMemsetAsync(d_cnt_.p, 0, d_cnt_.bytes, stream_main_));
     HCTR_CUDA(cudaStreamSynchronize(stream_main_));
   }
-  d_push_count_.ensure((size_t)nrank_ * sizeof(uint32_t));
-  d_push_base_.ensure((size_t)nrank_ * sizeof(uint32_t));
   d_recv_idx_.ensure((batch + 1) * sizeof(uint32_t));
   if (nrank_ > 1) {
     const size_t n = nrank_;
@@ -378,7 +378,7 @@ void HetuTable::preprocess(index_t *data_ptr, size_t batch_size) {
   // row is owned, nothing is ever pushed.
   const bool decide = n > 1 && prev.unique_size > 0;
   if (decide && !prev.decided) launchPushDecide(prev);  // normally done at the end of the previous push_pull
-  if (n > 1) HCTR_CUDA(cudaEventRecord(ev_decide_, stream_reduce_));
+  if (n > 1 && !use_p2p_) HCTR_CUDA(cudaEventRecord(ev_decide_, stream_reduce_));
   prev_push_valid_ = decide;
   if (n == 1) {
     // Single rank: nothing of this step reads what the dedupe produces (the expansion has the rows from the key
@@ -394,7 +394,7 @@ void HetuTable::preprocess(index_t *data_ptr, size_t batch_size) {
     // One packed count exchange instead of the reference's two all2allExchangeShape rounds
     // (csrc/core/preprocess.cu:135,176): per peer {keys I will query, rows I will push}.
     if (decide) HCTR_CUDA(cudaStreamWaitEvent(stream_main_, ev_decide_, 0));  // push counts come from the other stream
-    HCTR_LAUNCH(hctr_pack_counts(cur.meta.as<uint32_t>(), decide ? d_push_count_.as<uint32_t>() : nullptr, n,
+    HCTR_LAUNCH(hctr_pack_counts(cur.meta.as<uint32_t>(), decide ? prev.push_count.as<uint32_t>() : nullptr, n,
                                  d_cnt_s_.as<uint32_t>(), stream_main_));
     std::vector<XferItem> items;
     for (int p = 0; p < n; p++)
@@ -406,6 +406,8 @@ void HetuTable::preprocess(index_t *data_ptr, size_t batch_size) {
     HCTR_CUDA(cudaMemcpyAsync(h_cnt_r, d_cnt_r_.p, 2 * n * sizeof(uint32_t), cudaMemcpyDeviceToHost, stream_main_));
   }
   if (use_p2p_) {
+    if (keys_in_use_) HCTR_CUDA(cudaEventSynchronize(ev_keys_));  // the caller's buffer has been read
+    keys_in_use_ = false;
     // (The device-driven exchange, where counts never visit the host.)
     // Nothing on the host depends on the result before push_pull: the rest of the pipeline runs under the next
     // call's launches.
@@ -491,10 +493,14 @@ void HetuTable::ingestKeys(BatchDesc &b, const void *keys, size_t n, cudaStream_
                                     d_ingest_err_, s));
   HCTR_CUDA(cudaEventRecord(ev_keys_, s));
   if (n == 0 || (nrank_ > 1 && !use_p2p_)) return;  // (NCCL: the count exchange that follows waits for the stream)
+  if (nrank_ > 1) {  // preprocess waits, behind the launches of the dedupe
+    keys_in_use_ = true;
+    return;
+  }
   HCTR_CUDA(cudaEventSynchronize(ev_keys_));
   const bool bad = *h_ingest_err_ != 0;
   *h_ingest_err_ = 0;
-  if (bad && nrank_ == 1) dropBadBatch(b);  // (multi-rank tables hear of it from the dedupe, which also checks owners)
+  if (bad) dropBadBatch(b);  // (multi-rank tables hear of it from the dedupe, which also checks owners)
 }
 
 // A key outside the table: the batch is dropped (its dedupe is not enqueued yet) and the caller told right away.
@@ -540,15 +546,15 @@ void HetuTable::detectKeyStride(const BatchDesc &b) {
 }
 
 // Push decision for batch b (csrc/core/preprocess.cu:167-182), on the reduction's stream: only the reduction of
-// b's gradient (and the counts published after it) need the result.  It depends on the pending-update counts as
-// the previous reduction left them, so it can run as soon as b's own push_pull is over.
+// b's gradient (and the counts published after it) need the result.  It depends on b's runs and on the pending-update
+// counts as the previous reduction left them.
 void HetuTable::launchPushDecide(BatchDesc &b) {
   int spd = tic(kPhPushDecide, stream_reduce_);
-  HCTR_LAUNCH(hctr_push_decide_fused(b.meta.as<uint32_t>(), nrank_, rank_, b.unique_size, b.uniq_owner.as<uint8_t>(),
+  HCTR_LAUNCH(hctr_push_decide_fused(b.meta.as<uint32_t>(), nrank_, rank_, b.batch_size, b.uniq_owner.as<uint8_t>(),
                                      b.uniq_row.as<int32_t>(), b.run_start.as<uint32_t>(), d_updates_.as<int64_t>(),
                                      push_bound_, b.need_push.as<uint32_t>(), b.push_slot.as<uint32_t>(),
-                                     d_chain3_.as<uint32_t>(), nextEpoch(), d_push_count_.as<uint32_t>(),
-                                     d_push_base_.as<uint32_t>(), d_err_.as<uint32_t>(), stream_reduce_));
+                                     d_chain3_.as<uint32_t>(), nextEpoch(), b.push_count.as<uint32_t>(),
+                                     b.push_base.as<uint32_t>(), d_err_.as<uint32_t>(), stream_reduce_));
   toc(spd, stream_reduce_);
   b.decided = true;
 }
@@ -565,7 +571,7 @@ void HetuTable::flushDedupe(BatchDesc &b) {
   b.dedupe_in_flight = true;
   if (hctr_group_fits(b.batch_size, kEmbeddingIDMax, nrank_)) groupKeys(b);
   else rankKeys(b);
-  if (nrank_ == 1) return;  // whoever wants the sizes on the host copies them then
+  if (nrank_ == 1 || use_p2p_) return;  // whoever wants the sizes on the host has them copied then
   const size_t meta_words = HCTR_META_WORDS + nrank_ + 1;
   HCTR_CUDA(cudaMemcpyAsync(b.h_meta, b.meta.p, meta_words * sizeof(uint32_t), cudaMemcpyDeviceToHost, stream_main_));
 }
@@ -703,11 +709,10 @@ void HetuTable::finalizePending() {
   if (!cur_batch_.pending && !prev_batch_.pending) return;
   flushDedupe(prev_batch_);
   flushDedupe(cur_batch_);
-  if (nrank_ == 1)
-    for (BatchDesc *b : {&prev_batch_, &cur_batch_})
-      if (b->pending)
-        HCTR_CUDA(cudaMemcpyAsync(b->h_meta, b->meta.p, (HCTR_META_WORDS + 2) * sizeof(uint32_t), cudaMemcpyDeviceToHost,
-                                  stream_main_));
+  for (BatchDesc *b : {&prev_batch_, &cur_batch_})
+    if (b->pending)
+      HCTR_CUDA(cudaMemcpyAsync(b->h_meta, b->meta.p, (HCTR_META_WORDS + nrank_ + 1) * sizeof(uint32_t),
+                                cudaMemcpyDeviceToHost, stream_main_));
   HCTR_CUDA(cudaStreamSynchronize(stream_main_));
   collectSpans();
   finalizePrev();  // (the dedupe of the previous batch sits in front of this one's on the same stream)
@@ -770,7 +775,7 @@ void HetuTable::reduceGradients(BatchDesc &b, const embed_t *grad) {
   r.work_counter = d_err_.as<uint32_t>() + 32;
   r.p2p = use_p2p_ ? &p2p_->ctx() : nullptr;
   r.uniq_owner = b.uniq_owner.as<uint8_t>();
-  r.push_base = d_push_base_.as<uint32_t>();
+  r.push_base = b.push_base.as<uint32_t>();
   r.side_stream = stream_reduce_side_;
   r.fork_event = ev_rfork_;
   r.join_event = ev_rjoin_;
@@ -858,8 +863,7 @@ void HetuTable::pushPull(embed_t *grad, embed_t *dst) {
   // A. duplicate-gradient reduction + local apply + pack (generateGradient)
   if (prev.batch_size > 0 && (n == 1 || prev.unique_size > 0)) {
     // Own stream: overlaps the (still running) dedupe of the current batch.  It needs the runs of the previous batch
-    // (end of its dedupe), the push decision (ev_decide_) and nothing else from stream_main_.
-    if (n > 1) HCTR_CUDA(cudaStreamWaitEvent(stream_reduce_, ev_decide_, 0));
+    // (end of its dedupe), the push decision (in front of it on this stream) and nothing else from stream_main_.
     if (prev.scatter_recorded) HCTR_CUDA(cudaStreamWaitEvent(stream_reduce_, prev.ev_scatter, 0));
     if (prev.order_recorded) HCTR_CUDA(cudaStreamWaitEvent(stream_reduce_, prev.ev_order, 0));
     prev.dedupe_in_flight = false;
@@ -1156,23 +1160,21 @@ void HetuTable::exchangeP2P(embed_t *dst_dev) {
   d_ent_row_.ensure((slots + 1) * sizeof(int32_t));
   d_ent_next_.ensure((slots + 1) * sizeof(uint32_t));
   d_flag_r_.ensure(u_max + 16);
-  // In split mode every rank drains its stream after publishing and meets the others at a host barrier, so the
-  // kernel that consumes finds every sequence number in place and never polls.
-  auto meet = [&] {
-    if (!split) return;
-    HCTR_CUDA(cudaStreamSynchronize(stream_main_));
-    p2p_->hostBarrier();
+  // In split mode the stream goes on behind every rank's publishing kernel (events), so the kernel that consumes finds
+  // every sequence number in place and never polls.
+  auto meet = [&](int phase) {
+    if (split) p2p_->meet(phase, stream_main_);
   };
 
   // B. queries straight into the owners' mailboxes; the last thread block publishes counts + sequence number
   int sp = tic(kPhQuery);
   HCTR_LAUNCH(hctr_p2p_query_send(c, meta, u_max, cur.uniq.as<int64_t>(), cur.uniq_owner.as<uint8_t>(),
                                   cur.uniq_row.as<int32_t>(), d_version_.as<int64_t>(), seq,
-                                  prev_push_valid_ && prev_batch_.unique_size > 0 ? d_push_count_.as<uint32_t>()
+                                  prev_push_valid_ && prev_batch_.unique_size > 0 ? prev_batch_.push_count.as<uint32_t>()
                                                                                    : nullptr,
                                   stream_main_));
   toc(sp);
-  meet();
+  meet(0);
 
   // C. owner applies the pushed rows of each source in rank order
   const hctr_p2p_box mine = p2p_->mine();
@@ -1204,7 +1206,7 @@ void HetuTable::exchangeP2P(embed_t *dst_dev) {
   HCTR_LAUNCH(hctr_p2p_stale_gather(c, seq, d_row_of_.as<int32_t>(), kEmbeddingIDMax, kNonLocalStorageMax,
                                     d_embedding_.as<float>(), d_version_.as<int64_t>(), pull_bound_, stream_main_));
   toc(sp);
-  meet();
+  meet(1);
 
   // E. requester: wait for the owners, cache refresh and row expansion in one launch; or (HCTR_P2P_FUSED_EXPAND=0,
   // HCTR_EXPAND=bulk) in two: row index + flag of every unique key and cache refresh, then the expansion
@@ -1229,11 +1231,16 @@ void HetuTable::exchangeP2P(embed_t *dst_dev) {
     toc(sp);
   }
 
-  // counts, wait times and the error word come back with the step's final synchronisation
+  // counts, wait times, the error word and the batch's sizes come back with the step's final synchronisation
   uint32_t *h_cnt = h_pinned_ + HCTR_META_WORDS + n + 1 + 4 * n;  // [5n+7] + [n] push counts + error word
-  HCTR_CUDA(cudaMemcpyAsync(h_cnt, c->cnt_in, (5 * n + 7) * sizeof(uint32_t), cudaMemcpyDeviceToHost, stream_main_));
-  HCTR_CUDA(cudaMemcpyAsync(h_cnt + 5 * n + 7, d_push_count_.p, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, stream_main_));
-  HCTR_CUDA(cudaMemcpyAsync(h_cnt + 6 * n + 7, d_err_.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream_main_));
+  HCTR_LAUNCH(hctr_p2p_report(c, prev_batch_.push_count.as<uint32_t>(), meta, (unsigned)(HCTR_META_WORDS + n + 1), h_cnt,
+                              cur.h_meta, stream_main_));
+  // The push decision for this batch (its runs exist, the pending counts are as the reduction in front of it on
+  // stream_reduce_ left them) runs beside the exchange: the next step's reduction does not have to wait for it.
+  if (cur.batch_size > 0 && !cur.decided) {
+    HCTR_CUDA(cudaStreamWaitEvent(stream_reduce_, cur.ev_scatter, 0));
+    launchPushDecide(cur);
+  }
   p2p_counts_pending_ = true;
   p2p_pushed_valid_ = prev_push_valid_ && prev_batch_.unique_size > 0;
 }
@@ -1432,7 +1439,7 @@ void HetuTable::releaseAll() {
   transport_.reset();
   DevBuf *all[] = {&d_embedding_, &d_gradient_, &d_updates_, &d_version_, &d_root_, &d_row_of_, &d_stored_keys_,
                    &d_bits_, &d_blk_cnt_, &d_blk_flag_, &d_chain_, &d_chain3_, &d_ent_row_, &d_ent_next_, &d_row_mask_, &d_row_head_, &d_src_off_, &d_src_cnt_, &d_word_base_, &d_scan_, &d_sk_, &d_cnt_, &d_pairs_, &d_sort_keys_, &d_group_hist_, &d_group_tiles_,
-                   &d_push_count_, &d_push_base_, &d_recv_idx_, &d_err_, &d_cnt_s_, &d_cnt_r_, &d_qver_s_,
+                   &d_recv_idx_, &d_err_, &d_cnt_s_, &d_cnt_r_, &d_qver_s_,
                    &d_qkey_r_, &d_qver_r_, &d_pkey_s_, &d_pupd_s_, &d_pval_s_, &d_pkey_r_, &d_pupd_r_, &d_pval_r_,
                    &d_flag_s_, &d_flag_r_, &d_flag32_, &d_ret_slot_, &d_recv_slot_, &d_seg_r_, &d_retcnt_s_,
                    &d_retcnt_r_, &d_rver_s_, &d_rval_s_, &d_rver_r_, &d_rval_r_, &d_stage_grad_, &d_stage_dst_};
@@ -1451,7 +1458,8 @@ void HetuTable::releaseAll() {
   h_ingest_err_ = d_ingest_err_ = nullptr;
   for (BatchDesc *b : {&cur_batch_, &prev_batch_})
     for (DevBuf *d : {&b->keys, &b->idx_map, &b->sorted_pos, &b->uniq, &b->uniq_owner, &b->uniq_row,
-                      &b->run_start, &b->meta, &b->pos_row, &b->heavy, &b->chunk_key, &b->need_push, &b->push_slot, &b->rank})
+                      &b->run_start, &b->meta, &b->pos_row, &b->heavy, &b->chunk_key, &b->need_push, &b->push_slot,
+                      &b->push_count, &b->push_base, &b->rank})
       d->release();
   for (Span &sp : spans_) {
     cudaEventDestroy(sp.a);

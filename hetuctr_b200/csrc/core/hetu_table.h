@@ -71,7 +71,7 @@ struct BatchDesc {
   // Push decision of this batch (multi-rank tables): flag and send slot per unique key.  They belong to the batch
   // because the decision is taken at the end of the batch's own push_pull and consumed by the next one; a larger
   // batch arriving in between must not move them.
-  DevBuf need_push, push_slot;
+  DevBuf need_push, push_slot, push_count, push_base;
   // rank of every position inside its run; later the staging area of the batch's run ordering (its own buffer, so
   // that the ordering of one batch can overlap the dedupe of the next)
   DevBuf rank;
@@ -223,7 +223,7 @@ class HetuTable {
   bool key_stride_known_ = false;
   void detectKeyStride(const BatchDesc &b);
   bool batch_open_ = false;          // preprocess done, push_pull not yet
-  bool prev_push_valid_ = false;     // d_push_count_/d_push_base_ describe prev_batch_
+  bool prev_push_valid_ = false;     // prev_batch_'s push counts describe a push of this step
 
   // table state
   DevBuf d_embedding_, d_gradient_, d_updates_, d_version_, d_root_, d_row_of_, d_stored_keys_;
@@ -233,7 +233,7 @@ class HetuTable {
   DevBuf d_bits_, d_blk_cnt_, d_blk_flag_, d_chain_, d_chain3_, d_ent_row_, d_ent_next_, d_row_mask_, d_row_head_, d_src_off_, d_src_cnt_, d_word_base_, d_scan_, d_sk_, d_cnt_;
   DevBuf d_pairs_, d_sort_keys_, d_group_hist_, d_group_tiles_;  // radix grouping; d_sk_ holds its other half of the pairs
   bool rows_are_keys_ = false;  // single rank, every key stored in key order: row = key, no lookup
-  DevBuf d_push_count_, d_push_base_, d_recv_idx_, d_err_;
+  DevBuf d_recv_idx_, d_err_;
   size_t shared_capacity_ = 0;
   uint32_t dedupe_epoch_ = 0;
   uint32_t nextEpoch() { return ++dedupe_epoch_ ? dedupe_epoch_ : ++dedupe_epoch_; }  // never 0
@@ -253,6 +253,7 @@ class HetuTable {
   // Mapped pinned words: [0] the key ingest reports an out-of-range key through (the host reads it right after the
   // ingest without a copy), [1] error bits of the bulk-copy expansion.
   uint32_t *h_ingest_err_ = nullptr, *d_ingest_err_ = nullptr;
+  bool keys_in_use_ = false;  // the ingest kernel may still be reading the caller's key buffer
   void dropBadBatch(BatchDesc &b);
   void ingestKeys(BatchDesc &b, const void *keys, size_t n, cudaStream_t s);
   size_t h_pinned_words_ = 0;

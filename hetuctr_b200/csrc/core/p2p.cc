@@ -38,6 +38,11 @@ P2PMailbox::P2PMailbox(int rank, int nrank, int device_id, size_t width, Transpo
   bootstrap_->allgatherHost(&ok, oks.data(), sizeof(int));
   usable_ = true;
   for (int v : oks) usable_ = usable_ && v != 0;
+  if (usable_ && same_context_) {
+    for (cudaEvent_t &e : published_) HCTR_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    peer_published_.resize(2 * (size_t)nrank_);
+    bootstrap_->allgatherHost(published_, peer_published_.data(), sizeof(published_));
+  }
   ctx_.nrank = nrank_;
   ctx_.rank = rank_;
   ctx_.width = width_;
@@ -52,10 +57,13 @@ P2PMailbox::P2PMailbox(int rank, int nrank, int device_id, size_t width, Transpo
   }
 }
 
-void P2PMailbox::hostBarrier() {
-  int token = 0;
-  std::vector<int> tokens(nrank_);
-  bootstrap_->allgatherHost(&token, tokens.data(), sizeof(int));
+// An event is recorded again one step later at the earliest, behind a barrier that every peer joins after it has enqueued
+// its wait for the present recording.
+void P2PMailbox::meet(int phase, cudaStream_t stream) {
+  HCTR_CUDA(cudaEventRecord(published_[phase], stream));
+  bootstrap_->barrier(nrank_);
+  for (int p = 0; p < nrank_; p++)
+    if (p != rank_) HCTR_CUDA(cudaStreamWaitEvent(stream, peer_published_[2 * p + phase], 0));
 }
 
 size_t P2PMailbox::bytesFor(size_t cap) const {
@@ -107,7 +115,7 @@ void P2PMailbox::reserve(size_t cap, cudaStream_t stream) {
   HCTR_CHECK(usable_, "peer-to-peer exchange is not usable on this set of devices");
   HCTR_CHECK(cap < (size_t)1 << 31, "batch too large for the peer-to-peer exchange");
   HCTR_CUDA(cudaStreamSynchronize(stream));
-  if (same_context_) hostBarrier();  // thread ranks: nobody frees a mailbox while a peer's last step still runs
+  if (same_context_) bootstrap_->barrier(nrank_);  // thread ranks: nobody frees a mailbox while a peer's last step still runs
   // Every rank has finished the step that last used the old mailboxes before it gets here (a step only
   // ends after all peers' rows for it have arrived), so they can be unmapped and freed.
   releaseMappings();
@@ -149,15 +157,15 @@ void P2PMailbox::reserve(size_t cap, cudaStream_t stream) {
   ctx_.cnt_in = d_cnt_in_;
   seq_ = 0;
   // nobody may write into a mailbox before its owner has finished zeroing it and everyone has mapped it
-  int token = 0;
-  std::vector<int> tokens(nrank_);
-  bootstrap_->allgatherHost(&token, tokens.data(), sizeof(int));
+  bootstrap_->barrier(nrank_);
 }
 
 P2PMailbox::~P2PMailbox() {
   cudaSetDevice(device_id_);
   cudaDeviceSynchronize();
   releaseMappings();
+  for (cudaEvent_t e : published_)
+    if (e) cudaEventDestroy(e);
   if (d_boxes_) cudaFree(d_boxes_);
   if (d_cnt_in_) cudaFree(d_cnt_in_);
 }

@@ -19,10 +19,12 @@ class P2PMailbox {
   bool usable() const { return usable_; }
   // True when all ranks are threads of one process on one GPU: peers' mailboxes are plain pointers of the shared
   // context, and no kernel may wait for a peer's kernel (nothing guarantees that two launches on one GPU run at the
-  // same time).  The table then publishes with hctr_p2p_signal, drains its stream, meets the peers at a host
-  // barrier and only afterwards launches hctr_p2p_wait, which finds every sequence number already in place.
+  // same time).  Between publishing and consuming, the table then calls meet(): the consuming kernels come behind
+  // events that every rank's publishing kernel has completed, and find every sequence number already in place.
   bool sameContext() const { return same_context_; }
-  void hostBarrier();
+  // Thread ranks: `stream` goes on when the work every rank has in front of its own meet() of this phase (0 or 1) is
+  // done.  The calling thread only waits until all ranks have called.
+  void meet(int phase, cudaStream_t stream);
   // Collective: (re)allocates mailboxes for `cap` rows per source and exchanges the IPC handles.
   // Every rank must call it with the same cap at the same point of the step sequence.
   void reserve(size_t cap, cudaStream_t stream);
@@ -50,6 +52,8 @@ class P2PMailbox {
   hctr_p2p_ctx ctx_{};
   hctr_p2p_box mine_box_{};
   uint32_t seq_ = 0;
+  cudaEvent_t published_[2] = {};               // thread ranks: end of this rank's publishing kernel, per phase
+  std::vector<cudaEvent_t> peer_published_;     // [nrank * 2], every rank's
 };
 
 }  // namespace hetuCTR

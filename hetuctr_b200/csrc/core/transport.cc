@@ -2,6 +2,7 @@
 
 #include <nccl.h>
 
+#include <atomic>
 #include <chrono>
 #include <condition_variable>
 #include <cstdlib>
@@ -9,6 +10,7 @@
 #include <iostream>
 #include <map>
 #include <mutex>
+#include <vector>
 
 #include "utils/errors.h"
 #include "utils/rendezvous.h"
@@ -16,6 +18,12 @@
 namespace hetuCTR {
 
 void Transport::waitStream(cudaStream_t stream) { HCTR_CUDA(cudaStreamSynchronize(stream)); }
+
+void Transport::barrier(int nrank) {
+  const int token = 0;
+  std::vector<int> tokens(nrank);
+  allgatherHost(&token, tokens.data(), sizeof(int));
+}
 
 namespace {
 
@@ -98,21 +106,35 @@ struct InprocWorld {
   std::mutex mu;
   std::condition_variable cv;
   int arrived = 0;
-  long generation = 0;
+  std::atomic<long> generation{0};
   int attached = 0;
   std::vector<std::vector<XferItem>> posted;
 
   explicit InprocWorld(int n) : nrank(n), posted(n) {}
 
   void barrier() {
-    std::unique_lock<std::mutex> lk(mu);
-    const long gen = generation;
-    if (++arrived == nrank) {
-      arrived = 0;
-      generation++;
-      cv.notify_all();
-      return;
+    long gen;
+    {
+      std::unique_lock<std::mutex> lk(mu);
+      gen = generation.load(std::memory_order_relaxed);
+      if (++arrived == nrank) {
+        arrived = 0;
+        generation.store(gen + 1, std::memory_order_release);
+        lk.unlock();
+        cv.notify_all();
+        return;
+      }
     }
+    // The ranks of a step arrive within microseconds of each other, less than it takes to wake a sleeping thread: look for
+    // a while before going to sleep.
+    const auto until = std::chrono::steady_clock::now() + std::chrono::microseconds(100);
+    do {
+      for (int i = 0; i < 64; i++) {
+        if (generation.load(std::memory_order_acquire) != gen) return;
+        __builtin_ia32_pause();
+      }
+    } while (std::chrono::steady_clock::now() < until);
+    std::unique_lock<std::mutex> lk(mu);
     // a rank that never arrives must not hang the others forever
     if (!cv.wait_for(lk, std::chrono::seconds(120), [&] { return generation != gen; }))
       throw std::runtime_error("inproc transport: a rank did not reach the exchange within 120 s");
@@ -161,6 +183,7 @@ class InprocTransport : public Transport {
     HCTR_CUDA(cudaStreamSynchronize(stream));
     world_->barrier();  // nobody reuses a send range before every reader is done
   }
+  void barrier(int) override { world_->barrier(); }
   const char *name() const override { return "inproc"; }
   bool multiProcess() const override { return false; }
   void allgatherHost(const void *mine, void *all, size_t bytes) override {

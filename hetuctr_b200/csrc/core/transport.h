@@ -33,6 +33,8 @@ class Transport {
   virtual const char *name() const = 0;
   // Host-memory all-gather of `bytes` per rank (set-up paths only); acts as a barrier.
   virtual void allgatherHost(const void *mine, void *all, size_t bytes) = 0;
+  // Returns when every rank has called it.
+  virtual void barrier(int nrank);
   // True when ranks are separate processes that each drive their own GPU.
   virtual bool multiProcess() const = 0;
   // Waits until `stream` has drained.  The NCCL transport does not block inside the driver: it polls the stream

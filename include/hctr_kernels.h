@@ -340,6 +340,11 @@ int hctr_p2p_query_send(const hctr_p2p_ctx *c, const uint32_t *meta, size_t u_ma
                         const uint8_t *uniq_owner, const int32_t *uniq_row, const int64_t *version, uint32_t seq,
                         const uint32_t *push_counts, void *stream);
 
+/* End of a step: the words of c->cnt_in up to HCTR_P2P_SERVED, push_counts[0..nrank), the error word and the batch's meta
+ * words [0..meta_words) go to pinned (mapped) host memory in one launch: out = [5n + 7 | n | 1] words, out_meta. */
+int hctr_p2p_report(const hctr_p2p_ctx *c, const uint32_t *push_counts, const uint32_t *meta, unsigned meta_words,
+                    uint32_t *out, uint32_t *out_meta, void *stream);
+
 /* Publishes this rank's counts to every peer and releases sequence number `seq` (what the last thread block of
  * hctr_p2p_query_send / hctr_p2p_stale_gather does, as a launch of its own).
  * phase 0: query count (from meta's segments) + push_count (null = zeros); phase 1: ret_count. */
