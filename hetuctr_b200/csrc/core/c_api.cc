@@ -108,7 +108,7 @@ hctr_wait *hctr_table_push_pull_async(hctr_table *t, const float *grad, float *d
 
 int hctr_wait_finish(hctr_wait *w) {
   if (!w) return -1;
-  int rc = guarded([&] { w->fut.get(); });
+  int rc = guarded([&] { hetuCTR::wait_awake(w->fut); });
   delete w;
   return rc;
 }

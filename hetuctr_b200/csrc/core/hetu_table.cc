@@ -283,7 +283,7 @@ void HetuTable::reserveBatch(BatchDesc &b, size_t batch) {
   b.uniq_owner.ensure(batch);
   b.uniq_row.ensure(batch * sizeof(int32_t));
   b.run_start.ensure((batch + 1) * sizeof(uint32_t));
-  b.meta.ensure((HCTR_META_WORDS + nrank_ + 1) * sizeof(uint32_t));
+  b.meta.ensure((HCTR_META_WORDS + nrank_ + 1 + 2) * sizeof(uint32_t));  // behind them: the reduction's work counters
   b.pos_row.ensure(batch * sizeof(int32_t));
   b.heavy.ensure((batch / 32 + 2) * sizeof(uint32_t));
   if (!hctr_group_fits(batch, kEmbeddingIDMax, nrank_)) b.rank.ensure(batch * sizeof(uint32_t));
@@ -432,7 +432,7 @@ void HetuTable::ingestKeys(BatchDesc &b, const void *keys, size_t n, cudaStream_
   // transfer.
   constexpr size_t kStagePinned = 16384;
   constexpr size_t kChunk = 65536;
-  const unsigned meta_words = (unsigned)(HCTR_META_WORDS + nrank_ + 1);
+  const unsigned meta_words = (unsigned)(HCTR_META_WORDS + nrank_ + 1 + 2);
   const int32_t *row_of = rows_are_keys_ ? nullptr : d_row_of_.as<int32_t>();
   const void *in_place = n == 0 ? nullptr : keys;
   bool pageable = false;
@@ -772,7 +772,7 @@ void HetuTable::reduceGradients(BatchDesc &b, const embed_t *grad) {
   r.push_key = d_pkey_s_.as<int64_t>();
   r.push_updates = d_pupd_s_.as<int64_t>();
   r.push_val = d_pval_s_.as<float>();
-  r.work_counter = d_err_.as<uint32_t>() + 32;
+  r.work_counter = b.meta.as<uint32_t>() + HCTR_META_WORDS + nrank_ + 1;  // cleared by the batch's key ingest
   r.p2p = use_p2p_ ? &p2p_->ctx() : nullptr;
   r.uniq_owner = b.uniq_owner.as<uint8_t>();
   r.push_base = b.push_base.as<uint32_t>();

@@ -1170,8 +1170,6 @@ extern "C" int hctr_grad_reduce_apply_pack(const hctr_reduce_args *ap, void *str
       cudaError_t e = cudaStreamWaitEvent(ls, (cudaEvent_t)a.fork_event, 0);
       if (e != cudaSuccess) return (int)e;
     }
-    cudaError_t em = cudaMemsetAsync(a.work_counter, 0, 2 * sizeof(u32), ls);
-    if (em != cudaSuccess) return (int)em;
     const size_t per = need > 100 * 1024 ? 1 : (forked ? (size_t)long_per_sm : 3);
     const unsigned grid = (unsigned)min((size_t)a.n_heavy, (size_t)kSMs * per);
     if (al && a.width % 4 == 0) grad_reduce_long<true><<<grid, kLongThreads, need, ls>>>(ka, (u32)a.n_heavy, a.work_counter);

@@ -71,7 +71,7 @@ PYBIND11_MODULE(hetuCTR, m) {
   typedef std::future<void> wait_t;
   py::class_<wait_t>(m, "_waittype").def("wait", [](wait_t &w) {
     py::gil_scoped_release release;
-    w.get();  // rethrows a failure of the queued call
+    wait_awake(w);  // rethrows a failure of the queued call
   });
 
   py::enum_<InitType>(m, "InitType", py::module_local())

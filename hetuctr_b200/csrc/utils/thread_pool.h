@@ -2,6 +2,8 @@
 // on `n` threads (the table uses n = 1, so asynchronous calls keep program order).
 // Same role as the reference's ThreadPool (csrc/utils/thread_pool.h:16-50).
 #pragma once
+#include <atomic>
+#include <chrono>
 #include <condition_variable>
 #include <deque>
 #include <functional>
@@ -11,6 +13,26 @@
 #include <vector>
 
 namespace hetuCTR {
+
+// Looks for `ready()` for up to `us` microseconds; true when it came.  A step's calls follow each other within tens of
+// microseconds, and waking a thread that went to sleep in between costs about ten.
+template <class F>
+inline bool spin_for(int us, F ready) {
+  const auto until = std::chrono::steady_clock::now() + std::chrono::microseconds(us);
+  do {
+    for (int i = 0; i < 32; i++) {
+      if (ready()) return true;
+      __builtin_ia32_pause();
+    }
+  } while (std::chrono::steady_clock::now() < until);
+  return false;
+}
+
+// Waits for the result of a queued call, awake for the time a step takes; rethrows a failure of the call.
+inline void wait_awake(std::future<void> &f) {
+  spin_for(1000, [&] { return f.wait_for(std::chrono::seconds(0)) == std::future_status::ready; });
+  f.get();
+}
 
 class ThreadPool {
  public:
@@ -32,6 +54,7 @@ class ThreadPool {
       std::lock_guard<std::mutex> g(mu_);
       if (stop_) throw std::runtime_error("enqueue on stopped ThreadPool");
       queue_.emplace_back(std::move(task));
+      queued_.store(queue_.size(), std::memory_order_release);
     }
     cv_.notify_one();
     return f;
@@ -41,12 +64,14 @@ class ThreadPool {
   void run() {
     for (;;) {
       std::packaged_task<void()> task;
+      spin_for(100, [&] { return queued_.load(std::memory_order_acquire) != 0; });
       {
         std::unique_lock<std::mutex> lk(mu_);
         cv_.wait(lk, [this] { return stop_ || !queue_.empty(); });
         if (queue_.empty()) return;
         task = std::move(queue_.front());
         queue_.pop_front();
+        queued_.store(queue_.size(), std::memory_order_release);
       }
       task();
     }
@@ -55,6 +80,7 @@ class ThreadPool {
   std::condition_variable cv_;
   std::deque<std::packaged_task<void()>> queue_;
   std::vector<std::thread> workers_;
+  std::atomic<size_t> queued_{0};  // size of queue_, readable without the lock
   bool stop_ = false;
 };
 

@@ -425,7 +425,7 @@ typedef struct hctr_reduce_args {
   int64_t *push_key;          /* [P] packed ids of pushed rows */
   int64_t *push_updates;      /* [P] update counts */
   float *push_val;            /* [P, W] */
-  uint32_t *work_counter;     /* three device words of scratch (work queues of the kernels) */
+  uint32_t *work_counter;     /* two device words, zero on entry (work queues of the long-run kernel) */
   /* optional peer-to-peer routing of pushed rows: when p2p is non-null, a pushed row of a key owned by
    * rank p goes to slot (push_slot[u] - push_base[p]) of this rank's sub-region in p's mailbox instead
    * of push_key / push_updates / push_val */
