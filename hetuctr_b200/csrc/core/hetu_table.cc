@@ -896,9 +896,12 @@ void HetuTable::pushPull(embed_t *grad, embed_t *dst) {
                                           prev.uniq.as<int64_t>(), prev.meta.as<uint32_t>(), 1,
                                           d_embedding_.as<float>(), dst_dev, tail));
       HCTR_CUDA(cudaStreamWaitEvent(tail, ev_early_, 0));  // the step ends when both halves are in dst
+    } else if (expand_bulk_) {
+      HCTR_LAUNCH(hctr_expand_rows_bulk(cur.batch_size, W, cur.pos_row.as<int32_t>(), cur.idx_map.as<int32_t>(), nullptr,
+                                        nullptr, d_embedding_.as<float>(), dst_dev, d_ingest_err_ + 1, tail));
     } else {
-      HCTR_LAUNCH(expandRows(cur.batch_size, W, cur.pos_row.as<int32_t>(), cur.idx_map.as<int32_t>(), nullptr,
-                             nullptr, d_embedding_.as<float>(), dst_dev, d_ingest_err_ + 1, tail));
+      HCTR_LAUNCH(hctr_expand_rows_local(cur.batch_size, W, cur.pos_row.as<int32_t>(), d_embedding_.as<float>(), dst_dev,
+                                         tail));
     }
     toc(sp, tail);
     // The dedupe of this batch goes behind the step's critical path on stream_main_ (low priority): only the next

@@ -536,6 +536,11 @@ int hctr_expand_rows(size_t batch, size_t width, const int32_t *pos_row, const i
                      const uint32_t *recv_slot, const float *recv_val, const float *embedding,
                      float *dst, void *stream);
 
+/* hctr_expand_rows for a table that stores every key itself: dst[i] = embedding[pos_row[i]], zeros where pos_row[i] is
+ * HCTR_INVALID_ROW.  pos_row: 16-byte aligned. */
+int hctr_expand_rows_local(size_t batch, size_t width, const int32_t *pos_row, const float *embedding, float *dst,
+                           void *stream);
+
 /* Half of hctr_expand_rows for a table that stores every key itself: only the positions whose key is
  * (in_prev != 0) / is not (in_prev == 0) among prev_uniq[0 .. prev_meta[HCTR_META_UNIQUE]), the ascending unique
  * keys of the previous batch.  The two halves together write every row of dst exactly once; the "is not" half

@@ -143,3 +143,25 @@ def test_reduction_run_lengths(oracle_mod, width):
     grads = [None] + [[rng.normal(0, 1, size=(len(b[0]), width)).astype(np.float32)] for b in batches[:-1]]
     run_steps(gw, ow, batches, grads)
     gw.close()
+
+
+@pytest.mark.parametrize("width", [1, 3, 4, 6, 10, 12, 50, 64, 100, 128, 132, 258])
+@pytest.mark.parametrize("batch", [1, 2, 3, 4, 5, 37, 4097, 60_001])
+def test_expand_local(batch, width):
+    L = hb.lib()
+    L.hctr_expand_rows_local.argtypes = [sz, sz, vp, vp, vp, vp]
+    dev = torch.device("cuda:0")
+    g = torch.Generator(device=dev)
+    g.manual_seed(batch + width)
+    emb = torch.randn((3000, width), generator=g, device=dev)
+    rows = torch.randint(3000, (batch,), generator=g, device=dev, dtype=torch.int32)
+    rows[batch // 2] = -1  # no row: zeros
+    guard = torch.full((batch + 1, width), float("nan"), device=dev)
+    for dst in (guard[:batch], guard.reshape(-1)[1:1 + batch * width].reshape(batch, width)):  # the second misaligned
+        guard.fill_(float("nan"))
+        assert L.hctr_expand_rows_local(batch, width, rows.data_ptr(), emb.data_ptr(), dst.data_ptr(), None) == 0
+        torch.cuda.synchronize()
+        want = emb[rows.clamp(min=0).long()]
+        want[batch // 2] = 0
+        assert torch.equal(dst, want)
+        assert int(torch.isnan(guard).sum()) == width
