@@ -207,150 +207,125 @@ __device__ __forceinline__ void reduce_apply(const RowTarget &t, typename R::T s
   }
 }
 
-// Short runs (<= HCTR_LIGHT_RUN positions): one group of LANES lanes per unique key.
+// Short runs (<= HCTR_LIGHT_RUN positions): one group of LANES lanes per unique key, a resident round of groups that
+// walks the keys.  Bound: latency - run bounds, storage class and push slot, position, row, each loaded when the one
+// before it has arrived, were five round trips per key and 38 us for 26,500 or for 106,000 keys.  Now everything that
+// depends on the key's index alone is loaded two keys ahead and the first position one key ahead; the peers' addresses
+// wait in shared memory.  A key then costs the round trip of its rows.  (Two thread ranks of 212,992 x 32: 336 -> 313 us
+// per step.  At 128 floats the streaming kernel below stays ahead, 195 against 209 us: runs of ten and more rows are what
+// counts there.)
+struct KeyAhead {
+  u32 l, r;       // run
+  int32_t row;
+  u32 need, slot;
+  u32 owner;
+};
+
 template <int LANES, bool VEC>
-__global__ void __launch_bounds__(kThreads) grad_reduce_short(ReduceKernelArgs ka) {
+__global__ void __launch_bounds__(kThreads, 4) grad_reduce_short(ReduceKernelArgs ka) {
   const hctr_reduce_args &a = ka.a;
   typedef RowT<VEC> R;
   typedef typename R::T T;
-  const size_t u = ((size_t)blockIdx.x * kThreads + threadIdx.x) / LANES;
+  __shared__ PushDest s_peer[kMaxRanks];
+  __shared__ u32 s_base[kMaxRanks];
+  if (a.p2p) {
+    for (int p = threadIdx.x; p < ka.p2p.nrank; p += kThreads) {
+      const hctr_p2p_box b = ka.p2p.box[p];
+      const size_t first = (size_t)ka.p2p.rank * ka.p2p.cap;
+      s_peer[p].key = reinterpret_cast<long long *>(b.pkey) + first;
+      s_peer[p].upd = reinterpret_cast<long long *>(b.pupd) + first;
+      s_peer[p].val = b.pval + first * a.width;
+      s_base[p] = a.push_base[p];
+    }
+    __syncthreads();
+  }
+  const size_t groups = (size_t)gridDim.x * (kThreads / LANES);
   const unsigned gl = threadIdx.x % LANES;
-  if (u >= a.n_unique) return;
-  const u32 l = a.run_start[u], r = a.run_start[u + 1];
-  if (r - l > HCTR_LIGHT_RUN) return;  // handled by grad_reduce_long
-  PushDest dest;
-  const RowTarget t = reduce_bookkeeping(a, ka.p2p, u, r - l, gl == 0, &dest);
   const size_t E = R::elems(a.width);
   const T *grad = reinterpret_cast<const T *>(a.grad);
-  T *emb = reinterpret_cast<T *>(a.embedding) + (t.row >= 0 ? (size_t)t.row * E : 0);
-  T *pend = reinterpret_cast<T *>(a.pending) + (t.type >= 2 ? (size_t)t.row * E : 0);
-  T *out = reinterpret_cast<T *>(dest.val);
-  for (size_t c = gl; c < E; c += LANES) {
-    T sum = R::zero();
-    u32 j = l;
-    // the table row does not depend on the gradient chain: start its load first
-    T e_old = R::zero(), p_old = R::zero();
-    if (t.type != 0) e_old = emb[c];
-    if (t.type >= 2) p_old = pend[c];
-    // 4 independent loads in flight per lane; adds stay in position order
-    for (; j + 4 <= r; j += 4) {
-      const T g0 = R::ld_once(grad + (size_t)a.sorted_pos[j] * E + c);
-      const T g1 = R::ld_once(grad + (size_t)a.sorted_pos[j + 1] * E + c);
-      const T g2 = R::ld_once(grad + (size_t)a.sorted_pos[j + 2] * E + c);
-      const T g3 = R::ld_once(grad + (size_t)a.sorted_pos[j + 3] * E + c);
-      sum = R::add(R::add(R::add(R::add(sum, g0), g1), g2), g3);
+  auto ahead = [&](size_t u) {
+    KeyAhead k = {0u, 0u, 0, 0u, 0u, 0u};
+    if (u < a.n_unique) {
+      k.l = a.run_start[u];
+      k.r = a.run_start[u + 1];
+      k.row = a.uniq_row[u];
+      k.need = a.need_push[u];
+      k.slot = a.push_slot[u];
+      k.owner = a.uniq_owner[u];
     }
-    for (; j < r; j++) sum = R::add(sum, R::ld_once(grad + (size_t)a.sorted_pos[j] * E + c));
-    sum = R::scale(sum, a.neg_lr);
-    if (t.type == 0) {
-      out[c] = sum;
-    } else {
-      emb[c] = R::add(e_old, sum);
-      if (t.type >= 2) {
-        const T p = R::add(p_old, sum);
-        if (t.type == 2) {
-          out[c] = p;
-          pend[c] = R::zero();
+    return k;
+  };
+  size_t u = ((size_t)blockIdx.x * kThreads + threadIdx.x) / LANES;
+  KeyAhead now = ahead(u), then = ahead(u + groups);
+  u32 pos = now.r > now.l ? a.sorted_pos[now.l] : 0u;
+  for (; u < a.n_unique; u += groups) {
+    const KeyAhead after = ahead(u + 2 * groups);
+    const u32 pos_then = then.r > then.l ? a.sorted_pos[then.l] : 0u;
+    const u32 l = now.l, r = now.r;
+    if (r > l && r - l <= HCTR_LIGHT_RUN) {  // (longer: grad_reduce_long)
+      const int type = now.row < 0 ? 0 : (size_t)now.row >= a.n_cached ? 1 : now.need ? 2 : 3;
+      PushDest dest = {nullptr, nullptr, nullptr};
+      if (now.need) {
+        if (a.p2p) {
+          u32 j = now.slot - s_base[now.owner];
+          if (j >= ka.p2p.cap) {  // cannot happen when every rank uses the same batch size; never write out of bounds
+            atomicOr(ka.p2p.err, HCTR_ERR_CAPACITY);
+            j = 0;
+          }
+          dest.key = s_peer[now.owner].key + j;
+          dest.upd = s_peer[now.owner].upd + j;
+          dest.val = s_peer[now.owner].val + (size_t)j * a.width;
         } else {
-          pend[c] = p;
+          dest.key = reinterpret_cast<long long *>(a.push_key) + now.slot;
+          dest.upd = reinterpret_cast<long long *>(a.push_updates) + now.slot;
+          dest.val = a.push_val + (size_t)now.slot * a.width;
         }
       }
-    }
-  }
-}
-
-// Short runs, rows of at least 32 float4 (width >= 128): a warp takes kWideChunk consecutive unique
-// keys.  Run bounds, rows, push slots and first positions are fetched by the first lanes (one key per
-// lane) and the per-key bookkeeping runs one key per lane; the warp then walks the keys, and while it
-// sums and applies key k the first gradient row and the table row of the next key are already in
-// flight.  The chunk is small so that a batch still yields enough warps to fill every SM.
-constexpr unsigned kWideChunk = 8;
-// (Capping registers to raise occupancy was measured: 48 registers / 5 CTAs per SM made the warm kernel
-// slower, 84 us vs 71 us for the reduce phase, so the compiler keeps its 80.)
-__global__ void __launch_bounds__(kThreads) grad_reduce_short_wide(ReduceKernelArgs ka) {
-  const hctr_reduce_args &a = ka.a;
-  typedef RowT<true> R;
-  typedef float4 T;
-  const unsigned lane = threadIdx.x & 31;
-  const size_t warp = ((size_t)blockIdx.x * kThreads + threadIdx.x) >> 5;
-  const size_t n_warps = ((size_t)gridDim.x * kThreads) >> 5;
-  const size_t E = a.width / 4;
-  const T *grad = reinterpret_cast<const T *>(a.grad);
-  T *emb_base = reinterpret_cast<T *>(a.embedding);
-  T *pend_base = reinterpret_cast<T *>(a.pending);
-  // (A one-wave grid with chunks drawn from a shared counter was measured and was slower: 105 us vs 92 us.)
-  const size_t n_unique = a.n_unique;
-  for (size_t u0 = warp * kWideChunk; u0 < n_unique; u0 += n_warps * kWideChunk) {
-    const size_t my_u = u0 + lane;
-    u32 l = 0, len = 0, p0 = 0;
-    unsigned long long outp = 0;  // destination of this lane's key if it is pushed
-    int row = 0, type = -1;       // type -1: nothing to do for this lane's key
-    if (lane < kWideChunk && my_u < n_unique) {
-      l = a.run_start[my_u];
-      len = a.run_start[my_u + 1] - l;
-      if (len > 0 && len <= HCTR_LIGHT_RUN) {
-        p0 = a.sorted_pos[l];
-        PushDest dest;
-        const RowTarget t = reduce_bookkeeping(a, ka.p2p, my_u, len, true, &dest);
-        row = t.row;
-        type = t.type;
-        outp = (unsigned long long)dest.val;
-      }
-    }
-    unsigned todo = __ballot_sync(0xffffffffu, type >= 0);
-    if (!todo) continue;
-    // prefetch for the first key
-    int k = __ffs(todo) - 1;
-    todo &= todo - 1;
-    T g_next, e_next;
-    {
-      const u32 pk = __shfl_sync(0xffffffffu, p0, k);
-      const int rk = __shfl_sync(0xffffffffu, row, k), tk = __shfl_sync(0xffffffffu, type, k);
-      g_next = R::ld_once(grad + (size_t)pk * E + lane);
-      e_next = tk != 0 ? emb_base[(size_t)rk * E + lane] : R::zero();
-    }
-    while (k >= 0) {
-      const u32 lk = __shfl_sync(0xffffffffu, l, k), lenk = __shfl_sync(0xffffffffu, len, k);
-      const unsigned long long outk = __shfl_sync(0xffffffffu, outp, k);
-      const int rowk = __shfl_sync(0xffffffffu, row, k), typek = __shfl_sync(0xffffffffu, type, k);
-      const T g0 = g_next, e0 = e_next;
-      const int kn = todo ? __ffs(todo) - 1 : -1;
-      todo &= todo - 1;
-      if (kn >= 0) {
-        const u32 pk = __shfl_sync(0xffffffffu, p0, kn);
-        const int rk = __shfl_sync(0xffffffffu, row, kn), tk = __shfl_sync(0xffffffffu, type, kn);
-        g_next = R::ld_once(grad + (size_t)pk * E + lane);
-        e_next = tk != 0 ? emb_base[(size_t)rk * E + lane] : R::zero();
-      }
-      T *emb = emb_base + (typek != 0 ? (size_t)rowk * E : 0);
-      T *pend = pend_base + (typek >= 2 ? (size_t)rowk * E : 0);
-      T *out = reinterpret_cast<T *>(outk);
-      for (size_t c = lane; c < E; c += 32) {
-        T sum, e_old;
-        if (c == lane) {
-          sum = R::add(R::zero(), g0);
-          e_old = e0;
-        } else {
-          sum = R::add(R::zero(), R::ld_once(grad + (size_t)a.sorted_pos[lk] * E + c));
-          e_old = typek != 0 ? emb[c] : R::zero();
+      T *emb = reinterpret_cast<T *>(a.embedding) + (type != 0 ? (size_t)now.row * E : 0);
+      T *pend = reinterpret_cast<T *>(a.pending) + (type >= 2 ? (size_t)now.row * E : 0);
+      T *out = reinterpret_cast<T *>(dest.val);
+      for (size_t c = gl; c < E; c += LANES) {
+        const T g0 = R::ld_once(grad + (size_t)pos * E + c);
+        T e_old = R::zero(), p_old = R::zero();
+        if (type != 0) e_old = emb[c];
+        if (type >= 2) p_old = pend[c];
+        if (c == 0) {  // versions, pending counts, packed id + update count: once per key, while the rows are coming
+          long long cnt = (long long)(r - l);
+          if (type == 1) {
+            atomicAdd(reinterpret_cast<u64 *>(a.version) + now.row, (u64)cnt);  // (no other writer)
+          } else if (type >= 2) {
+            long long pc = a.pending_cnt[now.row] + cnt;
+            if (type == 2) {
+              cnt = pc;
+              pc = 0;
+              atomicAdd(reinterpret_cast<u64 *>(a.version) + now.row, (u64)cnt);
+            }
+            a.pending_cnt[now.row] = pc;
+          }
+          if (now.need) {
+            *dest.key = a.uniq[u];
+            *dest.upd = cnt;
+          }
         }
-        u32 j = 1;
-        for (; j + 4 <= lenk; j += 4) {
-          const T g1 = R::ld_once(grad + (size_t)a.sorted_pos[lk + j] * E + c);
-          const T g2 = R::ld_once(grad + (size_t)a.sorted_pos[lk + j + 1] * E + c);
-          const T g3 = R::ld_once(grad + (size_t)a.sorted_pos[lk + j + 2] * E + c);
-          const T g4 = R::ld_once(grad + (size_t)a.sorted_pos[lk + j + 3] * E + c);
+        T sum = R::add(R::zero(), g0);
+        u32 j = l + 1;
+        // 4 independent loads in flight per lane; adds stay in position order
+        for (; j + 4 <= r; j += 4) {
+          const T g1 = R::ld_once(grad + (size_t)a.sorted_pos[j] * E + c);
+          const T g2 = R::ld_once(grad + (size_t)a.sorted_pos[j + 1] * E + c);
+          const T g3 = R::ld_once(grad + (size_t)a.sorted_pos[j + 2] * E + c);
+          const T g4 = R::ld_once(grad + (size_t)a.sorted_pos[j + 3] * E + c);
           sum = R::add(R::add(R::add(R::add(sum, g1), g2), g3), g4);
         }
-        for (; j < lenk; j++) sum = R::add(sum, R::ld_once(grad + (size_t)a.sorted_pos[lk + j] * E + c));
+        for (; j < r; j++) sum = R::add(sum, R::ld_once(grad + (size_t)a.sorted_pos[j] * E + c));
         sum = R::scale(sum, a.neg_lr);
-        if (typek == 0) {
+        if (type == 0) {
           out[c] = sum;
         } else {
           emb[c] = R::add(e_old, sum);
-          if (typek >= 2) {
-            const T p = R::add(pend[c], sum);
-            if (typek == 2) {
+          if (type >= 2) {
+            const T p = R::add(p_old, sum);
+            if (type == 2) {
               out[c] = p;
               pend[c] = R::zero();
             } else {
@@ -359,12 +334,14 @@ __global__ void __launch_bounds__(kThreads) grad_reduce_short_wide(ReduceKernelA
           }
         }
       }
-      k = kn;
     }
+    now = then;
+    then = after;
+    pos = pos_then;
   }
 }
 
-// Work-balanced streaming variant of the kernel above (rows of 128..512 floats).
+// Short runs, rows of 128..512 floats: work-balanced and streaming.
 // Balance: a key costs (its gradient rows + 2) row transfers - the rows it sums plus the read and write of
 // its table row - and cost(k) = run_start[k] + 2k, the cost of all keys before k, grows strictly with k.
 // Warp w of n_warps takes the keys whose cost(k) falls into [w*T, (w+1)*T), T = ceil(cost(U) / n_warps): every
@@ -1133,6 +1110,7 @@ extern "C" int hctr_grad_reduce_apply_pack(const hctr_reduce_args *ap, void *str
   cudaStream_t s = (cudaStream_t)stream;
   const hctr_reduce_args a = *ap;
   if (a.n_unique == 0) return 0;
+  if (!a.need_push || !a.push_slot || !a.uniq_owner) return (int)cudaErrorInvalidValue;
   ReduceKernelArgs ka;
   ka.a = a;
   if (a.p2p) ka.p2p = *a.p2p;
@@ -1207,14 +1185,12 @@ extern "C" int hctr_grad_reduce_apply_pack(const hctr_reduce_args *ap, void *str
     const size_t wanted = (3 * a.n_unique / 48 * 32 + kThreads - 1) / kThreads + 1;
     const size_t ctas = std::min(wanted, slots);
     kernel<<<(unsigned)ctas, kThreads, smem, s>>>(ka);
-  } else if (al && a.width % 4 == 0 && a.width >= 128) {
-    size_t ctas = ((a.n_unique + kWideChunk - 1) / kWideChunk * 32 + kThreads - 1) / kThreads;
-    const size_t cap = (size_t)kSMs * 8;
-    if (ctas > cap) ctas = cap;
-    grad_reduce_short_wide<<<(unsigned)ctas, kThreads, 0, s>>>(ka);
   } else {
-#define CALL(L, V) \
-  grad_reduce_short<L, V><<<grid_for(a.n_unique * L, kThreads), kThreads, 0, s>>>(ka)
+#define CALL(L, V)                                                                                                      \
+  do {                                                                                                                  \
+    const size_t need = (a.n_unique * L + kThreads - 1) / kThreads;                                                     \
+    grad_reduce_short<L, V><<<(unsigned)std::min(need, (size_t)kSMs * 4), kThreads, 0, s>>>(ka); /* one resident round */ \
+  } while (0)
     HCTR_DISPATCH_ROWS(a.width, al, CALL);
 #undef CALL
   }

@@ -416,8 +416,8 @@ typedef struct hctr_reduce_args {
   size_t n_heavy;             /* entries in heavy_list (host value) */
   const int64_t *uniq;        /* [U] */
   const int32_t *uniq_row;    /* [U] */
-  const uint32_t *need_push;  /* [U] or null when nrank==1 */
-  const uint32_t *push_slot;  /* [U+1] or null */
+  const uint32_t *need_push;  /* [U] */
+  const uint32_t *push_slot;  /* [U+1] */
   float *embedding;           /* [S, W] */
   int64_t *version;           /* [S] */
   float *pending;             /* [n_cached, W] */
