@@ -1182,7 +1182,11 @@ void HetuTable::exchangeP2P(embed_t *dst_dev) {
   // C. owner applies the pushed rows of each source in rank order
   const hctr_p2p_box mine = p2p_->mine();
   sp = tic(kPhOwnerUpdate);
-  if (n <= 32) {
+  if (n == 2) {
+    HCTR_LAUNCH(hctr_p2p_owner_apply_pair(c, &mine, seq, d_row_of_.as<int32_t>(), kEmbeddingIDMax, kNonLocalStorageMax,
+                                          d_embedding_.as<float>(), d_version_.as<int64_t>(), stream_main_));
+    toc(sp);
+  } else if (n <= 32) {
     // pass A waits for the peers' counts, then marks sources, chains the entries of every row and finishes the
     // versions; pass B adds the rows
     HCTR_LAUNCH(hctr_p2p_owner_mark(c, &mine, seq, d_row_of_.as<int32_t>(), kEmbeddingIDMax, kNonLocalStorageMax,

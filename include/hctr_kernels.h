@@ -374,6 +374,10 @@ int hctr_p2p_owner_apply(const hctr_p2p_ctx *c, const hctr_p2p_box *mine, size_t
                          const unsigned long long *row_mask, unsigned long long *row_head, uint32_t *ent_next,
                          float *embedding, void *stream);
 
+/* Both passes in one launch for a job of two ranks (one peer: no row is pushed by more than one source). */
+int hctr_p2p_owner_apply_pair(const hctr_p2p_ctx *c, const hctr_p2p_box *mine, uint32_t seq, const int32_t *row_of,
+                              size_t length, size_t n_cached, float *embedding, int64_t *version, void *stream);
+
 /* Pull side.  Nothing is compacted: the row returned for the j-th query requester s sent to this owner goes to row
  * (owner * cap + j) of s's mailbox - a place s can compute for each of its unique keys without knowing what the
  * owner decided - so neither side scans flags.
