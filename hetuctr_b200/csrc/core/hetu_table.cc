@@ -103,14 +103,16 @@ HetuTable::HetuTable(const int rank, const int nrank, const int device_id, const
     // the side stream carries the run ordering of batches that are ranked through the bitmap
     HCTR_CUDA(cudaStreamCreateWithPriority(&stream_side_, cudaStreamNonBlocking, single ? lo : hi));
     HCTR_CUDA(cudaStreamCreateWithPriority(&stream_reduce_, cudaStreamNonBlocking, single ? hi : lo));
-    if (!single) HCTR_CUDA(cudaStreamCreateWithPriority(&stream_reduce_side_, cudaStreamNonBlocking, hi));
+    HCTR_CUDA(cudaStreamCreateWithPriority(&stream_reduce_side_, cudaStreamNonBlocking, hi));
+    if (single) HCTR_CUDA(cudaStreamCreateWithPriority(&stream_pieces_, cudaStreamNonBlocking, hi));
   }
   HCTR_CUDA(cudaEventCreateWithFlags(&ev_rfork_, cudaEventDisableTiming));
   HCTR_CUDA(cudaEventCreateWithFlags(&ev_rjoin_, cudaEventDisableTiming));
   HCTR_CUDA(cudaEventCreateWithFlags(&ev_decide_, cudaEventDisableTiming));
   HCTR_CUDA(cudaEventCreateWithFlags(&ev_reduce_, cudaEventDisableTiming));
   HCTR_CUDA(cudaEventCreateWithFlags(&ev_keys_, cudaEventDisableTiming));
-  HCTR_CUDA(cudaEventCreateWithFlags(&ev_early_, cudaEventDisableTiming));
+  for (cudaEvent_t *e : {&ev_early_, &ev_sizes_}) HCTR_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+  for (cudaEvent_t &e : ev_piece_) HCTR_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   if (const char *e = std::getenv("HCTR_SPLIT_HOST_EXPAND")) split_host_expand_ = std::atoi(e) != 0;
   if (const char *e = std::getenv("HCTR_P2P_FUSED_EXPAND")) fused_refresh_expand_ = std::atoi(e) != 0;
 
@@ -368,6 +370,7 @@ void HetuTable::preprocess(index_t *data_ptr, size_t batch_size) {
     cur.dedupe_in_flight = false;
   }
   cur.scatter_recorded = false;
+  cur.sizes_coming = false;
   cur.dedupe_pending = true;
   cur.pending = true;
   ingestKeys(cur, data_ptr, batch_size, ks);
@@ -719,21 +722,25 @@ void HetuTable::finalizePending() {
   if (cur_batch_.pending) finalizeBatch();
 }
 
-const void *HetuTable::stageIn(const void *ptr, size_t bytes, DevBuf &buf, cudaStream_t st) {
+static bool onDevice(const void *ptr) {
   cudaPointerAttributes attr;
-  cudaError_t e = cudaPointerGetAttributes(&attr, ptr);
-  if (e != cudaSuccess) {
+  if (cudaPointerGetAttributes(&attr, ptr) != cudaSuccess) {
     cudaGetLastError();
-    attr.type = cudaMemoryTypeUnregistered;
+    return false;
   }
-  if (attr.type == cudaMemoryTypeDevice || attr.type == cudaMemoryTypeManaged) return ptr;
+  return attr.type == cudaMemoryTypeDevice || attr.type == cudaMemoryTypeManaged;
+}
+
+const void *HetuTable::stageIn(const void *ptr, size_t bytes, DevBuf &buf, cudaStream_t st) {
+  if (onDevice(ptr)) return ptr;
   buf.ensure(bytes);
   HCTR_CUDA(cudaMemcpyAsync(buf.p, ptr, bytes, cudaMemcpyHostToDevice, st));
   return buf.p;
 }
 
 // Duplicate-gradient reduction + local apply (+ pack of pushed rows) of batch b, on stream_reduce_ (generateGradient).
-void HetuTable::reduceGradients(BatchDesc &b, const embed_t *grad) {
+// Single-rank tables: of the keys whose last batch position is in [last_lo, last_hi).
+void HetuTable::reduceGradients(BatchDesc &b, const embed_t *grad, size_t last_lo, size_t last_hi) {
   if (nrank_ == 1) {
     hctr_local_reduce_args r{};
     r.batch = b.batch_size;
@@ -748,7 +755,8 @@ void HetuTable::reduceGradients(BatchDesc &b, const embed_t *grad) {
     r.meta = b.meta.as<uint32_t>();
     r.embedding = d_embedding_.as<float>();
     r.version = d_version_.as<int64_t>();
-    HCTR_LAUNCH(hctr_grad_reduce_local(&r, stream_reduce_));
+    if (last_lo == 0 && last_hi == b.batch_size) HCTR_LAUNCH(hctr_grad_reduce_local(&r, stream_reduce_));
+    else HCTR_LAUNCH(hctr_grad_reduce_window(&r, (uint32_t)last_lo, (uint32_t)last_hi, stream_reduce_));
     return;
   }
   hctr_reduce_args r{};
@@ -780,6 +788,98 @@ void HetuTable::reduceGradients(BatchDesc &b, const embed_t *grad) {
   r.fork_event = ev_rfork_;
   r.join_event = ev_rjoin_;
   HCTR_LAUNCH(hctr_grad_reduce_apply_pack(&r, stream_reduce_));
+}
+
+// Single rank, gradients in host memory and dst in pinned host memory: the step is two transfers over the host link, which
+// overlap as far as the data allows.
+//  * Rows of dst whose keys the previous batch did not contain do not depend on the gradients: they are written (by the
+//    kernel, straight into dst) while those come in.
+//  * Large gradients come in pieces, and after each the keys that are complete with it are updated and their rows written.
+//    Each piece is half of what is left: early pieces complete few keys (the last position of a hot key is near the end
+//    of the batch).
+// 53,248 positions x 128, 30 % of them new keys: 955 us with one piece, 875 with five.  What is left is the link: the copy in
+// (500 us), and after it the rows of keys whose last position is in the last piece, at the 51 GB/s a kernel stores.
+void HetuTable::splitHostStep(BatchDesc &cur, BatchDesc &prev, const embed_t *grad, embed_t *dst) {
+  const size_t W = kEmbeddingWidth, n = prev.batch_size, B = cur.batch_size;
+  const float *rows = d_embedding_.as<float>();
+  d_stage_grad_.ensure(n * W * sizeof(embed_t));
+  embed_t *staged = d_stage_grad_.as<embed_t>();
+  const bool pieces = worthPieces(prev);
+  cudaStream_t copies = pieces ? stream_pieces_ : stream_reduce_;
+  auto fetch = [&](size_t i, size_t lo, size_t hi) {
+    HCTR_CUDA(cudaMemcpyAsync(staged + lo * W, grad + lo * W, (hi - lo) * W * sizeof(embed_t), cudaMemcpyHostToDevice, copies));
+    if (pieces) HCTR_CUDA(cudaEventRecord(ev_piece_[i], copies));
+  };
+  size_t hi = pieces ? pieceEnd(0, 0, n) : n;
+  fetch(0, 0, hi);
+
+  HCTR_CUDA(cudaStreamWaitEvent(stream_reduce_, prev.ev_scatter, 0));
+  if (prev.order_recorded) HCTR_CUDA(cudaStreamWaitEvent(stream_reduce_, prev.ev_order, 0));
+  prev.dedupe_in_flight = false;
+  cudaStream_t early = stream_reduce_side_;
+  HCTR_CUDA(cudaStreamWaitEvent(early, ev_keys_, 0));
+  HCTR_CUDA(cudaStreamWaitEvent(early, prev.ev_scatter, 0));
+  if (pieces) {
+    d_last_seen_.ensure(B * sizeof(uint32_t));
+    if (prev.order_recorded) HCTR_CUDA(cudaStreamWaitEvent(early, prev.ev_order, 0));
+    HCTR_LAUNCH(hctr_last_seen(B, cur.keys.as<int64_t>(), prev.uniq.as<int64_t>(), prev.meta.as<uint32_t>(),
+                               prev.run_start.as<uint32_t>(), prev.sorted_pos.as<uint32_t>(), d_last_seen_.as<uint32_t>(), early));
+    HCTR_CUDA(cudaEventRecord(ev_early_, early));
+    HCTR_CUDA(cudaStreamWaitEvent(stream_reduce_, ev_early_, 0));
+    HCTR_LAUNCH(hctr_expand_rows_window(B, W, cur.pos_row.as<int32_t>(), d_last_seen_.as<uint32_t>(), HCTR_NEVER, 1, rows,
+                                        dst, early));
+  } else {
+    HCTR_LAUNCH(hctr_expand_rows_subset(B, W, cur.pos_row.as<int32_t>(), cur.keys.as<int64_t>(), prev.uniq.as<int64_t>(),
+                                        prev.meta.as<uint32_t>(), 0, rows, dst, early));
+  }
+  HCTR_CUDA(cudaEventRecord(ev_early_, early));
+
+  flushDedupe(cur);  // (the host's launches hide behind the first copy)
+  if (pieceEnd(0, 0, B) < B) {  // worthPieces will ask
+    HCTR_CUDA(cudaMemcpyAsync(cur.h_meta, cur.meta.p, (HCTR_META_WORDS + nrank_ + 1) * sizeof(uint32_t),
+                              cudaMemcpyDeviceToHost, stream_main_));
+    HCTR_CUDA(cudaEventRecord(ev_sizes_, stream_main_));
+    cur.sizes_coming = true;
+  }
+
+  size_t lo = 0;
+  for (size_t i = 0; lo < n; i++) {
+    const size_t next = pieceEnd(i + 1, hi, n);
+    if (hi < n) fetch(i + 1, hi, next);
+    if (pieces) HCTR_CUDA(cudaStreamWaitEvent(stream_reduce_, ev_piece_[i], 0));
+    int sp = tic(kPhReduce, stream_reduce_);
+    reduceGradients(prev, staged, lo, hi);
+    toc(sp, stream_reduce_);
+    sp = tic(kPhExpand, stream_reduce_);
+    if (pieces)
+      HCTR_LAUNCH(hctr_expand_rows_window(B, W, cur.pos_row.as<int32_t>(), d_last_seen_.as<uint32_t>(), (uint32_t)lo,
+                                          (uint32_t)(hi - lo), rows, dst, stream_reduce_));
+    else
+      HCTR_LAUNCH(hctr_expand_rows_subset(B, W, cur.pos_row.as<int32_t>(), cur.keys.as<int64_t>(), prev.uniq.as<int64_t>(),
+                                          prev.meta.as<uint32_t>(), 1, rows, dst, stream_reduce_));
+    toc(sp, stream_reduce_);
+    lo = hi;
+    hi = next;
+  }
+  HCTR_CUDA(cudaStreamWaitEvent(stream_reduce_, ev_early_, 0));  // the step ends when all rows are in dst
+}
+
+// Pieces pay when the next batch asks for many of this one's keys again.  Nobody knows before the keys are compared, but the
+// next batch is as like this one as half of this one is like the other half: the share of duplicates says it.  53,248 x 128:
+// 61 % duplicates 955 -> 875 us, 38 % 938 -> 794 us, none 695 -> 746 us (so those go in one piece).
+bool HetuTable::worthPieces(BatchDesc &b) {
+  if (!b.sizes_coming) return false;
+  HCTR_CUDA(cudaEventSynchronize(ev_sizes_));  // (passed long ago)
+  return (size_t)b.h_meta[HCTR_META_UNIQUE] * 10 <= b.batch_size * 7;
+}
+
+// End of the i-th piece of n gradient rows, which starts at lo.
+// Pieces are at least kPiece bytes, 40 us on the link: the launches for one hide behind the copy of the next (53,248 x 128:
+// 875 us; at least 1 MB 892, 4 MB 900).
+size_t HetuTable::pieceEnd(size_t i, size_t lo, size_t n) const {
+  constexpr size_t kPiece = (size_t)2 << 20, kPieces = sizeof(ev_piece_) / sizeof(ev_piece_[0]);
+  const size_t half = (n - lo + 1) / 2;
+  return i + 1 >= kPieces || half * kEmbeddingWidth * sizeof(embed_t) < kPiece ? n : lo + half;
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -820,26 +920,20 @@ void HetuTable::pushPull(embed_t *grad, embed_t *dst) {
       dst_staged = true;
     }
   }
+  // Few rows for pinned host memory are written there by the expansion itself, with no copy behind it and no second
+  // expansion beside it: 3,900 x 16 (250 KB) 50.1 us, split 54.9, but 3,900 x 64 (1 MB) 81 against 78.
+  constexpr size_t kSplitBytes = (size_t)512 << 10;
   const embed_t *grad_dev = grad;
-  if (grad != nullptr && prev.batch_size > 0)
+  const bool split_expand = n == 1 && dst_mapped != nullptr && grad != nullptr && prev.batch_size > 0 &&
+                            prev.scatter_recorded && cur.batch_size > 0 && split_host_expand_ && !onDevice(grad) &&
+                            prev.batch_size * W * sizeof(embed_t) >= kSplitBytes;
+  if (grad != nullptr && prev.batch_size > 0 && !split_expand)
     grad_dev = static_cast<const embed_t *>(stageIn(grad, prev.batch_size * W * sizeof(embed_t), d_stage_grad_, stream_reduce_));
 
-  // Single rank, gradients arriving from host memory and dst in pinned host memory: the step is two transfers over
-  // the host link with a short computation between them.  The rows of dst whose keys the previous batch did not
-  // contain do not depend on the gradients, so they are written (by the kernel, straight into dst) while the
-  // gradients are still coming in, and only the other rows after the update: the two directions of the link overlap.
-  const bool split_expand = n == 1 && dst_mapped != nullptr && grad_dev != grad && prev.scatter_recorded &&
-                            cur.batch_size > 0 && split_host_expand_;
-  if (split_expand) {
+  if (split_expand || (n == 1 && dst_mapped != nullptr && !expand_bulk_ &&
+                       cur.batch_size * W * sizeof(embed_t) < kSplitBytes)) {
     dst_dev = dst_mapped;
     dst_staged = false;
-    // stream_main_ is idle here (the previous batch's dedupe ended long ago; this batch's is enqueued below) and
-    // already waits for the key ingest
-    HCTR_CUDA(cudaStreamWaitEvent(stream_main_, prev.ev_scatter, 0));
-    HCTR_LAUNCH(hctr_expand_rows_subset(cur.batch_size, W, cur.pos_row.as<int32_t>(), cur.keys.as<int64_t>(),
-                                        prev.uniq.as<int64_t>(), prev.meta.as<uint32_t>(), 0,
-                                        d_embedding_.as<float>(), dst_dev, stream_main_));
-    HCTR_CUDA(cudaEventRecord(ev_early_, stream_main_));
   } else if (dst_staged) {
     d_stage_dst_.ensure(cur.batch_size * W * sizeof(embed_t));
     dst_dev = d_stage_dst_.as<embed_t>();
@@ -861,14 +955,16 @@ void HetuTable::pushPull(embed_t *grad, embed_t *dst) {
   stats_.queried_keys = q_recv;
 
   // A. duplicate-gradient reduction + local apply + pack (generateGradient)
-  if (prev.batch_size > 0 && (n == 1 || prev.unique_size > 0)) {
+  if (split_expand) {
+    splitHostStep(cur, prev, grad, dst_dev);
+  } else if (prev.batch_size > 0 && (n == 1 || prev.unique_size > 0)) {
     // Own stream: overlaps the (still running) dedupe of the current batch.  It needs the runs of the previous batch
     // (end of its dedupe), the push decision (in front of it on this stream) and nothing else from stream_main_.
     if (prev.scatter_recorded) HCTR_CUDA(cudaStreamWaitEvent(stream_reduce_, prev.ev_scatter, 0));
     if (prev.order_recorded) HCTR_CUDA(cudaStreamWaitEvent(stream_reduce_, prev.ev_order, 0));
     prev.dedupe_in_flight = false;
     int sp = tic(kPhReduce, stream_reduce_);
-    reduceGradients(prev, grad_dev);
+    reduceGradients(prev, grad_dev, 0, prev.batch_size);
     toc(sp, stream_reduce_);
     // everything below reads rows / versions the reduction updates (a single-rank table runs it on the reduction's
     // own stream instead, and its dedupe on stream_main_ needs nothing from here)
@@ -892,10 +988,7 @@ void HetuTable::pushPull(embed_t *grad, embed_t *dst) {
       flushDedupe(cur);
     int sp = tic(kPhExpand, tail);
     if (split_expand) {
-      HCTR_LAUNCH(hctr_expand_rows_subset(cur.batch_size, W, cur.pos_row.as<int32_t>(), cur.keys.as<int64_t>(),
-                                          prev.uniq.as<int64_t>(), prev.meta.as<uint32_t>(), 1,
-                                          d_embedding_.as<float>(), dst_dev, tail));
-      HCTR_CUDA(cudaStreamWaitEvent(tail, ev_early_, 0));  // the step ends when both halves are in dst
+      // (written by splitHostStep)
     } else if (expand_bulk_) {
       HCTR_LAUNCH(hctr_expand_rows_bulk(cur.batch_size, W, cur.pos_row.as<int32_t>(), cur.idx_map.as<int32_t>(), nullptr,
                                         nullptr, d_embedding_.as<float>(), dst_dev, d_ingest_err_ + 1, tail));
@@ -1440,6 +1533,7 @@ void HetuTable::releaseAll() {
   cudaSetDevice(device_id_);
   if (stream_side_) cudaStreamSynchronize(stream_side_);
   if (stream_reduce_side_) cudaStreamSynchronize(stream_reduce_side_);
+  if (stream_pieces_) cudaStreamSynchronize(stream_pieces_);
   if (stream_reduce_) cudaStreamSynchronize(stream_reduce_);
   if (stream_main_) cudaStreamSynchronize(stream_main_);
   p2p_.reset();
@@ -1449,7 +1543,7 @@ void HetuTable::releaseAll() {
                    &d_recv_idx_, &d_err_, &d_cnt_s_, &d_cnt_r_, &d_qver_s_,
                    &d_qkey_r_, &d_qver_r_, &d_pkey_s_, &d_pupd_s_, &d_pval_s_, &d_pkey_r_, &d_pupd_r_, &d_pval_r_,
                    &d_flag_s_, &d_flag_r_, &d_flag32_, &d_ret_slot_, &d_recv_slot_, &d_seg_r_, &d_retcnt_s_,
-                   &d_retcnt_r_, &d_rver_s_, &d_rval_s_, &d_rver_r_, &d_rval_r_, &d_stage_grad_, &d_stage_dst_};
+                   &d_retcnt_r_, &d_rver_s_, &d_rval_s_, &d_rver_r_, &d_rval_r_, &d_stage_grad_, &d_stage_dst_, &d_last_seen_};
   for (DevBuf *b : all) b->release();
   for (BatchDesc *b : {&cur_batch_, &prev_batch_}) {
     if (b->ev_order) cudaEventDestroy(b->ev_order);
@@ -1480,8 +1574,14 @@ void HetuTable::releaseAll() {
   if (ev_epoch_) cudaEventDestroy(ev_epoch_);
   ev_epoch_ = nullptr;
   if (ev_keys_) cudaEventDestroy(ev_keys_);
-  if (ev_early_) cudaEventDestroy(ev_early_);
-  ev_early_ = nullptr;
+  for (cudaEvent_t *e : {&ev_early_, &ev_sizes_}) {
+    if (*e) cudaEventDestroy(*e);
+    *e = nullptr;
+  }
+  for (cudaEvent_t &e : ev_piece_) {
+    if (e) cudaEventDestroy(e);
+    e = nullptr;
+  }
   if (ev_decide_) cudaEventDestroy(ev_decide_);
   if (ev_reduce_) cudaEventDestroy(ev_reduce_);
   if (ev_rfork_) cudaEventDestroy(ev_rfork_);
@@ -1489,6 +1589,8 @@ void HetuTable::releaseAll() {
   ev_decide_ = ev_reduce_ = ev_rfork_ = ev_rjoin_ = nullptr;
   if (stream_reduce_side_) cudaStreamDestroy(stream_reduce_side_);
   stream_reduce_side_ = nullptr;
+  if (stream_pieces_) cudaStreamDestroy(stream_pieces_);
+  stream_pieces_ = nullptr;
   if (stream_reduce_) cudaStreamDestroy(stream_reduce_);
   stream_reduce_ = nullptr;
   ev_keys_ = nullptr;

@@ -79,6 +79,7 @@ struct BatchDesc {
   void *h_keys = nullptr;
   size_t h_keys_bytes = 0;
   bool h_keys_busy = false;        // an ingest kernel may still be reading it
+  bool sizes_coming = false;       // h_meta holds them once ev_sizes_ has passed (split steps of single-rank tables)
   uint32_t *h_meta = nullptr;      // pinned: the batch's meta words (sizes, segment starts, error bits) as read back
   std::vector<size_t> seg;         // [n+1] first unique of each owner
   std::vector<size_t> query_send;  // [n] unique keys addressed to each owner
@@ -189,7 +190,7 @@ class HetuTable {
   int expandRows(size_t batch, size_t width, const int32_t *pos_row, const int32_t *idx_map, const uint32_t *recv_slot,
                  const float *recv_val, const float *embedding, float *dst, uint32_t *err, cudaStream_t stream);
   void launchPushDecide(BatchDesc &b);
-  void reduceGradients(BatchDesc &b, const embed_t *grad);
+  void reduceGradients(BatchDesc &b, const embed_t *grad, size_t last_lo, size_t last_hi);
   void groupKeys(BatchDesc &b);
   void rankKeys(BatchDesc &b);
   void reserveBitmap();
@@ -204,10 +205,14 @@ class HetuTable {
   // batch on stream_main_ (they touch disjoint data); stream_main_ joins it before the first kernel that
   // reads updated rows or versions.
   cudaStream_t stream_reduce_ = nullptr;
-  cudaStream_t stream_reduce_side_ = nullptr;  // multi-rank tables: long-run reduce kernel, forked from stream_reduce_
+  cudaStream_t stream_reduce_side_ = nullptr;  // multi-rank tables: long-run reduce kernel, forked from stream_reduce_;
+                                               // single-rank tables: rows of a split step that need no gradients
+  cudaStream_t stream_pieces_ = nullptr;       // single-rank tables: gradients that come from host memory in pieces
   cudaEvent_t ev_decide_ = nullptr, ev_reduce_ = nullptr, ev_rfork_ = nullptr, ev_rjoin_ = nullptr;
   cudaEvent_t ev_keys_ = nullptr;
-  cudaEvent_t ev_early_ = nullptr;   // end of the gradient-independent half of a split row expansion
+  cudaEvent_t ev_early_ = nullptr;   // the rows of a split step that need no gradients are in dst
+  cudaEvent_t ev_sizes_ = nullptr;   // the sizes of the batch pulled by the last split step are on the host
+  cudaEvent_t ev_piece_[5] = {};     // a piece of the gradients has arrived from host memory
   bool split_host_expand_ = true;    // HCTR_SPLIT_HOST_EXPAND=0 switches the split off
   bool fused_refresh_expand_ = true; // HCTR_P2P_FUSED_EXPAND=0: cache refresh and row expansion as two launches
   std::unique_ptr<Transport> transport_;
@@ -246,6 +251,7 @@ class HetuTable {
   DevBuf d_retcnt_s_, d_retcnt_r_;
   DevBuf d_rver_s_, d_rval_s_, d_rver_r_, d_rval_r_;  // returned rows
   DevBuf d_stage_grad_, d_stage_dst_;
+  DevBuf d_last_seen_;
 
   void *h_src_ = nullptr;         // pinned staging of the per-source list descriptors
   size_t p2p_off_cap_ = 0;        // mailbox capacity d_src_off_ was filled for
@@ -254,6 +260,9 @@ class HetuTable {
   // ingest without a copy), [1] error bits of the bulk-copy expansion.
   uint32_t *h_ingest_err_ = nullptr, *d_ingest_err_ = nullptr;
   bool keys_in_use_ = false;  // the ingest kernel may still be reading the caller's key buffer
+  void splitHostStep(BatchDesc &cur, BatchDesc &prev, const embed_t *grad, embed_t *dst);
+  size_t pieceEnd(size_t i, size_t lo, size_t n) const;
+  bool worthPieces(BatchDesc &b);
   void dropBadBatch(BatchDesc &b);
   void ingestKeys(BatchDesc &b, const void *keys, size_t n, cudaStream_t s);
   size_t h_pinned_words_ = 0;

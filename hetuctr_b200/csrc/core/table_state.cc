@@ -80,7 +80,7 @@ void HetuTable::quiesce() {
       b->index_map_due = false;
     }
   }
-  for (cudaStream_t s : {stream_main_, stream_side_, stream_reduce_, stream_reduce_side_})
+  for (cudaStream_t s : {stream_main_, stream_side_, stream_reduce_, stream_reduce_side_, stream_pieces_})
     if (s) HCTR_CUDA(cudaStreamSynchronize(s));
 }
 

@@ -206,19 +206,19 @@ __global__ void __launch_bounds__(kThreads, 3) expand_rows_local(u32 batch, u32 
 // (in_prev == 0) among the unique keys of the previous batch.  The gradients of the previous batch change exactly the
 // rows of those keys, so the "is not" half can run before they are applied - while they are still on their way from
 // host memory - and the "is" half after.  prev_uniq is ascending (single owner); every lane of a group searches it
-// for the same key, which the hardware serves as one broadcast access per step.
-template <int LANES, bool VEC>
-__global__ void __launch_bounds__(kThreads) expand_rows_subset(size_t batch, size_t width, const int32_t *__restrict__ pos_row,
+// for the same key, which the hardware serves as one broadcast access per step.  Over the host link every store is a
+// transaction, so rows move in the widest elements their width allows: 53,248 x 30 644 us per step one float at a time, 287.
+template <int V, int LANES>
+__global__ void __launch_bounds__(kThreads) expand_rows_subset(size_t batch, size_t E, const int32_t *__restrict__ pos_row,
                                                                const long long *__restrict__ keys,
                                                                const long long *__restrict__ prev_uniq,
                                                                const u32 *__restrict__ prev_meta, int in_prev,
                                                                const float *__restrict__ embedding,
                                                                float *__restrict__ dst) {
-  typedef RowT<VEC> R;
+  typedef RowV<V> R;
   typedef typename R::T T;
   const size_t groups = ((size_t)gridDim.x * kThreads) / LANES;
   const unsigned gl = threadIdx.x % LANES;
-  const size_t E = R::elems(width);
   const size_t U = prev_meta[HCTR_META_UNIQUE];
   for (size_t i0 = (((size_t)blockIdx.x * kThreads + threadIdx.x) / LANES) * kExpandRows; i0 < batch;
        i0 += groups * kExpandRows) {
@@ -254,6 +254,63 @@ __global__ void __launch_bounds__(kThreads) expand_rows_subset(size_t batch, siz
   }
 }
 
+
+// Where the previous batch holds the key of each position for the last time (HCTR_NEVER: nowhere).  The search is a chain of
+// loads that hit L2: one thread per position has the most of them under way, and the passes that follow only compare.
+// (A pass that searched again for every piece made a step of 53,248 x 128 885 us instead of 875.)
+__global__ void __launch_bounds__(kThreads) last_seen_in(u32 batch, const long long *__restrict__ keys,
+                                                         const long long *__restrict__ prev_uniq,
+                                                         const u32 *__restrict__ prev_meta,
+                                                         const u32 *__restrict__ run_start,
+                                                         const u32 *__restrict__ sorted_pos, u32 *__restrict__ last_seen) {
+  const u32 U = prev_meta[HCTR_META_UNIQUE];
+  for (u32 i = blockIdx.x * kThreads + threadIdx.x; i < batch; i += gridDim.x * kThreads) {
+    const long long key = keys[i];
+    u32 lo = 0, hi = U;  // first entry >= key
+    while (lo < hi) {
+      const u32 mid = (lo + hi) >> 1;
+      if (prev_uniq[mid] < key) lo = mid + 1;
+      else hi = mid;
+    }
+    last_seen[i] = lo < U && prev_uniq[lo] == key ? sorted_pos[run_start[lo + 1] - 1] : HCTR_NEVER;
+  }
+}
+
+// Bound by the host link, where dst is; the scan over the other positions is 8 bytes each.
+// expand_rows_local for the positions with last_seen in [lo, lo + n) (modulo 2^32).
+template <int V, int LANES>
+__global__ void __launch_bounds__(kThreads, 3) expand_rows_window(u32 batch, u32 E, const int32_t *__restrict__ pos_row,
+                                                                  const u32 *__restrict__ last_seen, u32 lo, u32 n,
+                                                                  const float *__restrict__ embedding,
+                                                                  float *__restrict__ dst_f) {
+  typedef RowV<V> R;
+  typedef typename R::T T;
+  const u32 groups = gridDim.x * kThreads / LANES;
+  const unsigned gl = threadIdx.x % LANES;
+  const T *emb = reinterpret_cast<const T *>(embedding);
+  T *dst = reinterpret_cast<T *>(dst_f);
+  for (u32 i0 = ((blockIdx.x * kThreads + threadIdx.x) / LANES) * kExpandRows; i0 < batch; i0 += groups * kExpandRows) {
+    bool mine[kExpandRows];
+    int32_t row[kExpandRows];
+#pragma unroll
+    for (int k = 0; k < kExpandRows; k++) {
+      mine[k] = i0 + k < batch && last_seen[i0 + k] - lo < n;
+      row[k] = mine[k] ? pos_row[i0 + k] : HCTR_INVALID_ROW;
+    }
+    if (!(mine[0] || mine[1] || mine[2] || mine[3])) continue;
+    for (u32 c = gl; c < E; c += LANES) {
+      T v[kExpandRows];
+#pragma unroll
+      for (int k = 0; k < kExpandRows; k++) {
+        v[k] = R::zero();
+        if (row[k] >= 0) v[k] = emb[(size_t)row[k] * E + c];
+      }
+#pragma unroll
+      for (int k = 0; k < kExpandRows; k++)
+        if (mine[k]) R::st_once(dst + (size_t)(i0 + k) * E + c, v[k]);
+    }
+  }
+}
 
 // ---- expand through the bulk-copy engine ---------------------------------------------------------------
 // Each lane moves whole rows with two asynchronous bulk copies (cp.async.bulk): table (or receive-buffer) row ->
@@ -521,21 +578,49 @@ extern "C" int hctr_expand_rows_local(size_t batch, size_t width, const int32_t 
   return launch_status();
 }
 
+extern "C" int hctr_last_seen(size_t batch, const int64_t *keys, const int64_t *prev_uniq, const uint32_t *prev_meta,
+                              const uint32_t *run_start, const uint32_t *sorted_pos, uint32_t *last_seen, void *stream) {
+  if (batch == 0) return 0;
+  if (batch >= ((size_t)1 << 31)) return (int)cudaErrorInvalidValue;
+  const size_t need = (batch + kThreads - 1) / kThreads;
+  last_seen_in<<<(unsigned)(need < (size_t)kSMs * 8 ? need : (size_t)kSMs * 8), kThreads, 0, (cudaStream_t)stream>>>(
+      (u32)batch, (const long long *)keys, (const long long *)prev_uniq, prev_meta, run_start, sorted_pos, last_seen);
+  count_launches(1);
+  return launch_status();
+}
+
+extern "C" int hctr_expand_rows_window(size_t batch, size_t width, const int32_t *pos_row, const uint32_t *last_seen,
+                                       uint32_t lo, uint32_t n, const float *embedding, float *dst, void *stream) {
+  if (batch == 0) return 0;
+  if (batch >= ((size_t)1 << 31)) return (int)cudaErrorInvalidValue;
+  const uintptr_t addr = (uintptr_t)embedding | (uintptr_t)dst;
+#define CALL(V, L)                                                                                                 \
+  do {                                                                                                             \
+    const size_t need = ((batch + kExpandRows - 1) / kExpandRows * L + kThreads - 1) / kThreads;                   \
+    const unsigned g = (unsigned)(need < (size_t)kSMs * 3 ? need : (size_t)kSMs * 3);                              \
+    expand_rows_window<V, L><<<g, kThreads, 0, (cudaStream_t)stream>>>((u32)batch, (u32)(width / V), pos_row, last_seen, lo, \
+                                                                       n, embedding, dst);                         \
+  } while (0)
+  HCTR_DISPATCH_ELEMS(width, addr, CALL);
+#undef CALL
+  count_launches(1);
+  return launch_status();
+}
+
 extern "C" int hctr_expand_rows_subset(size_t batch, size_t width, const int32_t *pos_row, const int64_t *keys,
                                        const int64_t *prev_uniq, const uint32_t *prev_meta, int in_prev,
                                        const float *embedding, float *dst, void *stream) {
   cudaStream_t s = (cudaStream_t)stream;
   if (batch == 0) return 0;
-  const bool al = host_aligned16(embedding) && host_aligned16(dst);
-#define CALL(L, V)                                                                       \
-  do {                                                                                   \
-    size_t g_ = (((size_t)batch + kExpandRows - 1) / kExpandRows * L + kThreads - 1) / kThreads; \
-    const size_t cap_ = (size_t)kSMs * 3;                                                \
-    if (g_ > cap_) g_ = cap_;                                                            \
-    expand_rows_subset<L, V><<<(unsigned)g_, kThreads, 0, s>>>(                          \
-        batch, width, pos_row, (const long long *)keys, (const long long *)prev_uniq, prev_meta, in_prev, embedding, dst); \
+  const uintptr_t addr = (uintptr_t)embedding | (uintptr_t)dst;
+#define CALL(V, L)                                                                                                 \
+  do {                                                                                                             \
+    const size_t need = ((batch + kExpandRows - 1) / kExpandRows * L + kThreads - 1) / kThreads;                   \
+    const unsigned g = (unsigned)(need < (size_t)kSMs * 3 ? need : (size_t)kSMs * 3);                              \
+    expand_rows_subset<V, L><<<g, kThreads, 0, s>>>(batch, width / V, pos_row, (const long long *)keys,            \
+                                                    (const long long *)prev_uniq, prev_meta, in_prev, embedding, dst); \
   } while (0)
-  HCTR_DISPATCH_ROWS(width, al, CALL);
+  HCTR_DISPATCH_ELEMS(width, addr, CALL);
 #undef CALL
   count_launches(1);
   return launch_status();

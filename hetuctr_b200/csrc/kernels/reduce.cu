@@ -40,8 +40,16 @@ constexpr u32 kChunkMax = 64;       // positions of one chunk's short runs: 31 b
 constexpr u32 kRingBytes = 2 * kRound * 2 * 32 * 16;  // per warp: a gradient and a table row for each position in flight
 constexpr u32 kWarpBytes = kRingBytes + kChunkMax * sizeof(uint2);
 constexpr u32 kBlockBytes = kWarps * kWarpBytes;
+constexpr u32 kNoPosition = 0xffffffffu;
 static_assert(kStages * kStageRows * kSliceFloats * sizeof(float) <= kBlockBytes &&
                   kWarpStages * kWarpStageRows * kSliceFloats * sizeof(float) <= kRingBytes, "the rings share one area");
+
+// Gradients that arrive over the host link come in pieces of ascending batch positions, and a key can be summed as soon as
+// its last one is there: a launch with WINDOW takes the keys whose last position lies in [lo, hi).
+struct Window {
+  u32 lo, hi;
+  __device__ __forceinline__ bool has(u32 last) const { return last - lo < hi - lo; }
+};
 
 // More batch positions for the row's version.  Nobody else writes it: the atomic only saves waiting for the old value.
 __device__ __forceinline__ void count_updates(const hctr_local_reduce_args &a, int32_t row, u32 count) {
@@ -72,8 +80,8 @@ __device__ __forceinline__ void cp_async(void *smem, const void *gmem) {
 }
 
 // ---- very long runs ----------------------------------------------------------------------------
-template <int V>
-__device__ __forceinline__ void sum_very_long(const hctr_local_reduce_args &a, float *ring) {
+template <int V, bool WINDOW>
+__device__ __forceinline__ void sum_very_long(const hctr_local_reduce_args &a, Window win, float *ring) {
   const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const u32 W = (u32)a.width, slices = (W + kSliceFloats - 1) / kSliceFloats;
   const u32 n_tasks = a.meta[HCTR_META_NLONG] * slices;
@@ -84,6 +92,7 @@ __device__ __forceinline__ void sum_very_long(const hctr_local_reduce_args &a, f
     const u32 u = a.heavy_list[a.batch / 32 + 1 - task / slices];
     const u32 col0 = task % slices * kSliceFloats, cols = min(kSliceFloats, W - col0);
     const u32 l = a.run_start[u], len = a.run_start[u + 1] - l;
+    if (WINDOW && !win.has(a.sorted_pos[l + len - 1])) continue;  // (the same for the whole block)
     const u32 n_tiles = (len + kStageRows - 1) / kStageRows;
     // positions come two tiles at a time, one per lane: lane i has tile i / 16 of the two, row i % 16 of the warp's
     constexpr u32 kAtOnce = 32 / kRowsPerWarp;
@@ -144,12 +153,13 @@ __device__ __forceinline__ void sum_very_long(const hctr_local_reduce_args &a, f
 }
 
 // ---- long runs: one warp, 32 columns of one key -----------------------------------------------------
-template <int V>
-__device__ __forceinline__ void sum_long(const hctr_local_reduce_args &a, u32 u, u32 slice, float *ring) {
+template <int V, bool WINDOW>
+__device__ __forceinline__ void sum_long(const hctr_local_reduce_args &a, Window win, u32 u, u32 slice, float *ring) {
   const unsigned lane = threadIdx.x & 31;
   const u32 l = a.run_start[u], len = a.run_start[u + 1] - l;
   const int32_t row = a.uniq_row[u];
   if (len > HCTR_LONG_RUN) return;  // a block's work
+  if (WINDOW && !win.has(a.sorted_pos[l + len - 1])) return;
   const u32 W = (u32)a.width, col0 = slice * kSliceFloats, cols = min(kSliceFloats, W - col0);
   constexpr u32 kLanesPerRow = kSliceFloats / V, kRowsPerCopy = V;
   const unsigned sub = lane / kLanesPerRow, col = lane % kLanesPerRow * V;
@@ -230,9 +240,9 @@ __device__ __forceinline__ void load_chunk(const hctr_local_reduce_args &a, u32 
   }
 }
 
-template <int V, int LANES>
-__device__ __forceinline__ void sum_chunk(const hctr_local_reduce_args &a, u32 chunk, u32 slab, const ChunkMeta &ck,
-                                          unsigned char *smem, u64 once) {
+template <int V, int LANES, bool WINDOW>
+__device__ __forceinline__ void sum_chunk(const hctr_local_reduce_args &a, Window win, u32 chunk, u32 slab,
+                                          const ChunkMeta &ck, unsigned char *smem, u64 once) {
   typedef RowV<V> R;
   typedef typename R::T T;
   constexpr u32 kGroups = 32 / LANES;
@@ -242,7 +252,12 @@ __device__ __forceinline__ void sum_chunk(const hctr_local_reduce_args &a, u32 c
   // a chunk's last run may be a long one (any other ends inside the chunk)
   if (__any_sync(0xffffffffu, len > HCTR_LIGHT_RUN)) m--;
   if (m == 0) return;
-  if (slab == 0 && lane < m) count_updates(a, ck.row, len);
+  u32 wanted = 0xffffffffu;  // bit k: key k of the chunk is summed now
+  if (WINDOW) {
+    wanted = __ballot_sync(0xffffffffu, lane < m && win.has(a.sorted_pos[lane < m ? ck.next - 1 : 0u]));
+    if (wanted == 0) return;
+  }
+  if (slab == 0 && lane < m && (wanted >> lane & 1)) count_updates(a, ck.row, len);
   uint2 *s_row = reinterpret_cast<uint2 *>(smem + kRingBytes);
   const u32 base = __shfl_sync(0xffffffffu, ck.l, 0), P = __shfl_sync(0xffffffffu, ck.next, m - 1) - base;
   // bit p of `firsts`: a key's run starts at position p (of the P <= 63 positions of the chunk's short runs)
@@ -256,8 +271,9 @@ __device__ __forceinline__ void sum_chunk(const hctr_local_reduce_args &a, u32 c
     const u32 p = chunk * HCTR_CHUNK_POS + i * 32 + lane - base;  // (wraps to a large number in front of the base)
     const u32 key = p < P ? (u32)__popcll(firsts & ((2ull << p) - 1ull)) - 1u : 0u;
     const int32_t row = __shfl_sync(0xffffffffu, ck.row, key);
-    // {batch position, table row | last row of its key}
-    if (p < P) s_row[p] = make_uint2(ck.sp[i], (u32)row | ((u32)(lasts >> p) << 31));
+    // {batch position, table row | last row of its key}; a key that is not wanted now: no position, no last row
+    const bool now = !WINDOW || (wanted >> key & 1);
+    if (p < P) s_row[p] = now ? make_uint2(ck.sp[i], (u32)row | ((u32)(lasts >> p) << 31)) : make_uint2(kNoPosition, 0);
   }
   __syncwarp();
   // the lane groups take shares of the positions that begin and end with a key
@@ -279,6 +295,7 @@ __device__ __forceinline__ void sum_chunk(const hctr_local_reduce_args &a, u32 c
         const u32 p = p_lo + r * kRound + i;
         if (p < p_hi) {
           const uint2 w = s_row[p];
+          if (WINDOW && w.x == kNoPosition) continue;
           T *slot = mine + ((r & 1) * kRound + i) * 64;
           cp_async<V>(slot, grad + (u64)w.x * row_bytes, once);
           if ((int32_t)w.y < 0) cp_async<V>(slot + 32, emb + (u64)(w.y & 0x7fffffffu) * row_bytes);
@@ -296,6 +313,7 @@ __device__ __forceinline__ void sum_chunk(const hctr_local_reduce_args &a, u32 c
         const u32 p = p_lo + r * kRound + i;
         if (p < p_hi) {
           const T *slot = mine + ((r & 1) * kRound + i) * 64;
+          if (WINDOW && s_row[p].x == kNoPosition) continue;
           sum = R::add(sum, slot[0]);
           const u32 row = s_row[p].y;
           if ((int32_t)row < 0) {
@@ -311,11 +329,11 @@ __device__ __forceinline__ void sum_chunk(const hctr_local_reduce_args &a, u32 c
   __syncwarp();
 }
 
-template <int V, int LANES>
-__global__ void __launch_bounds__(kThreads, kResident) grad_reduce_local(hctr_local_reduce_args a) {
+template <int V, int LANES, bool WINDOW>
+__global__ void __launch_bounds__(kThreads, kResident) grad_reduce_local(hctr_local_reduce_args a, Window win) {
   extern __shared__ __align__(16) unsigned char reduce_smem[];
   const unsigned warp = threadIdx.x >> 5;
-  sum_very_long<V>(a, reinterpret_cast<float *>(reduce_smem));
+  sum_very_long<V, WINDOW>(a, win, reinterpret_cast<float *>(reduce_smem));
   __syncthreads();
   unsigned char *smem = reduce_smem + warp * kWarpBytes;
   // Long runs go to the warps of blocks that had no very long one, chunks first to warps with neither, then to those with a
@@ -328,7 +346,7 @@ __global__ void __launch_bounds__(kThreads, kResident) grad_reduce_local(hctr_lo
   const u32 n_chunks = (a.run_start[a.meta[HCTR_META_UNIQUE]] + HCTR_CHUNK_POS - 1) / HCTR_CHUNK_POS, n_pieces = n_chunks * slabs;
   const u64 once = l2_evict_first_policy();
   for (u32 t = place; t < n_long; t += n_warps)
-    sum_long<V>(a, a.heavy_list[t / slices], t % slices, reinterpret_cast<float *>(smem));
+    sum_long<V, WINDOW>(a, win, a.heavy_list[t / slices], t % slices, reinterpret_cast<float *>(smem));
   const u32 n_very = min(a.meta[HCTR_META_NLONG] * slices, gridDim.x) * kWarps;
   const u32 n_free = n_warps - n_very > n_long ? n_warps - n_very - n_long : 0u;
   u32 piece = n_free == 0 || place >= n_warps - n_very ? place : place < n_long ? n_free + place : place - n_long;
@@ -344,7 +362,7 @@ __global__ void __launch_bounds__(kThreads, kResident) grad_reduce_local(hctr_lo
     const u32 next = piece + n_warps;
     if (next < n_pieces) load_chunk(a, next / slabs, k0, k1, then);
     keys_of(next + n_warps);
-    sum_chunk<V, LANES>(a, piece / slabs, piece % slabs, now, smem, once);
+    sum_chunk<V, LANES, WINDOW>(a, win, piece / slabs, piece % slabs, now, smem, once);
     now = then;
   }
 }
@@ -353,9 +371,8 @@ __global__ void __launch_bounds__(kThreads, kResident) grad_reduce_local(hctr_lo
 
 using namespace hctr;
 
-extern "C" int hctr_grad_reduce_local(const hctr_local_reduce_args *ap, void *stream) {
-  cudaStream_t st = (cudaStream_t)stream;
-  const hctr_local_reduce_args a = *ap;
+template <bool WINDOW>
+static int launch_local(const hctr_local_reduce_args &a, Window win, cudaStream_t st) {
   if (a.batch == 0) return 0;
   // (32-bit piece and row-byte arithmetic: 2^31 positions, rows of up to 2^28 floats)
   if (a.batch >= ((size_t)1 << 31) || a.width >= ((size_t)1 << 28)) return (int)cudaErrorInvalidValue;
@@ -367,15 +384,24 @@ extern "C" int hctr_grad_reduce_local(const hctr_local_reduce_args *ap, void *st
   do {                                                                                                                 \
     static bool attr_set = false;                                                                                      \
     if (!attr_set) {                                                                                                   \
-      const cudaError_t e = cudaFuncSetAttribute(grad_reduce_local<V, L>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                                 (int)kBlockBytes);                                                    \
+      const cudaError_t e = cudaFuncSetAttribute(grad_reduce_local<V, L, WINDOW>,                                      \
+                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBlockBytes);       \
       if (e != cudaSuccess) return (int)e;                                                                             \
       attr_set = true;                                                                                                 \
     }                                                                                                                  \
-    grad_reduce_local<V, L><<<blocks, kThreads, kBlockBytes, st>>>(a);                                                 \
+    grad_reduce_local<V, L, WINDOW><<<blocks, kThreads, kBlockBytes, st>>>(a, win);                                    \
   } while (0)
   HCTR_DISPATCH_ELEMS(a.width, addr, CALL);
 #undef CALL
   count_launches(1);
   return launch_status();
+}
+
+extern "C" int hctr_grad_reduce_local(const hctr_local_reduce_args *a, void *stream) {
+  return launch_local<false>(*a, Window{}, (cudaStream_t)stream);
+}
+
+extern "C" int hctr_grad_reduce_window(const hctr_local_reduce_args *a, uint32_t last_lo, uint32_t last_hi, void *stream) {
+  if (last_lo > last_hi) return (int)cudaErrorInvalidValue;
+  return launch_local<true>(*a, Window{last_lo, last_hi}, (cudaStream_t)stream);
 }

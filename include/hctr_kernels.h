@@ -462,6 +462,8 @@ typedef struct hctr_local_reduce_args {
   int64_t *version;           /* [S] */
 } hctr_local_reduce_args;
 int hctr_grad_reduce_local(const hctr_local_reduce_args *a, void *stream);
+/* Only the keys whose last batch position is in [last_lo, last_hi): gradients of later positions need not be there yet. */
+int hctr_grad_reduce_window(const hctr_local_reduce_args *a, uint32_t last_lo, uint32_t last_hi, void *stream);
 
 /* ---------------------------------------------------------------------------------------------
  * Query generation.  Replaces lookup_version_kernel, csrc/core/generate_query.cu:91-106.
@@ -552,6 +554,14 @@ int hctr_expand_rows_local(size_t batch, size_t width, const int32_t *pos_row, c
 int hctr_expand_rows_subset(size_t batch, size_t width, const int32_t *pos_row, const int64_t *keys,
                             const int64_t *prev_uniq, const uint32_t *prev_meta, int in_prev,
                             const float *embedding, float *dst, void *stream);
+/* The same in more than two parts, for gradients that arrive in pieces.  hctr_last_seen: the batch position at which the
+ * previous batch (prev_uniq .. sorted_pos as above and from its grouping) holds each key for the last time, HCTR_NEVER where
+ * it does not.  hctr_expand_rows_window: the positions with last_seen in [lo, lo + n), counted modulo 2^32. */
+#define HCTR_NEVER 0xffffffffu
+int hctr_last_seen(size_t batch, const int64_t *keys, const int64_t *prev_uniq, const uint32_t *prev_meta,
+                   const uint32_t *run_start, const uint32_t *sorted_pos, uint32_t *last_seen, void *stream);
+int hctr_expand_rows_window(size_t batch, size_t width, const int32_t *pos_row, const uint32_t *last_seen, uint32_t lo,
+                            uint32_t n, const float *embedding, float *dst, void *stream);
 
 /* Same result through the bulk-copy engine (cp.async.bulk row -> shared memory -> dst, double-buffered per warp,
  * mbarrier completion with bounded waits: a wait that runs out sets HCTR_ERR_TIMEOUT in *err).  Needs 16-byte

@@ -145,6 +145,31 @@ def test_reduction_run_lengths(oracle_mod, width):
     gw.close()
 
 
+@pytest.mark.parametrize("width,scale", [(300, 1), (258, 1), (301, 1), (64, 4)])
+def test_host_gradients_in_pieces(oracle_mod, width, scale):
+    # gradients in pinned host memory, large enough to come in several pieces: short, long and very long runs that end
+    # in each piece, keys that span the pieces, and keys the batch before did not contain
+    from test_gpu_parity import make_worlds, run_steps
+
+    N = 9000 * scale
+    gw, ow = make_worlds(oracle_mod, 1, N, width, 0, 0, 0.1, np.zeros(N, dtype=np.uint8), [np.arange(N)],
+                         buffers="pinned", keys_on_device=False)
+    rng = np.random.RandomState(width)
+    runs = [1] * 800 * scale + [2, 3, 31, 32, 33, 64, 65, 255, 256, 257, 700]
+
+    def batch():
+        ids, parts = rng.permutation(N), []
+        for i in range(4):  # a part of the batch with keys of its own
+            part = np.repeat(ids[i * len(runs):(i + 1) * len(runs)], runs)
+            parts.append(rng.permutation(np.concatenate([part, ids[-40:]])))
+        return np.concatenate(parts)
+
+    batches = [[batch()] for _ in range(3)] + [[np.arange(N)]]
+    grads = [None] + [[rng.normal(0, 1, size=(len(b[0]), width)).astype(np.float32)] for b in batches[:-1]]
+    run_steps(gw, ow, batches, grads)
+    gw.close()
+
+
 @pytest.mark.parametrize("width", [1, 3, 4, 6, 10, 12, 50, 64, 100, 128, 132, 258])
 @pytest.mark.parametrize("batch", [1, 2, 3, 4, 5, 37, 4097, 60_001])
 def test_expand_local(batch, width):
