@@ -341,6 +341,8 @@ def run_ours(args):
         # latency-bound dedupe pipeline, whose working set lives in L2) are listed under `roofline_phases`
         kernels = {"reduce": "grad_reduce_apply_pack", "expand": "expand_rows", "owner_update": "owner_mark + owner_apply",
                    "stale_gather": "p2p_stale_gather", "dedupe": "dedupe pipeline (5 launches)"}
+        if world == 1:
+            kernels.update(reduce="grad_reduce_local", expand="expand_rows_local", dedupe="grouping (5 launches)")
         if world > 1 and per_phase.get("expand", 0.0) > 0 and per_phase.get("refresh", 0.0) == 0:
             # requester side of the mailbox exchange as one launch: the expansion plus the per-key flag look-ups of
             # the cache refresh (the refreshed rows themselves, 3D each, are not counted: their number stays on the
