@@ -797,7 +797,7 @@ void HetuTable::reduceGradients(BatchDesc &b, const embed_t *grad, size_t last_l
 //  * Large gradients come in pieces, and after each the keys that are complete with it are updated and their rows written.
 //    Each piece is half of what is left: early pieces complete few keys (the last position of a hot key is near the end
 //    of the batch).
-// 53,248 positions x 128, 30 % of them new keys: 955 us with one piece, 875 with five.  What is left is the link: the copy in
+// 53,248 positions x 128, 30 % of them new keys: 955 us with one piece, 875 with four.  What is left is the link: the copy in
 // (500 us), and after it the rows of keys whose last position is in the last piece, at the 51 GB/s a kernel stores.
 void HetuTable::splitHostStep(BatchDesc &cur, BatchDesc &prev, const embed_t *grad, embed_t *dst) {
   const size_t W = kEmbeddingWidth, n = prev.batch_size, B = cur.batch_size;
