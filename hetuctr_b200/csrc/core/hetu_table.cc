@@ -147,7 +147,7 @@ HetuTable::HetuTable(const int rank, const int nrank, const int device_id, const
       reserveBatch(*b, 1);
     }
     HCTR_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&h_ingest_err_), 64, cudaHostAllocMapped));
-    h_ingest_err_[0] = h_ingest_err_[1] = 0;
+    h_ingest_err_[0] = h_ingest_err_[1] = h_ingest_err_[2] = 0;
     HCTR_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void **>(&d_ingest_err_), h_ingest_err_, 0));
     reserveShared(1);
     h_pinned_words_ = HCTR_META_WORDS + (size_t)nrank_ + 1 + 12 * (size_t)nrank_ + 16;
@@ -271,6 +271,14 @@ void HetuTable::reserveBitmap() {
   d_blk_flag_.ensure(blocks + 1);
   HCTR_CUDA(cudaMemsetAsync(d_blk_cnt_.p, 0, d_blk_cnt_.bytes, stream_main_));
   HCTR_CUDA(cudaMemsetAsync(d_blk_flag_.p, 0, d_blk_flag_.bytes, stream_main_));
+  HCTR_CUDA(cudaStreamSynchronize(stream_main_));
+}
+
+// Brings that scratch back to rest after a ranking that broke off half-way.
+void HetuTable::clearBitmap() {
+  if (!d_bits_.p) return;
+  HCTR_CUDA(cudaStreamSynchronize(stream_side_));
+  for (DevBuf *d : {&d_bits_, &d_blk_flag_, &d_cnt_}) HCTR_CUDA(cudaMemsetAsync(d->p, 0, d->bytes, stream_main_));
   HCTR_CUDA(cudaStreamSynchronize(stream_main_));
 }
 
@@ -688,8 +696,7 @@ void HetuTable::finalizeBatch() {
     prev.push_send[p] = host_counts ? h_cnt_s[2 * p + 1] : 0;
     prev.push_recv[p] = host_counts ? h_cnt_r[2 * p + 1] : 0;
   }
-  if (err & HCTR_ERR_TIMEOUT)
-    throw std::runtime_error("preprocess: a chained scan gave up waiting for an earlier thread block");
+  if (err & HCTR_ERR_TIMEOUT) dropBrokenBatch(cur);
   if (err & HCTR_ERR_KEY_RANGE) {
     // leave a consistent (empty) batch behind, then report
     cur.batch_size = 0;
@@ -703,9 +710,17 @@ void HetuTable::finalizeBatch() {
 // them for the previous batch (dump, stats) gets them here.  stream_main_ must have drained.
 void HetuTable::finalizePrev() {
   if (!prev_batch_.pending) return;
-  const uint32_t err = readSizes(prev_batch_);
-  if (err & HCTR_ERR_TIMEOUT)
-    throw std::runtime_error("preprocess: a chained scan gave up waiting for an earlier thread block");
+  if (readSizes(prev_batch_) & HCTR_ERR_TIMEOUT) dropBrokenBatch(prev_batch_);
+}
+
+// The grouping of b gave up a wait: the device takes it for a batch without keys (HCTR_META_ERR), and so does the host from
+// here on.
+void HetuTable::dropBrokenBatch(BatchDesc &b) {
+  b.batch_size = b.unique_size = b.n_heavy = 0;
+  std::fill(b.seg.begin(), b.seg.end(), 0);
+  std::fill(b.query_send.begin(), b.query_send.end(), 0);
+  clearBitmap();
+  throw std::runtime_error("preprocess: the grouping of a batch gave up waiting for an earlier thread block");
 }
 
 void HetuTable::finalizePending() {
@@ -755,6 +770,7 @@ void HetuTable::reduceGradients(BatchDesc &b, const embed_t *grad, size_t last_l
     r.meta = b.meta.as<uint32_t>();
     r.embedding = d_embedding_.as<float>();
     r.version = d_version_.as<int64_t>();
+    r.err = d_ingest_err_ + 2;
     if (last_lo == 0 && last_hi == b.batch_size) HCTR_LAUNCH(hctr_grad_reduce_local(&r, stream_reduce_));
     else HCTR_LAUNCH(hctr_grad_reduce_window(&r, (uint32_t)last_lo, (uint32_t)last_hi, stream_reduce_));
     return;
@@ -1200,6 +1216,12 @@ void HetuTable::pushPull(embed_t *grad, embed_t *dst) {
   if (h_ingest_err_[1]) {
     h_ingest_err_[1] = 0;
     throw std::runtime_error("push_pull: the row expansion gave up waiting for a bulk copy");
+  }
+  if (h_ingest_err_[2]) {
+    h_ingest_err_[2] = 0;
+    clearBitmap();
+    throw std::runtime_error("push_pull: the gradients were not applied: the grouping of their batch gave up waiting for an "
+                             "earlier thread block (the rows pulled are those before the update)");
   }
   if (cur.pending && n > 1) {
     finalizeBatch();

@@ -194,6 +194,8 @@ class HetuTable {
   void groupKeys(BatchDesc &b);
   void rankKeys(BatchDesc &b);
   void reserveBitmap();
+  void clearBitmap();
+  void dropBrokenBatch(BatchDesc &b);
   void flushDedupe(BatchDesc &b);    // enqueues a batch's deferred dedupe pipeline (single-rank tables)
   void quiesce();  // every stream drained, pending batch sizes read back
   void exchangeP2P(embed_t *dst_dev);
@@ -257,7 +259,7 @@ class HetuTable {
   size_t p2p_off_cap_ = 0;        // mailbox capacity d_src_off_ was filled for
   uint32_t *h_pinned_ = nullptr;  // pinned mirror for counts read back from the device
   // Mapped pinned words: [0] the key ingest reports an out-of-range key through (the host reads it right after the
-  // ingest without a copy), [1] error bits of the bulk-copy expansion.
+  // ingest without a copy), [1] error bits of the bulk-copy expansion, [2] of the gradient reduction (single-rank tables).
   uint32_t *h_ingest_err_ = nullptr, *d_ingest_err_ = nullptr;
   bool keys_in_use_ = false;  // the ingest kernel may still be reading the caller's key buffer
   void splitHostStep(BatchDesc &cur, BatchDesc &prev, const embed_t *grad, embed_t *dst);

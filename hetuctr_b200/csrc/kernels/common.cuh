@@ -81,6 +81,11 @@ __device__ __forceinline__ u32 chained_cta_prefix(u64 *agg, u32 epoch, u32 cta, 
   return s_prefix;
 }
 
+// A batch whose grouping gave up a bounded wait (HCTR_ERR_TIMEOUT in its meta words) has holes in its runs and lists: to
+// everybody who reads them on the device it has no keys.
+__device__ __forceinline__ bool grouping_broke_off(const u32 *meta) { return (meta[HCTR_META_ERR] & HCTR_ERR_TIMEOUT) != 0; }
+__device__ __forceinline__ u32 unique_of(const u32 *meta) { return grouping_broke_off(meta) ? 0u : meta[HCTR_META_UNIQUE]; }
+
 // Number of lanes that cooperate on one row: W/4 float4 per row, capped at a warp, at least 1.
 // Power of two so groups tile a warp.
 static inline int lanes_per_row(size_t width) {

@@ -188,7 +188,9 @@ __global__ void __launch_bounds__(kThreads) dedupe_rank(hctr_dedupe_args a) {
 
 __global__ void __launch_bounds__(kThreads) dedupe_scatter(hctr_dedupe_args a) {
   const size_t t = (size_t)blockIdx.x * kThreads + threadIdx.x;
-  if (t >= a.batch) return;
+  // (after a wait that ran out, run starts are missing; the bitmap and the counters then stay as they are: the owner of the
+  // scratch clears them)
+  if (t >= a.batch || grouping_broke_off(a.meta)) return;
   const size_t i = mapped_pos(t, a.batch, a.stride);
   const u64 sk = a.sk[i];
   if (sk == ~0ull) {
@@ -216,7 +218,7 @@ __global__ void __launch_bounds__(kThreads) dedupe_order_light(hctr_dedupe_args 
   const unsigned lane = threadIdx.x & 31;
   const size_t warp = ((size_t)blockIdx.x * kThreads + threadIdx.x) >> 5;
   const size_t n_warps = ((size_t)gridDim.x * kThreads) >> 5;
-  const size_t U = a.meta[HCTR_META_UNIQUE];
+  const size_t U = unique_of(a.meta);
   for (size_t u0 = warp * 32; u0 < U; u0 += n_warps * 32) {
     const size_t u = u0 + lane;
     u32 l = 0, len = 0;
@@ -245,7 +247,7 @@ __global__ void __launch_bounds__(1024) dedupe_order_heavy(hctr_dedupe_args a, u
   extern __shared__ u32 win[];  // window_bits / 32 words
   __shared__ u32 warp_tot[32];
   __shared__ u32 carry;
-  const u32 n_heavy = a.meta[HCTR_META_NHEAVY];
+  const u32 n_heavy = grouping_broke_off(a.meta) ? 0u : a.meta[HCTR_META_NHEAVY];
   const unsigned tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const size_t batch = a.batch;
   for (u32 h = blockIdx.x; h < n_heavy; h += gridDim.x) {

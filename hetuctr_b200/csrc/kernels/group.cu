@@ -161,16 +161,18 @@ __device__ __forceinline__ void rank_tile(TileSmem &s, const u32 (&digit)[ITEMS]
 
 // The sorted pairs of one tile -> unique keys, runs, positions.  before(heads) returns the number of heads (first pairs
 // of a key) in the tiles in front, given the tile's own; every thread calls it.
+// broken: a pass gave up its wait, so pairs may be missing and old ones in their place - none of them is looked at, and
+// the batch comes out with no keys.
 template <int ITEMS, class F>
 __device__ __forceinline__ void finish_tile(TileSmem &s, const hctr_group_args &a, const GroupPlan &g,
-                                            const u64 *pairs, u32 tile, F before) {
+                                            const u64 *pairs, u32 tile, bool broken, F before) {
   const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const u32 n = (u32)a.batch;
   u32 sk[ITEMS], pos[ITEMS], prev[ITEMS], next[ITEMS], heads[ITEMS];
 #pragma unroll
   for (int j = 0; j < ITEMS; j++) {
     const u32 q = pair_index<ITEMS>(tile, j);
-    const u64 w = q < n ? __ldcg(pairs + q) : ((u64)g.sentinel << 32);
+    const u64 w = q < n && !broken ? __ldcg(pairs + q) : ((u64)g.sentinel << 32 | q);
     sk[j] = (u32)(w >> 32);
     pos[j] = (u32)w;
     // neighbours across the warp's edges (the others come by shuffle)
@@ -294,7 +296,7 @@ __global__ void __launch_bounds__(kTileThreads) group_cluster(hctr_group_args a,
     in = out;
     out = reinterpret_cast<u64 *>(in == reinterpret_cast<u64 *>(a.pairs0) ? a.pairs1 : a.pairs0);
   }
-  finish_tile<ITEMS>(s, a, g, in, tile, [&](u32 heads) -> u32 {
+  finish_tile<ITEMS>(s, a, g, in, tile, false, [&](u32 heads) -> u32 {
     if (tiles == 1) return 0u;
     if (tid == 0) s.heads = heads;
     sync_cluster();
@@ -386,7 +388,8 @@ __global__ void __launch_bounds__(kTileThreads) group_finish(hctr_group_args a, 
   const u64 *in = reinterpret_cast<const u64 *>(g.passes & 1 ? a.pairs0 : a.pairs1);
   if (blockIdx.x == 0)
     for (int i = threadIdx.x; i < g.passes * kMaxDigits; i += kTileThreads) a.hist[i] = 0;  // at rest again
-  finish_tile<ITEMS>(s, a, g, in, blockIdx.x, [&](u32 heads) {
+  // (the passes are over; a bit that a tile of this launch sets while others start changes nothing that they index)
+  finish_tile<ITEMS>(s, a, g, in, blockIdx.x, grouping_broke_off(a.meta), [&](u32 heads) {
     return chained_cta_prefix(reinterpret_cast<u64 *>(a.chain_scratch), a.epoch, blockIdx.x, heads,
                               &a.meta[HCTR_META_ERR]);
   });
@@ -395,7 +398,7 @@ __global__ void __launch_bounds__(kTileThreads) group_finish(hctr_group_args a, 
 // idx_map[position] = unique index, from the finished grouping (for callers that did not ask for it there)
 __global__ void __launch_bounds__(256) group_index_map(const u32 *__restrict__ meta, const u32 *__restrict__ run_start,
                                                        const u32 *__restrict__ sorted_pos, int32_t *__restrict__ idx_map) {
-  const u32 U = meta[HCTR_META_UNIQUE];
+  const u32 U = unique_of(meta);
   const u32 lane = threadIdx.x & 31, n_warps = gridDim.x * 8;
   for (u32 u = blockIdx.x * 8 + (threadIdx.x >> 5); u < U; u += n_warps)
     for (u32 q = run_start[u] + lane; q < run_start[u + 1]; q += 32) idx_map[sorted_pos[q]] = (int32_t)u;
@@ -404,6 +407,7 @@ __global__ void __launch_bounds__(256) group_index_map(const u32 *__restrict__ m
 // What hctr_group_keys leaves for the reduction, from runs that were made otherwise.
 __global__ void __launch_bounds__(256) run_chunks(u32 n, const u32 *__restrict__ run_start, u32 *__restrict__ chunk_key,
                                                   u32 *__restrict__ heavy_list, u32 *meta) {
+  if (grouping_broke_off(meta)) return;
   const u32 U = meta[HCTR_META_UNIQUE];
   for (u32 u = blockIdx.x * 256 + threadIdx.x; u <= U; u += gridDim.x * 256) {
     // chunks that begin behind the start of the key before and not behind this one's

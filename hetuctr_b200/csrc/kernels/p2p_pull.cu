@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(kPullThreads) p2p_refresh_index(hctr_p2p_ctx c
   __shared__ u32 s_flagged;
   if (threadIdx.x == 0) s_flagged = 0;
   wait_returns(c, seq, ret_base, false, blockIdx.x == 0);  // (ends with a block barrier)
-  const size_t U = meta[HCTR_META_UNIQUE];
+  const size_t U = unique_of(meta);
   const u32 *seg = meta + HCTR_META_SEG;
   const unsigned lane = threadIdx.x & 31;
   const size_t warp = ((size_t)blockIdx.x * kPullThreads + threadIdx.x) >> 5;
@@ -229,7 +229,7 @@ __global__ void __launch_bounds__(kFusedThreads) p2p_refresh_expand(hctr_p2p_ctx
   if (threadIdx.x == 0) s_flagged = s_n = 0;
   for (int i = threadIdx.x; i <= c.nrank; i += kFusedThreads) seg[i] = meta[HCTR_META_SEG + i];
   wait_returns(c, seq, ret_base, false, blockIdx.x == 0);  // (ends with a block barrier)
-  const size_t U = meta[HCTR_META_UNIQUE];
+  const size_t U = unique_of(meta);
   const unsigned lane = threadIdx.x & 31;
   const u32 E = (u32)R::elems(c.width);
   const hctr_p2p_box me = c.box[c.rank];
@@ -302,7 +302,8 @@ __global__ void __launch_bounds__(kFusedThreads) p2p_refresh_expand(hctr_p2p_ctx
         if (row >= 0 && (size_t)row >= n_cached) {
           src[k] = reinterpret_cast<const T *>(embedding) + (size_t)row * E;
         } else {
-          const int32_t u = idx_map[i];  // < 0: key was out of range (the host reports it); write zeros
+          // < 0: key was out of range, or the grouping broke off (the host reports either); write zeros
+          const int32_t u = U > 0 ? idx_map[i] : -1;
           if (u >= 0) {
             const unsigned p = uniq_owner[u];
             const u32 j = (u32)u - seg[p];

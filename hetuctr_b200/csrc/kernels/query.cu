@@ -48,7 +48,7 @@ __global__ void pack_counts(const u32 *__restrict__ meta, const u32 *__restrict_
   const int p = threadIdx.x;
   if (p < nrank) {
     const u32 *seg = meta + HCTR_META_SEG;
-    out[2 * p] = seg[p + 1] - seg[p];
+    out[2 * p] = grouping_broke_off(meta) ? 0u : seg[p + 1] - seg[p];
     out[2 * p + 1] = push_count ? push_count[p] : 0u;
   }
 }
@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(kThreads) expand_rows_subset(size_t batch, siz
   typedef typename R::T T;
   const size_t groups = ((size_t)gridDim.x * kThreads) / LANES;
   const unsigned gl = threadIdx.x % LANES;
-  const size_t U = prev_meta[HCTR_META_UNIQUE];
+  const size_t U = unique_of(prev_meta);
   for (size_t i0 = (((size_t)blockIdx.x * kThreads + threadIdx.x) / LANES) * kExpandRows; i0 < batch;
        i0 += groups * kExpandRows) {
     const T *src[kExpandRows];
@@ -263,7 +263,7 @@ __global__ void __launch_bounds__(kThreads) last_seen_in(u32 batch, const long l
                                                          const u32 *__restrict__ prev_meta,
                                                          const u32 *__restrict__ run_start,
                                                          const u32 *__restrict__ sorted_pos, u32 *__restrict__ last_seen) {
-  const u32 U = prev_meta[HCTR_META_UNIQUE];
+  const u32 U = unique_of(prev_meta);
   for (u32 i = blockIdx.x * kThreads + threadIdx.x; i < batch; i += gridDim.x * kThreads) {
     const long long key = keys[i];
     u32 lo = 0, hi = U;  // first entry >= key

@@ -333,6 +333,10 @@ template <int V, int LANES, bool WINDOW>
 __global__ void __launch_bounds__(kThreads, kResident) grad_reduce_local(hctr_local_reduce_args a, Window win) {
   extern __shared__ __align__(16) unsigned char reduce_smem[];
   const unsigned warp = threadIdx.x >> 5;
+  if (grouping_broke_off(a.meta)) {  // no runs to go by: nothing is updated, and the host hears of it
+    if (a.err && blockIdx.x == 0 && threadIdx.x == 0) *a.err = HCTR_ERR_TIMEOUT;
+    return;
+  }
   sum_very_long<V, WINDOW>(a, win, reinterpret_cast<float *>(reduce_smem));
   __syncthreads();
   unsigned char *smem = reduce_smem + warp * kWarpBytes;

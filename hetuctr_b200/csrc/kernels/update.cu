@@ -21,7 +21,7 @@ __global__ void __launch_bounds__(kThreads) push_decide(const u32 *__restrict__ 
                                                         const long long *__restrict__ pending_cnt,
                                                         long long push_bound, u32 *__restrict__ need_push) {
   const size_t u = (size_t)blockIdx.x * kThreads + threadIdx.x;
-  if (u >= meta[HCTR_META_UNIQUE]) return;
+  if (u >= unique_of(meta)) return;
   u32 need;
   const int32_t row = uniq_row[u];
   if (uniq_owner[u] == rank) need = 0;
@@ -45,7 +45,7 @@ __global__ void __launch_bounds__(kDecideThreads) push_decide_scan(const u32 *__
                                                                    u32 *__restrict__ push_slot, u64 *agg, u32 epoch,
                                                                    u32 *err) {
   __shared__ u32 warp_sums[32];
-  const size_t U = meta[HCTR_META_UNIQUE];
+  const size_t U = unique_of(meta);
   const size_t base = ((size_t)blockIdx.x * kDecideThreads + threadIdx.x) * kDecideItems;
   const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   u32 v[kDecideItems];
@@ -100,8 +100,10 @@ __global__ void push_counts(const u32 *__restrict__ meta, int nrank, const u32 *
   const int p = threadIdx.x;
   if (p < nrank) {
     const u32 *seg = meta + HCTR_META_SEG;
-    push_count[p] = push_slot[seg[p + 1]] - push_slot[seg[p]];
-    if (push_base) push_base[p] = push_slot[seg[p]];
+    const bool none = grouping_broke_off(meta);
+    const u32 first = none ? 0u : seg[p], end = none ? 0u : seg[p + 1];
+    push_count[p] = push_slot[end] - push_slot[first];
+    if (push_base) push_base[p] = push_slot[first];
   }
 }
 

@@ -173,7 +173,7 @@ typedef struct hctr_dedupe_args {
 } hctr_dedupe_args;
 
 #define HCTR_META_UNIQUE 0   /* number of unique keys U                         */
-#define HCTR_META_ERR 1      /* error word (HCTR_ERR_*)                         */
+#define HCTR_META_ERR 1      /* error word (HCTR_ERR_*); with HCTR_ERR_TIMEOUT the batch counts as one without keys */
 #define HCTR_META_NHEAVY 2   /* number of runs longer than HCTR_LIGHT_RUN       */
 #define HCTR_META_SEG 4      /* seg_start[0..nrank]: first unique of each owner */
 #define HCTR_META_NLONG 3    /* number of runs longer than HCTR_LONG_RUN (hctr_group_keys) */
@@ -460,6 +460,8 @@ typedef struct hctr_local_reduce_args {
   const uint32_t *meta;
   float *embedding;           /* [S, W] */
   int64_t *version;           /* [S] */
+  uint32_t *err;              /* null, or a word (mapped host memory or device) that receives HCTR_ERR_TIMEOUT when nothing
+                                 was updated because the batch's grouping had given up a wait */
 } hctr_local_reduce_args;
 int hctr_grad_reduce_local(const hctr_local_reduce_args *a, void *stream);
 /* Only the keys whose last batch position is in [last_lo, last_hi): gradients of later positions need not be there yet. */
