@@ -4,8 +4,11 @@
 #include <stdint.h>
 
 #include "hctr_kernels.h"
+#include "utils/per_device.h"
 
 namespace hctr {
+
+using hetuCTR::PerDevice;
 
 constexpr int kSMs = 148;  // B200: 2 dies x 74 SMs; persistent grids are sized in multiples of this
 
@@ -17,6 +20,17 @@ static inline int launch_status() { return (int)cudaGetLastError(); }
 // Kernels enqueued by this library since load (every launcher adds what it launched).
 extern unsigned long long g_launches;
 static inline void count_launches(int n) { __atomic_fetch_add(&g_launches, (unsigned long long)n, __ATOMIC_RELAXED); }
+
+// Lets `kernel` have `bytes` of dynamic shared memory on the current device; 0 or a cudaError_t.
+template <class K>
+static inline int allow_shared(PerDevice &done, K *kernel, size_t bytes) {
+  int device = -1;
+  const cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return (int)e;
+  return done.once(device, [&] {
+    return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  });
+}
 
 static inline unsigned grid_for(size_t n, unsigned block) {
   size_t g = (n + block - 1) / block;

@@ -471,13 +471,8 @@ extern "C" int hctr_dedupe_order_light(const hctr_dedupe_args *ap, void *stream)
 
 extern "C" int hctr_dedupe_order_heavy(const hctr_dedupe_args *ap, void *stream) {
   const hctr_dedupe_args a = *ap;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(dedupe_order_heavy, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         kHeavyWindowBits / 8);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+  static PerDevice allowed;
+  if (const int e = allow_shared(allowed, dedupe_order_heavy, kHeavyWindowBits / 8)) return e;
   // window = the batch when it fits (small windows let several CTAs share an SM)
   size_t wbits = (a.batch + 1023) / 1024 * 1024;
   if (wbits > (size_t)kHeavyWindowBits) wbits = kHeavyWindowBits;

@@ -455,17 +455,20 @@ static cudaLaunchConfig_t cluster_config(u32 tiles, cudaStream_t s, cudaLaunchAt
 
 // Blocks a cluster of this kernel may have here: 16 where the device places such a cluster, else the portable 8.
 static u32 cluster_blocks() {
-  static u32 most = 0;
-  if (most) return most;
-  bool big = true;
-  for (const void *k : {(const void *)group_cluster<1>, (const void *)group_cluster<2>, (const void *)group_cluster<4>})
-    big = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess && big;
-  int clusters = 0;
-  cudaLaunchAttribute at;
-  const cudaLaunchConfig_t cfg = cluster_config<4>(kMaxCluster, nullptr, &at);
-  big = big && cudaOccupancyMaxActiveClusters(&clusters, group_cluster<4>, &cfg) == cudaSuccess && clusters > 0;
-  cudaGetLastError();
-  return most = big ? kMaxCluster : 8u;
+  static PerDevice most;
+  int device = -1;
+  if (cudaGetDevice(&device) != cudaSuccess) return 8u;
+  return (u32)most.get(device, [] {
+    bool big = true;
+    for (const void *k : {(const void *)group_cluster<1>, (const void *)group_cluster<2>, (const void *)group_cluster<4>})
+      big = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess && big;
+    int clusters = 0;
+    cudaLaunchAttribute at;
+    const cudaLaunchConfig_t cfg = cluster_config<4>(kMaxCluster, nullptr, &at);
+    big = big && cudaOccupancyMaxActiveClusters(&clusters, group_cluster<4>, &cfg) == cudaSuccess && clusters > 0;
+    cudaGetLastError();
+    return big ? (int)kMaxCluster : 8;
+  });
 }
 
 template <int ITEMS>

@@ -524,12 +524,8 @@ extern "C" int hctr_expand_rows_bulk(size_t batch, size_t width, const int32_t *
   unsigned rows_per_round = (unsigned)(kBulkBufBytes / row_bytes);
   if (rows_per_round > 32) rows_per_round = 32;
   const size_t smem = (size_t)kBulkWarps * 2 * kBulkBufBytes;  // 64 KB
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(expand_rows_bulk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+  static PerDevice allowed;
+  if (const int e = allow_shared(allowed, expand_rows_bulk, smem)) return e;
   const size_t rounds = (batch + rows_per_round - 1) / rows_per_round;
   size_t ctas = (rounds + kBulkWarps - 1) / kBulkWarps;
   const size_t cap = (size_t)kSMs * 3;  // 3 blocks of 64 KB per SM

@@ -386,13 +386,8 @@ static int launch_local(const hctr_local_reduce_args &a, Window win, cudaStream_
   const unsigned blocks = (unsigned)std::min((pieces + kWarps - 1) / kWarps, (size_t)kSMs * kResident);
 #define CALL(V, L)                                                                                                     \
   do {                                                                                                                 \
-    static bool attr_set = false;                                                                                      \
-    if (!attr_set) {                                                                                                   \
-      const cudaError_t e = cudaFuncSetAttribute(grad_reduce_local<V, L, WINDOW>,                                      \
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBlockBytes);       \
-      if (e != cudaSuccess) return (int)e;                                                                             \
-      attr_set = true;                                                                                                 \
-    }                                                                                                                  \
+    static PerDevice allowed;                                                                                          \
+    if (const int e = allow_shared(allowed, grad_reduce_local<V, L, WINDOW>, kBlockBytes)) return e;                   \
     grad_reduce_local<V, L, WINDOW><<<blocks, kThreads, kBlockBytes, st>>>(a, win);                                    \
   } while (0)
   HCTR_DISPATCH_ELEMS(a.width, addr, CALL);

@@ -1193,16 +1193,11 @@ extern "C" int hctr_grad_reduce_apply_pack(const hctr_reduce_args *ap, void *str
   const bool forked = a.n_heavy > 0 && a.side_stream && a.fork_event && a.join_event;
   cudaStream_t ls = forked ? (cudaStream_t)a.side_stream : s;
   if (a.n_heavy > 0) {
-    static bool attr_set = false;
     size_t need = (size_t)kLongStages * max((size_t)kLongStageBytes, a.width * sizeof(float));
     if (need > 200 * 1024) return (int)cudaErrorInvalidValue;  // rows wider than 12800 floats
-    if (!attr_set) {
-      cudaError_t e1 = cudaFuncSetAttribute(grad_reduce_long<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-      cudaError_t e2 = cudaFuncSetAttribute(grad_reduce_long<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-      if (e1 != cudaSuccess) return (int)e1;
-      if (e2 != cudaSuccess) return (int)e2;
-      attr_set = true;
-    }
+    static PerDevice allowed[2];
+    if (const int e = allow_shared(allowed[0], grad_reduce_long<true>, 200 * 1024)) return e;
+    if (const int e = allow_shared(allowed[1], grad_reduce_long<false>, 200 * 1024)) return e;
     if (forked) {
       cudaError_t e = cudaStreamWaitEvent(ls, (cudaEvent_t)a.fork_event, 0);
       if (e != cudaSuccess) return (int)e;
@@ -1229,13 +1224,15 @@ extern "C" int hctr_grad_reduce_apply_pack(const hctr_reduce_args *ap, void *str
                                                       : grad_reduce_short_stream<2, 4, 0>;
     const int depth = variant == 0 ? 8 : variant == 1 ? 4 : 2;
     const size_t smem = (size_t)(kThreads / 32) * depth * E * sizeof(float4);  // at most 32 KB
-    static int per_sm_of[3][3] = {};  // resident thread blocks per SM, by kernel variant and ring size class
-    int &per_sm = per_sm_of[variant][smem <= 16384 ? 0 : smem <= 24576 ? 1 : 2];
-    if (per_sm == 0) {
-      cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kThreads, smem);
-      if (e != cudaSuccess) return (int)e;
-      if (per_sm < 1) per_sm = 1;
-    }
+    static PerDevice per_sm_of[3][3];  // resident thread blocks per SM, by kernel variant and ring size class
+    int device = -1;
+    cudaError_t e = cudaGetDevice(&device);
+    const int per_sm = per_sm_of[variant][smem <= 16384 ? 0 : smem <= 24576 ? 1 : 2].get(device, [&] {
+      int blocks = 0;
+      if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kernel, kThreads, smem);
+      return e != cudaSuccess ? 0 : std::max(blocks, 1);
+    });
+    if (per_sm == 0) return (int)e;
     // Equal-cost thread blocks, at most one resident round of them (one, two and three rounds measured the
     // same; a few blocks left over for another round would double the kernel's duration).  A warp should get
     // at least ~48 row transfers; every key costs at least 3, so 3U bounds the total from below.  Next to the
