@@ -12,6 +12,7 @@
 #include <mutex>
 #include <vector>
 
+#include "utils/cpu_relax.h"
 #include "utils/errors.h"
 #include "utils/rendezvous.h"
 
@@ -131,7 +132,7 @@ struct InprocWorld {
     do {
       for (int i = 0; i < 64; i++) {
         if (generation.load(std::memory_order_acquire) != gen) return;
-        __builtin_ia32_pause();
+        cpu_relax();
       }
     } while (std::chrono::steady_clock::now() < until);
     std::unique_lock<std::mutex> lk(mu);

@@ -12,6 +12,8 @@
 #include <thread>
 #include <vector>
 
+#include "utils/cpu_relax.h"
+
 namespace hetuCTR {
 
 // Looks for `ready()` for up to `us` microseconds; true when it came.  A step's calls follow each other within tens of
@@ -22,7 +24,7 @@ inline bool spin_for(int us, F ready) {
   do {
     for (int i = 0; i < 32; i++) {
       if (ready()) return true;
-      __builtin_ia32_pause();
+      cpu_relax();
     }
   } while (std::chrono::steady_clock::now() < until);
   return false;
