@@ -361,7 +361,7 @@ void HetuTable::preprocess(index_t *data_ptr, size_t batch_size) {
   profile_ = profile_every_ > 0 && (profile_step_++ % (size_t)profile_every_) == 0;
   std::swap(cur_batch_, prev_batch_);
   BatchDesc &cur = cur_batch_, &prev = prev_batch_;
-  cur.decided = false;
+  cur.decided = cur.reduced = false;
   reserveBatch(cur, std::max<size_t>(batch_size, 1));
   reserveShared(std::max<size_t>(batch_size, 1));
   if (use_p2p_) p2p_->reserve(std::max<size_t>(batch_size, 1), stream_main_);  // collective when it grows
@@ -796,7 +796,10 @@ void HetuTable::reduceGradients(BatchDesc &b, const embed_t *grad, size_t last_l
   r.push_key = d_pkey_s_.as<int64_t>();
   r.push_updates = d_pupd_s_.as<int64_t>();
   r.push_val = d_pval_s_.as<float>();
-  r.work_counter = b.meta.as<uint32_t>() + HCTR_META_WORDS + nrank_ + 1;  // cleared by the batch's key ingest
+  // the work counters are cleared by the batch's key ingest; a second push_pull for the same batch finds them used up
+  r.work_counter = b.meta.as<uint32_t>() + HCTR_META_WORDS + nrank_ + 1;
+  if (b.reduced) HCTR_CUDA(cudaMemsetAsync(r.work_counter, 0, 2 * sizeof(uint32_t), stream_reduce_));
+  b.reduced = true;
   r.p2p = use_p2p_ ? &p2p_->ctx() : nullptr;
   r.uniq_owner = b.uniq_owner.as<uint8_t>();
   r.push_base = b.push_base.as<uint32_t>();

@@ -65,6 +65,7 @@ struct BatchDesc {
   bool scatter_recorded = false;
   bool dedupe_in_flight = false;     // the dedupe was enqueued and the reduction's stream has not waited for it yet
   bool decided = false;            // the push decision for this batch has been enqueued
+  bool reduced = false;            // its gradients have been applied (multi-rank tables)
   bool dedupe_pending = false;     // the dedupe pipeline of this batch is not enqueued yet
   bool index_map_due = false;      // idx_map has not been filled (nothing but dump reads it on a single-rank table)
   DevBuf keys, idx_map, sorted_pos, uniq, uniq_owner, uniq_row, run_start, meta, pos_row, heavy, chunk_key;
