@@ -910,6 +910,7 @@ void HetuTable::pushPull(embed_t *grad, embed_t *dst) {
   BatchDesc &cur = cur_batch_, &prev = prev_batch_;
   const int n = nrank_;
   const size_t W = kEmbeddingWidth;
+  cur.decided = false;  // (a second push_pull for this batch moves the pending counts once more)
 
   // No gradient = inference step: the previous batch is dropped (all ranks must do this together).
   if (grad == nullptr) {

@@ -45,3 +45,28 @@ def test_every_call_applies_its_gradients(nrank, exchange, width):
         version, stored = gw.get(r, "version"), gw.get(r, "stored_keys")
         assert np.array_equal(version, count[stored])
     gw.close()
+
+
+@pytest.mark.parametrize("exchange", ["inproc", "p2p"])
+def test_push_decision_counts_both_calls(exchange):
+    # rank 0 caches key 5 of rank 1 and may hold back 10 updates: 4 + 4 of one batch, pushed with the 4 of the next
+    N, W = 16, 4
+    root = np.array([0] * 4 + [1] * 12, dtype=np.uint8)
+    gw = GpuWorld(2, N, W, 100, 10, 1.0, root, [np.arange(8), np.flatnonzero(root == 1)], exchange=exchange)
+    a, other = np.full(4, 5), np.array([0, 1, 2, 3])
+    g = [np.ones((4, W), dtype=np.float32), np.zeros((4, W), dtype=np.float32)]
+    held = lambda: int(gw.get(0, "updates")[np.flatnonzero(gw.get(0, "stored_keys") == 5)[0]])  # noqa: E731
+    gw.preprocess([a, other])
+    gw.push_pull(None)
+    gw.preprocess([a, other])
+    gw.push_pull(g)
+    assert held() == 4
+    gw.push_pull(g)
+    assert held() == 8
+    gw.preprocess([a, other])
+    gw.push_pull(g)  # 8 + 4 > 10
+    assert held() == 0
+    owner = np.flatnonzero(gw.get(1, "stored_keys") == 5)[0]
+    assert int(gw.get(1, "version")[owner]) == 12
+    assert np.array_equal(gw.get_f32(1, "embedding")[owner], np.full(W, -12, dtype=np.float32))
+    gw.close()
