@@ -436,8 +436,8 @@ void HetuTable::preprocess(index_t *data_ptr, size_t batch_size) {
 //  * Keys in pageable memory (and small pinned batches) are copied into pinned staging by this thread, which checks
 //    their range on the way: nothing is left to wait for, and the kernel reads the staged keys over the host link.
 //    Big batches go in chunks, so that the link works while the next chunk is being copied.
-//  * Keys the device can address - device, managed or pinned memory - are read in place and the call waits for the
-//    kernel that has read them all.
+//  * Keys the device can address - device, managed or pinned memory, at a multiple of their size - are read in place and
+//    the call waits for the kernel that has read them all.
 void HetuTable::ingestKeys(BatchDesc &b, const void *keys, size_t n, cudaStream_t s) {
   // Staging a pinned batch costs ~0.2 us per 1000 keys, waiting for the kernel to read it in place ~8 us plus the
   // transfer.
@@ -446,7 +446,7 @@ void HetuTable::ingestKeys(BatchDesc &b, const void *keys, size_t n, cudaStream_
   const unsigned meta_words = (unsigned)(HCTR_META_WORDS + nrank_ + 1 + 2);
   const int32_t *row_of = rows_are_keys_ ? nullptr : d_row_of_.as<int32_t>();
   const void *in_place = n == 0 ? nullptr : keys;
-  bool pageable = false;
+  bool pageable = false, odd = false;
   if (n > 0) {
     cudaPointerAttributes attr;
     if (cudaPointerGetAttributes(&attr, keys) != cudaSuccess) {
@@ -456,7 +456,9 @@ void HetuTable::ingestKeys(BatchDesc &b, const void *keys, size_t n, cudaStream_
     const bool pinned = attr.type == cudaMemoryTypeHost && attr.devicePointer != nullptr;
     pageable = !(attr.type == cudaMemoryTypeDevice || attr.type == cudaMemoryTypeManaged || pinned);
     if (pinned) in_place = attr.devicePointer;
-    if (pageable || (pinned && n <= kStagePinned)) {
+    // a kernel reads keys at multiples of their size only; a copy takes them from anywhere
+    odd = reinterpret_cast<uintptr_t>(keys) % sizeof(index_t) != 0;
+    if (pageable || (pinned && (odd || n <= kStagePinned))) {
       const bool narrow = kEmbeddingIDMax <= ((size_t)1 << 31);
       const size_t each = narrow ? sizeof(int32_t) : sizeof(int64_t);
       if (b.h_keys_busy) HCTR_CUDA(cudaEventSynchronize(ev_keys_));
@@ -495,7 +497,7 @@ void HetuTable::ingestKeys(BatchDesc &b, const void *keys, size_t n, cudaStream_
       // a multi-rank table takes the whole batch to the dedupe, which reports the key at the end of the step
     }
   }
-  if (pageable) {
+  if (pageable || odd) {
     HCTR_CUDA(cudaMemcpyAsync(b.keys.p, keys, sizeof(index_t) * n, cudaMemcpyDefault, s));
     in_place = b.keys.p;
   }
@@ -936,7 +938,9 @@ void HetuTable::pushPull(embed_t *grad, embed_t *dst) {
       attr.type = cudaMemoryTypeUnregistered;
     }
     if (!(attr.type == cudaMemoryTypeDevice || attr.type == cudaMemoryTypeManaged)) {
-      dst_mapped = attr.type == cudaMemoryTypeHost ? static_cast<embed_t *>(attr.devicePointer) : nullptr;
+      // (kernels store rows there, which takes an address that is a multiple of a float's size)
+      const bool odd = reinterpret_cast<uintptr_t>(dst) % sizeof(embed_t) != 0;
+      dst_mapped = attr.type == cudaMemoryTypeHost && !odd ? static_cast<embed_t *>(attr.devicePointer) : nullptr;
       dst_staged = true;
     }
   }

@@ -1,5 +1,7 @@
 #include "utils/stage_keys.h"
 
+#include <cstring>
+
 #if defined(__x86_64__)
 #include <immintrin.h>
 #endif
@@ -16,7 +18,8 @@ __attribute__((optimize("O3"))) bool copy_checked(const int64_t *__restrict__ sr
   const uint64_t last = (uint64_t)length - 1;
   uint64_t bad = 0;
   for (size_t i = 0; i < n; i++) {
-    const uint64_t k = (uint64_t)src[i];
+    uint64_t k;
+    std::memcpy(&k, src + i, sizeof(k));  // (keys may stand at any address)
     bad |= k | (last - k);
     dst[i] = (T)k;
   }
