@@ -748,6 +748,12 @@ static bool onDevice(const void *ptr) {
   return attr.type == cudaMemoryTypeDevice || attr.type == cudaMemoryTypeManaged;
 }
 
+// Rows of a split step are written while gradients are still read.
+static bool overlap(const embed_t *a, size_t na, const embed_t *b, size_t nb) {
+  const uintptr_t a0 = reinterpret_cast<uintptr_t>(a), b0 = reinterpret_cast<uintptr_t>(b);
+  return a0 < b0 + nb * sizeof(embed_t) && b0 < a0 + na * sizeof(embed_t);
+}
+
 const void *HetuTable::stageIn(const void *ptr, size_t bytes, DevBuf &buf, cudaStream_t st) {
   if (onDevice(ptr)) return ptr;
   buf.ensure(bytes);
@@ -950,7 +956,8 @@ void HetuTable::pushPull(embed_t *grad, embed_t *dst) {
   const embed_t *grad_dev = grad;
   const bool split_expand = n == 1 && dst_mapped != nullptr && grad != nullptr && prev.batch_size > 0 &&
                             prev.scatter_recorded && cur.batch_size > 0 && split_host_expand_ && !onDevice(grad) &&
-                            prev.batch_size * W * sizeof(embed_t) >= kSplitBytes;
+                            prev.batch_size * W * sizeof(embed_t) >= kSplitBytes &&
+                            !overlap(grad, prev.batch_size * W, dst, cur.batch_size * W);
   if (grad != nullptr && prev.batch_size > 0 && !split_expand)
     grad_dev = static_cast<const embed_t *>(stageIn(grad, prev.batch_size * W * sizeof(embed_t), d_stage_grad_, stream_reduce_));
 

@@ -1,5 +1,5 @@
 """Keys, gradients and rows in host memory that is laid out in unusual ways: at addresses that are no multiple of an
-element's size (fields of a packed record)."""
+element's size (fields of a packed record), or rows that take the gradients' place."""
 import numpy as np
 import pytest
 
@@ -61,4 +61,27 @@ def test_device_keys_at_an_odd_address(n):
     t.preprocess(raw.data_ptr() + 4, n)
     t.push_pull(None, out)
     assert np.array_equal(out.cpu().numpy(), emb[keys])
+    t.close()
+
+
+@pytest.mark.parametrize("n,width", [(300, 16), (4000, 64), (20_000, 128)])  # copied, split in two, in pieces
+@pytest.mark.parametrize("shift", [0, 7, -3000])
+def test_rows_take_the_place_of_the_gradients(n, width, shift):
+    # one pinned buffer for both directions, the rows `shift` floats behind the gradients
+    rows = 3000
+    t, emb = _table(rows, width)
+    rng = np.random.RandomState(n)
+    pinned = torch.zeros(n * width + 8000).pin_memory()
+    buf, at = pinned.numpy(), 4000
+    batch = None
+    for step in range(4):
+        keys = rng.randint(rows, size=n) if step % 2 else rng.randint(rows // 2, size=n)
+        grad = rng.randint(-4, 5, size=(n, width)).astype(np.float32)
+        buf[at:at + n * width] = grad.reshape(-1)
+        t.preprocess(keys, n)
+        t.push_pull(pinned.data_ptr() + 4 * at if step else None, pinned.data_ptr() + 4 * (at + shift))
+        if step:
+            np.add.at(emb, batch, -grad)
+        assert np.array_equal(buf[at + shift:at + shift + n * width].reshape(n, width), emb[keys])
+        batch = keys
     t.close()
