@@ -231,6 +231,7 @@ class HetuTable {
   bool key_stride_known_ = false;
   void detectKeyStride(const BatchDesc &b);
   bool batch_open_ = false;          // preprocess done, push_pull not yet
+  bool serving_ = false;             // the last push_pull brought no gradients (single-rank tables)
   bool prev_push_valid_ = false;     // prev_batch_'s push counts describe a push of this step
 
   // table state
@@ -267,6 +268,7 @@ class HetuTable {
   size_t pieceEnd(size_t i, size_t lo, size_t n) const;
   bool worthPieces(BatchDesc &b);
   void dropBadBatch(BatchDesc &b);
+  void reserveStaging(BatchDesc &b, size_t bytes, size_t each);
   void ingestKeys(BatchDesc &b, const void *keys, size_t n, cudaStream_t s);
   size_t h_pinned_words_ = 0;
 
