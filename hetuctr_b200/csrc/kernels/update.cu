@@ -1186,10 +1186,12 @@ extern "C" int hctr_grad_reduce_apply_pack(const hctr_reduce_args *ap, void *str
   // `long_per_sm` blocks per SM, the short-run kernel then fills what is left of every SM: launched the other way
   // round, the short-run kernel's single resident round of blocks occupies all SMs and the long runs only start
   // when it ends.
-  // A multi-rank table runs the dedupe of the next batch beside this reduction, and both are on the step's critical
-  // path: two short-run blocks per SM leave its small kernels room (config 2, two GPUs: 0.314 ms per step against
-  // 0.323 with three blocks and 0.369 with one; the dedupe 108 against 122 us, the reduction 113 against 120 us).
-  const int long_per_sm = 1, short_cap = 3;
+  // The grouping of the next batch runs beside this reduction, and both are on the step's critical path: two short-run
+  // blocks per SM leave its kernels room.  One process per GPU, two GPUs, 212,992 x 128 each, when the next batch was
+  // ranked through the bitmap: 0.314 ms per step against 0.323 with three blocks and 0.369 with one (its ranking 108
+  // against 122 us, this reduction 113 against 120).  Two ranks that share a GPU do not tell two from three up to there
+  // (13,312 to 212,992 x 128, 53,248 x 256: within 2 %); at 425,984 x 128 three are 2 to 6 % faster (525 us).
+  const int long_per_sm = 1, short_cap = 2;
   const bool forked = a.n_heavy > 0 && a.side_stream && a.fork_event && a.join_event;
   cudaStream_t ls = forked ? (cudaStream_t)a.side_stream : s;
   if (a.n_heavy > 0) {
@@ -1234,9 +1236,11 @@ extern "C" int hctr_grad_reduce_apply_pack(const hctr_reduce_args *ap, void *str
     });
     if (per_sm == 0) return (int)e;
     // Equal-cost thread blocks, at most one resident round of them (one, two and three rounds measured the
-    // same; a few blocks left over for another round would double the kernel's duration).  A warp should get
-    // at least ~48 row transfers; every key costs at least 3, so 3U bounds the total from below.  Next to the
-    // long-run kernel the round is one block per SM smaller.
+    // same; a few blocks left over for another round would double the kernel's duration).  A warp should get at
+    // least ~16 row transfers; every key costs at least 3, so 3U bounds the total from below.  (At least 48 left SMs
+    // idle in small batches: two ranks on one GPU, 13,312 x 128 124 us per step against 115, 26,624 x 128 140 against
+    // 133, 53,248 x 256 220 against 208; no difference from 106,496 on.)  Next to the long-run kernel an SM takes
+    // short_cap of its blocks at most.
     const size_t slots = (size_t)kSMs * (forked ? std::min(per_sm, short_cap) : per_sm);
     const size_t wanted = (3 * a.n_unique / 16 * 32 + kThreads - 1) / kThreads + 1;
     const size_t ctas = std::min(wanted, slots);
