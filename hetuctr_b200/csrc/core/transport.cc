@@ -2,6 +2,7 @@
 
 #include <nccl.h>
 
+#include <algorithm>
 #include <atomic>
 #include <chrono>
 #include <condition_variable>
@@ -12,9 +13,9 @@
 #include <mutex>
 #include <vector>
 
-#include "utils/cpu_relax.h"
 #include "utils/errors.h"
 #include "utils/rendezvous.h"
+#include "utils/spin.h"
 
 namespace hetuCTR {
 
@@ -128,13 +129,7 @@ struct InprocWorld {
     }
     // The ranks of a step arrive within microseconds of each other, less than it takes to wake a sleeping thread: look for
     // a while before going to sleep.
-    const auto until = std::chrono::steady_clock::now() + std::chrono::microseconds(100);
-    do {
-      for (int i = 0; i < 64; i++) {
-        if (generation.load(std::memory_order_acquire) != gen) return;
-        cpu_relax();
-      }
-    } while (std::chrono::steady_clock::now() < until);
+    if (spin_for(100, std::max(nrank, queue_workers() + 1), [&] { return generation.load(std::memory_order_acquire) != gen; })) return;
     std::unique_lock<std::mutex> lk(mu);
     // a rank that never arrives must not hang the others forever
     if (!cv.wait_for(lk, std::chrono::seconds(120), [&] { return generation != gen; }))

@@ -12,33 +12,20 @@
 #include <thread>
 #include <vector>
 
-#include "utils/cpu_relax.h"
+#include "utils/spin.h"
 
 namespace hetuCTR {
 
-// Looks for `ready()` for up to `us` microseconds; true when it came.  A step's calls follow each other within tens of
-// microseconds, and waking a thread that went to sleep in between costs about ten.
-template <class F>
-inline bool spin_for(int us, F ready) {
-  const auto until = std::chrono::steady_clock::now() + std::chrono::microseconds(us);
-  do {
-    for (int i = 0; i < 32; i++) {
-      if (ready()) return true;
-      cpu_relax();
-    }
-  } while (std::chrono::steady_clock::now() < until);
-  return false;
-}
-
 // Waits for the result of a queued call, awake for the time a step takes; rethrows a failure of the call.
 inline void wait_awake(std::future<void> &f) {
-  spin_for(1000, [&] { return f.wait_for(std::chrono::seconds(0)) == std::future_status::ready; });
+  spin_for(1000, queue_workers() + 1, [&] { return f.wait_for(std::chrono::seconds(0)) == std::future_status::ready; });
   f.get();
 }
 
 class ThreadPool {
  public:
   explicit ThreadPool(size_t n) {
+    queue_workers() += (int)n;
     for (size_t i = 0; i < n; i++) workers_.emplace_back([this] { run(); });
   }
   ~ThreadPool() {
@@ -48,6 +35,7 @@ class ThreadPool {
     }
     cv_.notify_all();
     for (auto &t : workers_) t.join();
+    queue_workers() -= (int)workers_.size();
   }
   std::future<void> Enqueue(std::function<void()> fn) {
     std::packaged_task<void()> task(std::move(fn));
@@ -66,7 +54,8 @@ class ThreadPool {
   void run() {
     for (;;) {
       std::packaged_task<void()> task;
-      spin_for(100, [&] { return queued_.load(std::memory_order_acquire) != 0; });
+      // a step's calls follow each other within tens of microseconds
+      spin_for(100, queue_workers() + 1, [&] { return queued_.load(std::memory_order_acquire) != 0; });
       {
         std::unique_lock<std::mutex> lk(mu_);
         cv_.wait(lk, [this] { return stop_ || !queue_.empty(); });
