@@ -45,7 +45,7 @@ inline std::atomic<int> &queue_workers() {
 // Looks for `ready()` for up to `us` microseconds; true when it came.  A thread that waits awake must not keep from its work
 // whoever it waits for:
 //  * the `threads` that run together (waiting ones among them) have a processor each, or all of them sleep;
-//  * a thread whose processor has been given to somebody else since it last waited sleeps the next 64 times.
+//  * a thread whose processor has been given to somebody else meanwhile - it looks every 16 waits - sleeps 64 times.
 // Two and four ranks of 53,248 x 128 in one process and the thread that waits for them, us per pass, always awake (100 to
 // 1000 us) -> so -> always asleep (an earlier build, 100 us slower elsewhere):
 //   16 free processors       163 / 305 -> 166 / 305 -> 270 / 410       (3 threads / 5 threads)
@@ -53,17 +53,25 @@ inline std::atomic<int> &queue_workers() {
 //   16, all computing       1600 / 2200 -> 480..760 / 730..1330 -> 670..830 / 1530..1790
 template <class F>
 inline bool spin_for(int us, int threads, F ready) {
+  static thread_local int processors_here = 1, looks = 0, asleep = 0;
   static thread_local long pushed = 0;
-  static thread_local int asleep = 0;
   if (ready()) return true;
-  if (threads > processors()) return false;
-  const long seen = pushed_aside();
-  if (seen != pushed) asleep = 64;
-  pushed = seen;
   if (asleep > 0) {
     asleep--;
     return false;
   }
+  if (looks-- == 0) {  // (two system calls)
+    looks = 15;
+    processors_here = processors();
+    const long seen = pushed_aside();
+    if (seen != pushed) {
+      pushed = seen;
+      asleep = 63;
+      looks = 0;
+      return false;
+    }
+  }
+  if (threads > processors_here) return false;
   const auto until = std::chrono::steady_clock::now() + std::chrono::microseconds(us);
   do {
     for (int i = 0; i < 32; i++) {
