@@ -3,8 +3,9 @@
 // Mirrors the reference's class of the same name (csrc/core/hetu_gpu_table.h:21-145): same
 // constructor arguments, same preprocess()/pushPull() call pattern and semantics, one table per
 // process/GPU.  The implementation underneath is new: all GPU work goes through the C-ABI launchers
-// of hctr_kernels.h, the key->row map is a dense array instead of a managed-memory hash map, and the
-// exchanges are packed into three NCCL groups per step with one mid-step host synchronisation.
+// of hctr_kernels.h and the key->row map is a dense array instead of a managed-memory hash map.  Ranks
+// exchange through each other's mailboxes in peer memory, with every count on the device; where peer
+// memory cannot be mapped, through three NCCL groups per step with one host synchronisation in between.
 #pragma once
 #include <cuda_runtime.h>
 #include <cstdint>
@@ -101,7 +102,7 @@ struct StepStats {  // sizes of the last push_pull, for roofline arithmetic
 // Phases timed with CUDA events on the table's stream when profiling is enabled.
 enum Phase {
   kPhDedupe = 0,      // hctr_dedupe_map
-  kPhPushDecide,      // hctr_push_decide
+  kPhPushDecide,      // hctr_push_decide_fused
   kPhReduce,          // hctr_grad_reduce_apply_pack
   kPhQuery,           // hctr_query_versions
   kPhExchange,        // transport groups (all of a step)

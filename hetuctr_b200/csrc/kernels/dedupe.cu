@@ -459,7 +459,7 @@ extern "C" int hctr_dedupe_map(const hctr_dedupe_args *ap, void *stream) {
   return hctr_dedupe_order(ap, stream);
 }
 
-extern "C" int hctr_dedupe_order_light(const hctr_dedupe_args *ap, void *stream) {
+static int order_light(const hctr_dedupe_args *ap, void *stream) {
   const hctr_dedupe_args a = *ap;
   size_t ctas = ((a.batch + 31) / 32 * 32 + kThreads - 1) / kThreads;  // one warp per 32 unique keys
   if (ctas > (size_t)kSMs * 8) ctas = (size_t)kSMs * 8;
@@ -469,7 +469,7 @@ extern "C" int hctr_dedupe_order_light(const hctr_dedupe_args *ap, void *stream)
   return launch_status();
 }
 
-extern "C" int hctr_dedupe_order_heavy(const hctr_dedupe_args *ap, void *stream) {
+static int order_heavy(const hctr_dedupe_args *ap, void *stream) {
   const hctr_dedupe_args a = *ap;
   static PerDevice allowed;
   if (const int e = allow_shared(allowed, dedupe_order_heavy, kHeavyWindowBits / 8)) return e;
@@ -487,6 +487,6 @@ extern "C" int hctr_dedupe_order_heavy(const hctr_dedupe_args *ap, void *stream)
 }
 
 extern "C" int hctr_dedupe_order(const hctr_dedupe_args *ap, void *stream) {
-  const int rc = hctr_dedupe_order_light(ap, stream);
-  return rc ? rc : hctr_dedupe_order_heavy(ap, stream);
+  const int rc = order_light(ap, stream);
+  return rc ? rc : order_heavy(ap, stream);
 }

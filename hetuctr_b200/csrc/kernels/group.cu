@@ -43,7 +43,6 @@ struct TileSmem {
   u32 start[kMaxDigits];                 // where the tile's first pair of a digit goes
   u32 warp_sum[kTileWarps];
   u32 heads;                             // heads in the tile (cluster)
-  u32 misc[2];
 };
 
 struct GroupPlan {

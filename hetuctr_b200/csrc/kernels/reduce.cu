@@ -217,12 +217,13 @@ __device__ __forceinline__ void sum_long(const hctr_local_reduce_args &a, Window
 }
 
 // ---- short runs: the keys of one chunk ------------------------------------------------------------
-// What a warp must know of a chunk, one key and up to three positions per lane.
+// What a warp must know of a chunk, one key and up to two positions per lane.
+static_assert(HCTR_CHUNK_POS - 1 + HCTR_LIGHT_RUN < 64, "the short runs of a chunk end within 64 positions of its start");
 struct ChunkMeta {
   u32 m;                   // number of keys
   u32 l, next;             // start of the lane's run and of the one behind it
   int32_t row;
-  u32 sp[3];               // sorted_pos[32 chunk + lane + 32 i]
+  u32 sp[2];               // sorted_pos[32 chunk + lane + 32 i]
 };
 
 __device__ __forceinline__ void load_chunk(const hctr_local_reduce_args &a, u32 chunk, u32 k0, u32 k1, ChunkMeta &c) {
@@ -232,7 +233,7 @@ __device__ __forceinline__ void load_chunk(const hctr_local_reduce_args &a, u32 
   c.row = 0;
   if (c.m == 0) return;
 #pragma unroll
-  for (u32 i = 0; i < 3; i++) c.sp[i] = a.sorted_pos[min(chunk * HCTR_CHUNK_POS + i * 32 + lane, (u32)a.batch - 1)];
+  for (u32 i = 0; i < 2; i++) c.sp[i] = a.sorted_pos[min(chunk * HCTR_CHUNK_POS + i * 32 + lane, (u32)a.batch - 1)];
   if (lane < c.m) {
     c.l = a.run_start[k0 + lane];
     c.next = a.run_start[k0 + lane + 1];
@@ -267,7 +268,7 @@ __device__ __forceinline__ void sum_chunk(const hctr_local_reduce_args &a, Windo
   const u64 firsts = (u64)lo | (u64)hi << 32, lasts = firsts >> 1 | 1ull << (P - 1);
   __syncwarp();
 #pragma unroll
-  for (u32 i = 0; i < 3; i++) {
+  for (u32 i = 0; i < 2; i++) {
     const u32 p = chunk * HCTR_CHUNK_POS + i * 32 + lane - base;  // (wraps to a large number in front of the base)
     const u32 key = p < P ? (u32)__popcll(firsts & ((2ull << p) - 1ull)) - 1u : 0u;
     const int32_t row = __shfl_sync(0xffffffffu, ck.row, key);

@@ -14,22 +14,6 @@ namespace hctr {
 constexpr int kThreads = 256;
 
 // ---- push decision ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kThreads) push_decide(const u32 *__restrict__ meta, int rank,
-                                                        const uint8_t *__restrict__ uniq_owner,
-                                                        const int32_t *__restrict__ uniq_row,
-                                                        const u32 *__restrict__ run_start,
-                                                        const long long *__restrict__ pending_cnt,
-                                                        long long push_bound, u32 *__restrict__ need_push) {
-  const size_t u = (size_t)blockIdx.x * kThreads + threadIdx.x;
-  if (u >= unique_of(meta)) return;
-  u32 need;
-  const int32_t row = uniq_row[u];
-  if (uniq_owner[u] == rank) need = 0;
-  else if (row < 0) need = 1;
-  else need = (pending_cnt[row] + (long long)(run_start[u + 1] - run_start[u]) <= push_bound) ? 0u : 1u;
-  need_push[u] = need;
-}
-
 // Decision + slot assignment in one launch: every CTA decides a tile of 4096 unique keys, scans the flags
 // locally and chains the tile totals (chained_cta_prefix), so need_push[] and push_slot[] (U+1 entries)
 // come out of a single kernel.
@@ -1126,23 +1110,6 @@ extern "C" int hctr_p2p_owner_update(const hctr_p2p_ctx *cp, const int32_t *row_
 #undef CALL
   count_launches(1);
   return (int)e;
-}
-
-extern "C" int hctr_push_decide(const uint32_t *meta, int nrank, int rank, size_t u_max,
-                                const uint8_t *uniq_owner, const int32_t *uniq_row, const uint32_t *run_start,
-                                const int64_t *pending_cnt, int64_t push_bound, uint32_t *need_push,
-                                uint32_t *push_slot, uint32_t *scan_scratch, uint32_t *push_count,
-                                uint32_t *push_base, void *stream) {
-  cudaStream_t s = (cudaStream_t)stream;
-  if (nrank > 1024) return (int)cudaErrorInvalidValue;
-  push_decide<<<grid_for(u_max, kThreads), kThreads, 0, s>>>(meta, rank, uniq_owner, uniq_row, run_start,
-                                                              (const long long *)pending_cnt, push_bound,
-                                                              need_push);
-  int rc = hctr_scan_exclusive_u32(need_push, push_slot, u_max, meta + HCTR_META_UNIQUE, scan_scratch, stream);
-  if (rc) return rc;
-  push_counts<<<1, 1024, 0, s>>>(meta, nrank, push_slot, push_count, push_base);
-  count_launches(2);
-  return launch_status();
 }
 
 extern "C" int hctr_push_decide_fused(const uint32_t *meta, int nrank, int rank, size_t u_max,

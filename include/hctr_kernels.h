@@ -248,10 +248,6 @@ int hctr_group_index_map(const uint32_t *meta, const uint32_t *run_start, const 
  * stream that has waited for that call's fork_event.  Nothing but the next gradient reduction (and a reader
  * of sorted_pos) needs it. */
 int hctr_dedupe_order(const hctr_dedupe_args *a, void *stream);
-/* The two halves of hctr_dedupe_order: runs of 2..HCTR_LIGHT_RUN positions (one warp per run) and longer runs
- * (a thread block per run). */
-int hctr_dedupe_order_light(const hctr_dedupe_args *a, void *stream);
-int hctr_dedupe_order_heavy(const hctr_dedupe_args *a, void *stream);
 
 /* ---------------------------------------------------------------------------------------------
  * Gradient push decision (previous batch).  Replaces decide_update_kernel + scan,
@@ -260,13 +256,15 @@ int hctr_dedupe_order_heavy(const hctr_dedupe_args *a, void *stream);
 
 /* need_push[u] = 0 if owner==rank; 1 if not stored; else pending_cnt[row] + occurrences(u) > push_bound,
  * with occurrences(u) = run_start[u+1] - run_start[u].
- * Then push_slot = exclusive scan of need_push (U+1 entries) and push_count[p] = pushes to owner p.
- * U is read from meta (device). */
-/* push_base[p] (optional output, device [nrank]) = push_slot at the first unique key of owner p. */
-int hctr_push_decide(const uint32_t *meta, int nrank, int rank, size_t u_max, const uint8_t *uniq_owner,
-                     const int32_t *uniq_row, const uint32_t *run_start, const int64_t *pending_cnt,
-                     int64_t push_bound, uint32_t *need_push, uint32_t *push_slot,
-                     uint32_t *scan_scratch, uint32_t *push_count, uint32_t *push_base, void *stream);
+ * Then push_slot = exclusive scan of need_push (U+1 entries), push_count[p] = pushes to owner p and push_base[p]
+ * (optional, [nrank]) = push_slot at the first unique key of owner p.  U is read from meta (device).  Two launches:
+ * decision, scan and slot assignment are one (tile totals chained with bounded waits, HCTR_ERR_TIMEOUT in *err).
+ * chain_scratch: hctr_scan_chained_scratch_words(u_max) words, 8-byte aligned, zero-initialised once; epoch: non-zero,
+ * different from the previous call's. */
+int hctr_push_decide_fused(const uint32_t *meta, int nrank, int rank, size_t u_max, const uint8_t *uniq_owner,
+                           const int32_t *uniq_row, const uint32_t *run_start, const int64_t *pending_cnt,
+                           int64_t push_bound, uint32_t *need_push, uint32_t *push_slot, uint32_t *chain_scratch,
+                           uint32_t epoch, uint32_t *push_count, uint32_t *push_base, uint32_t *err, void *stream);
 
 /* Packs the per-peer counts a rank announces after preprocess: out[2p] = unique keys of the current
  * batch owned by p (from meta's segment starts), out[2p+1] = push_count[p] (0 when push_count is null).
@@ -277,14 +275,6 @@ int hctr_pack_counts(const uint32_t *meta, const uint32_t *push_count, int nrank
  * Gradient aggregation + local SGD apply + pack of pushed rows (previous batch).
  * Replaces gradient_index_kernel and gradient_reduction_kernel, csrc/core/generate_query.cu:8-89.
  * ------------------------------------------------------------------------------------------- */
-
-/* Same result in two launches instead of four (decision, scan and slot assignment fused; tile totals
- * chained with bounded waits, HCTR_ERR_TIMEOUT in *err).  chain_scratch: hctr_scan_chained_scratch_words(u_max)
- * words, 8-byte aligned, zero-initialised once; epoch: non-zero, different from the previous call's. */
-int hctr_push_decide_fused(const uint32_t *meta, int nrank, int rank, size_t u_max, const uint8_t *uniq_owner,
-                           const int32_t *uniq_row, const uint32_t *run_start, const int64_t *pending_cnt,
-                           int64_t push_bound, uint32_t *need_push, uint32_t *push_slot, uint32_t *chain_scratch,
-                           uint32_t epoch, uint32_t *push_count, uint32_t *push_base, uint32_t *err, void *stream);
 
 /* ---------------------------------------------------------------------------------------------
  * Peer-to-peer exchange (one process per GPU, all GPUs of one NVLink domain).
@@ -344,12 +334,6 @@ int hctr_p2p_query_send(const hctr_p2p_ctx *c, const uint32_t *meta, size_t u_ma
  * words [0..meta_words) go to pinned (mapped) host memory in one launch: out = [5n + 7 | n | 1] words, out_meta. */
 int hctr_p2p_report(const hctr_p2p_ctx *c, const uint32_t *push_counts, const uint32_t *meta, unsigned meta_words,
                     uint32_t *out, uint32_t *out_meta, void *stream);
-
-/* Publishes this rank's counts to every peer and releases sequence number `seq` (what the last thread block of
- * hctr_p2p_query_send / hctr_p2p_stale_gather does, as a launch of its own).
- * phase 0: query count (from meta's segments) + push_count (null = zeros); phase 1: ret_count. */
-int hctr_p2p_signal(const hctr_p2p_ctx *c, int phase, uint32_t seq, const uint32_t *meta,
-                    const uint32_t *counts, void *stream);
 
 /* Waits (bounded by c->timeout_ns) until every peer has released `seq` for `phase`; copies the announced counts
  * into c->cnt_in.  On timeout sets HCTR_ERR_TIMEOUT in *c->err, records zero counts for the silent peers and
