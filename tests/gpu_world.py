@@ -6,9 +6,10 @@ threads of this process (ip="inproc") and there are two ways for them to exchang
   exchange="inproc"  the kernels of the NCCL path; bytes move between the ranks' buffers with cudaMemcpyAsync
   exchange="p2p"     the kernels of the peer-to-peer mailbox exchange, the default of a one-process-per-GPU job:
                      queries, pushed rows, flags and returned rows are stored straight into the destination rank's
-                     mailbox.  The ranks share one CUDA context here, so a peer's mailbox is a plain pointer; the
-                     table drains its stream and meets the other ranks at a host barrier between publishing and
-                     consuming, so no kernel ever waits for another launch on the same GPU.
+                     mailbox.  The ranks share one CUDA context here, so a peer's mailbox is a plain pointer; between
+                     publishing and consuming the table records an event, meets the other ranks at a host barrier
+                     and makes its stream wait for their events, so no kernel ever waits for another launch on the
+                     same GPU.
 """
 import itertools
 import os
