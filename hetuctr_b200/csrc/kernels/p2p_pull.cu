@@ -57,12 +57,15 @@ __device__ __forceinline__ V warp_compact(unsigned mask, V value) {
   return __shfl_sync(0xffffffffu, value, from < 32 ? (int)from : 0);
 }
 
-// Owner.  For every received query (flat index q over the sources' sub-regions; counts and starts were recorded
-// in c.cnt_in by the kernel that waited for them): stale = (requester's version is INT64_MIN or version +
-// pull_bound < owner's version) and the requester is not this rank (csrc/core/handle_query.cu:7-22).  The flag
-// byte goes to the requester's mailbox; a stale key's row and version follow, to row rank * cap + j of that
-// mailbox (write_return_value_kernel, csrc/core/handle_query.cu:24-40).  A warp takes 32 queries, one per lane for
-// the decision, then moves the rows of the stale ones together.  The block that finishes last releases `seq`
+// Owner.  For every query received from another rank (flat index q over the sources' sub-regions; counts and starts were
+// recorded in c.cnt_in by the kernel that waited for them): stale = (requester's version is INT64_MIN or version +
+// pull_bound < owner's version) (csrc/core/handle_query.cu:7-22; a rank's queries to itself are never stale, and nobody reads
+// a flag for them).  The flag byte goes to the requester's mailbox; a stale key's row and version follow, to row rank * cap + j
+// of that mailbox (write_return_value_kernel, csrc/core/handle_query.cu:24-40).  A warp takes up to 32 queries, one per lane
+// for the decision, then moves the rows of the stale ones together; so many that all warps of the grid have some: with 32
+// each, 26,500 queries kept 26 SMs busy.  Their addresses go through shared memory, and a power of two of lanes moves a row.
+// (Two ranks on one GPU, 53,248 x 128: 21.5 -> 18 us a launch, half of the queries a rank's own before; what is left is four
+// dependent accesses and the fences.)  The block that finishes last releases `seq`
 // (phase 1) to every peer, all2allReturnOutdated / all2allReturnValue in one, csrc/core/all2all.cu:89-130.
 template <bool VEC>
 __global__ void __launch_bounds__(kPullThreads) p2p_stale_gather(hctr_p2p_ctx c, u32 seq,
@@ -74,26 +77,35 @@ __global__ void __launch_bounds__(kPullThreads) p2p_stale_gather(hctr_p2p_ctx c,
   typedef typename R::T T;
   __shared__ u32 qstart[kMaxRanks + 1];
   __shared__ u32 s_served;
+  __shared__ const T *s_src[kPullThreads / 32][32];  // rows to move, per warp
+  __shared__ T *s_dst[kPullThreads / 32][32];
   for (int i = threadIdx.x; i <= c.nrank; i += kPullThreads) qstart[i] = c.cnt_in[3 * c.nrank + i];
   if (threadIdx.x == 0) s_served = 0;
   __syncthreads();
-  const u32 Q = qstart[c.nrank];
+  // (the queries of the others: those of this rank stand between own_at and own_at + own)
+  const u32 own_at = qstart[c.rank], own = qstart[c.rank + 1] - own_at, Q = qstart[c.nrank] - own;
   const unsigned lane = threadIdx.x & 31;
-  const size_t warp = ((size_t)blockIdx.x * kPullThreads + threadIdx.x) >> 5;
-  const size_t n_warps = ((size_t)gridDim.x * kPullThreads) >> 5;
+  const u32 warp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x, n_warps = gridDim.x * (kPullThreads / 32);
+  const u32 per = min(32u, max(4u, (Q + n_warps - 1) / n_warps));
   const u32 E = (u32)R::elems(c.width);
+  // a row is moved by the smallest power of two of lanes that covers it, at most a warp
+  const int lane_bits = E > 16 ? 5 : E > 8 ? 4 : E > 4 ? 3 : E > 2 ? 2 : E > 1 ? 1 : 0;
+  const u32 lanes = 1u << lane_bits, at_once = 32u >> lane_bits, sub = lane >> lane_bits, col0 = lane & (lanes - 1);
+  const T **src_of = s_src[threadIdx.x >> 5];
+  T **dst_of = s_dst[threadIdx.x >> 5];
   const hctr_p2p_box me = c.box[c.rank];
   u32 served = 0;
-  for (size_t q0 = warp * 32; q0 < Q; q0 += n_warps * 32) {
-    const size_t q = q0 + lane;
+  for (size_t q0 = (size_t)warp * per; q0 < Q; q0 += (size_t)n_warps * per) {
+    size_t q = q0 + lane;
     bool stale = false;
     const T *src_row = nullptr;
     T *dst_row = nullptr;
-    if (q < Q) {
+    if (lane < per && q < Q) {
+      if (q >= own_at) q += own;
       const unsigned s = segment_of(qstart, c.nrank, (u32)q);
       const u32 j = (u32)q - qstart[s];
       const size_t slot = (size_t)s * c.cap + j;
-      const long long key = me.qkey[slot];
+      const long long key = me.qkey[slot], lv = me.qver[slot];
       int32_t row = -1;
       if (key >= 0 && (size_t)key < length) row = row_of[key];
       const size_t out = (size_t)c.rank * c.cap + j;
@@ -101,8 +113,8 @@ __global__ void __launch_bounds__(kPullThreads) p2p_stale_gather(hctr_p2p_ctx c,
       if (row < 0 || (size_t)row < n_cached) {
         atomicOr(c.err, HCTR_ERR_NOT_OWNER);
       } else {
-        const long long lv = me.qver[slot], gv = version[row];
-        stale = (lv == kInvalidVersion || (long long)((u64)lv + (u64)pull_bound) < gv) && s != (unsigned)c.rank;
+        const long long gv = version[row];
+        stale = lv == kInvalidVersion || (long long)((u64)lv + (u64)pull_bound) < gv;
         if (stale) {
           b.rver[out] = gv;
           src_row = reinterpret_cast<const T *>(embedding) + (size_t)row * E;
@@ -115,9 +127,24 @@ __global__ void __launch_bounds__(kPullThreads) p2p_stale_gather(hctr_p2p_ctx c,
     if (m == 0) continue;
     const u32 cnt = __popc(m);
     served += cnt;
-    const T *sp = reinterpret_cast<const T *>(warp_compact(m, (unsigned long long)src_row));
-    T *dp = reinterpret_cast<T *>(warp_compact(m, (unsigned long long)dst_row));
-    warp_move_rows<R, false>(cnt, E, sp, nullptr, dp);
+    if (stale) {
+      const u32 place = __popc(m & ((1u << lane) - 1u));
+      src_of[place] = src_row;
+      dst_of[place] = dst_row;
+    }
+    __syncwarp();
+    for (u32 r0 = sub; r0 < cnt; r0 += kCopyUnroll * at_once) {
+      for (u32 col = col0; col < E; col += lanes) {
+        T v[kCopyUnroll];
+#pragma unroll
+        for (int k = 0; k < kCopyUnroll; k++)
+          if (r0 + k * at_once < cnt) v[k] = src_of[r0 + k * at_once][col];
+#pragma unroll
+        for (int k = 0; k < kCopyUnroll; k++)
+          if (r0 + k * at_once < cnt) dst_of[r0 + k * at_once][col] = v[k];
+      }
+    }
+    __syncwarp();
   }
   if (lane == 0 && served) atomicAdd(&s_served, served);
   __syncthreads();
@@ -172,7 +199,7 @@ __global__ void __launch_bounds__(kPullThreads) p2p_refresh_index(hctr_p2p_ctx c
       u32 idx = 0;
       if (j < c.cap) {  // (a larger j was reported when the query was sent)
         idx = p * c.cap + j;
-        f = me.flag[idx] != 0;
+        f = p != (unsigned)c.rank && me.flag[idx] != 0;
       }
       flags[u] = f ? 1 : 0;
       recv_index[u] = idx;
@@ -247,7 +274,7 @@ __global__ void __launch_bounds__(kFusedThreads) p2p_refresh_expand(hctr_p2p_ctx
       if (u < U) {
         const unsigned p = uniq_owner[u];
         const u32 j = (u32)u - seg[p];
-        if (j < c.cap) {  // (a larger j was reported when the query was sent)
+        if (p != (unsigned)c.rank && j < c.cap) {  // (a larger j was reported when the query was sent)
           const u32 idx = p * c.cap + j;
           f = me.flag[idx] != 0;
           const int32_t row = uniq_row[u];
@@ -345,8 +372,8 @@ extern "C" int hctr_p2p_stale_gather(const hctr_p2p_ctx *c, uint32_t seq, const 
                                      int64_t pull_bound, void *stream) {
   cudaStream_t st = (cudaStream_t)stream;
   if (c->nrank > kMaxRanks) return (int)cudaErrorInvalidValue;
-  // one warp per 32 queries; a publishing kernel runs one block per SM at most
-  size_t g = ((size_t)c->nrank * c->cap / 32 + 1 + kPullThreads / 32 - 1) / (kPullThreads / 32);
+  // a warp per four queries; a publishing kernel runs one block per SM at most
+  size_t g = ((size_t)c->nrank * c->cap / 4 + 1 + kPullThreads / 32 - 1) / (kPullThreads / 32);
   if (g > (size_t)kSMs) g = kSMs;
   if (g == 0) g = 1;
   const bool vec = host_aligned16(embedding) && c->width % 4 == 0;

@@ -594,19 +594,22 @@ __global__ void __launch_bounds__(kLongThreads) grad_reduce_long(ReduceKernelArg
   while (lpr > 1 && (size_t)(lpr / 2) >= E) lpr /= 2;
   const unsigned rows_per_warp_iter = 32 / lpr, sub = lane / lpr, sl = lane % lpr;
 
-  // two passes over the list: the longest runs bound the kernel's duration, so they start first
+  // Two passes over the list: the longest runs bound the kernel's duration, so they start first.  With a block per run there
+  // is nothing to draw.
+  const bool dealt = n_heavy <= gridDim.x;
   for (int pass = 0; pass < 2;) {
     __syncthreads();
-    if (tid == 0) next_item = atomicAdd(work_counter + pass, 1u);
+    if (!dealt && tid == 0) next_item = atomicAdd(work_counter + pass, 1u);
     __syncthreads();
-    const u32 h = next_item;
+    const u32 h = dealt ? (pass == 0 ? blockIdx.x : n_heavy) : next_item;
     if (h >= n_heavy) {
       pass++;
       continue;
     }
     const size_t u = a.heavy_list[h];
     const u32 l = a.run_start[u], len = a.run_start[u + 1] - l;
-    if ((len >= kVeryLongRun) != (pass == 0)) continue;
+    if (dealt) pass = 1;  // (its only one)
+    else if ((len >= kVeryLongRun) != (pass == 0)) continue;
     PushDest dest;
     const RowTarget t = reduce_bookkeeping(a, ka.p2p, u, len, tid == 0, &dest);
     // columns are processed in slabs of up to 4 per thread (width <= 1024 needs a single pass)
