@@ -114,6 +114,11 @@ HetuTable::HetuTable(const int rank, const int nrank, const int device_id, const
   for (cudaEvent_t *e : {&ev_early_, &ev_sizes_}) HCTR_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
   for (cudaEvent_t &e : ev_piece_) HCTR_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   if (const char *e = std::getenv("HCTR_SPLIT_HOST_EXPAND")) split_host_expand_ = std::atoi(e) != 0;
+  if (const char *e = std::getenv("HCTR_FOLLOW_LIMIT_US")) {
+    const long v = std::strtol(e, nullptr, 10);
+    HCTR_CHECK(v >= 0 && v <= 1000000, "HCTR_FOLLOW_LIMIT_US must be 0..1000000");
+    follow_limit_us_ = (unsigned)v;
+  }
   if (const char *e = std::getenv("HCTR_P2P_FUSED_EXPAND")) fused_refresh_expand_ = std::atoi(e) != 0;
 
   try {
@@ -148,8 +153,11 @@ HetuTable::HetuTable(const int rank, const int nrank, const int device_id, const
       reserveBatch(*b, 1);
     }
     HCTR_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&h_ingest_err_), 64, cudaHostAllocMapped));
-    h_ingest_err_[0] = h_ingest_err_[1] = h_ingest_err_[2] = 0;
+    for (int i = 0; i < 4; i++) h_ingest_err_[i] = 0;
     HCTR_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void **>(&d_ingest_err_), h_ingest_err_, 0));
+    HCTR_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&h_progress_), 64, cudaHostAllocMapped));
+    *h_progress_ = 0;
+    HCTR_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void **>(&d_progress_), h_progress_, 0));
     reserveShared(1);
     hctr_group_is_small(1);  // asks the device about clusters, once; a step would wait for the answer
     h_pinned_words_ = HCTR_META_WORDS + (size_t)nrank_ + 1 + 12 * (size_t)nrank_ + 16;
@@ -363,6 +371,7 @@ void HetuTable::preprocess(index_t *data_ptr, size_t batch_size) {
   profile_ = profile_every_ > 0 && (profile_step_++ % (size_t)profile_every_) == 0;
   std::swap(cur_batch_, prev_batch_);
   BatchDesc &cur = cur_batch_, &prev = prev_batch_;
+  settleIngest(prev);  // (no push_pull in between) its event is about to be recorded again
   cur.decided = cur.reduced = false;
   reserveBatch(cur, std::max<size_t>(batch_size, 1));
   // The other descriptor holds nothing yet on a table's first batch: the next one, which brings gradients, then has to
@@ -440,7 +449,8 @@ void HetuTable::preprocess(index_t *data_ptr, size_t batch_size) {
 // without waiting for the dedupe.  Records ev_keys_; returns when the caller's buffer may be reused.
 //  * Keys in pageable memory (and small pinned batches) are copied into pinned staging by this thread, which checks
 //    their range on the way: nothing is left to wait for, and the kernel reads the staged keys over the host link.
-//    Big batches go in chunks, so that the link works while the next chunk is being copied.
+//    On a single-rank table the kernel of a big batch is launched first and follows the copy (stageAndFollow); elsewhere big
+//    batches go in chunks with a launch each, so that the link works while the next chunk is being copied.
 //  * Keys the device can address - device, managed or pinned memory, at a multiple of their size - are read in place and
 //    the call waits for the kernel that has read them all.
 void HetuTable::ingestKeys(BatchDesc &b, const void *keys, size_t n, cudaStream_t s) {
@@ -448,6 +458,9 @@ void HetuTable::ingestKeys(BatchDesc &b, const void *keys, size_t n, cudaStream_
   // transfer.
   constexpr size_t kStagePinned = 16384;
   constexpr size_t kChunk = 65536;
+  // Launched in front of the copy, the kernel that waits for it takes 26,624 keys no earlier (36.9 us per step of x 16, 35.8
+  // with the launch behind), 53,248 6 us earlier (67 for 73 us of x 128).
+  constexpr size_t kFollow = 32768;
   const unsigned meta_words = (unsigned)(HCTR_META_WORDS + nrank_ + 1 + 2);
   const int32_t *row_of = rows_are_keys_ ? nullptr : d_row_of_.as<int32_t>();
   const void *in_place = n == 0 ? nullptr : keys;
@@ -474,8 +487,12 @@ void HetuTable::ingestKeys(BatchDesc &b, const void *keys, size_t n, cudaStream_
       void *dev = nullptr;
       HCTR_CUDA(cudaHostGetDevicePointer(&dev, b.h_keys, 0));
       const int64_t *src = static_cast<const int64_t *>(keys);
-      bool good = true;
-      for (size_t off = 0; off < n && good; off += kChunk) {
+      bool good = true, done = false;
+      if (nrank_ == 1 && n >= kFollow && n < ((size_t)1 << 31) && can_follow_) {
+        done = stageAndFollow(b, src, n, each, dev, s);
+        good = done || !can_follow_;
+      }
+      for (size_t off = 0; off < n && good && !done; off += kChunk) {
         const size_t m = std::min(kChunk, n - off);
         char *to = static_cast<char *>(b.h_keys) + off * each;
         good = narrow ? stage_keys(src + off, reinterpret_cast<int32_t *>(to), m, kEmbeddingIDMax)
@@ -493,6 +510,7 @@ void HetuTable::ingestKeys(BatchDesc &b, const void *keys, size_t n, cudaStream_
       }
       HCTR_CUDA(cudaStreamSynchronize(s));  // chunks in front of the bad one may still be on their way
       b.h_keys_busy = false;
+      h_ingest_err_[3] = 0;
       if (nrank_ == 1) dropBadBatch(b);
       // a multi-rank table takes the whole batch to the dedupe, which reports the key at the end of the step
     }
@@ -514,6 +532,55 @@ void HetuTable::ingestKeys(BatchDesc &b, const void *keys, size_t n, cudaStream_
   const bool bad = *h_ingest_err_ != 0;
   *h_ingest_err_ = 0;
   if (bad) dropBadBatch(b);  // (multi-rank tables hear of it from the dedupe, which also checks owners)
+}
+
+// Launches the ingest of n keys, then puts them into b's staging (`staged` on the device), chunk by chunk, with the kernel
+// behind.  False: a key is out of range (the kernel has been told), or launches wait for their kernels here and this one has
+// given up (can_follow_ is false from then on).  What the kernel has made of it is seen to by settleIngest.
+bool HetuTable::stageAndFollow(BatchDesc &b, const int64_t *keys, size_t n, size_t each, void *staged, cudaStream_t s) {
+  constexpr size_t kKeys = 4096;  // between two words about it: 2 us of copying
+  const uint32_t epoch = nextEpoch();
+  const int32_t *row_of = rows_are_keys_ ? nullptr : d_row_of_.as<int32_t>();
+  HCTR_LAUNCH(hctr_ingest_keys_following(staged, (int)each, b.keys.as<int64_t>(), n, b.meta.as<uint32_t>(),
+                                         (unsigned)(HCTR_META_WORDS + nrank_ + 1 + 2), row_of, kEmbeddingIDMax,
+                                         b.pos_row.as<int32_t>(), d_progress_,
+                                         reinterpret_cast<unsigned long long *>(d_err_.as<char>() + 128), epoch,
+                                         d_ingest_err_ + 3, follow_limit_us_, s));
+  if (reinterpret_cast<volatile uint32_t *>(h_ingest_err_)[3]) {  // it has run, before a single key was there
+    HCTR_CUDA(cudaStreamSynchronize(s));
+    h_ingest_err_[3] = 0;
+    can_follow_ = false;
+    return false;
+  }
+  b.h_keys_busy = b.following = true;
+  bool good = true;
+  for (size_t off = 0; off < n && good; off += kKeys) {
+    const size_t m = std::min(kKeys, n - off);
+    char *to = static_cast<char *>(b.h_keys) + off * each;
+    good = each == sizeof(int32_t) ? stage_keys(keys + off, reinterpret_cast<int32_t *>(to), m, kEmbeddingIDMax)
+                                   : stage_keys(keys + off, reinterpret_cast<int64_t *>(to), m, kEmbeddingIDMax);
+    const unsigned long long there = good ? off + m : 0xffffffffu;
+    __atomic_store_n(h_progress_, (unsigned long long)epoch << 32 | there, __ATOMIC_RELEASE);
+  }
+  if (!good) b.following = false;
+  return good;
+}
+
+// An ingest that followed the staging of batch b: did it see all of it?  Called before anything reads what it made, behind
+// launches that do not.
+void HetuTable::settleIngest(BatchDesc &b) {
+  if (!b.following) return;
+  b.following = false;
+  HCTR_CUDA(cudaEventSynchronize(ev_keys_));
+  if (!h_ingest_err_[3]) return;
+  h_ingest_err_[3] = 0;
+  const size_t each = kEmbeddingIDMax <= ((size_t)1 << 31) ? sizeof(int32_t) : sizeof(int64_t);
+  void *staged = nullptr;
+  HCTR_CUDA(cudaHostGetDevicePointer(&staged, b.h_keys, 0));
+  HCTR_LAUNCH(hctr_ingest_keys_rows(staged, (int)each, b.keys.as<int64_t>(), b.batch_size, b.meta.as<uint32_t>(),
+                                    (unsigned)(HCTR_META_WORDS + nrank_ + 1 + 2), rows_are_keys_ ? nullptr : d_row_of_.as<int32_t>(),
+                                    kEmbeddingIDMax, b.pos_row.as<int32_t>(), nullptr, stream_reduce_));
+  HCTR_CUDA(cudaEventRecord(ev_keys_, stream_reduce_));
 }
 
 void HetuTable::reserveStaging(BatchDesc &b, size_t bytes, size_t each) {
@@ -587,6 +654,7 @@ void HetuTable::launchPushDecide(BatchDesc &b) {
 void HetuTable::flushDedupe(BatchDesc &b) {
   if (!b.dedupe_pending) return;
   b.dedupe_pending = false;
+  settleIngest(b);
   if (nrank_ == 1) HCTR_CUDA(cudaStreamWaitEvent(stream_main_, ev_keys_, 0));
   b.scatter_recorded = true;
   b.dedupe_in_flight = true;
@@ -836,6 +904,7 @@ void HetuTable::reduceGradients(BatchDesc &b, const embed_t *grad, size_t last_l
 // (500 us), and after it the rows of keys whose last position is in the last piece, at the 51 GB/s a kernel stores.
 void HetuTable::splitHostStep(BatchDesc &cur, BatchDesc &prev, const embed_t *grad, embed_t *dst) {
   const size_t W = kEmbeddingWidth, n = prev.batch_size, B = cur.batch_size;
+  settleIngest(cur);
   const float *rows = d_embedding_.as<float>();
   // (rows of such a step need no staging: the gradients take the buffer that a pull without gradients has left)
   d_stage_dst_.ensure(n * W * sizeof(embed_t));
@@ -1014,6 +1083,7 @@ void HetuTable::pushPull(embed_t *grad, embed_t *dst) {
     }
   }
 
+  settleIngest(cur);  // (the reduction, on its way, has nothing to do with this batch)
   // the stream the step ends on
   cudaStream_t tail = n == 1 ? stream_reduce_ : stream_main_;
   if (n == 1) {
@@ -1605,6 +1675,8 @@ void HetuTable::releaseAll() {
   }
   if (h_ingest_err_) cudaFreeHost(h_ingest_err_);
   h_ingest_err_ = d_ingest_err_ = nullptr;
+  if (h_progress_) cudaFreeHost(h_progress_);
+  h_progress_ = d_progress_ = nullptr;
   for (BatchDesc *b : {&cur_batch_, &prev_batch_})
     for (DevBuf *d : {&b->keys, &b->idx_map, &b->sorted_pos, &b->uniq, &b->uniq_owner, &b->uniq_row,
                       &b->run_start, &b->meta, &b->pos_row, &b->heavy, &b->chunk_key, &b->need_push, &b->push_slot,

@@ -81,6 +81,7 @@ struct BatchDesc {
   void *h_keys = nullptr;
   size_t h_keys_bytes = 0;
   bool h_keys_busy = false;        // an ingest kernel may still be reading it
+  bool following = false;          // its ingest followed the staging; nobody has looked yet whether it gave up
   bool sizes_coming = false;       // h_meta holds them once ev_sizes_ has passed (split steps of single-rank tables)
   uint32_t *h_meta = nullptr;      // pinned: the batch's meta words (sizes, segment starts, error bits) as read back
   std::vector<size_t> seg;         // [n+1] first unique of each owner
@@ -262,7 +263,8 @@ class HetuTable {
   size_t p2p_off_cap_ = 0;        // mailbox capacity d_src_off_ was filled for
   uint32_t *h_pinned_ = nullptr;  // pinned mirror for counts read back from the device
   // Mapped pinned words: [0] the key ingest reports an out-of-range key through (the host reads it right after the
-  // ingest without a copy), [1] error bits of the bulk-copy expansion, [2] of the gradient reduction (single-rank tables).
+  // ingest without a copy), [1] error bits of the bulk-copy expansion, [2] of the gradient reduction (single-rank tables),
+  // [3] an ingest that follows the staging gave up.
   uint32_t *h_ingest_err_ = nullptr, *d_ingest_err_ = nullptr;
   bool keys_in_use_ = false;  // the ingest kernel may still be reading the caller's key buffer
   void splitHostStep(BatchDesc &cur, BatchDesc &prev, const embed_t *grad, embed_t *dst);
@@ -271,6 +273,11 @@ class HetuTable {
   void dropBadBatch(BatchDesc &b);
   void reserveStaging(BatchDesc &b, size_t bytes, size_t each);
   void ingestKeys(BatchDesc &b, const void *keys, size_t n, cudaStream_t s);
+  bool stageAndFollow(BatchDesc &b, const int64_t *keys, size_t n, size_t each, void *staged, cudaStream_t s);
+  void settleIngest(BatchDesc &b);
+  unsigned follow_limit_us_ = 20000;  // HCTR_FOLLOW_LIMIT_US: a thread that lost its processor for longer finds the keys ingested anew
+  unsigned long long *h_progress_ = nullptr, *d_progress_ = nullptr;  // mapped pinned: how far the staging of a batch has got
+  bool can_follow_ = true;    // launches return while their kernels run (not under tools that take launches one by one)
   size_t h_pinned_words_ = 0;
 
   BatchDesc cur_batch_, prev_batch_;

@@ -340,13 +340,82 @@ __global__ void __launch_bounds__(kThreads) ingest_keys(const long long *__restr
 // Bound: the latency of two dependent accesses (key, row), so a thread takes ITEMS independent ones; on a table of 1e8
 // keys the second one misses the address translation caches nearly every time (851,968 keys: 26 us), which a table
 // whose rows stand in key order (row_of = null) does without.
-template <class K, int ITEMS>
+//
+// FOLLOW: the keys are on their way into src, mapped host memory, while the kernel runs.  Block 0 alone looks at the host's
+// progress and passes it on in device memory, where the others wait (bounded) for their keys: every look is a round trip over
+// the host link in front of the keys' own (with a look per 1024 keys 53,248 of them came no earlier than with the launch
+// behind the copy, with one per 256 25 us later).  The launch and the link then work while the host copies: a step of 53,248 x 128 with pageable
+// keys 73 -> 67 us.
+struct Follow {
+  const u64 *progress;  // mapped host memory: epoch << 32 | keys that are there (kLost: no more will come)
+  u64 *seen;            // the same in device memory
+  u32 epoch;
+  u32 *gave_up;
+  u64 limit_ns;
+};
+constexpr u32 kLost = 0xffffffffu;
+
+__device__ __forceinline__ u64 nanoseconds() {
+  u64 t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+
+__device__ __forceinline__ void pass_progress_on(const Follow &f, u32 n) {
+  const u64 t0 = nanoseconds();
+  u32 last = 0;
+  while (last < n) {  // (kLost is not)
+    u64 v;
+    asm volatile("ld.acquire.sys.global.u64 %0, [%1];" : "=l"(v) : "l"(f.progress) : "memory");
+    u32 now = (u32)(v >> 32) == f.epoch ? (u32)v : 0u;
+    if (now == last && nanoseconds() - t0 > f.limit_ns) {
+      *f.gave_up = 1;
+      now = kLost;
+    }
+    if (now == last) continue;
+    last = now;
+    asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(f.seen), "l"((u64)f.epoch << 32 | now) : "memory");
+  }
+}
+
+// Have the first `need` keys arrived?  (Waits; the same answer for the whole block.)
+__device__ __forceinline__ bool keys_arrived(const Follow &f, u32 need) {
+  __shared__ bool here;
+  if (threadIdx.x == 0) {
+    const u64 t0 = nanoseconds();
+    u32 now = 0;
+    for (;;) {
+      u64 v;
+      asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(f.seen) : "memory");
+      now = (u32)(v >> 32) == f.epoch ? (u32)v : 0u;
+      if (now >= need) break;
+      if (nanoseconds() - t0 > 2 * f.limit_ns + 1000000) {  // (block 0 gives up long before)
+        *f.gave_up = 1;
+        now = kLost;
+        break;
+      }
+      __nanosleep(100);
+    }
+    here = now != kLost;
+  }
+  __syncthreads();
+  return here;
+}
+
+template <class K, int ITEMS, bool FOLLOW>
 __global__ void __launch_bounds__(kThreads) ingest_keys_rows(const K *src, long long *dst, size_t n,
                                                              u32 *__restrict__ meta, unsigned meta_words,
                                                              const int32_t *__restrict__ row_of, size_t length,
-                                                             int32_t *__restrict__ pos_row, u32 *err) {
-  const size_t base = (size_t)blockIdx.x * kThreads * ITEMS + threadIdx.x;
+                                                             int32_t *__restrict__ pos_row, u32 *err, Follow follow) {
   for (unsigned m = blockIdx.x * kThreads + threadIdx.x; m < meta_words; m += gridDim.x * kThreads) meta[m] = 0;
+  const size_t block = blockIdx.x - (FOLLOW ? 1 : 0), base = block * kThreads * ITEMS + threadIdx.x;
+  if (FOLLOW) {
+    if (blockIdx.x == 0) {
+      if (threadIdx.x == 0) pass_progress_on(follow, (u32)n);
+      return;
+    }
+    if (!keys_arrived(follow, (u32)min((block + 1) * kThreads * ITEMS, n))) return;
+  }
   long long k[ITEMS];
   int32_t row[ITEMS];
   bool bad = false;
@@ -385,11 +454,30 @@ static int launch_ingest(const K *src, int64_t *dst, size_t n, uint32_t *meta, u
   cudaStream_t s = (cudaStream_t)stream;
   // four keys per thread where that still leaves every SM a block
   if (n >= (size_t)kThreads * 4 * kSMs)
-    ingest_keys_rows<K, 4><<<grid_for(n, kThreads * 4), kThreads, 0, s>>>(src, (long long *)dst, n, meta, meta_words,
-                                                                         row_of, length, pos_row, err);
+    ingest_keys_rows<K, 4, false><<<grid_for(n, kThreads * 4), kThreads, 0, s>>>(
+        src, (long long *)dst, n, meta, meta_words, row_of, length, pos_row, err, Follow{});
   else
-    ingest_keys_rows<K, 1><<<grid_for(n, kThreads), kThreads, 0, s>>>(src, (long long *)dst, n, meta, meta_words,
-                                                                     row_of, length, pos_row, err);
+    ingest_keys_rows<K, 1, false><<<grid_for(n, kThreads), kThreads, 0, s>>>(
+        src, (long long *)dst, n, meta, meta_words, row_of, length, pos_row, err, Follow{});
+  count_launches(1);
+  return launch_status();
+}
+
+extern "C" int hctr_ingest_keys_following(const void *src, int key_bytes, int64_t *dst, size_t n, uint32_t *meta,
+                                          unsigned meta_words, const int32_t *row_of, size_t length, int32_t *pos_row,
+                                          const unsigned long long *progress, unsigned long long *seen, uint32_t epoch,
+                                          uint32_t *gave_up, unsigned limit_us, void *stream) {
+  cudaStream_t s = (cudaStream_t)stream;
+  constexpr int kItems = 4;
+  if (epoch == 0 || n >= ((size_t)1 << 31) || (key_bytes != 4 && key_bytes != 8)) return (int)cudaErrorInvalidValue;
+  const Follow f = {progress, seen, epoch, gave_up, (u64)limit_us * 1000};
+  const unsigned grid = grid_for(n, kThreads * kItems) + 1;
+  if (key_bytes == 8)
+    ingest_keys_rows<long long, kItems, true><<<grid, kThreads, 0, s>>>((const long long *)src, (long long *)dst, n, meta,
+                                                                        meta_words, row_of, length, pos_row, nullptr, f);
+  else
+    ingest_keys_rows<int32_t, kItems, true><<<grid, kThreads, 0, s>>>((const int32_t *)src, (long long *)dst, n, meta,
+                                                                      meta_words, row_of, length, pos_row, nullptr, f);
   count_launches(1);
   return launch_status();
 }

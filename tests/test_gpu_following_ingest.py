@@ -1,0 +1,142 @@
+"""The key ingest that is launched before its keys are staged: chunks that arrive one by one, that will not come and that do
+not come in time (the kernel then says so and returns), on caller-owned buffers; and tables whose ingest gives up, or whose
+launches wait for their kernels, against the oracle."""
+import ctypes
+import os
+import subprocess
+import sys
+
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+if not torch.cuda.is_available():
+    pytest.skip("needs a CUDA device", allow_module_level=True)
+
+import hetuctr_b200 as hb  # noqa: E402
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+vp, sz, u32 = ctypes.c_void_p, ctypes.c_size_t, ctypes.c_uint32
+CHUNK, LOST = 1000, 0xffffffff
+
+
+@pytest.mark.parametrize("width", [4, 8])
+@pytest.mark.parametrize("n", [1, 1023, 1024, 1025, 9000])
+@pytest.mark.parametrize("lost", ["none", "last", "never"])
+def test_chunks(n, width, lost):
+    L = hb.lib()
+    L.hctr_ingest_keys_following.argtypes = [vp, ctypes.c_int, vp, sz, vp, u32, vp, sz, vp, vp, vp, u32, vp, u32, vp]
+    dev, length, epoch = torch.device("cuda:0"), 70_000, 5
+    rng = np.random.RandomState(n)
+    keys = rng.randint(length, size=n)
+    row_of = rng.permutation(length).astype(np.int32)
+    dt = torch.int32 if width == 4 else torch.int64
+    src = torch.zeros(n, dtype=dt).pin_memory()
+    progress = torch.full((1,), (epoch - 1) << 32 | n).pin_memory()  # (an earlier call's)
+    gave_up = torch.zeros(1, dtype=torch.int32).pin_memory()
+    seen = torch.full((1,), (epoch - 1) << 32 | n, device=dev)
+    dst = torch.full((n,), -7, dtype=torch.int64, device=dev)
+    rows = torch.full((n,), -7, dtype=torch.int32, device=dev)
+    meta = torch.full((9,), 3, dtype=torch.int32, device=dev)
+    row_d = torch.from_numpy(row_of).to(dev)
+    torch.cuda.synchronize()
+    starts = list(range(0, n, CHUNK))
+    # a chunk that is not coming in time ends the wait after a millisecond; the others get as long as they need
+    limit = 1000 if lost == "never" else 1_000_000
+    if lost == "never":  # (all but the last are there beforehand)
+        src.copy_(torch.from_numpy(keys).to(dt))
+        progress[0] = epoch << 32 | starts[-1]
+    assert L.hctr_ingest_keys_following(src.data_ptr(), width, dst.data_ptr(), n, meta.data_ptr(), 9, row_d.data_ptr(),
+                                        length, rows.data_ptr(), progress.data_ptr(), seen.data_ptr(), epoch,
+                                        gave_up.data_ptr(), limit, None) == 0
+    if lost != "never":
+        for at in starts:
+            part = slice(at, min(n, at + CHUNK))
+            src[part] = torch.from_numpy(keys[part]).to(dt)
+            progress[0] = epoch << 32 | (LOST if lost == "last" and at == starts[-1] else part.stop)
+    torch.cuda.synchronize()
+    assert int(gave_up[0]) == (1 if lost == "never" else 0)
+    got, at = dst.cpu().numpy(), rows.cpu().numpy()
+    for first in range(0, n, 1024):  # a block takes all of its keys or none
+        block = slice(first, min(n, first + 1024))
+        if got[block][0] != -7:
+            assert np.array_equal(got[block], keys[block]) and np.array_equal(at[block], row_of[keys[block]])
+        else:
+            assert (got[block] == -7).all() and (at[block] == -7).all()
+    there = int((got != -7).sum())
+    if lost == "none":
+        assert there == n
+    elif lost == "never":
+        assert there == starts[-1] // 1024 * 1024
+    else:  # (a block that looks late finds that the rest is lost)
+        assert there <= starts[-1]
+    assert not bool(meta.any())
+
+
+def _steps(oracle_mod, sizes, bad=()):
+    """Training and serving steps with pageable keys, against the oracle; a batch of `bad` has one key out of range."""
+    from test_gpu_parity import assert_state_parity, make_worlds
+
+    N, W = 60_000, 4
+    rng = np.random.RandomState(3)
+    gw, ow = make_worlds(oracle_mod, 1, N, W, 0, 0, 0.5, np.zeros(N, dtype=np.uint8), [rng.permutation(N)],
+                         keys_on_device=False)
+    before = None
+    for s, n in enumerate(sizes):
+        keys = [rng.randint(N, size=n)]
+        if s in bad:
+            broken = keys[0].copy()
+            broken[n - 1 - n // 3] = N
+            with pytest.raises(RuntimeError, match="outside"):
+                gw.preprocess([broken])
+            before = None
+            gw.push_pull(None)
+            continue
+        gw.preprocess(keys)
+        ow.preprocess(keys)
+        grads = None if before is None or s % 4 == 3 else [rng.normal(0, 1, size=(before, W)).astype(np.float32)]
+        got, want = gw.push_pull(grads), ow.push_pull(grads)
+        assert np.array_equal(got[0], want[0]), s
+        before = n
+    assert_state_parity(gw, ow, exact=True)
+    gw.close()
+
+
+SIZES = [40_000, 32_768, 32_767, 70_000, 45_057, 300, 50_000, 36_864, 140_001]
+
+
+@pytest.mark.parametrize("limit", ["20000", "3", "0"])  # (3 us: the kernel gives up while the keys are being staged)
+def test_tables(oracle_mod, monkeypatch, limit):
+    monkeypatch.setenv("HCTR_FOLLOW_LIMIT_US", limit)
+    _steps(oracle_mod, SIZES)
+
+
+def test_bad_key(oracle_mod):
+    _steps(oracle_mod, SIZES + SIZES, bad=(3, 10))
+
+
+def test_two_batches_in_a_row(oracle_mod):
+    from test_gpu_parity import make_worlds
+
+    N, W = 60_000, 4
+    rng = np.random.RandomState(5)
+    gw, ow = make_worlds(oracle_mod, 1, N, W, 0, 0, 0.5, np.zeros(N, dtype=np.uint8), [np.arange(N)], keys_on_device=False)
+    for n in (50_000, 80_000):
+        keys = [rng.randint(N, size=n)]
+        gw.preprocess(keys)
+        ow.preprocess(keys)
+    grad = [rng.normal(0, 1, size=(50_000, W)).astype(np.float32)]
+    assert np.array_equal(gw.push_pull(grad)[0], ow.push_pull(grad)[0])
+    gw.close()
+
+
+def test_launches_that_wait_for_their_kernels():
+    code = ("import sys; sys.path[:0] = [%r, %r]\n"
+            "from oracle import build, hetu_oracle\n"
+            "import test_gpu_following_ingest as t\n"
+            "t._steps(hetu_oracle, t.SIZES)\nprint('same')\n" % (ROOT, os.path.join(ROOT, "tests")))
+    r = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, CUDA_LAUNCH_BLOCKING="1"), cwd=ROOT,
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "same" in r.stdout, r.stderr[-2000:]
