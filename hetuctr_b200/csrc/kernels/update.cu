@@ -82,6 +82,7 @@ __global__ void __launch_bounds__(kDecideThreads) push_decide_scan(const u32 *__
 __global__ void push_counts(const u32 *__restrict__ meta, int nrank, const u32 *__restrict__ push_slot,
                             u32 *__restrict__ push_count, u32 *__restrict__ push_base) {
   const int p = threadIdx.x;
+  wait_predecessor();
   if (p < nrank) {
     const u32 *seg = meta + HCTR_META_SEG;
     const bool none = grouping_broke_off(meta);
@@ -923,6 +924,7 @@ __global__ void __launch_bounds__(kThreads) owner_apply_pair(PushLists p, hctr_p
   typedef RowT<VEC> R;
   typedef typename R::T T;
   __shared__ u32 qstart[kMaxRanks + 1], gstart[kMaxRanks + 1];
+  wait_predecessor();
   wait_queries(c, seq, qstart, gstart, blockIdx.x == 0);
   const int peer = 1 - c.rank;
   const size_t first = push_list_base(p, peer), n = gstart[peer + 1] - gstart[peer];
@@ -1081,8 +1083,10 @@ extern "C" int hctr_p2p_owner_apply_pair(const hctr_p2p_ctx *c, const hctr_p2p_b
 #define CALL(L, V)                                                                                                  \
   do {                                                                                                              \
     const size_t need = ((size_t)c->cap * L + kThreads - 1) / kThreads;                                             \
-    owner_apply_pair<L, V><<<(unsigned)std::max<size_t>(1, std::min(need, (size_t)kSMs * 4)), kThreads, 0,          \
-                             (cudaStream_t)stream>>>(p, *c, seq, row_of, length, n_cached, embedding, (long long *)version); \
+    const unsigned g_ = (unsigned)std::max<size_t>(1, std::min(need, (size_t)kSMs * 4));                             \
+    if (const cudaError_t e_ = launch_chained(owner_apply_pair<L, V>, g_, kThreads, 0, (cudaStream_t)stream, p, *c, seq, \
+                                              row_of, length, n_cached, embedding, (long long *)version))           \
+      return (int)e_;                                                                                               \
   } while (0)
   HCTR_DISPATCH_ROWS(c->width, al, CALL);
 #undef CALL
@@ -1128,7 +1132,7 @@ extern "C" int hctr_push_decide_fused(const uint32_t *meta, int nrank, int rank,
                                                              (const long long *)pending_cnt, push_bound, need_push,
                                                              push_slot, reinterpret_cast<u64 *>(chain_scratch), epoch,
                                                              err);
-  push_counts<<<1, 1024, 0, s>>>(meta, nrank, push_slot, push_count, push_base);
+  if (const cudaError_t e = launch_chained(push_counts, 1, 1024, 0, s, meta, nrank, push_slot, push_count, push_base)) return (int)e;
   count_launches(2);
   return launch_status();
 }
