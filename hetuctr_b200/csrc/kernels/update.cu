@@ -557,7 +557,13 @@ __global__ void __launch_bounds__(kThreads) grad_reduce_short_stream(ReduceKerne
 constexpr int kLongThreads = 256;
 constexpr int kLongWarps = kLongThreads / 32;
 constexpr int kLongStages = 4;
-constexpr int kLongStageBytes = 16 * 1024;
+// Sixteen rows per stage, within 8 and 16 KB: beside it an SM holds the short-run blocks of two ranks when its ring is small
+// (two ranks on one GPU: 53,248 x 128 177 -> 169 us per step, 212,992 x 128 351 -> 345, x 64 265 -> 259), but rows of 256
+// floats in stages of eight cost 191 -> 196.
+static __host__ __device__ __forceinline__ size_t long_stage_bytes(size_t width) {
+  const size_t want = 16 * width * sizeof(float);
+  return want < 8192 ? 8192 : want > 16384 ? 16384 : want;
+}
 constexpr int kLongPosChunk = 2048;  // positions staged in shared memory at a time
 constexpr u32 kVeryLongRun = 256;     // runs at least this long are started first
 
@@ -583,7 +589,7 @@ __global__ void __launch_bounds__(kLongThreads) grad_reduce_long(ReduceKernelArg
   __shared__ u32 next_item;
   const size_t E = R::elems(a.width);  // T elements per row
   const size_t W = a.width;            // floats per row
-  const u32 rows_per_stage = (u32)max((size_t)1, (size_t)kLongStageBytes / (W * sizeof(float)));
+  const u32 rows_per_stage = (u32)max((size_t)1, long_stage_bytes(W) / (W * sizeof(float)));
   const size_t stage_elems = (size_t)rows_per_stage * E;
   const size_t stage_floats = (size_t)rows_per_stage * W;
   T *stage = reinterpret_cast<T *>(smem_raw);
@@ -1169,7 +1175,7 @@ extern "C" int hctr_grad_reduce_apply_pack(const hctr_reduce_args *ap, void *str
   const bool forked = a.n_heavy > 0 && a.side_stream && a.fork_event && a.join_event;
   cudaStream_t ls = forked ? (cudaStream_t)a.side_stream : s;
   if (a.n_heavy > 0) {
-    size_t need = (size_t)kLongStages * max((size_t)kLongStageBytes, a.width * sizeof(float));
+    size_t need = (size_t)kLongStages * max(long_stage_bytes(a.width), a.width * sizeof(float));
     if (need > 200 * 1024) return (int)cudaErrorInvalidValue;  // rows wider than 12800 floats
     static PerDevice allowed[2];
     if (const int e = allow_shared(allowed[0], grad_reduce_long<true>, 200 * 1024)) return e;
