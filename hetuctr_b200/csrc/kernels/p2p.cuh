@@ -42,8 +42,11 @@ __device__ __forceinline__ bool poll_seq(const u32 *flag, u32 seq, u64 timeout_n
 // True in exactly one thread block of the launch: the one that arrives last.  Every thread of every block must
 // call it after its last store of the launch.  The block barrier orders the block's stores before thread 0's
 // system-scope fence and arrival, and the last arriver has therefore observed every other block's arrival (and,
-// through their fences, their stores): what it releases afterwards is ordered after all stores of the launch.
-// The counter is left at zero for the next launch.
+// through their fences, their stores): what it releases afterwards (st_release_sys, by any of its threads) is
+// ordered after all stores of the launch.  Seeing the other blocks' arrivals takes a fence on this GPU only, they
+// are on it; a second system-scope fence there and a third before each flag cost the exchange 3 to 4 us a step
+// (two ranks on one GPU, 53,248 x 128 172 -> 167 us, 212,992 x 32 248 -> 242, with the expansion's first indices
+// fetched ahead of its wait).  The counter is left at zero for the next launch.
 __device__ __forceinline__ bool last_block_of_launch(u32 *ticket) {
   __shared__ bool s_last;
   __syncthreads();
@@ -53,7 +56,7 @@ __device__ __forceinline__ bool last_block_of_launch(u32 *ticket) {
     s_last = t == gridDim.x - 1;
     if (s_last) {
       *ticket = 0;
-      __threadfence_system();
+      __threadfence();
     }
   }
   __syncthreads();

@@ -152,7 +152,6 @@ __global__ void __launch_bounds__(kPullThreads) p2p_stale_gather(hctr_p2p_ctx c,
   if (threadIdx.x == 0 && s_served) atomicAdd(c.cnt_in + HCTR_P2P_SERVED(c.nrank), s_served);
   if (!last_block_of_launch(c.cnt_in + HCTR_P2P_TICKET1(c.nrank))) return;
   for (int p = threadIdx.x; p < c.nrank; p += kPullThreads) {
-    __threadfence_system();
     u32 *hdr = c.box[p].hdr + (size_t)c.rank * kHdrWords;
     hdr[9] = 0;
     st_release_sys(hdr + 8, seq);
@@ -256,6 +255,20 @@ __global__ void __launch_bounds__(kFusedThreads, LANES >= 4 ? 4 : 3) p2p_refresh
   wait_predecessor();
   if (threadIdx.x == 0) s_flagged = s_n = 0;
   for (int i = threadIdx.x; i <= c.nrank; i += kFusedThreads) seg[i] = meta[HCTR_META_SEG + i];
+  // (the expansion's first indices, on their way while the block waits)
+  const u32 stride = (u32)((size_t)gridDim.x * kFusedThreads / LANES * kFusedRows), n_pos = (u32)batch;
+  const unsigned gl = threadIdx.x % LANES;
+  static_assert(kFusedRows == 4, "indices come four at a time");
+  auto four_at = [&](const int32_t *p, u32 i) {
+    if (i + 3 < n_pos) return *reinterpret_cast<const int4 *>(p + i);
+    int4 r = make_int4(HCTR_INVALID_ROW, HCTR_INVALID_ROW, HCTR_INVALID_ROW, HCTR_INVALID_ROW);
+    if (i < n_pos) r.x = p[i];
+    if (i + 1 < n_pos) r.y = p[i + 1];
+    if (i + 2 < n_pos) r.z = p[i + 2];
+    return r;
+  };
+  u32 i0 = (u32)(((size_t)blockIdx.x * kFusedThreads + threadIdx.x) / LANES) * kFusedRows;
+  int4 next_row = four_at(pos_row, i0), next_u = four_at(idx_map, i0);
   wait_returns(c, seq, ret_base, false, blockIdx.x == 0);  // (ends with a block barrier)
   const size_t U = unique_of(meta);
   const unsigned lane = threadIdx.x & 31;
@@ -317,19 +330,6 @@ __global__ void __launch_bounds__(kFusedThreads, LANES >= 4 ? 4 : 3) p2p_refresh
   // Expansion: a group of LANES lanes takes kFusedRows positions per iteration; the next iteration's row and unique indices
   // arrive meanwhile, and a key's owner is the segment its unique index falls into (no access to wait for: two ranks on one
   // GPU, 212,992 x 32 20.5 -> 16.6 us a launch, 53,248 x 128 21.4 -> 20.3).
-  const u32 stride = (u32)((size_t)gridDim.x * kFusedThreads / LANES * kFusedRows), n_pos = (u32)batch;
-  const unsigned gl = threadIdx.x % LANES;
-  static_assert(kFusedRows == 4, "indices come four at a time");
-  auto four_at = [&](const int32_t *p, u32 i) {
-    if (i + 3 < n_pos) return *reinterpret_cast<const int4 *>(p + i);
-    int4 r = make_int4(HCTR_INVALID_ROW, HCTR_INVALID_ROW, HCTR_INVALID_ROW, HCTR_INVALID_ROW);
-    if (i < n_pos) r.x = p[i];
-    if (i + 1 < n_pos) r.y = p[i + 1];
-    if (i + 2 < n_pos) r.z = p[i + 2];
-    return r;
-  };
-  u32 i0 = (u32)(((size_t)blockIdx.x * kFusedThreads + threadIdx.x) / LANES) * kFusedRows;
-  int4 next_row = four_at(pos_row, i0), next_u = four_at(idx_map, i0);
   for (; i0 < n_pos; i0 += stride) {
     const int32_t row4[kFusedRows] = {next_row.x, next_row.y, next_row.z, next_row.w};
     const int32_t u4[kFusedRows] = {next_u.x, next_u.y, next_u.z, next_u.w};
