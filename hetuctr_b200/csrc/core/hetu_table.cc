@@ -152,12 +152,12 @@ HetuTable::HetuTable(const int rank, const int nrank, const int device_id, const
       HCTR_CUDA(cudaMallocHost(&b->h_meta, (HCTR_META_WORDS + (size_t)nrank_ + 1) * sizeof(uint32_t)));
       reserveBatch(*b, 1);
     }
-    HCTR_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&h_ingest_err_), 64, cudaHostAllocMapped));
+    HCTR_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&h_ingest_err_), 128, cudaHostAllocMapped));
     for (int i = 0; i < 4; i++) h_ingest_err_[i] = 0;
     HCTR_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void **>(&d_ingest_err_), h_ingest_err_, 0));
-    HCTR_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&h_progress_), 64, cudaHostAllocMapped));
+    h_progress_ = reinterpret_cast<unsigned long long *>(h_ingest_err_ + 16);  // (a cache line of its own)
+    d_progress_ = reinterpret_cast<unsigned long long *>(d_ingest_err_ + 16);
     *h_progress_ = 0;
-    HCTR_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void **>(&d_progress_), h_progress_, 0));
     reserveShared(1);
     hctr_group_is_small(1);  // asks the device about clusters, once; a step would wait for the answer
     h_pinned_words_ = HCTR_META_WORDS + (size_t)nrank_ + 1 + 12 * (size_t)nrank_ + 16;
@@ -1675,7 +1675,6 @@ void HetuTable::releaseAll() {
   }
   if (h_ingest_err_) cudaFreeHost(h_ingest_err_);
   h_ingest_err_ = d_ingest_err_ = nullptr;
-  if (h_progress_) cudaFreeHost(h_progress_);
   h_progress_ = d_progress_ = nullptr;
   for (BatchDesc *b : {&cur_batch_, &prev_batch_})
     for (DevBuf *d : {&b->keys, &b->idx_map, &b->sorted_pos, &b->uniq, &b->uniq_owner, &b->uniq_row,
