@@ -890,6 +890,7 @@ void HetuTable::reduceGradients(BatchDesc &b, const embed_t *grad, size_t last_l
   r.side_stream = stream_reduce_side_;
   r.fork_event = ev_rfork_;
   r.join_event = ev_rjoin_;
+  r.shared_gpu = use_p2p_ && p2p_->sameContext();  // (thread ranks on one GPU)
   HCTR_LAUNCH(hctr_grad_reduce_apply_pack(&r, stream_reduce_));
 }
 

@@ -557,12 +557,16 @@ __global__ void __launch_bounds__(kThreads) grad_reduce_short_stream(ReduceKerne
 constexpr int kLongThreads = 256;
 constexpr int kLongWarps = kLongThreads / 32;
 constexpr int kLongStages = 4;
-// Sixteen rows per stage, within 8 and 16 KB: beside it an SM holds the short-run blocks of two ranks when its ring is small
-// (two ranks on one GPU: 53,248 x 128 177 -> 169 us per step, 212,992 x 128 351 -> 345, x 64 265 -> 259), but rows of 256
-// floats in stages of eight cost 191 -> 196.
-static __host__ __device__ __forceinline__ size_t long_stage_bytes(size_t width) {
-  const size_t want = 16 * width * sizeof(float);
-  return want < 8192 ? 8192 : want > 16384 ? 16384 : want;
+// Every stage costs a barrier and the slowest of its rows, so large ones are better - where there is room.  With a GPU to
+// itself the kernel takes 32 KB for rows of 128 floats or more, else 16 KB: two short-run blocks still fit an SM beside it
+// (the reduction's two kernels with 32 / 16 / 8 KB: 212,992 x 128 79 / 82 / 100 us, with hotter keys 86 / 94 / 123,
+// 53,248 x 256 39 / 45 / 45, 53,248 x 128 33 / 33 / 37, 212,992 x 64 70 / 68 / 75).  Where ranks share a GPU, sixteen rows
+// within 8 and 16 KB: an SM then holds the short-run blocks of two ranks beside both rings (two ranks on one GPU, against
+// 16 KB: 53,248 x 128 177 -> 169 us per step, 212,992 x 128 351 -> 345, x 64 265 -> 259; rows of 256 floats in stages of
+// eight 191 -> 196).  On one stream several blocks per SM run long runs: 16 KB.
+static size_t long_stage_bytes(size_t width, bool forked, bool shared_gpu) {
+  if (!shared_gpu) return forked && width >= 128 ? 32768 : 16384;
+  return std::min<size_t>(std::max<size_t>(16 * width * sizeof(float), 8192), 16384);
 }
 constexpr int kLongPosChunk = 2048;  // positions staged in shared memory at a time
 constexpr u32 kVeryLongRun = 256;     // runs at least this long are started first
@@ -579,7 +583,8 @@ __device__ __forceinline__ void cp_async_elem(void *smem_dst, const void *gsrc, 
 }
 
 template <bool VEC>
-__global__ void __launch_bounds__(kLongThreads) grad_reduce_long(ReduceKernelArgs ka, u32 n_heavy, u32 *work_counter) {
+__global__ void __launch_bounds__(kLongThreads) grad_reduce_long(ReduceKernelArgs ka, u32 n_heavy, u32 *work_counter,
+                                                                  u32 stage_bytes) {
   const hctr_reduce_args &a = ka.a;
   const u64 once = l2_evict_first_policy();
   typedef RowT<VEC> R;
@@ -589,7 +594,7 @@ __global__ void __launch_bounds__(kLongThreads) grad_reduce_long(ReduceKernelArg
   __shared__ u32 next_item;
   const size_t E = R::elems(a.width);  // T elements per row
   const size_t W = a.width;            // floats per row
-  const u32 rows_per_stage = (u32)max((size_t)1, long_stage_bytes(W) / (W * sizeof(float)));
+  const u32 rows_per_stage = (u32)max((size_t)1, stage_bytes / (W * sizeof(float)));
   const size_t stage_elems = (size_t)rows_per_stage * E;
   const size_t stage_floats = (size_t)rows_per_stage * W;
   T *stage = reinterpret_cast<T *>(smem_raw);
@@ -1175,7 +1180,8 @@ extern "C" int hctr_grad_reduce_apply_pack(const hctr_reduce_args *ap, void *str
   const bool forked = a.n_heavy > 0 && a.side_stream && a.fork_event && a.join_event;
   cudaStream_t ls = forked ? (cudaStream_t)a.side_stream : s;
   if (a.n_heavy > 0) {
-    size_t need = (size_t)kLongStages * max(long_stage_bytes(a.width), a.width * sizeof(float));
+    const size_t stage = long_stage_bytes(a.width, forked, a.shared_gpu != 0);
+    size_t need = (size_t)kLongStages * max(stage, a.width * sizeof(float));
     if (need > 200 * 1024) return (int)cudaErrorInvalidValue;  // rows wider than 12800 floats
     static PerDevice allowed[2];
     if (const int e = allow_shared(allowed[0], grad_reduce_long<true>, 200 * 1024)) return e;
@@ -1186,8 +1192,8 @@ extern "C" int hctr_grad_reduce_apply_pack(const hctr_reduce_args *ap, void *str
     }
     const size_t per = need > 100 * 1024 ? 1 : (forked ? (size_t)long_per_sm : 3);
     const unsigned grid = (unsigned)min((size_t)a.n_heavy, (size_t)kSMs * per);
-    if (al && a.width % 4 == 0) grad_reduce_long<true><<<grid, kLongThreads, need, ls>>>(ka, (u32)a.n_heavy, a.work_counter);
-    else grad_reduce_long<false><<<grid, kLongThreads, need, ls>>>(ka, (u32)a.n_heavy, a.work_counter);
+    if (al && a.width % 4 == 0) grad_reduce_long<true><<<grid, kLongThreads, need, ls>>>(ka, (u32)a.n_heavy, a.work_counter, (u32)stage);
+    else grad_reduce_long<false><<<grid, kLongThreads, need, ls>>>(ka, (u32)a.n_heavy, a.work_counter, (u32)stage);
     count_launches(1);
     if (forked) {
       cudaError_t e = cudaEventRecord((cudaEvent_t)a.join_event, ls);

@@ -434,6 +434,7 @@ typedef struct hctr_reduce_args {
   void *side_stream;
   void *fork_event;
   void *join_event;
+  int shared_gpu;             /* other ranks' kernels run on this GPU meanwhile: leave them room on an SM */
 } hctr_reduce_args;
 
 int hctr_grad_reduce_apply_pack(const hctr_reduce_args *a, void *stream);
