@@ -890,7 +890,7 @@ void HetuTable::reduceGradients(BatchDesc &b, const embed_t *grad, size_t last_l
   r.side_stream = stream_reduce_side_;
   r.fork_event = ev_rfork_;
   r.join_event = ev_rjoin_;
-  r.shared_gpu = use_p2p_ && p2p_->sameContext();  // (thread ranks on one GPU)
+  r.shared_gpu = use_p2p_ ? p2p_->sameContext() : std::strcmp(transport_->name(), "inproc") == 0;  // (thread ranks)
   HCTR_LAUNCH(hctr_grad_reduce_apply_pack(&r, stream_reduce_));
 }
 
