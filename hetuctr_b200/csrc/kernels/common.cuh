@@ -37,6 +37,9 @@ static inline int allow_shared(PerDevice &done, K *kernel, size_t bytes) {
 // kernel of a stream to the next that takes 2 us off.  (Predecessors do not let the successor's blocks in any earlier than
 // when all of their own have ended: waiting blocks kept those of other streams' kernels off the SMs, 108 -> 127 us for a
 // step of 212,992 x 128 whose grouping did so.)
+// Such a kernel begins while its predecessor still writes, so none of its pointers is __restrict__ but those to what is constant
+// from a table's construction on (row_of): the qualifier would promise that nobody else touches the memory for as long as
+// the kernel runs, and loads under that promise need not stay behind the wait.
 __device__ __forceinline__ void wait_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 template <class... P, class... A>
 static inline cudaError_t launch_chained(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, A... args) {

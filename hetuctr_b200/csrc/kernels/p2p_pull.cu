@@ -70,9 +70,8 @@ __device__ __forceinline__ V warp_compact(unsigned mask, V value) {
 template <bool VEC>
 __global__ void __launch_bounds__(kPullThreads) p2p_stale_gather(hctr_p2p_ctx c, u32 seq,
                                                                  const int32_t *__restrict__ row_of, size_t length,
-                                                                 size_t n_cached, const float *__restrict__ embedding,
-                                                                 const long long *__restrict__ version,
-                                                                 long long pull_bound) {
+                                                                 size_t n_cached, const float *embedding,
+                                                                 const long long *version, long long pull_bound) {
   typedef RowT<VEC> R;
   typedef typename R::T T;
   __shared__ u32 qstart[kMaxRanks + 1];
@@ -238,14 +237,11 @@ constexpr int kFusedRows = 4;  // rows per lane group and iteration, as in the p
 constexpr int kFusedThreads = 256;  // >= kMaxRanks: thread s of every block polls owner s
 
 template <int LANES, bool VEC>
-__global__ void __launch_bounds__(kFusedThreads, LANES >= 4 ? 4 : 3) p2p_refresh_expand(hctr_p2p_ctx c, u32 seq, const u32 *__restrict__ meta,
-                                                               const int32_t *__restrict__ uniq_row, size_t n_cached,
-                                                               const float *__restrict__ pending,
-                                                               float *__restrict__ embedding,
-                                                               long long *__restrict__ version, size_t batch,
-                                                               const int32_t *__restrict__ pos_row,
-                                                               const int32_t *__restrict__ idx_map,
-                                                               float *__restrict__ dst) {
+__global__ void __launch_bounds__(kFusedThreads, LANES >= 4 ? 4 : 3) p2p_refresh_expand(hctr_p2p_ctx c, u32 seq, const u32 *meta,
+                                                               const int32_t *uniq_row, size_t n_cached,
+                                                               const float *pending, float *embedding,
+                                                               long long *version, size_t batch, const int32_t *pos_row,
+                                                               const int32_t *idx_map, float *dst) {
   typedef RowT<VEC> R;
   typedef typename R::T T;
   __shared__ u32 ret_base[kMaxRanks + 1];

@@ -166,9 +166,8 @@ __global__ void __launch_bounds__(kThreads) expand_rows(size_t batch, size_t wid
 // 47.2 (50.9).  A chained launch, behind the ingest or the reduction: 26 keys x 16 16.9 -> 15.1 us per request, steps of
 // 5,661 x 50 34.9 -> 32.8 and of 26,624 x 16 35.8 -> 33.4.
 template <int V, int LANES>
-__global__ void __launch_bounds__(kThreads, 3) expand_rows_local(u32 batch, u32 E, const int32_t *__restrict__ pos_row,
-                                                                 const float *__restrict__ embedding,
-                                                                 float *__restrict__ dst_f) {
+__global__ void __launch_bounds__(kThreads, 3) expand_rows_local(u32 batch, u32 E, const int32_t *pos_row,
+                                                                 const float *embedding, float *dst_f) {
   typedef RowV<V> R;
   typedef typename R::T T;
   static_assert(kExpandRows == 4, "row indices come four at a time");

@@ -79,8 +79,7 @@ __global__ void __launch_bounds__(kDecideThreads) push_decide_scan(const u32 *__
   }
 }
 
-__global__ void push_counts(const u32 *__restrict__ meta, int nrank, const u32 *__restrict__ push_slot,
-                            u32 *__restrict__ push_count, u32 *__restrict__ push_base) {
+__global__ void push_counts(const u32 *meta, int nrank, const u32 *push_slot, u32 *push_count, u32 *push_base) {
   const int p = threadIdx.x;
   wait_predecessor();
   if (p < nrank) {
@@ -930,8 +929,7 @@ __global__ void __launch_bounds__(kThreads) owner_apply_sources(PushLists p, siz
 template <int LANES, bool VEC>
 __global__ void __launch_bounds__(kThreads) owner_apply_pair(PushLists p, hctr_p2p_ctx c, u32 seq,
                                                              const int32_t *__restrict__ row_of, size_t length,
-                                                             size_t n_cached, float *__restrict__ embedding,
-                                                             long long *__restrict__ version) {
+                                                             size_t n_cached, float *embedding, long long *version) {
   typedef RowT<VEC> R;
   typedef typename R::T T;
   __shared__ u32 qstart[kMaxRanks + 1], gstart[kMaxRanks + 1];
