@@ -16,6 +16,12 @@ typedef unsigned long long u64;
 typedef uint32_t u32;
 
 static inline int launch_status() { return (int)cudaGetLastError(); }
+// For launches that return their status: a failure is reported once, not by the next launch_status as well.
+static inline int launch_status(cudaError_t e) {
+  if (e == cudaSuccess) return launch_status();
+  cudaGetLastError();
+  return (int)e;
+}
 
 // Kernels enqueued by this library since load (every launcher adds what it launched).
 extern unsigned long long g_launches;
@@ -42,7 +48,7 @@ static inline int allow_shared(PerDevice &done, K *kernel, size_t bytes) {
 // the kernel runs, and loads under that promise need not stay behind the wait.
 __device__ __forceinline__ void wait_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 template <class... P, class... A>
-static inline cudaError_t launch_chained(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, A... args) {
+static inline int launch_chained(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, A... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(block);
@@ -53,7 +59,7 @@ static inline cudaError_t launch_chained(void (*kernel)(P...), unsigned grid, un
   at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+  return launch_status(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
 }
 
 static inline unsigned grid_for(size_t n, unsigned block) {

@@ -479,7 +479,7 @@ static int launch_cluster(const hctr_group_args &a, const GroupPlan &g, cudaStre
   const cudaLaunchConfig_t cfg = cluster_config<ITEMS>(tiles, s, &at);
   const cudaError_t e = cudaLaunchKernelEx(&cfg, group_cluster<ITEMS>, a, g);
   count_launches(1);
-  return e != cudaSuccess ? (int)e : launch_status();
+  return launch_status(e);
 }
 
 template <int ITEMS>
@@ -487,8 +487,8 @@ static int launch_passes(const hctr_group_args &a, const GroupPlan &g, cudaStrea
   const u32 tiles = (u32)((a.batch + kTileThreads * ITEMS - 1) / (kTileThreads * ITEMS));
   group_histogram<<<kSMs, 512, 0, s>>>(a, g);
   for (int p = 0; p < g.passes; p++)
-    if (const cudaError_t e = launch_chained(group_pass<ITEMS>, tiles, kTileThreads, sizeof(TileSmem), s, a, g, p)) return (int)e;
-  if (const cudaError_t e = launch_chained(group_finish<ITEMS>, tiles, kTileThreads, 0, s, a, g)) return (int)e;
+    if (const int e = launch_chained(group_pass<ITEMS>, tiles, kTileThreads, sizeof(TileSmem), s, a, g, p)) return e;
+  if (const int e = launch_chained(group_finish<ITEMS>, tiles, kTileThreads, 0, s, a, g)) return e;
   count_launches(g.passes + 2);
   return launch_status();
 }

@@ -390,9 +390,9 @@ extern "C" int hctr_p2p_stale_gather(const hctr_p2p_ctx *c, uint32_t seq, const 
   if (g == 0) g = 1;
   const bool vec = host_aligned16(embedding) && c->width % 4 == 0;
   const auto kernel = vec ? p2p_stale_gather<true> : p2p_stale_gather<false>;
-  if (const cudaError_t e = launch_chained(kernel, (unsigned)g, kPullThreads, 0, st, *c, seq, row_of, length, n_cached, embedding,
+  if (const int e = launch_chained(kernel, (unsigned)g, kPullThreads, 0, st, *c, seq, row_of, length, n_cached, embedding,
                                            (const long long *)version, pull_bound))
-    return (int)e;
+    return e;
   count_launches(1);
   return launch_status();
 }
@@ -435,10 +435,10 @@ extern "C" int hctr_p2p_refresh_expand(const hctr_p2p_ctx *c, uint32_t seq, cons
     const size_t cap_ = (size_t)kSMs * 4; /* one resident round (64 registers); every block polls the headers */ \
     if (g_ > cap_) g_ = cap_;                                                                              \
     if (g_ == 0) g_ = 1; /* an empty batch still waits for the peers: the step's protocol */               \
-    if (const cudaError_t e_ = launch_chained(p2p_refresh_expand<L, V>, (unsigned)g_, kFusedThreads, 0, st, *c, seq, meta, \
+    if (const int e_ = launch_chained(p2p_refresh_expand<L, V>, (unsigned)g_, kFusedThreads, 0, st, *c, seq, meta, \
                                               uniq_row, n_cached, pending, embedding, (long long *)version, batch, pos_row, \
                                               idx_map, dst))                                               \
-      return (int)e_;                                                                                      \
+      return e_;                                                                                      \
   } while (0)
   HCTR_DISPATCH_ROWS(width, al, CALL);
 #undef CALL

@@ -567,8 +567,8 @@ extern "C" int hctr_expand_rows_local(size_t batch, size_t width, const int32_t 
   do {                                                                                                             \
     const size_t need = ((batch + kExpandRows - 1) / kExpandRows * L + kThreads - 1) / kThreads;                   \
     const unsigned g = (unsigned)(need < (size_t)kSMs * 3 ? need : (size_t)kSMs * 3); /* one resident round */     \
-    if (const cudaError_t e = launch_chained(expand_rows_local<V, L>, g, kThreads, 0, (cudaStream_t)stream, (u32)batch,   \
-                                             (u32)(width / V), pos_row, embedding, dst)) return (int)e;            \
+    if (const int e = launch_chained(expand_rows_local<V, L>, g, kThreads, 0, (cudaStream_t)stream, (u32)batch,   \
+                                             (u32)(width / V), pos_row, embedding, dst)) return e;            \
   } while (0)
   HCTR_DISPATCH_ELEMS(width, addr, CALL);
 #undef CALL

@@ -1093,9 +1093,9 @@ extern "C" int hctr_p2p_owner_apply_pair(const hctr_p2p_ctx *c, const hctr_p2p_b
   do {                                                                                                              \
     const size_t need = ((size_t)c->cap * L + kThreads - 1) / kThreads;                                             \
     const unsigned g_ = (unsigned)std::max<size_t>(1, std::min(need, (size_t)kSMs * 4));                             \
-    if (const cudaError_t e_ = launch_chained(owner_apply_pair<L, V>, g_, kThreads, 0, (cudaStream_t)stream, p, *c, seq, \
+    if (const int e_ = launch_chained(owner_apply_pair<L, V>, g_, kThreads, 0, (cudaStream_t)stream, p, *c, seq, \
                                               row_of, length, n_cached, embedding, (long long *)version))           \
-      return (int)e_;                                                                                               \
+      return e_;                                                                                               \
   } while (0)
   HCTR_DISPATCH_ROWS(c->width, al, CALL);
 #undef CALL
@@ -1125,7 +1125,7 @@ extern "C" int hctr_p2p_owner_update(const hctr_p2p_ctx *cp, const int32_t *row_
   HCTR_DISPATCH_ROWS(c.width, al, CALL);
 #undef CALL
   count_launches(1);
-  return (int)e;
+  return launch_status(e);
 }
 
 extern "C" int hctr_push_decide_fused(const uint32_t *meta, int nrank, int rank, size_t u_max,
@@ -1141,7 +1141,7 @@ extern "C" int hctr_push_decide_fused(const uint32_t *meta, int nrank, int rank,
                                                              (const long long *)pending_cnt, push_bound, need_push,
                                                              push_slot, reinterpret_cast<u64 *>(chain_scratch), epoch,
                                                              err);
-  if (const cudaError_t e = launch_chained(push_counts, 1, 1024, 0, s, meta, nrank, push_slot, push_count, push_base)) return (int)e;
+  if (const int e = launch_chained(push_counts, 1, 1024, 0, s, meta, nrank, push_slot, push_count, push_base)) return e;
   count_launches(2);
   return launch_status();
 }
