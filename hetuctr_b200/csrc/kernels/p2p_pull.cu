@@ -255,12 +255,14 @@ __global__ void __launch_bounds__(kFusedThreads, LANES >= 4 ? 4 : 3) p2p_refresh
   const u32 stride = (u32)((size_t)gridDim.x * kFusedThreads / LANES * kFusedRows), n_pos = (u32)batch;
   const unsigned gl = threadIdx.x % LANES;
   static_assert(kFusedRows == 4, "indices come four at a time");
+  const bool fours = aligned16(pos_row) && aligned16(idx_map);  // (a table's own arrays are)
   auto four_at = [&](const int32_t *p, u32 i) {
-    if (i + 3 < n_pos) return *reinterpret_cast<const int4 *>(p + i);
+    if (fours && i + 3 < n_pos) return *reinterpret_cast<const int4 *>(p + i);
     int4 r = make_int4(HCTR_INVALID_ROW, HCTR_INVALID_ROW, HCTR_INVALID_ROW, HCTR_INVALID_ROW);
     if (i < n_pos) r.x = p[i];
     if (i + 1 < n_pos) r.y = p[i + 1];
     if (i + 2 < n_pos) r.z = p[i + 2];
+    if (i + 3 < n_pos) r.w = p[i + 3];
     return r;
   };
   u32 i0 = (u32)(((size_t)blockIdx.x * kFusedThreads + threadIdx.x) / LANES) * kFusedRows;
@@ -424,8 +426,8 @@ extern "C" int hctr_p2p_refresh_expand(const hctr_p2p_ctx *c, uint32_t seq, cons
                                        const float *pending, float *embedding, int64_t *version, size_t batch,
                                        const int32_t *pos_row, const int32_t *idx_map, float *dst, void *stream) {
   cudaStream_t st = (cudaStream_t)stream;
-  if (c->nrank > kMaxRanks || batch >= ((size_t)1 << 31) || !host_aligned16(pos_row) || !host_aligned16(idx_map))
-    return (int)cudaErrorInvalidValue;
+  // (positions are 32-bit, up to one round of the grid beyond the last)
+  if (c->nrank > kMaxRanks || batch > 0xfff00000u) return (int)cudaErrorInvalidValue;
   const size_t width = c->width;
   // (the mailbox arrays are device allocations of their own: aligned; c->box is a device array)
   const bool al = host_aligned16(embedding) && host_aligned16(pending) && host_aligned16(dst);

@@ -186,6 +186,19 @@ def test_requester_side_kernel_on_synthetic_mailbox(ranks, width):
     assert (pos >= r.C).any() and ((pos >= 0) & (pos < r.C)).any() and (pos < 0).any()
 
 
+@pytest.mark.parametrize("batch", [5999, 6001, 6002])
+@pytest.mark.parametrize("array,elements", [("pos_row", 1), ("idx_map", 2), ("pos_row", 3)])
+def test_requester_side_kernel_takes_indices_at_any_address(array, elements, batch):
+    from hetuctr_b200.requester_replay import RequesterReplay
+
+    r = RequesterReplay(ranks=3, batch=batch, unique=2500, width=12, owned_rows=5000, seed=batch)
+    t = getattr(r, array)
+    moved = torch.cat([torch.full((elements,), 1 << 30, dtype=t.dtype, device=t.device), t])[elements:]
+    assert moved.data_ptr() % 16 != 0
+    setattr(r, array, moved)
+    assert r.check()
+
+
 def test_ingest_keys_and_deferred_ordering():
     """hctr_ingest_keys (copy + cleared meta in one launch) and the split pipeline: hctr_dedupe_map without the
     run ordering (fork event only), hctr_dedupe_order later on another stream."""
