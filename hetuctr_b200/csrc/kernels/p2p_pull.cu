@@ -235,13 +235,15 @@ __global__ void __launch_bounds__(kPullThreads) p2p_refresh_index(hctr_p2p_ctx c
 // The refresh writes only flagged cached rows, which the expansion never reads: the two parts are independent.
 constexpr int kFusedRows = 4;  // rows per lane group and iteration, as in the plain expansion
 constexpr int kFusedThreads = 256;  // >= kMaxRanks: thread s of every block polls owner s
+// Blocks an SM holds and the grid counts on: one resident round, since every block polls the headers.  From four lanes per row
+// on 64 registers do; with one or two the column loop is unrolled into more (80, three blocks).
+constexpr int fused_blocks(int lanes) { return lanes >= 4 ? 4 : 3; }
 
 template <int LANES, bool VEC>
-__global__ void __launch_bounds__(kFusedThreads, LANES >= 4 ? 4 : 3) p2p_refresh_expand(hctr_p2p_ctx c, u32 seq, const u32 *meta,
-                                                               const int32_t *uniq_row, size_t n_cached,
-                                                               const float *pending, float *embedding,
-                                                               long long *version, size_t batch, const int32_t *pos_row,
-                                                               const int32_t *idx_map, float *dst) {
+__global__ void __launch_bounds__(kFusedThreads, fused_blocks(LANES))
+    p2p_refresh_expand(hctr_p2p_ctx c, u32 seq, const u32 *meta, const int32_t *uniq_row, size_t n_cached,
+                       const float *pending, float *embedding, long long *version, size_t batch, const int32_t *pos_row,
+                       const int32_t *idx_map, float *dst) {
   typedef RowT<VEC> R;
   typedef typename R::T T;
   __shared__ u32 ret_base[kMaxRanks + 1];
@@ -434,7 +436,7 @@ extern "C" int hctr_p2p_refresh_expand(const hctr_p2p_ctx *c, uint32_t seq, cons
 #define CALL(L, V)                                                                                         \
   do {                                                                                                     \
     size_t g_ = (((size_t)batch + kFusedRows - 1) / kFusedRows * L + kFusedThreads - 1) / kFusedThreads;              \
-    const size_t cap_ = (size_t)kSMs * 4; /* one resident round (64 registers); every block polls the headers */ \
+    const size_t cap_ = (size_t)kSMs * fused_blocks(L);                                                    \
     if (g_ > cap_) g_ = cap_;                                                                              \
     if (g_ == 0) g_ = 1; /* an empty batch still waits for the peers: the step's protocol */               \
     if (const int e_ = launch_chained(p2p_refresh_expand<L, V>, (unsigned)g_, kFusedThreads, 0, st, *c, seq, meta, \

@@ -26,13 +26,20 @@ def test_pointers_that_a_predecessor_writes_are_not_restrict():
     found, seen = [], 0
     for name, text in _sources().items():
         for kernel in _chained(text):
-            m = re.search(r"__global__ void (?:__launch_bounds__\((?:[^()]|\([^()]*\))*\) )?%s\(([^{]*)\) \{(.*?)\n}\n" % kernel, text, re.S)
+            m = re.search(r"__global__ void (?:__launch_bounds__\((?:[^()]|\([^()]*\))*\)\s+)?%s\(([^{]*)\) \{(.*?)\n}\n" % kernel, text, re.S)
             assert m, (name, kernel)
             seen += 1
             found += [(name, kernel, p) for p in re.findall(r"__restrict__\s+(\w+)", m[1]) if p not in CONSTANT]
             assert "wait_predecessor();" in m[2], (name, kernel)
     assert seen == 8, seen
     assert not found, found
+
+
+def test_grid_of_the_fused_expansion_is_what_its_launch_bounds_keep_resident():
+    text = _sources()["p2p_pull.cu"]
+    assert "__launch_bounds__(kFusedThreads, fused_blocks(LANES))" in text
+    launcher = text[text.index("int hctr_p2p_refresh_expand"):]
+    assert re.findall(r"cap_ = \(size_t\)kSMs \* ([^;]+);", launcher) == ["fused_blocks(L)"]
 
 
 PROGRAM = r"""
