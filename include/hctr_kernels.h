@@ -330,8 +330,9 @@ typedef struct hctr_p2p_ctx {
 #define HCTR_P2P_TICKET1(n) (5 * (n) + 5)
 #define HCTR_P2P_SERVED(n) (5 * (n) + 6)  /* rows this rank returned to its peers in the last step */
 
-/* Requester: (key, local version) of every unique key, written into its owner's mailbox; the thread block that
- * finishes last then publishes this rank's counts for the step (queries per owner from the batch's meta words,
+/* Requester: (key, local version) of every unique key that another rank owns, written into its owner's mailbox; this rank's
+ * own keys are counted only, and one that is not stored here sets HCTR_ERR_NOT_OWNER.  The thread block that finishes
+ * last then publishes this rank's counts for the step (queries per owner from the batch's meta words, its own among them;
  * pushed rows per owner from push_counts, null = none) and releases sequence number `seq` to every peer.
  * Replaces generateQuery + the first half of all2allExchangeQuery, csrc/core/generate_query.cu:91-106,
  * csrc/core/all2all.cu:18-44.  nrank <= 256. */
@@ -374,10 +375,9 @@ int hctr_p2p_owner_apply_pair(const hctr_p2p_ctx *c, const hctr_p2p_box *mine, u
 /* Pull side.  Nothing is compacted: the row returned for the j-th query requester s sent to this owner goes to row
  * (owner * cap + j) of s's mailbox - a place s can compute for each of its unique keys without knowing what the
  * owner decided - so neither side scans flags.
- * hctr_p2p_stale_gather (owner; after the pushed rows have been applied): for every received query, indexed FLAT
- * (q in [0, Q) runs over the queries of source 0, then source 1, ...; Q and the per-source starts are in c->cnt_in),
- * stale = (requester's version is INT64_MIN or version + pull_bound < owner's version) and the requester is not
- * this rank.  Flag bytes, and rows + versions of the stale keys, go straight into the requesters' mailboxes; the
+ * hctr_p2p_stale_gather (owner; after the pushed rows have been applied): for every query received from another rank
+ * (counts and per-source starts in c->cnt_in, in which this rank's queries to itself are counted but not answered),
+ * stale = requester's version is INT64_MIN or version + pull_bound < owner's version.  Flag bytes, and rows + versions of the stale keys, go straight into the requesters' mailboxes; the
  * thread block that finishes last releases `seq` (phase 1).  Replaces decide_outdated_kernel, the scan, the
  * segmented reduce, the select and write_return_value_kernel of csrc/core/handle_query.cu:7-78 and
  * all2allReturnOutdated / all2allReturnValue, csrc/core/all2all.cu:89-130.

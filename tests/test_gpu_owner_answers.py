@@ -1,4 +1,4 @@
-"""The owner's staleness test and row gather where the queries change their share per warp: fewer than a warp each, a
+"""What a rank asks the owners, and the owner's staleness test and row gather where the queries change their share per warp: fewer than a warp each, a
 remainder, more than one round of 32, with the rank's own (unanswered) queries in front of, between and behind the others.
 Oracle: numpy."""
 import ctypes
@@ -76,3 +76,43 @@ def test_queries(counts, width, rank):
         assert np.array_equal(rval[stale], e[at[stale]]) and np.isnan(rval[~stale]).all()
         assert np.array_equal(rver[stale], version[at[stale]]) and (rver[~stale] == -1).all()
         assert int(b["hdr"][rank * 16 + 8]) == 7
+
+
+@pytest.mark.parametrize("lost", [False, True])
+def test_queries_of_a_rank(lost):
+    """Own keys are counted and not written; one that is not stored here is reported, as its owner would."""
+    L = hb.lib()
+    L.hctr_p2p_query_send.argtypes = [vp, vp, sz, vp, vp, vp, vp, u32, vp, vp]
+    dev, n, rank, cap, rows = torch.device("cuda:0"), 3, 1, 2000, 4000
+    rng = np.random.RandomState(4)
+    counts = [700, 1100, 1]
+    seg, U = np.r_[0, np.cumsum(counts)], sum(counts)
+    owner = np.repeat(np.arange(n), counts)
+    uniq, version = rng.permutation(100_000)[:U], rng.randint(0, 99, size=rows)
+    row = rng.permutation(rows)[:U]
+    row[(owner != rank) & (rng.rand(U) < 0.5)] = -1
+    if lost:
+        row[seg[rank] + 1050] = -1
+    put = lambda a, dt: torch.from_numpy(np.ascontiguousarray(a).astype(dt)).to(dev)  # noqa: E731
+    boxes = [dict(hdr=torch.zeros(n * 16, dtype=torch.int32, device=dev), qkey=torch.full((n * cap,), -5, device=dev),
+                  qver=torch.full((n * cap,), -5, device=dev)) for _ in range(n)]
+    raw = np.array([[b[k].data_ptr() if k in b else 0 for k, _ in Box._fields_] for b in boxes], dtype=np.uint64)
+    box_d, cnt, err = torch.from_numpy(raw.view(np.int64)).to(dev), put(np.zeros(cnt_words(n)), np.int32), put([0], np.int32)
+    meta = put(np.r_[U, 0, 0, 0, seg], np.int32)
+    d = [put(uniq, np.int64), put(owner, np.uint8), put(row, np.int32), put(version, np.int64)]
+    c = Ctx(nrank=n, rank=rank, cap=cap, width=4, box=box_d.data_ptr(), cnt_in=cnt.data_ptr(), err=err.data_ptr(),
+            timeout_ns=10 ** 9)
+    assert L.hctr_p2p_query_send(ctypes.byref(c), meta.data_ptr(), U, *[t.data_ptr() for t in d], 9, None, None) == 0
+    torch.cuda.synchronize()
+    assert int(err[0]) == (2 if lost else 0)  # HCTR_ERR_NOT_OWNER
+    for p, b in enumerate(boxes):
+        hdr = b["hdr"].cpu().numpy()[rank * 16:]
+        assert (hdr[0], hdr[1], hdr[2]) == (9, counts[p], 0)
+        key, ver = (b[k].cpu().numpy() for k in ("qkey", "qver"))
+        at = slice(rank * cap, rank * cap + counts[p])
+        if p != rank:
+            mine = slice(seg[p], seg[p + 1])
+            assert np.array_equal(key[at], uniq[mine])
+            assert np.array_equal(ver[at], np.where(row[mine] >= 0, version[row[mine]], NEVER))
+            key[at] = ver[at] = -5
+        assert (key == -5).all() and (ver == -5).all()
