@@ -890,8 +890,8 @@ void HetuTable::reduceGradients(BatchDesc &b, const embed_t *grad, size_t last_l
   r.side_stream = stream_reduce_side_;
   r.fork_event = ev_rfork_;
   r.join_event = ev_rjoin_;
-  r.shared_gpu = use_p2p_ ? p2p_->sameContext() : std::strcmp(transport_->name(), "inproc") == 0;  // (thread ranks)
-  HCTR_LAUNCH(hctr_grad_reduce_apply_pack(&r, stream_reduce_));
+  const bool shared = use_p2p_ ? p2p_->sameContext() : std::strcmp(transport_->name(), "inproc") == 0;  // (thread ranks)
+  HCTR_LAUNCH(shared ? hctr_grad_reduce_apply_pack_shared(&r, stream_reduce_) : hctr_grad_reduce_apply_pack(&r, stream_reduce_));
 }
 
 // Single rank, gradients in host memory and dst in pinned host memory: the step is two transfers over the host link, which

@@ -1148,9 +1148,7 @@ extern "C" int hctr_push_decide_fused(const uint32_t *meta, int nrank, int rank,
 
 static bool streaming_shape(size_t width, bool aligned) { return aligned && width % 4 == 0 && width >= 128 && width <= 512; }
 
-extern "C" int hctr_grad_reduce_apply_pack(const hctr_reduce_args *ap, void *stream) {
-  cudaStream_t s = (cudaStream_t)stream;
-  const hctr_reduce_args a = *ap;
+static int reduce_apply_pack(const hctr_reduce_args &a, bool shared_gpu, cudaStream_t s) {
   if (a.n_unique == 0) return 0;
   if (!a.need_push || !a.push_slot || !a.uniq_owner) return (int)cudaErrorInvalidValue;
   ReduceKernelArgs ka;
@@ -1178,7 +1176,7 @@ extern "C" int hctr_grad_reduce_apply_pack(const hctr_reduce_args *ap, void *str
   const bool forked = a.n_heavy > 0 && a.side_stream && a.fork_event && a.join_event;
   cudaStream_t ls = forked ? (cudaStream_t)a.side_stream : s;
   if (a.n_heavy > 0) {
-    const size_t stage = long_stage_bytes(a.width, forked, a.shared_gpu != 0);
+    const size_t stage = long_stage_bytes(a.width, forked, shared_gpu);
     size_t need = (size_t)kLongStages * max(stage, a.width * sizeof(float));
     if (need > 200 * 1024) return (int)cudaErrorInvalidValue;  // rows wider than 12800 floats
     static PerDevice allowed[2];
@@ -1244,6 +1242,14 @@ extern "C" int hctr_grad_reduce_apply_pack(const hctr_reduce_args *ap, void *str
     if (e != cudaSuccess) return (int)e;
   }
   return launch_status();
+}
+
+extern "C" int hctr_grad_reduce_apply_pack(const hctr_reduce_args *a, void *stream) {
+  return reduce_apply_pack(*a, false, (cudaStream_t)stream);
+}
+
+extern "C" int hctr_grad_reduce_apply_pack_shared(const hctr_reduce_args *a, void *stream) {
+  return reduce_apply_pack(*a, true, (cudaStream_t)stream);
 }
 
 extern "C" int hctr_owner_update_dev(size_t n_rows_max, const uint32_t *n_rows_dev, size_t width, const int64_t *key,

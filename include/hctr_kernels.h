@@ -434,10 +434,11 @@ typedef struct hctr_reduce_args {
   void *side_stream;
   void *fork_event;
   void *join_event;
-  int shared_gpu;             /* other ranks' kernels run on this GPU meanwhile: leave them room on an SM */
 } hctr_reduce_args;
 
 int hctr_grad_reduce_apply_pack(const hctr_reduce_args *a, void *stream);
+/* The same where other ranks' kernels run on this GPU meanwhile: leaves them room on an SM. */
+int hctr_grad_reduce_apply_pack_shared(const hctr_reduce_args *a, void *stream);
 
 /* The same for a single-rank table (every key owned: rows and versions are all there is to update), in one launch.  The
  * batch's sizes are read from its meta words on the device. */

@@ -2,6 +2,7 @@
 declared in include/*.h; the drop-in module exposes the reference's names."""
 import os
 import re
+import subprocess
 
 import numpy as np
 import pytest
@@ -66,3 +67,16 @@ def test_no_device_fails_loudly():
 def test_scan_scratch_size_helper(built):
     assert built.hctr_scan_scratch_words(0) >= 1
     assert built.hctr_scan_scratch_words(1 << 20) >= (1 << 20) // 4096
+
+
+# Structs that callers fill: a field at the end of one would be read beyond the end of what a caller built before passes.
+SIZES = {"hctr_reduce_args": 27 * 8, "hctr_local_reduce_args": 13 * 8, "hctr_p2p_ctx": 56, "hctr_p2p_box": 9 * 8}
+
+
+def test_argument_structs_keep_their_size(tmp_path):
+    src, exe = tmp_path / "t.c", tmp_path / "t"
+    src.write_text('#include <stdio.h>\n#include "hctr_kernels.h"\nint main(void) {\n' +
+                   "".join(f'  printf("%zu ", sizeof({n}));\n' for n in SIZES) + "  return 0;\n}\n")
+    subprocess.run(["gcc", "-std=c11", "-I", os.path.join(ROOT, "include"), str(src), "-o", str(exe)], check=True)
+    out = subprocess.run([str(exe)], capture_output=True, text=True, check=True).stdout
+    assert [int(x) for x in out.split()] == list(SIZES.values())

@@ -22,14 +22,15 @@ class Args(ctypes.Structure):
                 ("sorted_pos", vp), ("heavy_list", vp), ("n_heavy", sz), ("uniq", vp), ("uniq_row", vp), ("need_push", vp),
                 ("push_slot", vp), ("embedding", vp), ("version", vp), ("pending", vp), ("pending_cnt", vp), ("push_key", vp),
                 ("push_updates", vp), ("push_val", vp), ("work_counter", vp), ("p2p", vp), ("uniq_owner", vp),
-                ("push_base", vp), ("side_stream", vp), ("fork_event", vp), ("join_event", vp), ("shared_gpu", ctypes.c_int)]
+                ("push_base", vp), ("side_stream", vp), ("fork_event", vp), ("join_event", vp)]
 
 
 @pytest.mark.parametrize("forked,shared", [(True, 0), (True, 1), (False, 0), (False, 1)])
 @pytest.mark.parametrize("width", [3, 64, 127, 128, 132, 256, 512, 1100])
 def test_stage_sizes(width, forked, shared):
     L = hb.lib()
-    L.hctr_grad_reduce_apply_pack.argtypes = [vp, vp]
+    reduce = L.hctr_grad_reduce_apply_pack_shared if shared else L.hctr_grad_reduce_apply_pack
+    reduce.argtypes = [vp, vp]
     rng = np.random.RandomState(width)
     dev, rows = torch.device("cuda:0"), 400
     fits = {max(1, s // (4 * width)) for s in (8192, 16384, 32768)}  # rows of a stage
@@ -60,10 +61,10 @@ def test_stage_sizes(width, forked, shared):
     for e in ev:
         e.record(s)
     torch.cuda.synchronize()
-    a = Args(n_unique=U, width=width, neg_lr=-0.25, n_heavy=len(heavy), shared_gpu=shared, **{k: v.data_ptr() for k, v in d.items()})
+    a = Args(n_unique=U, width=width, neg_lr=-0.25, n_heavy=len(heavy), **{k: v.data_ptr() for k, v in d.items()})
     if forked:
         a.side_stream, a.fork_event, a.join_event = side.cuda_stream, ev[0].cuda_event, ev[1].cuda_event
-    assert L.hctr_grad_reduce_apply_pack(ctypes.byref(a), s.cuda_stream) == 0
+    assert reduce(ctypes.byref(a), s.cuda_stream) == 0
     torch.cuda.synchronize()
     sums = np.zeros((U, width), np.float32)
     for u in range(U):
