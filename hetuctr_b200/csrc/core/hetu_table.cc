@@ -10,6 +10,7 @@
 #include "core/transport.h"
 #include "hctr_kernels.h"
 #include "utils/errors.h"
+#include "utils/same_device.h"
 #include "utils/stage_keys.h"
 
 namespace hetuCTR {
@@ -172,6 +173,16 @@ HetuTable::HetuTable(const int rank, const int nrank, const int device_id, const
 void HetuTable::initComm(const std::string &ip, int port) {
   if (nrank_ == 1) return;  // a single-rank table has nobody to talk to
   transport_ = make_transport(rank_, nrank_, ip, port, verbose_);
+  {
+    cudaDeviceProp prop;
+    HCTR_CUDA(cudaGetDeviceProperties(&prop, device_id_));
+    DeviceIdentity mine;
+    static_assert(sizeof(prop.uuid) == sizeof(mine.uuid), "");
+    std::memcpy(mine.uuid, &prop.uuid, sizeof(mine.uuid));
+    std::vector<DeviceIdentity> all(nrank_);
+    transport_->allgatherHost(&mine, all.data(), sizeof(mine));
+    shares_gpu_ = shares_device(all, rank_);
+  }
   // Exchange flavour: HCTR_EXCHANGE = auto (default) | p2p | nccl.  The peer-to-peer exchange needs one
   // process per GPU and peer access between all of them; all ranks take the same decision.
   const char *env = std::getenv("HCTR_EXCHANGE");
@@ -890,8 +901,7 @@ void HetuTable::reduceGradients(BatchDesc &b, const embed_t *grad, size_t last_l
   r.side_stream = stream_reduce_side_;
   r.fork_event = ev_rfork_;
   r.join_event = ev_rjoin_;
-  const bool shared = use_p2p_ ? p2p_->sameContext() : std::strcmp(transport_->name(), "inproc") == 0;  // (thread ranks)
-  HCTR_LAUNCH(shared ? hctr_grad_reduce_apply_pack_shared(&r, stream_reduce_) : hctr_grad_reduce_apply_pack(&r, stream_reduce_));
+  HCTR_LAUNCH(shares_gpu_ ? hctr_grad_reduce_apply_pack_shared(&r, stream_reduce_) : hctr_grad_reduce_apply_pack(&r, stream_reduce_));
 }
 
 // Single rank, gradients in host memory and dst in pinned host memory: the step is two transfers over the host link, which

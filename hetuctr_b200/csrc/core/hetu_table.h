@@ -223,6 +223,7 @@ class HetuTable {
   std::unique_ptr<Transport> transport_;
   std::unique_ptr<P2PMailbox> p2p_;  // device-driven exchange (one process per GPU, peer access); else NCCL groups
   bool use_p2p_ = false;
+  bool shares_gpu_ = false;          // another rank of the job runs on this device
   bool p2p_counts_pending_ = false;
   bool p2p_pushed_valid_ = false;    // the push counts read back with the step describe a real previous batch
   bool expand_bulk_ = false;         // HCTR_EXPAND=bulk

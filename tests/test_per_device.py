@@ -52,3 +52,30 @@ def test_launchers_keep_no_plain_static():
             if re.match(r"\s+static (bool|int|u32|unsigned|size_t)\b[^(]*[;=]", line) and "constexpr" not in line:
                 found.append(f"{os.path.basename(path)}:{n}: {line.strip()}")
     assert not found, found
+
+
+SHARED = r"""
+#include "utils/same_device.h"
+using namespace hetuCTR;
+static DeviceIdentity id(char last) {
+  DeviceIdentity d = {};
+  d.uuid[15] = last;
+  return d;
+}
+int main() {
+  const std::vector<DeviceIdentity> two_threads = {id(1), id(1)}, a_gpu_each = {id(0), id(1), id(2)}, mixed = {id(4), id(5), id(4)};
+  if (!shares_device(two_threads, 0) || !shares_device(two_threads, 1)) return 1;
+  for (int r = 0; r < 3; r++)
+    if (shares_device(a_gpu_each, r)) return 2;
+  return shares_device(mixed, 0) && !shares_device(mixed, 1) && shares_device(mixed, 2) ? 0 : 3;
+}
+"""
+
+
+def test_ranks_share_a_device_by_its_identity(tmp_path):
+    src, exe = tmp_path / "t.cc", tmp_path / "t"
+    src.write_text(SHARED)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-Wall", "-Werror", "-I", CSRC, str(src), "-o", str(exe)], check=True)
+    assert subprocess.run([str(exe)]).returncode == 0
+    table = open(os.path.join(CSRC, "core", "hetu_table.cc")).read()
+    assert "shares_device(" in table and "transport_->name()," not in table  # (not guessed from how they are connected)
