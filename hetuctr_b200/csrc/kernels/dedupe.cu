@@ -344,8 +344,9 @@ __global__ void __launch_bounds__(kThreads) ingest_keys(const long long *__restr
 // FOLLOW: the keys are on their way into src, mapped host memory, while the kernel runs.  Block 0 alone looks at the host's
 // progress and passes it on in device memory, where the others wait (bounded) for their keys: every look is a round trip over
 // the host link in front of the keys' own (with a look per 1024 keys 53,248 of them came no earlier than with the launch
-// behind the copy, with one per 256 25 us later).  The launch and the link then work while the host copies: a step of 53,248 x 128 with pageable
-// keys 73 -> 67 us.
+// behind the copy, with one per 256 25 us later).  The launch and the link then work while the host copies.  A few blocks
+// keep up with a copying thread (32,768 keys at a time arrive in 16 us); with one per 1024 keys, waiting, a batch of 150,000
+// held every SM, and blocks of other streams' kernels that need an empty one found none until the copy was done.
 struct Follow {
   const u64 *progress;  // mapped host memory: epoch << 32 | keys that are there (kLost: no more will come)
   u64 *seen;            // the same in device memory
@@ -378,13 +379,13 @@ __device__ __forceinline__ void pass_progress_on(const Follow &f, u32 n) {
   }
 }
 
-// Have the first `need` keys arrived?  (Waits; the same answer for the whole block.)
-__device__ __forceinline__ bool keys_arrived(const Follow &f, u32 need) {
+// Have the first `need` keys arrived?  (Waits; the same answer for the whole block.)  now: what thread 0 has seen, 0 at first.
+__device__ __forceinline__ bool keys_arrived(const Follow &f, u32 need, u32 &now) {
   __shared__ bool here;
+  __syncthreads();  // (the last answer has been read)
   if (threadIdx.x == 0) {
     const u64 t0 = nanoseconds();
-    u32 now = 0;
-    for (;;) {
+    while (now < need) {
       u64 v;
       asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(f.seen) : "memory");
       now = (u32)(v >> 32) == f.epoch ? (u32)v : 0u;
@@ -402,20 +403,10 @@ __device__ __forceinline__ bool keys_arrived(const Follow &f, u32 need) {
   return here;
 }
 
-template <class K, int ITEMS, bool FOLLOW>
-__global__ void __launch_bounds__(kThreads) ingest_keys_rows(const K *src, long long *dst, size_t n,
-                                                             u32 *__restrict__ meta, unsigned meta_words,
-                                                             const int32_t *__restrict__ row_of, size_t length,
-                                                             int32_t *__restrict__ pos_row, u32 *err, Follow follow) {
-  for (unsigned m = blockIdx.x * kThreads + threadIdx.x; m < meta_words; m += gridDim.x * kThreads) meta[m] = 0;
-  const size_t block = blockIdx.x - (FOLLOW ? 1 : 0), base = block * kThreads * ITEMS + threadIdx.x;
-  if (FOLLOW) {
-    if (blockIdx.x == 0) {
-      if (threadIdx.x == 0) pass_progress_on(follow, (u32)n);
-      return;
-    }
-    if (!keys_arrived(follow, (u32)min((block + 1) * kThreads * ITEMS, n))) return;
-  }
+// Keys base, base + kThreads, ... of the batch.  True: one of them is out of range.
+template <class K, int ITEMS>
+__device__ __forceinline__ bool ingest_at(size_t base, const K *src, long long *dst, size_t n, const int32_t *row_of,
+                                          size_t length, int32_t *pos_row) {
   long long k[ITEMS];
   int32_t row[ITEMS];
   bool bad = false;
@@ -441,7 +432,38 @@ __global__ void __launch_bounds__(kThreads) ingest_keys_rows(const K *src, long 
       pos_row[i] = row[j];
     }
   }
+  return bad;
+}
+
+template <class K, int ITEMS>
+__global__ void __launch_bounds__(kThreads) ingest_keys_rows(const K *src, long long *dst, size_t n,
+                                                             u32 *__restrict__ meta, unsigned meta_words,
+                                                             const int32_t *__restrict__ row_of, size_t length,
+                                                             int32_t *__restrict__ pos_row, u32 *err) {
+  for (unsigned m = blockIdx.x * kThreads + threadIdx.x; m < meta_words; m += gridDim.x * kThreads) meta[m] = 0;
+  const size_t base = (size_t)blockIdx.x * kThreads * ITEMS + threadIdx.x;
+  const bool bad = ingest_at<K, ITEMS>(base, src, dst, n, row_of, length, pos_row);
   if (bad && err) atomicOr(err, HCTR_ERR_KEY_RANGE);
+}
+
+constexpr int kFollowItems = 4;
+constexpr unsigned kFollowBlocks = 32;
+template <class K>
+__global__ void __launch_bounds__(kThreads) ingest_keys_following(const K *src, long long *dst, size_t n,
+                                                                  u32 *__restrict__ meta, unsigned meta_words,
+                                                                  const int32_t *__restrict__ row_of, size_t length,
+                                                                  int32_t *__restrict__ pos_row, Follow follow) {
+  for (unsigned m = blockIdx.x * kThreads + threadIdx.x; m < meta_words; m += gridDim.x * kThreads) meta[m] = 0;
+  if (blockIdx.x == 0) {
+    if (threadIdx.x == 0) pass_progress_on(follow, (u32)n);
+    return;
+  }
+  constexpr size_t kSpan = kThreads * kFollowItems;
+  u32 seen = 0;
+  for (size_t first = (blockIdx.x - 1) * kSpan; first < n; first += (gridDim.x - 1) * kSpan) {
+    if (!keys_arrived(follow, (u32)min(first + kSpan, n), seen)) return;
+    ingest_at<K, kFollowItems>(first + threadIdx.x, src, dst, n, row_of, length, pos_row);
+  }
 }
 
 }  // namespace hctr
@@ -454,11 +476,11 @@ static int launch_ingest(const K *src, int64_t *dst, size_t n, uint32_t *meta, u
   cudaStream_t s = (cudaStream_t)stream;
   // four keys per thread where that still leaves every SM a block
   if (n >= (size_t)kThreads * 4 * kSMs)
-    ingest_keys_rows<K, 4, false><<<grid_for(n, kThreads * 4), kThreads, 0, s>>>(
-        src, (long long *)dst, n, meta, meta_words, row_of, length, pos_row, err, Follow{});
+    ingest_keys_rows<K, 4><<<grid_for(n, kThreads * 4), kThreads, 0, s>>>(src, (long long *)dst, n, meta, meta_words,
+                                                                         row_of, length, pos_row, err);
   else
-    ingest_keys_rows<K, 1, false><<<grid_for(n, kThreads), kThreads, 0, s>>>(
-        src, (long long *)dst, n, meta, meta_words, row_of, length, pos_row, err, Follow{});
+    ingest_keys_rows<K, 1><<<grid_for(n, kThreads), kThreads, 0, s>>>(src, (long long *)dst, n, meta, meta_words,
+                                                                     row_of, length, pos_row, err);
   count_launches(1);
   return launch_status();
 }
@@ -468,16 +490,15 @@ extern "C" int hctr_ingest_keys_following(const void *src, int key_bytes, int64_
                                           const unsigned long long *progress, unsigned long long *seen, uint32_t epoch,
                                           uint32_t *gave_up, unsigned limit_us, void *stream) {
   cudaStream_t s = (cudaStream_t)stream;
-  constexpr int kItems = 4;
   if (epoch == 0 || n >= ((size_t)1 << 31) || (key_bytes != 4 && key_bytes != 8)) return (int)cudaErrorInvalidValue;
   const Follow f = {progress, seen, epoch, gave_up, (u64)limit_us * 1000};
-  const unsigned grid = grid_for(n, kThreads * kItems) + 1;
+  const unsigned grid = min(grid_for(n, kThreads * kFollowItems), kFollowBlocks) + 1;
   if (key_bytes == 8)
-    ingest_keys_rows<long long, kItems, true><<<grid, kThreads, 0, s>>>((const long long *)src, (long long *)dst, n, meta,
-                                                                        meta_words, row_of, length, pos_row, nullptr, f);
+    ingest_keys_following<<<grid, kThreads, 0, s>>>((const long long *)src, (long long *)dst, n, meta, meta_words, row_of,
+                                                    length, pos_row, f);
   else
-    ingest_keys_rows<int32_t, kItems, true><<<grid, kThreads, 0, s>>>((const int32_t *)src, (long long *)dst, n, meta,
-                                                                      meta_words, row_of, length, pos_row, nullptr, f);
+    ingest_keys_following<<<grid, kThreads, 0, s>>>((const int32_t *)src, (long long *)dst, n, meta, meta_words, row_of,
+                                                    length, pos_row, f);
   count_launches(1);
   return launch_status();
 }

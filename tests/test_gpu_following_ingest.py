@@ -5,6 +5,7 @@ import ctypes
 import os
 import subprocess
 import sys
+import time
 
 import numpy as np
 import pytest
@@ -73,6 +74,46 @@ def test_chunks(n, width, lost):
     else:  # (a block that looks late finds that the rest is lost)
         assert there <= starts[-1]
     assert not bool(meta.any())
+
+
+def test_a_waiting_ingest_leaves_room_for_other_streams():
+    """A kernel whose blocks need an empty SM (a tile of the grouping: 1024 threads) runs while the ingest of a batch that would
+    fill every SM waits for its keys."""
+    from test_gpu_group_keys import GroupArgs
+
+    L = hb.lib()
+    L.hctr_ingest_keys_following.argtypes = [vp, ctypes.c_int, vp, sz, vp, u32, vp, sz, vp, vp, vp, u32, vp, u32, vp]
+    L.hctr_group_keys.argtypes = [ctypes.POINTER(GroupArgs), vp]
+    dev, n, m, length = torch.device("cuda:0"), 1_300_000, 1000, 5000
+
+    def z(count, dt=torch.int32):
+        return torch.zeros(count, dtype=dt, device=dev)
+
+    keys = torch.arange(n) % length
+    src, progress, gave_up = keys.int().pin_memory(), torch.zeros(1, dtype=torch.int64).pin_memory(), torch.zeros(1).int().pin_memory()
+    seen, dst, rows, meta = z(1, torch.int64), z(n, torch.int64), z(n), z(9)
+    t = dict(keys=keys[:m].to(dev), owner_of=z(length, torch.uint8), pos_row=z(m), pairs0=z(m, torch.int64), pairs1=z(m, torch.int64),
+             sort_keys=z(m), tile_counts=z(512 * 256), hist=z(2048), tile_flags=z(1024), chain_scratch=z(512), uniq=z(m, torch.int64),
+             uniq_owner=z(m, torch.uint8), uniq_row=z(m), run_start=z(m + 1), sorted_pos=z(m), idx_map=z(m), chunk_key=z(m),
+             heavy_list=z(m), meta=z(6))
+    a = GroupArgs(batch=m, length=length, nrank=1, epoch=1, **{k: v.data_ptr() for k, v in t.items()})
+    first, other = torch.cuda.Stream(), torch.cuda.Stream()
+    assert L.hctr_group_keys(ctypes.byref(a), other.cuda_stream) == 0  # (loads the kernel)
+    torch.cuda.synchronize()
+    assert L.hctr_ingest_keys_following(src.data_ptr(), 4, dst.data_ptr(), n, meta.data_ptr(), 9, None, length, rows.data_ptr(),
+                                        progress.data_ptr(), seen.data_ptr(), 3, gave_up.data_ptr(), 1_000_000,
+                                        first.cuda_stream) == 0
+    time.sleep(0.01)
+    assert L.hctr_group_keys(ctypes.byref(a), other.cuda_stream) == 0
+    done = other.record_event()
+    until = time.time() + 0.3
+    while not done.query() and time.time() < until:
+        time.sleep(0.001)
+    ran = done.query()
+    progress[0] = 3 << 32 | n
+    torch.cuda.synchronize()
+    assert ran and int(gave_up[0]) == 0
+    assert torch.equal(dst.cpu(), keys) and torch.equal(rows.cpu(), keys.int()) and int(t["meta"][0]) == m
 
 
 def _steps(oracle_mod, sizes, bad=()):
