@@ -276,7 +276,7 @@ class HetuTable {
   void ingestKeys(BatchDesc &b, const void *keys, size_t n, cudaStream_t s);
   bool stageAndFollow(BatchDesc &b, const int64_t *keys, size_t n, size_t each, void *staged, cudaStream_t s);
   void settleIngest(BatchDesc &b);
-  unsigned follow_limit_us_ = 20000;  // HCTR_FOLLOW_LIMIT_US: a thread that lost its processor for longer finds the keys ingested anew
+  unsigned follow_limit_us_ = 1000;  // HCTR_FOLLOW_LIMIT_US: a thread that lost its processor for longer finds the keys ingested anew
   // how far the staging of a batch has got (in the same mapped memory)
   unsigned long long *h_progress_ = nullptr, *d_progress_ = nullptr;
   bool can_follow_ = true;    // launches return while their kernels run (not under tools that take launches one by one)

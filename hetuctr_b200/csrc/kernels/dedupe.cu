@@ -352,7 +352,7 @@ struct Follow {
   u64 *seen;            // the same in device memory
   u32 epoch;
   u32 *gave_up;
-  u64 limit_ns;
+  u64 limit_ns;  // without a further key
 };
 constexpr u32 kLost = 0xffffffffu;
 
@@ -363,18 +363,19 @@ __device__ __forceinline__ u64 nanoseconds() {
 }
 
 __device__ __forceinline__ void pass_progress_on(const Follow &f, u32 n) {
-  const u64 t0 = nanoseconds();
+  u64 since = nanoseconds();  // when something last came
   u32 last = 0;
   while (last < n) {  // (kLost is not)
     u64 v;
     asm volatile("ld.acquire.sys.global.u64 %0, [%1];" : "=l"(v) : "l"(f.progress) : "memory");
     u32 now = (u32)(v >> 32) == f.epoch ? (u32)v : 0u;
-    if (now == last && nanoseconds() - t0 > f.limit_ns) {
+    if (now <= last && nanoseconds() - since > f.limit_ns) {
       *f.gave_up = 1;
       now = kLost;
     }
-    if (now == last) continue;
+    if (now <= last) continue;
     last = now;
+    since = nanoseconds();
     asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(f.seen), "l"((u64)f.epoch << 32 | now) : "memory");
   }
 }
@@ -384,13 +385,15 @@ __device__ __forceinline__ bool keys_arrived(const Follow &f, u32 need, u32 &now
   __shared__ bool here;
   __syncthreads();  // (the last answer has been read)
   if (threadIdx.x == 0) {
-    const u64 t0 = nanoseconds();
+    u64 since = nanoseconds();
     while (now < need) {
       u64 v;
       asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(f.seen) : "memory");
+      const u32 before = now;
       now = (u32)(v >> 32) == f.epoch ? (u32)v : 0u;
       if (now >= need) break;
-      if (nanoseconds() - t0 > 2 * f.limit_ns + 1000000) {  // (block 0 gives up long before)
+      if (now != before) since = nanoseconds();
+      if (nanoseconds() - since > 2 * f.limit_ns + 1000000) {  // (block 0 gives up long before)
         *f.gave_up = 1;
         now = kLost;
         break;

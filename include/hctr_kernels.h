@@ -203,7 +203,7 @@ int hctr_ingest_keys_rows(const void *src, int key_bytes, int64_t *dst, size_t n
 /* The same for keys that the caller goes on putting into src (mapped host memory, range already checked) after this call, in
  * ascending order: *progress (mapped host memory) = epoch << 32 | number of keys that are in place, the low word 0xffffffff
  * when the rest will not come; epoch is non-zero and no earlier call's.  seen: a device word of the same kind that nobody else
- * uses meanwhile.  After limit_us without the last key the kernel stores 1 to *gave_up (mapped host memory) and returns with
+ * uses meanwhile.  After limit_us without a further key the kernel stores 1 to *gave_up (mapped host memory) and returns with
  * the keys it has seen ingested.  n < 2^31. */
 int hctr_ingest_keys_following(const void *src, int key_bytes, int64_t *dst, size_t n, uint32_t *meta, unsigned meta_words,
                                const int32_t *row_of, size_t length, int32_t *pos_row, const unsigned long long *progress,

@@ -76,6 +76,25 @@ def test_chunks(n, width, lost):
     assert not bool(meta.any())
 
 
+def test_the_limit_is_for_the_next_keys():
+    """Twelve chunks, the last of them long after the limit has passed since the launch, but none of them late by itself."""
+    L = hb.lib()
+    L.hctr_ingest_keys_following.argtypes = [vp, ctypes.c_int, vp, sz, vp, u32, vp, sz, vp, vp, vp, u32, vp, u32, vp]
+    dev, n, limit = torch.device("cuda:0"), 12 * 4096, 0.2
+    keys = torch.arange(n)
+    src, progress, gave_up = keys.int().pin_memory(), torch.zeros(1, dtype=torch.int64).pin_memory(), torch.zeros(1).int().pin_memory()
+    seen, dst = torch.zeros(1, dtype=torch.int64, device=dev), torch.zeros(n, dtype=torch.int64, device=dev)
+    rows, meta = torch.zeros(n, dtype=torch.int32, device=dev), torch.zeros(9, dtype=torch.int32, device=dev)
+    torch.cuda.synchronize()
+    assert L.hctr_ingest_keys_following(src.data_ptr(), 4, dst.data_ptr(), n, meta.data_ptr(), 9, None, n, rows.data_ptr(),
+                                        progress.data_ptr(), seen.data_ptr(), 3, gave_up.data_ptr(), int(limit * 1e6), None) == 0
+    for chunk in range(12):
+        time.sleep(limit / 4)
+        progress[0] = 3 << 32 | (chunk + 1) * 4096
+    torch.cuda.synchronize()
+    assert int(gave_up[0]) == 0 and torch.equal(dst.cpu(), keys) and torch.equal(rows.cpu(), keys.int())
+
+
 def test_a_waiting_ingest_leaves_room_for_other_streams():
     """A kernel whose blocks need an empty SM (a tile of the grouping: 1024 threads) runs while the ingest of a batch that would
     fill every SM waits for its keys."""
