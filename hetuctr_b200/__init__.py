@@ -78,6 +78,7 @@ def lib():
     L.hctr_table_export.argtypes = [vp, ctypes.c_char_p]
     L.hctr_table_import.argtypes = [vp, ctypes.c_char_p]
     L.hctr_table_stats.argtypes = [vp, vp]
+    L.hctr_table_ingest_counts.argtypes = [vp, vp]
     L.hctr_table_exchange_name.restype = c.c_char_p
     L.hctr_table_exchange_name.argtypes = [vp]
     L.hctr_table_stream.restype = vp
@@ -219,6 +220,12 @@ class Table:
         out = (ctypes.c_longlong * len(self._STATS))()
         self._lib.hctr_table_stats(self._h, out)
         return dict(zip(self._STATS, list(out)))
+
+    def ingest_counts(self):
+        """Batches of host keys whose ingest followed the copy, of those the ones ingested anew, and the ones given up at once."""
+        out = (ctypes.c_longlong * 3)()
+        self._lib.hctr_table_ingest_counts(self._h, out)
+        return dict(zip(("followed", "redone", "not_started"), list(out)))
 
     PHASES = ("dedupe", "push_decide", "reduce", "query", "exchange", "owner_update", "stale_gather", "refresh",
               "expand", "owner_apply")

@@ -158,6 +158,14 @@ int hctr_table_stats(hctr_table *t, long long out[13]) {
   return 0;
 }
 
+int hctr_table_ingest_counts(hctr_table *t, long long out[3]) {
+  const hetuCTR::IngestCounts &c = t->impl->ingestCounts();
+  out[0] = (long long)c.followed;
+  out[1] = (long long)c.redone;
+  out[2] = (long long)c.not_started;
+  return 0;
+}
+
 int hctr_table_profile(hctr_table *t, int enable) {
   t->impl->setProfile(enable);
   return 0;

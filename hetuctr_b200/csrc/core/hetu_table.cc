@@ -498,12 +498,10 @@ void HetuTable::ingestKeys(BatchDesc &b, const void *keys, size_t n, cudaStream_
       void *dev = nullptr;
       HCTR_CUDA(cudaHostGetDevicePointer(&dev, b.h_keys, 0));
       const int64_t *src = static_cast<const int64_t *>(keys);
-      bool good = true, done = false;
-      if (nrank_ == 1 && n >= kFollow && n < ((size_t)1 << 31) && can_follow_) {
-        done = stageAndFollow(b, src, n, each, dev, s);
-        good = done || !can_follow_;
-      }
-      for (size_t off = 0; off < n && good && !done; off += kChunk) {
+      Following how = Following::kNot;
+      if (nrank_ == 1 && n >= kFollow && n < ((size_t)1 << 31) && follow_.tryNow()) how = stageAndFollow(b, src, n, each, dev, s);
+      bool good = how != Following::kBadKey;
+      for (size_t off = 0; off < n && how == Following::kNot && good; off += kChunk) {
         const size_t m = std::min(kChunk, n - off);
         char *to = static_cast<char *>(b.h_keys) + off * each;
         good = narrow ? stage_keys(src + off, reinterpret_cast<int32_t *>(to), m, kEmbeddingIDMax)
@@ -546,9 +544,10 @@ void HetuTable::ingestKeys(BatchDesc &b, const void *keys, size_t n, cudaStream_
 }
 
 // Launches the ingest of n keys, then puts them into b's staging (`staged` on the device), chunk by chunk, with the kernel
-// behind.  False: a key is out of range (the kernel has been told), or launches wait for their kernels here and this one has
-// given up (can_follow_ is false from then on).  What the kernel has made of it is seen to by settleIngest.
-bool HetuTable::stageAndFollow(BatchDesc &b, const int64_t *keys, size_t n, size_t each, void *staged, cudaStream_t s) {
+// behind.  kBadKey: a key is out of range (the kernel has been told).  kNot: the kernel has given up before a single key was
+// there - the thread has lost its processor, or launches wait for their kernels here, as some tools make them.  What the kernel
+// has made of it otherwise is seen to by settleIngest.
+HetuTable::Following HetuTable::stageAndFollow(BatchDesc &b, const int64_t *keys, size_t n, size_t each, void *staged, cudaStream_t s) {
   constexpr size_t kKeys = 4096;  // between two words about it: 2 us of copying
   const uint32_t epoch = nextEpoch();
   const int32_t *row_of = rows_are_keys_ ? nullptr : d_row_of_.as<int32_t>();
@@ -557,12 +556,14 @@ bool HetuTable::stageAndFollow(BatchDesc &b, const int64_t *keys, size_t n, size
                                          b.pos_row.as<int32_t>(), d_progress_,
                                          reinterpret_cast<unsigned long long *>(d_err_.as<char>() + 128), epoch,
                                          d_ingest_err_ + 3, follow_limit_us_, s));
-  if (reinterpret_cast<volatile uint32_t *>(h_ingest_err_)[3]) {  // it has run, before a single key was there
+  if (reinterpret_cast<volatile uint32_t *>(h_ingest_err_)[3]) {
     HCTR_CUDA(cudaStreamSynchronize(s));
     h_ingest_err_[3] = 0;
-    can_follow_ = false;
-    return false;
+    follow_.failed();
+    ingest_counts_.not_started++;
+    return Following::kNot;
   }
+  ingest_counts_.followed++;
   b.h_keys_busy = b.following = true;
   bool good = true;
   for (size_t off = 0; off < n && good; off += kKeys) {
@@ -574,7 +575,7 @@ bool HetuTable::stageAndFollow(BatchDesc &b, const int64_t *keys, size_t n, size
     __atomic_store_n(h_progress_, (unsigned long long)epoch << 32 | there, __ATOMIC_RELEASE);
   }
   if (!good) b.following = false;
-  return good;
+  return good ? Following::kDone : Following::kBadKey;
 }
 
 // An ingest that followed the staging of batch b: did it see all of it?  Called before anything reads what it made, behind
@@ -583,8 +584,13 @@ void HetuTable::settleIngest(BatchDesc &b) {
   if (!b.following) return;
   b.following = false;
   HCTR_CUDA(cudaEventSynchronize(ev_keys_));
-  if (!h_ingest_err_[3]) return;
+  if (!h_ingest_err_[3]) {
+    follow_.worked();
+    return;
+  }
   h_ingest_err_[3] = 0;
+  follow_.failed();
+  ingest_counts_.redone++;
   const size_t each = kEmbeddingIDMax <= ((size_t)1 << 31) ? sizeof(int32_t) : sizeof(int64_t);
   void *staged = nullptr;
   HCTR_CUDA(cudaHostGetDevicePointer(&staged, b.h_keys, 0));

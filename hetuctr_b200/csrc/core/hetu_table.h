@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "hctr_kernels.h"
+#include "utils/backoff.h"
 
 namespace hetuCTR {
 
@@ -100,6 +101,10 @@ struct StepStats {  // sizes of the last push_pull, for roofline arithmetic
   size_t wait_queries_us = 0, wait_returns_us = 0;
 };
 
+struct IngestCounts {  // batches since the table was made, see hctr_table_ingest_counts
+  size_t followed = 0, redone = 0, not_started = 0;
+};
+
 // Phases timed with CUDA events on the table's stream when profiling is enabled.
 enum Phase {
   kPhDedupe = 0,      // hctr_dedupe_map
@@ -167,6 +172,7 @@ class HetuTable {
     stats_.prev_unique = stats_.prev_batch ? prev_batch_.unique_size : 0;
     return stats_;
   }
+  const IngestCounts &ingestCounts() const { return ingest_counts_; }
   // "none" (single rank), "nccl", "inproc" or "p2p"
   const char *exchangeName() const;
   // Per-phase device time.  While enabled, every phase is bracketed by two events on the table's
@@ -274,12 +280,14 @@ class HetuTable {
   void dropBadBatch(BatchDesc &b);
   void reserveStaging(BatchDesc &b, size_t bytes, size_t each);
   void ingestKeys(BatchDesc &b, const void *keys, size_t n, cudaStream_t s);
-  bool stageAndFollow(BatchDesc &b, const int64_t *keys, size_t n, size_t each, void *staged, cudaStream_t s);
+  enum class Following { kNot, kDone, kBadKey };
+  Following stageAndFollow(BatchDesc &b, const int64_t *keys, size_t n, size_t each, void *staged, cudaStream_t s);
   void settleIngest(BatchDesc &b);
   unsigned follow_limit_us_ = 1000;  // HCTR_FOLLOW_LIMIT_US: a thread that lost its processor for longer finds the keys ingested anew
   // how far the staging of a batch has got (in the same mapped memory)
   unsigned long long *h_progress_ = nullptr, *d_progress_ = nullptr;
-  bool can_follow_ = true;    // launches return while their kernels run (not under tools that take launches one by one)
+  Backoff follow_;  // (a thread that keeps losing its processor, tools that take launches one by one)
+  IngestCounts ingest_counts_;
   size_t h_pinned_words_ = 0;
 
   BatchDesc cur_batch_, prev_batch_;

@@ -89,6 +89,11 @@ int hctr_table_import(hctr_table *t, const char *path);
  * peer's returned rows (peer-to-peer exchange; 0 otherwise). */
 int hctr_table_stats(hctr_table *t, long long out[13]);
 
+/* Batches of host keys since the table was made: {followed: the ingest was launched first and followed the keys; redone: of
+ * those, it gave up waiting (HCTR_FOLLOW_LIMIT_US) and the batch was ingested anew; not_started: it gave up before the first
+ * key was there and the batch went another way}. */
+int hctr_table_ingest_counts(hctr_table *t, long long out[3]);
+
 /* Per-phase device time.  hctr_table_profile(t, k): k = 0 off, 1 every step, k > 1 every k-th step (the
  * timing events cost the step a few microseconds per phase, sampling keeps that out of a benchmark).  In a
  * timed step each phase of preprocess/push_pull is bracketed by two CUDA events on the stream it runs on; hctr_table_phase_times returns the accumulated milliseconds and

@@ -136,7 +136,8 @@ def test_a_waiting_ingest_leaves_room_for_other_streams():
 
 
 def _steps(oracle_mod, sizes, bad=()):
-    """Training and serving steps with pageable keys, against the oracle; a batch of `bad` has one key out of range."""
+    """Training and serving steps with pageable keys, against the oracle; a batch of `bad` has one key out of range.  Returns how
+    the keys were ingested."""
     from test_gpu_parity import assert_state_parity, make_worlds
 
     N, W = 60_000, 4
@@ -160,43 +161,87 @@ def _steps(oracle_mod, sizes, bad=()):
         got, want = gw.push_pull(grads), ow.push_pull(grads)
         assert np.array_equal(got[0], want[0]), s
         before = n
+    counts = gw.tables[0].ingest_counts()
     assert_state_parity(gw, ow, exact=True)
     gw.close()
+    return counts
 
 
 SIZES = [40_000, 32_768, 32_767, 70_000, 45_057, 300, 50_000, 36_864, 140_001]
 
 
-@pytest.mark.parametrize("limit", ["20000", "3", "0"])  # (3 us: the kernel gives up while the keys are being staged)
-def test_tables(oracle_mod, monkeypatch, limit):
-    monkeypatch.setenv("HCTR_FOLLOW_LIMIT_US", limit)
-    _steps(oracle_mod, SIZES)
+# No limit: the kernel gives up when it looks twice without a further chunk in between (2 us of copying), so it hardly ever keeps
+# up; a second: it always does.
+AT_ONCE, PATIENT = "0", "1000000"
+
+
+def test_tables_keep_up(oracle_mod, monkeypatch):
+    monkeypatch.setenv("HCTR_FOLLOW_LIMIT_US", PATIENT)
+    assert _steps(oracle_mod, SIZES) == {"followed": sum(n >= 32_768 for n in SIZES), "redone": 0, "not_started": 0}
+
+
+def test_tables_give_up(oracle_mod, monkeypatch):
+    monkeypatch.setenv("HCTR_FOLLOW_LIMIT_US", AT_ONCE)
+    counts = _steps(oracle_mod, SIZES * 4)
+    assert counts["redone"] >= 1
+    # given up is not given up for good
+    assert counts["followed"] + counts["not_started"] >= 4
 
 
 def test_bad_key(oracle_mod):
     _steps(oracle_mod, SIZES + SIZES, bad=(3, 10))
 
 
-def test_two_batches_in_a_row(oracle_mod):
+@pytest.mark.parametrize("limit", [PATIENT, AT_ONCE])
+def test_two_batches_in_a_row(oracle_mod, monkeypatch, limit):
     from test_gpu_parity import make_worlds
 
-    N, W = 60_000, 4
-    rng = np.random.RandomState(5)
-    gw, ow = make_worlds(oracle_mod, 1, N, W, 0, 0, 0.5, np.zeros(N, dtype=np.uint8), [np.arange(N)], keys_on_device=False)
-    for n in (50_000, 80_000):
-        keys = [rng.randint(N, size=n)]
-        gw.preprocess(keys)
-        ow.preprocess(keys)
-    grad = [rng.normal(0, 1, size=(50_000, W)).astype(np.float32)]
-    assert np.array_equal(gw.push_pull(grad)[0], ow.push_pull(grad)[0])
-    gw.close()
+    monkeypatch.setenv("HCTR_FOLLOW_LIMIT_US", limit)
+    N, W, redone = 60_000, 4, 0
+    for seed in range(6):
+        rng = np.random.RandomState(seed)
+        gw, ow = make_worlds(oracle_mod, 1, N, W, 0, 0, 0.5, np.zeros(N, dtype=np.uint8), [np.arange(N)], keys_on_device=False)
+        for n in (50_000, 80_000):
+            keys = [rng.randint(N, size=n)]
+            gw.preprocess(keys)
+            ow.preprocess(keys)
+        grad = [rng.normal(0, 1, size=(50_000, W)).astype(np.float32)]
+        assert np.array_equal(gw.push_pull(grad)[0], ow.push_pull(grad)[0])
+        redone += gw.tables[0].ingest_counts()["redone"]
+        gw.close()
+    assert (redone > 0) == (limit == AT_ONCE)
+
+
+@pytest.mark.parametrize("limit", [PATIENT, AT_ONCE])
+def test_gradients_and_rows_in_pinned_memory(oracle_mod, monkeypatch, limit):
+    """The step that writes rows while gradients still come in reads the batch's rows earlier than the others."""
+    from test_gpu_parity import make_worlds
+
+    monkeypatch.setenv("HCTR_FOLLOW_LIMIT_US", limit)
+    N, W, redone = 60_000, 8, 0
+    for seed in range(6):
+        rng = np.random.RandomState(seed)
+        gw, ow = make_worlds(oracle_mod, 1, N, W, 0, 0, 0.5, np.zeros(N, dtype=np.uint8), [np.arange(N)], keys_on_device=False,
+                             buffers="pinned")
+        before = None
+        for n in (20_000, 50_000):  # (only the second one is followed)
+            keys = [rng.randint(N, size=n)]
+            gw.preprocess(keys)
+            ow.preprocess(keys)
+            grad = None if before is None else [rng.normal(0, 1, size=(before, W)).astype(np.float32)]
+            assert np.array_equal(gw.push_pull(grad)[0], ow.push_pull(grad)[0])
+            before = n
+        redone += gw.tables[0].ingest_counts()["redone"]
+        gw.close()
+    assert (redone > 0) == (limit == AT_ONCE)
 
 
 def test_launches_that_wait_for_their_kernels():
     code = ("import sys; sys.path[:0] = [%r, %r]\n"
             "from oracle import build, hetu_oracle\n"
             "import test_gpu_following_ingest as t\n"
-            "t._steps(hetu_oracle, t.SIZES)\nprint('same')\n" % (ROOT, os.path.join(ROOT, "tests")))
+            "c = t._steps(hetu_oracle, t.SIZES * 3)\n"
+            "assert c['followed'] == 0 and c['not_started'] >= 3, c\nprint('same')\n" % (ROOT, os.path.join(ROOT, "tests")))
     r = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, CUDA_LAUNCH_BLOCKING="1"), cwd=ROOT,
                        capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and "same" in r.stdout, r.stderr[-2000:]

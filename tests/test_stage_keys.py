@@ -1,5 +1,6 @@
 """The checked copy of a host key batch, compiled on its own: what it copies, and that it refuses a key outside the table
-wherever it stands - in the vector body, in the tail behind it, first or last."""
+wherever it stands - in the vector body, in the tail behind it, first or last; and when a way of ingesting keys that has failed
+is tried again."""
 import os
 import subprocess
 
@@ -62,3 +63,35 @@ def test_keys_are_copied_and_checked(tmp_path):
         subprocess.run(["g++", "-std=c++17", "-O2", "-I", CSRC, str(src), "-o", str(exe)], check=True)
         r = subprocess.run([str(exe)], stdout=subprocess.PIPE, text=True)
         assert r.returncode == 0, r.stdout
+
+
+BACKOFF = r"""
+#include "utils/backoff.h"
+int main() {
+  hetuCTR::Backoff b;
+  for (int i = 0; i < 5; i++) {
+    if (!b.tryNow()) return 1;
+    b.worked();
+  }
+  unsigned pause = 1;
+  for (int i = 0; i < 14; i++) {  // never off for good
+    if (!b.tryNow()) return 2;
+    b.failed();
+    for (unsigned k = 0; k < pause; k++)
+      if (b.tryNow()) return 3;
+    pause = pause < 1024 ? 2 * pause : 1024;
+  }
+  if (!b.tryNow()) return 4;
+  b.worked();
+  if (!b.tryNow()) return 5;
+  b.failed();
+  return !b.tryNow() && b.tryNow() ? 0 : 6;
+}
+"""
+
+
+def test_a_failed_way_is_tried_again(tmp_path):
+    src, exe = tmp_path / "t.cc", tmp_path / "t"
+    src.write_text(BACKOFF)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-Wall", "-Werror", "-I", CSRC, str(src), "-o", str(exe)], check=True)
+    assert subprocess.run([str(exe)]).returncode == 0
