@@ -470,7 +470,9 @@ void HetuTable::ingestKeys(BatchDesc &b, const void *keys, size_t n, cudaStream_
   constexpr size_t kStagePinned = 16384;
   constexpr size_t kChunk = 65536;
   // Launched in front of the copy, the kernel that waits for it takes 26,624 keys no earlier (36.9 us per step of x 16, 35.8
-  // with the launch behind), 53,248 6 us earlier (67 for 73 us of x 128).
+  // with the launch behind), 53,248 6 us earlier (67 for 73 us of x 128).  A table that serves does not follow: nothing runs
+  // in front of the expansion there, and the host's look at what the kernel has made of the batch would stand between the
+  // two (53,248 x 16 42.6 us per request, 46.5 followed; x 128 48.3, 52.0).
   constexpr size_t kFollow = 32768;
   const unsigned meta_words = (unsigned)(HCTR_META_WORDS + nrank_ + 1 + 2);
   const int32_t *row_of = rows_are_keys_ ? nullptr : d_row_of_.as<int32_t>();
@@ -499,7 +501,8 @@ void HetuTable::ingestKeys(BatchDesc &b, const void *keys, size_t n, cudaStream_
       HCTR_CUDA(cudaHostGetDevicePointer(&dev, b.h_keys, 0));
       const int64_t *src = static_cast<const int64_t *>(keys);
       Following how = Following::kNot;
-      if (nrank_ == 1 && n >= kFollow && n < ((size_t)1 << 31) && follow_.tryNow()) how = stageAndFollow(b, src, n, each, dev, s);
+      const bool training = pulls_in_a_row_ < 2;
+      if (nrank_ == 1 && training && n >= kFollow && n < ((size_t)1 << 31) && follow_.tryNow()) how = stageAndFollow(b, src, n, each, dev, s);
       bool good = how != Following::kBadKey;
       for (size_t off = 0; off < n && how == Following::kNot && good; off += kChunk) {
         const size_t m = std::min(kChunk, n - off);
@@ -1131,6 +1134,7 @@ void HetuTable::pushPull(embed_t *grad, embed_t *dst) {
     // do.  (The first one is how every training loop starts.)
     if (grad != nullptr || !serving_) flushDedupe(cur);
     serving_ = grad == nullptr;
+    pulls_in_a_row_ = serving_ ? pulls_in_a_row_ + 1 : 0;
   } else if (use_p2p_) {
     exchangeP2P(dst_dev);
   } else {

@@ -241,6 +241,7 @@ class HetuTable {
   void detectKeyStride(const BatchDesc &b);
   bool batch_open_ = false;          // preprocess done, push_pull not yet
   bool serving_ = false;             // the last push_pull brought no gradients (single-rank tables)
+  size_t pulls_in_a_row_ = 0;        // push_pulls without gradients, the last ones
   bool prev_push_valid_ = false;     // prev_batch_'s push counts describe a push of this step
 
   // table state

@@ -180,6 +180,25 @@ def test_tables_keep_up(oracle_mod, monkeypatch):
     assert _steps(oracle_mod, SIZES) == {"followed": sum(n >= 32_768 for n in SIZES), "redone": 0, "not_started": 0}
 
 
+def test_a_table_that_serves_does_not_follow(oracle_mod, monkeypatch):
+    from test_gpu_parity import make_worlds
+
+    monkeypatch.setenv("HCTR_FOLLOW_LIMIT_US", PATIENT)
+    N, W, n = 60_000, 4, 40_000
+    rng = np.random.RandomState(7)
+    gw, ow = make_worlds(oracle_mod, 1, N, W, 0, 0, 0.5, np.zeros(N, dtype=np.uint8), [np.arange(N)], keys_on_device=False)
+    followed = []
+    for grads in (False, False, False, False, True, True):
+        keys = [rng.randint(N, size=n)]
+        gw.preprocess(keys)
+        ow.preprocess(keys)
+        grad = [rng.normal(0, 1, size=(n, W)).astype(np.float32)] if grads else None
+        assert np.array_equal(gw.push_pull(grad)[0], ow.push_pull(grad)[0])
+        followed.append(gw.tables[0].ingest_counts()["followed"])
+    assert followed == [1, 2, 2, 2, 2, 3]  # (two pulls in a row are how it is told)
+    gw.close()
+
+
 def test_tables_give_up(oracle_mod, monkeypatch):
     monkeypatch.setenv("HCTR_FOLLOW_LIMIT_US", AT_ONCE)
     counts = _steps(oracle_mod, SIZES * 4)
