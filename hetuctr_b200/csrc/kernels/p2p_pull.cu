@@ -13,12 +13,11 @@ constexpr int kPullThreads = 1024;  // fat blocks, at most a few per SM: every b
 constexpr long long kInvalidVersion = INT64_MIN;
 constexpr int kCopyUnroll = 4;
 
-// The elements of `cnt` rows (cnt <= 32; lane i holds the pointers of row i) moved as ONE flat range by the
-// warp, kCopyUnroll independent loads in flight per lane.  COMBINE: dst = src + add (the cache refresh), else a
-// plain copy.  All 32 lanes must call it.
-template <class R, bool COMBINE>
-__device__ __forceinline__ void warp_move_rows(u32 cnt, u32 E, const typename R::T *src_row,
-                                               const typename R::T *add_row, typename R::T *dst_row) {
+// dst = src + add (the cache refresh) for `cnt` rows (cnt <= 32; lane i holds the pointers of row i): their elements as ONE
+// flat range for the warp, kCopyUnroll independent loads in flight per lane.  All 32 lanes must call it.
+template <class R>
+__device__ __forceinline__ void warp_refresh_rows(u32 cnt, u32 E, const typename R::T *src_row,
+                                                  const typename R::T *add_row, typename R::T *dst_row) {
   typedef typename R::T T;
   const unsigned lane = threadIdx.x & 31;
   const u32 total = cnt * E;
@@ -38,14 +37,14 @@ __device__ __forceinline__ void warp_move_rows(u32 cnt, u32 E, const typename R:
       d[k] = reinterpret_cast<T *>(__shfl_sync(0xffffffffu, (unsigned long long)dst_row, act ? j : 0));
       if (act) {
         v[k] = sp[e];
-        if (COMBINE) w[k] = ap[e];
+        w[k] = ap[e];
       } else {
         d[k] = nullptr;
       }
     }
 #pragma unroll
     for (int k = 0; k < kCopyUnroll; k++)
-      if (d[k]) d[k][ee[k]] = COMBINE ? R::add(v[k], w[k]) : v[k];
+      if (d[k]) d[k][ee[k]] = R::add(v[k], w[k]);
   }
 }
 
@@ -217,7 +216,7 @@ __global__ void __launch_bounds__(kPullThreads) p2p_refresh_index(hctr_p2p_ctx c
     const T *sp = reinterpret_cast<const T *>(warp_compact(m, (unsigned long long)src_row));
     const T *ap = reinterpret_cast<const T *>(warp_compact(m, (unsigned long long)add_row));
     T *dp = reinterpret_cast<T *>(warp_compact(m, (unsigned long long)dst_row));
-    warp_move_rows<R, true>(__popc(m), E, sp, ap, dp);
+    warp_refresh_rows<R>(__popc(m), E, sp, ap, dp);
   }
   if (lane == 0 && flagged) atomicAdd(&s_flagged, flagged);
   __syncthreads();

@@ -395,6 +395,8 @@ int hctr_p2p_refresh_index(const hctr_p2p_ctx *c, uint32_t seq, const uint32_t *
  * them: after the (bounded) wait for the owners' phase-1 release the kernel refreshes the flagged cached rows and
  * writes dst[i] for every batch position - from the table (key owned, or cached and not flagged), from the mailbox
  * (key not stored here) or as mailbox row + pending row (key cached and flagged: the value the refresh stores).
+ * uniq_owner is not read (the segments in the batch's meta words say whose a unique key is).  Indices at 16-byte aligned
+ * addresses are read four at a time.  batch <= 0xfff00000.
  * Replaces update_cache_kernel, the scan and write_back_kernel of csrc/core/writeback.cu:8-71. */
 int hctr_p2p_refresh_expand(const hctr_p2p_ctx *c, uint32_t seq, const uint32_t *meta, const uint8_t *uniq_owner,
                             const int32_t *uniq_row, size_t n_cached, const float *pending, float *embedding,
