@@ -469,11 +469,14 @@ void HetuTable::ingestKeys(BatchDesc &b, const void *keys, size_t n, cudaStream_
   // transfer.
   constexpr size_t kStagePinned = 16384;
   constexpr size_t kChunk = 65536;
-  // Launched in front of the copy, the kernel that waits for it takes 26,624 keys no earlier (36.9 us per step of x 16, 35.8
-  // with the launch behind), 53,248 6 us earlier (67 for 73 us of x 128).  A table that serves does not follow: nothing runs
-  // in front of the expansion there, and the host's look at what the kernel has made of the batch would stand between the
-  // two (53,248 x 16 42.6 us per request, 46.5 followed; x 128 48.3, 52.0).
-  constexpr size_t kFollow = 32768;
+  // Launched in front of the copy, the kernel that waits for it takes 26,624 keys no earlier, and the host's look at what it has
+  // made of them stands in front of the expansion's launch: so from 32,768 keys on where the reduction of as many gradients
+  // hides that, else from 65,536.  Per training step, launched behind -> followed: 33,800 x 128 51.2 -> 47.0 us, x 64 46.6 -> 42.9,
+  // x 32 45.1 -> 41.2 (keys nearly all distinct: 41.7 -> 43.2), 53,248 x 128 66.2 -> 60.9, x 16 53.3 -> 51.4, 212,992 x 128 198 -> 187,
+  // 638,976 x 64 475 -> 444; but 46,800 x 16 49.3 -> 50.5, 33,800 x 16 42.4 -> 45.9, x 4 42.5 -> 45.9.  A table that serves
+  // does not follow: nothing runs in front of the expansion there (53,248 x 16 42.6 us per request, 46.5 followed;
+  // x 128 48.3, 52.0).
+  constexpr size_t kFollow = 32768, kFollowAll = 65536, kFollowRows = (size_t)3 << 20;
   const unsigned meta_words = (unsigned)(HCTR_META_WORDS + nrank_ + 1 + 2);
   const int32_t *row_of = rows_are_keys_ ? nullptr : d_row_of_.as<int32_t>();
   const void *in_place = n == 0 ? nullptr : keys;
@@ -501,8 +504,8 @@ void HetuTable::ingestKeys(BatchDesc &b, const void *keys, size_t n, cudaStream_
       HCTR_CUDA(cudaHostGetDevicePointer(&dev, b.h_keys, 0));
       const int64_t *src = static_cast<const int64_t *>(keys);
       Following how = Following::kNot;
-      const bool training = pulls_in_a_row_ < 2;
-      if (nrank_ == 1 && training && n >= kFollow && n < ((size_t)1 << 31) && follow_.tryNow()) how = stageAndFollow(b, src, n, each, dev, s);
+      const bool training = pulls_in_a_row_ < 2, hidden = n * kEmbeddingWidth * sizeof(embed_t) >= kFollowRows || n >= kFollowAll;
+      if (nrank_ == 1 && training && n >= kFollow && hidden && n < ((size_t)1 << 31) && follow_.tryNow()) how = stageAndFollow(b, src, n, each, dev, s);
       bool good = how != Following::kBadKey;
       for (size_t off = 0; off < n && how == Following::kNot && good; off += kChunk) {
         const size_t m = std::min(kChunk, n - off);

@@ -135,12 +135,12 @@ def test_a_waiting_ingest_leaves_room_for_other_streams():
     assert torch.equal(dst.cpu(), keys) and torch.equal(rows.cpu(), keys.int()) and int(t["meta"][0]) == m
 
 
-def _steps(oracle_mod, sizes, bad=()):
+def _steps(oracle_mod, sizes, bad=(), width=32):
     """Training and serving steps with pageable keys, against the oracle; a batch of `bad` has one key out of range.  Returns how
     the keys were ingested."""
     from test_gpu_parity import assert_state_parity, make_worlds
 
-    N, W = 60_000, 4
+    N, W = 60_000, width
     rng = np.random.RandomState(3)
     gw, ow = make_worlds(oracle_mod, 1, N, W, 0, 0, 0.5, np.zeros(N, dtype=np.uint8), [rng.permutation(N)],
                          keys_on_device=False)
@@ -175,16 +175,18 @@ SIZES = [40_000, 32_768, 32_767, 70_000, 45_057, 300, 50_000, 36_864, 140_001]
 AT_ONCE, PATIENT = "0", "1000000"
 
 
-def test_tables_keep_up(oracle_mod, monkeypatch):
+@pytest.mark.parametrize("width,least", [(32, 32_768), (4, 65_536), (16, 49_152)])  # (3 MB of rows, else 65,536 keys)
+def test_tables_keep_up(oracle_mod, monkeypatch, width, least):
     monkeypatch.setenv("HCTR_FOLLOW_LIMIT_US", PATIENT)
-    assert _steps(oracle_mod, SIZES) == {"followed": sum(n >= 32_768 for n in SIZES), "redone": 0, "not_started": 0}
+    sizes = SIZES + [least, least - 1]
+    assert _steps(oracle_mod, sizes, width=width) == {"followed": sum(n >= least for n in sizes), "redone": 0, "not_started": 0}
 
 
 def test_a_table_that_serves_does_not_follow(oracle_mod, monkeypatch):
     from test_gpu_parity import make_worlds
 
     monkeypatch.setenv("HCTR_FOLLOW_LIMIT_US", PATIENT)
-    N, W, n = 60_000, 4, 40_000
+    N, W, n = 60_000, 32, 40_000
     rng = np.random.RandomState(7)
     gw, ow = make_worlds(oracle_mod, 1, N, W, 0, 0, 0.5, np.zeros(N, dtype=np.uint8), [np.arange(N)], keys_on_device=False)
     followed = []
@@ -216,7 +218,7 @@ def test_two_batches_in_a_row(oracle_mod, monkeypatch, limit):
     from test_gpu_parity import make_worlds
 
     monkeypatch.setenv("HCTR_FOLLOW_LIMIT_US", limit)
-    N, W, redone = 60_000, 4, 0
+    N, W, redone = 60_000, 32, 0
     for seed in range(6):
         rng = np.random.RandomState(seed)
         gw, ow = make_worlds(oracle_mod, 1, N, W, 0, 0, 0.5, np.zeros(N, dtype=np.uint8), [np.arange(N)], keys_on_device=False)
@@ -237,7 +239,7 @@ def test_gradients_and_rows_in_pinned_memory(oracle_mod, monkeypatch, limit):
     from test_gpu_parity import make_worlds
 
     monkeypatch.setenv("HCTR_FOLLOW_LIMIT_US", limit)
-    N, W, redone = 60_000, 8, 0
+    N, W, redone = 60_000, 32, 0
     for seed in range(6):
         rng = np.random.RandomState(seed)
         gw, ow = make_worlds(oracle_mod, 1, N, W, 0, 0, 0.5, np.zeros(N, dtype=np.uint8), [np.arange(N)], keys_on_device=False,
